@@ -135,7 +135,7 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
     // as dependent launches (a kernel's blocks come in while the previous kernel drains and wait for its completion
     // before touching anything a neighbour writes)
     nsl::PdlScope pdl(m->pdl);
-    const bool fused = T <= MV_MAXT && d % 64 == 0 && d <= 2048 && (d & (d - 1)) == 0;
+    const bool fused = T <= MV_MAXT && d % 64 == 0 && d <= 32768 && nsl::aligned16(x);
     // on request, one launch for the whole step where the fused kernel serves the sizes (measured slower than the three
     // dependent launches: 126.3 against 114.2 us at 8 rows, 70.1 / 65.5 at 4, 26.7 / 26.2 at 1)
     if (fused && m->one_launch &&

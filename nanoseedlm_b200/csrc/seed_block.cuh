@@ -7,16 +7,16 @@
 // weight c = fl((float) isum_c * fl(R32 2^e)), isum_c = sum_p (state_(4c+p+1) - 32768) q_p.
 //
 // How the expansion is laid out here.  On this part the integer/logic pipe issues at half the FP32 rate (measured:
-// 63 LOP3/SHF/PRMT vs 119 FFMA lane-ops per clock per SM) and packed FP32 pairs (fma.rn.f32x2) halve the FP issue
-// count again, so a block costs what its integer operations cost.  They are kept to one shift per weight and one
-// AND per state:
-//   Y_c  = the window shifted so that stream bit 4c+1 sits at bit 4            (one shift per weight)
-//   v_cp = as_float(Y_c & (0xFFFF << (4+p))) = state_(4c+p+1) * 2^(p-145)      (one AND with a literal; a subnormal float)
+// 63 LOP3/SHF/PRMT vs 119 FFMA lane-ops per clock per SM), so a block costs what its integer operations cost -- and what its
+// packed multiply-adds take of the register file (fma.rn.f32x2: 3.0 cycles a sub-partition with six distinct operand
+// registers, 2.4 when neighbours share one).  The integer operations are kept to one AND per state:
+//   v = as_float(word & (0xFFFF << n)) = state * 2^(n-149)
 // FP32 subnormals are exact multiples of 2^-149 and this GPU's FMA takes them at full rate, so no exponent has to be
 // merged in (a second constant per logic operation costs a second instruction or a register move).  The mat-vec
-// kernels scale their inputs by 2^64 when they load them, so every product is a normal number; the powers of two and
-// the centring (-32768 per state) fold into per-block constants.  The window is held as two words, A = stream bits
-// 0..31 (weights 0..3) and G = stream bits 16..47 (weights 4..7), so no shift crosses a word.
+// kernels scale their inputs when they stage them, so every product is a normal number; the powers of two and the
+// centring (-32768 per state) fold into per-block constants.  In the pair kernels one word serves two weights or three
+// (state_bit below); the single-block forms shift once per weight, so that stream bit 4c+1 sits at bit 4.  The window is
+// held as two words, A = stream bits 0..31 (weights 0..3) and G = stream bits 16..47 (weights 4..7).
 // Two adjacent blocks are expanded side by side and their state values packed as f32x2 pairs {block A, block B}, so
 // the 32 multiply-adds of each block issue as 32 packed operations per block pair.
 #pragma once
@@ -129,12 +129,6 @@ __device__ __forceinline__ float state_value(uint32_t y) {
 template <int P>
 __device__ __forceinline__ float coef_raw(uint32_t cw, uint32_t cx) {
     return __uint_as_float(and_xor<(0xFu << (4 * P))>(cw, cx));
-}
-// 2^(code - 15) for block i (0..7) of a chunk whose eight codes are the nibbles of cd.
-__device__ __forceinline__ float code_scale(uint32_t cd, int i, const KConst& k) {   // i: a constant after unrolling
-    const int sh = 23 - 4 * i;
-    const uint32_t f = sh >= 0 ? cd * (1u << (sh & 31)) : cd >> ((-sh) & 31);
-    return __uint_as_float(and_or<0x07800000u>(f, k.cor));
 }
 // {2^(code - 15) of block 2 bp, of block 2 bp + 1} of the chunk.
 __device__ __forceinline__ unsigned long long code_scale_pair(uint32_t cd, int bp, const KConst& k) {
@@ -302,6 +296,46 @@ __device__ __forceinline__ u64 add2(u64 a, u64 b) {
     return d;
 }
 
+// ---- where a pair kernel finds weight c's states -------------------------------------------------------------------------
+// A float whose bit pattern is below 2^24 equals pattern * 2^-149: exponent field 0 (subnormal) and exponent field 1 have the
+// same unit.  So a state may lie anywhere in bits 0..23 of a word, and one shifted word serves several weights: no shift per
+// weight, only one more word per half window.
+//   P = 4: weight c's states start at bit 4c + 1 of the stream.  Words: the window's low half a (stream bits 0..31), a >> 8,
+//          its high half g (stream bits 16..47), g >> 8; weight c lies at bit 1 (even c) or 5 (odd c) of word c / 2.
+//   P = 3: weight c's states start at stream bit 3c + 1.  Words: a (weights 0, 1), a >> 7 (2, 3, 4), g (5, 6, 7).
+// The differing powers of two go into the scale of the staged inputs: input c is multiplied by 2^(64 - start bit), every
+// product is then x state 2^(p - 85).
+template <int P, int C>
+__device__ __forceinline__ constexpr int state_bit() {
+    return P == 4 ? ((C & 1) ? 5 : 1) : C == 0 ? 1 : C == 1 ? 4 : C <= 4 ? 3 * C - 6 : 3 * C - 15;
+}
+template <int P>
+__device__ __forceinline__ float input_scale(int c) {      // 2^(64 - start bit); c: a constant after unrolling
+    const int bit = P == 4 ? ((c & 1) ? 5 : 1) : c == 0 ? 1 : c == 1 ? 4 : c <= 4 ? 3 * c - 6 : 3 * c - 15;
+    return __uint_as_float((uint32_t) (127 + 64 - bit) << 23);
+}
+template <int BIT, int P>
+__device__ __forceinline__ float state_at(uint32_t y) { return __uint_as_float(y & (0xFFFFu << (BIT + P))); }
+// The words of a block's window, from its seed (the low or high half of sw) and its stream bits g.
+struct Words { uint32_t w[4]; };
+template <int P, int HALF>
+__device__ __forceinline__ Words window_words(uint32_t sw, uint32_t g) {
+    Words r;
+    r.w[0] = __byte_perm(sw, g, HALF ? 0x5432 : 0x5410);
+    if (P == 4) {
+        r.w[1] = __byte_perm(sw, g, HALF ? 0x6543 : 0x6541);      // a >> 8; the byte above bit 23 is masked off
+        r.w[2] = g;
+        r.w[3] = g >> 8;
+    } else {
+        r.w[1] = r.w[0] >> 7;
+        r.w[2] = g;
+        r.w[3] = g;
+    }
+    return r;
+}
+template <int P, int C>
+__device__ __forceinline__ constexpr int word_of() { return P == 4 ? C / 2 : C < 2 ? 0 : C <= 4 ? 1 : 2; }
+
 // t[idx] for a table in shared memory with the address formed by a multiply-add whose factor 4 comes from constant
 // memory, so that it stays a multiply-add: it issues on the FMA pipe, where the logic pipe is the one that binds
 // (measured on config 1: 115.4 -> 113.9 us per step; doing the right shifts as high products the same way lost 1 %).
@@ -312,22 +346,11 @@ __device__ __forceinline__ uint32_t lut_word(const uint32_t* t, uint32_t idx) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
-// The 32 state-value pairs of the blocks whose seeds are the two halves of sw: v[4c+p] = {even, odd}.
-__device__ __forceinline__ void pair_states(const StreamTab& tab, uint32_t sw, u64* v) {
-    // table indices and the two windows by byte permutes: one logic-pipe operation each
-    const uint32_t g0 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4440)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4441));
-    const uint32_t g1 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4442)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4443));
-    const uint32_t a0 = __byte_perm(sw, g0, 0x5410), a1 = __byte_perm(sw, g1, 0x5432);
-#define NSL_V2(C)                                                                  \
-    {                                                                              \
-        const uint32_t y0 = weight_word<C>(a0, g0), y1 = weight_word<C>(a1, g1);   \
-        v[4 * C + 0] = pack2(state_value<0>(y0), state_value<0>(y1));              \
-        v[4 * C + 1] = pack2(state_value<1>(y0), state_value<1>(y1));              \
-        v[4 * C + 2] = pack2(state_value<2>(y0), state_value<2>(y1));              \
-        v[4 * C + 3] = pack2(state_value<3>(y0), state_value<3>(y1));              \
-    }
-    NSL_V2(0) NSL_V2(1) NSL_V2(2) NSL_V2(3) NSL_V2(4) NSL_V2(5) NSL_V2(6) NSL_V2(7)
-#undef NSL_V2
+// The stream bits of the two seeds packed in sw.
+__device__ __forceinline__ void pair_stream(const StreamTab& tab, uint32_t sw, uint32_t& g0, uint32_t& g1) {
+    // table indices by byte permutes: one logic-pipe operation each
+    g0 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4440)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4441));
+    g1 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4442)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4443));
 }
 // The four coefficient pairs of the two words packed in cw.
 __device__ __forceinline__ void pair_coefs(uint32_t cw, const KConst& k, u64* q) {
@@ -337,39 +360,49 @@ __device__ __forceinline__ void pair_coefs(uint32_t cw, const KConst& k, u64* q)
     q[2] = add2(and_xor_pair<0x0F00u>(cw, c1, k.cxor[2]), pack2(k.coff[2], k.coff[2]));
     q[3] = add2(and_xor_pair<0xF000u>(cw, c1, k.cxor[3]), pack2(k.coff[3], k.coff[3]));
 }
-// Both blocks' dot forms at once: x2[c] = {x of the even block, x of the odd block}, xm2[p] likewise.
-__device__ __forceinline__ u64 pair_dot(const u64* v, const u64* q, const u64* x2, const u64* xm2) {
-    u64 d0 = xm2[0], d1 = xm2[1], d2 = xm2[2], d3 = xm2[3];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        d0 = fma2(x2[c], v[4 * c + 0], d0);
-        d1 = fma2(x2[c], v[4 * c + 1], d1);
-        d2 = fma2(x2[c], v[4 * c + 2], d2);
-        d3 = fma2(x2[c], v[4 * c + 3], d3);
-    }
-    return fma2(q[3], d3, fma2(q[2], d2, fma2(q[1], d1, mul2(q[0], d0))));
-}
-
-// pair_states + pair_dot written weight by weight: the two shifts and eight ANDs of weight c, then its four packed
-// multiply-adds, so that logic-pipe and FMA-pipe instructions alternate in program order.  Same operations, same order
-// per accumulator: the same bits.  Measured on the config-1 step at 8 rows: 112.9 us against 114.2 us with all 32 state
-// values formed first (by halves, 16 at a time: 114.2; gate and up side by side per weight: 114.4).
+// Both blocks' dot forms at once: x2[c] = {x of the even block, x of the odd block} (scaled by input_scale), xm2[p] the
+// centring; d_p = xm_p + sum_c x_c v_cp (c ascending), result = ((q0 d0 + q1 d1) + q2 d2) + q3 d3.  Written weight by weight:
+// its eight ANDs, then its four packed multiply-adds, which share x2[c] (a shared operand saves a register-file read).
+// Words instead of one shift per weight (two shifts and byte permutes a block instead of eight shifts): config 1 at 8 rows
+// 134.3 -> 130.1 us a step.
 __device__ __forceinline__ u64 pair_expand_dot(const StreamTab& tab, uint32_t sw, const u64* q, const u64* x2, const u64* xm2) {
-    const uint32_t g0 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4440)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4441));
-    const uint32_t g1 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4442)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4443));
-    const uint32_t a0 = __byte_perm(sw, g0, 0x5410), a1 = __byte_perm(sw, g1, 0x5432);
+    uint32_t g0, g1;
+    pair_stream(tab, sw, g0, g1);
+    const Words wa = window_words<4, 0>(sw, g0), wb = window_words<4, 1>(sw, g1);
     u64 d0 = xm2[0], d1 = xm2[1], d2 = xm2[2], d3 = xm2[3];
-#define NSL_W2(C)                                                                  \
-    {                                                                              \
-        const uint32_t y0 = weight_word<C>(a0, g0), y1 = weight_word<C>(a1, g1);   \
-        d0 = fma2(x2[C], pack2(state_value<0>(y0), state_value<0>(y1)), d0);       \
-        d1 = fma2(x2[C], pack2(state_value<1>(y0), state_value<1>(y1)), d1);       \
-        d2 = fma2(x2[C], pack2(state_value<2>(y0), state_value<2>(y1)), d2);       \
-        d3 = fma2(x2[C], pack2(state_value<3>(y0), state_value<3>(y1)), d3);       \
+#define NSL_W2(C)                                                                                                            \
+    {                                                                                                                        \
+        constexpr int B = state_bit<4, C>(), W = word_of<4, C>();                                                            \
+        d0 = fma2(x2[C], pack2(state_at<B, 0>(wa.w[W]), state_at<B, 0>(wb.w[W])), d0);                                       \
+        d1 = fma2(x2[C], pack2(state_at<B, 1>(wa.w[W]), state_at<B, 1>(wb.w[W])), d1);                                       \
+        d2 = fma2(x2[C], pack2(state_at<B, 2>(wa.w[W]), state_at<B, 2>(wb.w[W])), d2);                                       \
+        d3 = fma2(x2[C], pack2(state_at<B, 3>(wa.w[W]), state_at<B, 3>(wb.w[W])), d3);                                       \
     }
     NSL_W2(0) NSL_W2(1) NSL_W2(2) NSL_W2(3) NSL_W2(4) NSL_W2(5) NSL_W2(6) NSL_W2(7)
 #undef NSL_W2
     return fma2(q[3], d3, fma2(q[2], d2, fma2(q[1], d1, mul2(q[0], d0))));
+}
+
+// ---- the weight form: the two blocks' weights (without their power-of-two block scale), to be multiplied into several rows of
+// inputs.  A weight costs one packed operation more per state than it does in the dot form of one row, but each further row
+// then costs 8 packed multiply-adds a block pair instead of 37.
+// The centring, -32768 sum_p q_p in the units of (unscaled input sum) x (weight).
+template <int P>
+__device__ __forceinline__ u64 pair_centre(const u64* q) {
+    u64 t = fma2(q[1], pack2(-1.6940658945086007e-21f, -1.6940658945086007e-21f), mul2(q[0], pack2(-8.470329472543003e-22f, -8.470329472543003e-22f)));
+    t = fma2(q[2], pack2(-3.3881317890172014e-21f, -3.3881317890172014e-21f), t);      // -2^-70, -2^-69, -2^-68, -2^-67
+    if (P == 4) t = fma2(q[3], pack2(-6.776263578034403e-21f, -6.776263578034403e-21f), t);
+    return t;
+}
+// Weight C of the two blocks: sum_p q'_p state_(C,p) 2^(start bit + p - 149).
+template <int P, int C>
+__device__ __forceinline__ u64 pair_weight(const Words& wa, const Words& wb, const u64* q) {
+    constexpr int B = state_bit<P, C>(), W = word_of<P, C>();
+    u64 t = mul2(q[0], pack2(state_at<B, 0>(wa.w[W]), state_at<B, 0>(wb.w[W])));
+    t = fma2(q[1], pack2(state_at<B, 1>(wa.w[W]), state_at<B, 1>(wb.w[W])), t);
+    t = fma2(q[2], pack2(state_at<B, 2>(wa.w[W]), state_at<B, 2>(wb.w[W])), t);
+    if (P == 4) t = fma2(q[P - 1], pack2(state_at<B, P - 1>(wa.w[W]), state_at<B, P - 1>(wb.w[W])), t);
+    return t;
 }
 
 // The same for two adjacent P = 3 blocks (see block_states3 / block_coefs3 / states_dot3): 24 state-value pairs, the three
@@ -384,16 +417,16 @@ __device__ __forceinline__ void pair_coefs3(uint32_t nw, const KConst& k, u64* q
 // The P = 3 form of pair_expand_dot: 24 state-value pairs, weight by weight; d_p = xm_p + sum_c x_c v_cp (c ascending),
 // result = (q0 d0 + q1 d1) + q2 d2.
 __device__ __forceinline__ u64 pair_expand_dot3(const StreamTab& tab, uint32_t sw, const u64* q, const u64* x2, const u64* xm2) {
-    const uint32_t g0 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4440)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4441));
-    const uint32_t g1 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4442)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4443));
-    const uint32_t a0 = __byte_perm(sw, g0, 0x5410), a1 = __byte_perm(sw, g1, 0x5432);
+    uint32_t g0, g1;
+    pair_stream(tab, sw, g0, g1);
+    const Words wa = window_words<3, 0>(sw, g0), wb = window_words<3, 1>(sw, g1);
     u64 d0 = xm2[0], d1 = xm2[1], d2 = xm2[2];
-#define NSL_W23(C)                                                                   \
-    {                                                                                \
-        const uint32_t y0 = weight_word3<C>(a0, g0), y1 = weight_word3<C>(a1, g1);   \
-        d0 = fma2(x2[C], pack2(state_value<0>(y0), state_value<0>(y1)), d0);         \
-        d1 = fma2(x2[C], pack2(state_value<1>(y0), state_value<1>(y1)), d1);         \
-        d2 = fma2(x2[C], pack2(state_value<2>(y0), state_value<2>(y1)), d2);         \
+#define NSL_W23(C)                                                                                                           \
+    {                                                                                                                        \
+        constexpr int B = state_bit<3, C>(), W = word_of<3, C>();                                                            \
+        d0 = fma2(x2[C], pack2(state_at<B, 0>(wa.w[W]), state_at<B, 0>(wb.w[W])), d0);                                       \
+        d1 = fma2(x2[C], pack2(state_at<B, 1>(wa.w[W]), state_at<B, 1>(wb.w[W])), d1);                                       \
+        d2 = fma2(x2[C], pack2(state_at<B, 2>(wa.w[W]), state_at<B, 2>(wb.w[W])), d2);                                       \
     }
     NSL_W23(0) NSL_W23(1) NSL_W23(2) NSL_W23(3) NSL_W23(4) NSL_W23(5) NSL_W23(6) NSL_W23(7)
 #undef NSL_W23

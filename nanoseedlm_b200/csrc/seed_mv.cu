@@ -3,16 +3,14 @@
 // (engine/kernels_moe.cu:130-159, 222-348, 2308-2328) and the weight reader used by its tests.
 //
 // Data movement.  A row of K weights is K/8 blocks; a "chunk" is 8 consecutive blocks = one 16-byte load of seeds, one
-// of coefficient words and one 4-byte load of exponent codes.  A lane owns one chunk position of the row (64 inputs),
-// so a warp reads a row's streams as contiguous 512 + 512 + 128 bytes, and the lane's 64 inputs (plus the per-block
-// centring constants) stay in registers while the warp walks over many rows: the only per-row traffic is the packed
-// streams.  Rows shorter than 32 chunks share a warp (K = 512: four rows per step, eight lanes each).
+// of coefficient words and one 4-byte load of exponent codes.  A lane takes one chunk of a row at a time (64 inputs), so a
+// warp reads a row's streams as contiguous runs; the inputs sit in shared memory.  Rows shorter than 32 chunks share a warp
+// (K = 512: four rows per step, eight lanes each); rows of another length than 2^j <= 32 chunks are cut into groups of lanes.
 //
-// Arithmetic per block: the dot form of seed_block.cuh (32 fused multiply-adds on 32 masked stream words, then the
-// four coefficients and the block's 2^code).  A token's sum is formed in the same order whatever the number of tokens
-// in the call (chunks ascending within a lane, blocks ascending within a chunk, then a butterfly over the row's
-// lanes), so a row of a multi-token call equals the single-token call bit for bit, as the reference requires
-// (tests/test_mova_kernels.c:173-183).
+// Arithmetic per block: the dot form of seed_block.cuh for gathers (32 fused multiply-adds on 32 masked stream words, then the
+// four coefficients and the block's 2^code), the weight form for dense calls, whose rows of inputs share each expansion.  A
+// token's sum is formed in the same order whatever the number of tokens in the call, so a row of a multi-token call equals the
+// single-token call bit for bit, as the reference requires (tests/test_mova_kernels.c:173-183).
 #include <math.h>
 
 #include "common.cuh"
@@ -112,51 +110,68 @@ __device__ __forceinline__ void store_out(const MvParams& a, int pair, int r, fl
     else *yo = a.add ? bf16_round(*yo + bf16_round(s)) : bf16_round(s);   // engine/kernels_moe.cu:214
 }
 
-// One thread's share of staging a pair's inputs: 16 inputs (two blocks: chunk j of the row, block pair bp), scaled, as
-// the f32x2 operands of pair_dot plus the two blocks' input sums (2^-64 of them), from which the consumer forms the
-// centring constants: xm[p] = -2^(p-66) * sum, an exact scaling, so the bits are those of block_offsets.
-__device__ __forceinline__ float block_sum(const float* xs) {      // the order of block_offsets
-    return (((xs[0] + xs[4]) + (xs[1] + xs[5])) + ((xs[2] + xs[6]) + (xs[3] + xs[7]))) * 5.421010862427522e-20f;   // 2^-64
-}
+// Inputs in shared memory.  A staged chunk (64 inputs) is CX 16-byte units: the f32x2 operands of the block pairs
+// ({x of the even block, x of the odd block}, scaled by input_scale; unit 4 bp + cq holds operands 2 cq and 2 cq + 1 of block
+// pair bp), then the block pairs' input sums (unscaled, two u64 a unit), and one unit of padding: chunks are 304 bytes apart,
+// so that the 16-byte loads of eight neighbouring lanes (one chunk each) touch all 32 banks once.  Every offset inside a
+// chunk is an immediate.
+constexpr int CX = 19;
+
+// The centring of pair_expand_dot: xm[p] = -32768 2^(p-85) sum(x), from the (unscaled) input sums of the pair's blocks.
 __device__ __forceinline__ void offsets_from_sum(u64 s2, u64* xm2) {
-    xm2[0] = mul2(s2, pack2(-1.3552527156068805e-20f, -1.3552527156068805e-20f));   // -2^-66
-    xm2[1] = mul2(s2, pack2(-2.710505431213761e-20f, -2.710505431213761e-20f));     // -2^-65
-    xm2[2] = mul2(s2, pack2(-5.421010862427522e-20f, -5.421010862427522e-20f));     // -2^-64
-    xm2[3] = mul2(s2, pack2(-1.0842021724855044e-19f, -1.0842021724855044e-19f));   // -2^-63
+    xm2[0] = mul2(s2, pack2(-8.470329472543003e-22f, -8.470329472543003e-22f));     // -2^-70
+    xm2[1] = mul2(s2, pack2(-1.6940658945086007e-21f, -1.6940658945086007e-21f));   // -2^-69
+    xm2[2] = mul2(s2, pack2(-3.3881317890172014e-21f, -3.3881317890172014e-21f));   // -2^-68
+    xm2[3] = mul2(s2, pack2(-6.776263578034403e-21f, -6.776263578034403e-21f));     // -2^-67
 }
-__device__ __forceinline__ void stage_load(const MvParams& a, int xr, int j, int bp, float* x) {
-    if (a.xbf16) {
-        const uint4* xp = (const uint4*) ((const uint16_t*) a.x + (size_t) xr * a.xs + (size_t) j * 64 + bp * 16);
+__device__ __forceinline__ float input_sum(const float* x) { return ((x[0] + x[4]) + (x[1] + x[5])) + ((x[2] + x[6]) + (x[3] + x[7])); }
+
+// 16 inputs (chunk j of the row, block pair bp): from memory, and into a staged row.
+template <bool CG = false>      // CG: memory that other blocks of this grid have written (the loads bypass the non-coherent path)
+__device__ __forceinline__ void stage_load(const void* row, int bf16, int j, int bp, float* x) {
+    if (bf16) {
+        const uint4* xp = (const uint4*) ((const uint16_t*) row + (size_t) j * 64 + bp * 16);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const uint4 t = __ldg(xp + i);
             const uint32_t u[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                x[8 * i + 2 * q] = __uint_as_float(u[q] << 16) * NSL_XSCALE;
-                x[8 * i + 2 * q + 1] = __uint_as_float(u[q] & 0xFFFF0000u) * NSL_XSCALE;
+                x[8 * i + 2 * q] = __uint_as_float(u[q] << 16);
+                x[8 * i + 2 * q + 1] = __uint_as_float(u[q] & 0xFFFF0000u);
             }
         }
     } else {
-        const float4* xp = (const float4*) (a.x + (size_t) xr * a.xs + (size_t) j * 64 + bp * 16);
+        const float4* xp = (const float4*) ((const float*) row + (size_t) j * 64 + bp * 16);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float4 t = __ldg(xp + i);
-            x[4 * i] = t.x * NSL_XSCALE; x[4 * i + 1] = t.y * NSL_XSCALE; x[4 * i + 2] = t.z * NSL_XSCALE; x[4 * i + 3] = t.w * NSL_XSCALE;
+            const float4 t = CG ? __ldcg(xp + i) : __ldg(xp + i);
+            x[4 * i] = t.x; x[4 * i + 1] = t.y; x[4 * i + 2] = t.z; x[4 * i + 3] = t.w;
         }
     }
 }
-__device__ __forceinline__ void stage_store(const float* x, int j, int bp, ulonglong2* sx, u64* ss) {
+template <int PF>
+__device__ __forceinline__ void stage_store(const float* x, int j, int bp, ulonglong2* sx) {
+    ulonglong2* c = sx + j * CX;
 #pragma unroll
     for (int cq = 0; cq < 4; ++cq) {
+        const float s0 = input_scale<PF>(2 * cq), s1 = input_scale<PF>(2 * cq + 1);
         ulonglong2 t;
-        t.x = pack2(x[2 * cq], x[8 + 2 * cq]);
-        t.y = pack2(x[2 * cq + 1], x[8 + 2 * cq + 1]);
-        sx[(bp * 4 + cq) * 32 + j] = t;
+        t.x = pack2(x[2 * cq] * s0, x[8 + 2 * cq] * s0);
+        t.y = pack2(x[2 * cq + 1] * s1, x[8 + 2 * cq + 1] * s1);
+        c[bp * 4 + cq] = t;
     }
-    ss[bp * 32 + j] = pack2(block_sum(x), block_sum(x + 8));
+    ((u64*) (c + 16))[bp] = pack2(input_sum(x), input_sum(x + 8));
 }
-
+__device__ __forceinline__ const void* input_row(const MvParams& a, int xr) {
+    return a.xbf16 ? (const void*) ((const uint16_t*) a.x + (size_t) xr * a.xs) : (const void*) (a.x + (size_t) xr * a.xs);
+}
+// The operands of block pair bp of a staged chunk.
+__device__ __forceinline__ void staged_pair(const ulonglong2* c, int bp, u64* x2) {
+#pragma unroll
+    for (int cq = 0; cq < 4; ++cq) { const ulonglong2 t = c[bp * 4 + cq]; x2[2 * cq] = t.x; x2[2 * cq + 1] = t.y; }
+}
+__device__ __forceinline__ u64 staged_sum(const ulonglong2* c, int bp) { return ((const u64*) (c + 16))[bp]; }
 
 struct RouteFuse {        // the router folded into the prologue (logits == NULL: the pair list comes from MvParams.sel)
     const float* logits;
@@ -165,71 +180,169 @@ struct RouteFuse {        // the router folded into the prologue (logits == NULL
     float* wt_out;
 };
 
-// One thread's share of staging a pair's inputs: 16 inputs (two blocks: chunk j of the row, block pair bp), scaled, as
-// the f32x2 operands of pair_dot plus their centring constants.
-__device__ __forceinline__ void stage_pair_inputs(const MvParams& a, int xr, int j, int bp, ulonglong2* sx, ulonglong2* sm) {
-    float x[16], xm[8];
-    if (a.xbf16) {
-        const uint4* xp = (const uint4*) ((const uint16_t*) a.x + (size_t) xr * a.xs + (size_t) j * 64 + bp * 16);
+// How a row is cut.  Its sum is defined on 32 VIRTUAL lanes: virtual lane v sums chunks v, v + 32, ... in order, and the 32 sums
+// are added by the tree of a butterfly (distance 16 first).  A warp may give a row any power of two lpr of real lanes: lane jc
+// then plays the virtual lanes jc + i lpr one after the other (in the order in which the tree adds them) and adds them as the
+// tree does, so the split never shows in the bits.  Virtual lanes beyond the row's chunks are zeros: lv = log2 of those kept.
+//   fewer lanes a row: more rows a step, so fewer shuffles and fewer distinct 16-byte inputs a load of the warp fetches, and
+//   less idling when the chunks do not fill 32 lanes (45 chunks: 64 lane slots with 32 lanes, 48 with 8);
+//   more lanes a row: more steps to deal to the warps of a small call.
+struct RowShape { int ch, lpr_log2, lv, groups; };
+
+__host__ __device__ __forceinline__ int pass_offset(int pass, int lv) {      // the first virtual lane of a pass: the pass number's bits reversed
+    return ((pass & 1) << lv >> 1) | ((pass >> 1 & 1) << lv >> 2) | ((pass >> 2 & 1) << lv >> 3);
+}
+// s = the sum of pass `pass`: the tree's partial sums that it completes, or into the stack to wait for their other half.
+__device__ __forceinline__ float tree_push(float* stk, int pass, float s) {
+    if (pass & 1) s = stk[0] + s; else stk[0] = s;
+    if ((pass & 1) && (pass & 2)) s = stk[1] + s; else if (pass & 1) stk[1] = s;
+    if ((pass & 3) == 3 && (pass & 4)) s = stk[2] + s; else if ((pass & 3) == 3) stk[2] = s;
+    return s;      // the whole lane's sum after its last pass
+}
+
+// One chunk of the gate (or only) matrix and of the up matrix against its staged inputs.
+template <int MODE, int PF>
+__device__ __forceinline__ void chunk_dots(const StreamTab& tab, const KConst& kc, const Chunk& ka, const Chunk& kb, const ulonglong2* cx, u64& acc, u64& accu) {
+    const uint32_t swa[4] = {ka.s.x, ka.s.y, ka.s.z, ka.s.w}, cwa[4] = {ka.c.x, ka.c.y, ka.c.z, ka.c.w};
+    const uint32_t swb[4] = {kb.s.x, kb.s.y, kb.s.z, kb.s.w}, cwb[4] = {kb.c.x, kb.c.y, kb.c.z, kb.c.w};
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const uint4 t = __ldg(xp + i);
-            const uint32_t u[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                x[8 * i + 2 * q] = __uint_as_float(u[q] << 16) * NSL_XSCALE;
-                x[8 * i + 2 * q + 1] = __uint_as_float(u[q] & 0xFFFF0000u) * NSL_XSCALE;
+    for (int bp = 0; bp < 4; ++bp) {
+        u64 x2[8], xm2[4];
+        staged_pair(cx, bp, x2);
+        offsets_from_sum(staged_sum(cx, bp), xm2);
+        if (PF == 4) {
+            u64 q[4];
+            pair_coefs(cwa[bp], kc, q);
+            acc = fma2(pair_expand_dot(tab, swa[bp], q, x2, xm2), code_scale_pair(ka.cd, bp, kc), acc);
+        } else {
+            u64 q[3];
+            pair_coefs3(cwa[bp], kc, q);
+            acc = fma2(pair_expand_dot3(tab, swa[bp], q, x2, xm2), code_scale_pair3(cwa[bp], kc), acc);
+        }
+        if (MODE == MODE_GU && PF == 4) {
+            u64 q[4];
+            pair_coefs(cwb[bp], kc, q);
+            accu = fma2(pair_expand_dot(tab, swb[bp], q, x2, xm2), code_scale_pair(kb.cd, bp, kc), accu);
+        } else if (MODE == MODE_GU) {
+            u64 q[3];
+            pair_coefs3(cwb[bp], kc, q);
+            accu = fma2(pair_expand_dot3(tab, swb[bp], q, x2, xm2), code_scale_pair3(cwb[bp], kc), accu);
+        }
+    }
+}
+
+// The row steps [s_lo, s_hi) of one pair that fall to this warp (every MV_WARPS-th), for rows of 2^j <= 32 chunks: a step = the
+// 32 / lpr rows a warp expands at once, a lane owning one chunk of its row.  ka / kb: the first step's streams, requested by
+// the caller before the inputs were staged; the next ones are requested before the current ones are expanded.
+// store(r, s, su): row r's sum (and the up matrix's).
+template <int MODE, int PF, typename Store>
+__device__ __forceinline__ void pair_rows(const StreamTab& tab, const KConst& kc, const WSlice& wa, const WSlice& wb, const ulonglong2* sx,
+                                          int lpr_log2, int R, int s_lo, int s_hi, Chunk ka, Chunk kb, Store store) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
+    const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
+    const float sca = slice_scale(wa.eb + (8 - PF)), scb = slice_scale(wb.eb + (8 - PF));      // P = 3 products are half as large
+    const ulonglong2* cx = sx + jc * CX;
+    int st = s_lo + warp, r = st * rpw + ro;
+    for (; st < s_hi; st += MV_WARPS, r += MV_WARPS * rpw) {
+        const bool ok = r < R;
+        const int rn = r + MV_WARPS * rpw;
+        Chunk na, nb;
+        if (st + MV_WARPS < s_hi && rn < R) {
+            na = load_chunk<PF>(wa, (size_t) rn * lpr + jc);
+            if (MODE == MODE_GU) nb = load_chunk<PF>(wb, (size_t) rn * lpr + jc);
+        }
+        u64 acc = 0ull, accu = 0ull;
+        if (ok) chunk_dots<MODE, PF>(tab, kc, ka, kb, cx, acc, accu);
+        const float s = group_sum(pair_total(acc), lpr) * sca;
+        float su = 0.0f;
+        if (MODE == MODE_GU) su = group_sum(pair_total(accu), lpr) * scb;
+        if (ok && jc == 0) store(r, s, su);
+        ka = na;
+        if (MODE == MODE_GU) kb = nb;
+    }
+}
+
+// The same for rows of any number of chunks: a row is cut into groups of lpr chunks, an ITEM is one group of the 32 / lpr rows of
+// a row step, and a block's warps take the items of its share one by one, so the work is even to within one chunk a warp
+// whatever the row's length.  A group's sum (the butterfly over its lanes) waits in shared memory; the row's is the groups'
+// sum in order.  PART_STEPS row steps at a time.
+constexpr int PART_FLOATS = 2048;
+__host__ __device__ __forceinline__ int part_steps(int groups, int lpr_log2, int mats) { return PART_FLOATS / (groups * (32 >> lpr_log2) * mats); }
+
+template <int MODE, int PF, typename Store>
+__device__ __forceinline__ void pair_items(const StreamTab& tab, const KConst& kc, const WSlice& wa, const WSlice& wb, const ulonglong2* sx, float* part,
+                                           RowShape sh, int R, int s_lo, int s_hi, Chunk ka, Chunk kb, Store store) {
+    constexpr int MATS = MODE == MODE_GU ? 2 : 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lpr = 1 << sh.lpr_log2, rpw = 32 >> sh.lpr_log2, ch = sh.ch, groups = sh.groups;
+    const int jc = lane & (lpr - 1), ro = lane >> sh.lpr_log2;
+    const float sca = slice_scale(wa.eb + (8 - PF)), scb = slice_scale(wb.eb + (8 - PF));
+    const int span = part_steps(groups, sh.lpr_log2, MATS);
+    int done = s_lo, st = s_lo + warp / groups, g = warp % groups;      // this warp's item; its streams are in ka / kb
+    while (done < s_hi) {
+        const int upto = min(s_hi, done + span);
+        while (st < upto) {
+            int gn = g + MV_WARPS, sn = st;
+            while (gn >= groups) { gn -= groups; ++sn; }
+            const int r = st * rpw + ro, j = g * lpr + jc, rn = sn * rpw + ro, jn = gn * lpr + jc;
+            Chunk na, nb;
+            if (sn < s_hi && rn < R && jn < ch) {
+                na = load_chunk<PF>(wa, (size_t) rn * ch + jn);
+                if (MODE == MODE_GU) nb = load_chunk<PF>(wb, (size_t) rn * ch + jn);
             }
+            u64 acc = 0ull, accu = 0ull;
+            if (r < R && j < ch) chunk_dots<MODE, PF>(tab, kc, ka, kb, sx + j * CX, acc, accu);
+            const float s = group_sum(pair_total(acc), lpr);
+            float su = 0.0f;
+            if (MODE == MODE_GU) su = group_sum(pair_total(accu), lpr);
+            if (jc == 0) {
+                float* at = part + (((st - done) * rpw + ro) * groups + g) * MATS;
+                at[0] = s;
+                if (MODE == MODE_GU) at[1] = su;
+            }
+            ka = na;
+            if (MODE == MODE_GU) kb = nb;
+            st = sn; g = gn;
         }
-    } else {
-        const float4* xp = (const float4*) (a.x + (size_t) xr * a.xs + (size_t) j * 64 + bp * 16);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 t = __ldg(xp + i);
-            x[4 * i] = t.x * NSL_XSCALE; x[4 * i + 1] = t.y * NSL_XSCALE; x[4 * i + 2] = t.z * NSL_XSCALE; x[4 * i + 3] = t.w * NSL_XSCALE;
+        __syncthreads();
+        for (int i = threadIdx.x; i < (upto - done) * rpw; i += MV_THREADS) {
+            const float* at = part + i * groups * MATS;
+            float s = at[0], su = MODE == MODE_GU ? at[1] : 0.0f;
+            for (int q = 1; q < groups; ++q) {
+                s += at[q * MATS];
+                if (MODE == MODE_GU) su += at[q * MATS + 1];
+            }
+            if (done * rpw + i < R) store(done * rpw + i, s * sca, su * scb);
         }
-    }
-    block_offsets(x, xm);
-    block_offsets(x + 8, xm + 4);
-#pragma unroll
-    for (int cq = 0; cq < 4; ++cq) {
-        ulonglong2 t;
-        t.x = pack2(x[2 * cq], x[8 + 2 * cq]);
-        t.y = pack2(x[2 * cq + 1], x[8 + 2 * cq + 1]);
-        sx[(bp * 4 + cq) * 32 + j] = t;
-    }
-#pragma unroll
-    for (int pq = 0; pq < 2; ++pq) {
-        ulonglong2 t;
-        t.x = pack2(xm[2 * pq], xm[4 + 2 * pq]);
-        t.y = pack2(xm[2 * pq + 1], xm[4 + 2 * pq + 1]);
-        sm[(bp * 2 + pq) * 32 + j] = t;
+        done = upto;
+        if (done < s_hi) __syncthreads();      // the sums are read before the next span's are written
     }
 }
 
 // ---- one expansion per pair, inputs in shared memory, two blocks of 8 warps per SM ----------------------------------------
-// Rows of 1, 2, 4, .. 32 chunks (K = 64 .. 2048).  The pair's inputs sit in shared memory as the f32x2 operands of pair_dot,
-// laid out [block pair][operand pair][lane] so that a warp's 16-byte loads are conflict-free; a thread fits in 128
-// registers and 16 warps per SM hide the logic pipe's latencies.  The work is the pair-major sequence of row steps (a
-// step = the 32 / lanes-per-row rows a warp expands at once); blocks take contiguous equal shares of it, inside a pair the
-// block's warps take its steps round-robin, and the next row's streams are prefetched while the current row is expanded.
+// Any row of whole chunks.  The pair's inputs sit in shared memory; a thread fits in 128 registers and 16 warps per SM hide
+// the logic pipe's latencies.  The work is the pair-major sequence of row steps (pair_rows); blocks take contiguous equal
+// shares of it, inside a pair the block's warps take its steps round-robin.
+// Bound: the logic pipe (38 LOP3 + 4 PRMT + 2 SHF a block of 8 weights) together with the register file's read ports (a packed
+// multiply-add reads three register pairs, three cycles alone, 2.4 with one of them shared by neighbours): the arithmetic
+// alone runs at 0.875 clk a block and SM (256 threads x 2 blocks, a loop without streams).
 // Optionally the block first ROUTES: with logits given, warp t picks token t's top-k experts (route.cuh) and the pair
 // list is the T * top_k (token, expert) pairs; block 0 also stores ids and weights for the kernels that follow.
-// PF: coefficients per block.  4: SEED4P4; 3: SEED4 (24 states, the nibble word; the products are half as large, which the
-// slice scale makes up).
-template <int MODE, int PF>
-__global__ void __launch_bounds__(MV_THREADS, 2) mv_pair_kernel(MvParams a, KConst kc, int lpr_log2, RouteFuse rf) {
+// PF: coefficients per block.  4: SEED4P4; 3: SEED4 (24 states, the nibble word).
+template <int MODE, int PF, bool MULTI>
+__global__ void __launch_bounds__(MV_THREADS, 2) mv_pair_kernel(MvParams a, KConst kc, RowShape sh, RouteFuse rf) {
+    extern __shared__ __align__(16) ulonglong2 pair_sx[];
     __shared__ StreamTab tab;
+    __shared__ float part[MULTI ? PART_FLOATS : 1];
     __shared__ int32_t r_ind[256];   // the fused router's picks
     __shared__ float r_wt[256];
-    __shared__ __align__(16) ulonglong2 sx[4 * 4 * 32];   // [bp][c / 2][lane] = {x2[c], x2[c + 1]}
-    __shared__ __align__(16) ulonglong2 sm[4 * 2 * 32];   // [bp][p / 2][lane] = {xm2[p], xm2[p + 1]}
     load_stream_tab(tab, a.G, threadIdx.x, MV_THREADS);
     grid_dependents_go();
     grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
-    const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
+    const int lpr = 1 << sh.lpr_log2, rpw = 32 >> sh.lpr_log2;
+    const int ch = MULTI ? sh.ch : lpr;
     int P = a.count ? min(*a.count, a.P) : a.P;
     if (rf.logits) {          // the router: one warp per token, every block the same picks; block 0 stores them
         if (warp < rf.T) {
@@ -258,66 +371,24 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_pair_kernel(MvParams a, KCon
         WSlice wb = wa;
         if (MODE == MODE_GU) wb = a.wu[slice];
         // this warp's first streams are requested before the inputs are staged: their DRAM latency runs under it
-        int st = s_lo + warp;
-        int r = st * rpw + ro;
+        const int st = s_lo + (MULTI ? warp / sh.groups : warp), r = st * rpw + (lane >> sh.lpr_log2);
+        const int jc = (lane & (lpr - 1)) + (MULTI ? warp % sh.groups * lpr : 0);
         Chunk ka, kb;
-        if (st < s_hi && r < a.R) {
-            ka = load_chunk<PF>(wa, (size_t) r * lpr + jc);
-            if (MODE == MODE_GU) kb = load_chunk<PF>(wb, (size_t) r * lpr + jc);
+        if (st < s_hi && r < a.R && (!MULTI || jc < ch)) {
+            ka = load_chunk<PF>(wa, (size_t) r * ch + jc);
+            if (MODE == MODE_GU) kb = load_chunk<PF>(wb, (size_t) r * ch + jc);
         }
         if (pair != p_first) __syncthreads();   // the previous pair's inputs are no longer read
-        if (threadIdx.x < lpr * 4) {
-            const int j = threadIdx.x & (lpr - 1), bp = threadIdx.x >> lpr_log2;
-            stage_pair_inputs(a, a.xrow ? a.xrow[pair] : pair / a.xdiv, j, bp, sx, sm);
+        const void* row = input_row(a, a.xrow ? a.xrow[pair] : pair / a.xdiv);
+        for (int i = threadIdx.x; i < ch * 4; i += MV_THREADS) {
+            float x[16];
+            stage_load(row, a.xbf16, i >> 2, i & 3, x);
+            stage_store<PF>(x, i >> 2, i & 3, pair_sx);
         }
         __syncthreads();   // inputs staged (and, for the block's first pair, the stream table loaded)
-        const float sca = slice_scale(wa.eb + (4 - PF)), scb = slice_scale(wb.eb + (4 - PF));
-        for (; st < s_hi; st += MV_WARPS, r += MV_WARPS * rpw) {
-            const bool ok = r < a.R;
-            const int rn = r + MV_WARPS * rpw;
-            Chunk na, nb;
-            if (st + MV_WARPS < s_hi && rn < a.R) {
-                na = load_chunk<PF>(wa, (size_t) rn * lpr + jc);
-                if (MODE == MODE_GU) nb = load_chunk<PF>(wb, (size_t) rn * lpr + jc);
-            }
-            u64 acc = 0ull, accu = 0ull;
-            if (ok) {
-                const uint32_t swa[4] = {ka.s.x, ka.s.y, ka.s.z, ka.s.w}, cwa[4] = {ka.c.x, ka.c.y, ka.c.z, ka.c.w};
-                const uint32_t swb[4] = {kb.s.x, kb.s.y, kb.s.z, kb.s.w}, cwb[4] = {kb.c.x, kb.c.y, kb.c.z, kb.c.w};
-#pragma unroll
-                for (int bp = 0; bp < 4; ++bp) {
-                    u64 x2[8], xm2[4];
-#pragma unroll
-                    for (int cq = 0; cq < 4; ++cq) { const ulonglong2 t = sx[(bp * 4 + cq) * 32 + jc]; x2[2 * cq] = t.x; x2[2 * cq + 1] = t.y; }
-#pragma unroll
-                    for (int pq = 0; pq < 2; ++pq) { const ulonglong2 t = sm[(bp * 2 + pq) * 32 + jc]; xm2[2 * pq] = t.x; xm2[2 * pq + 1] = t.y; }
-                    if (PF == 4) {
-                        u64 q[4];
-                        pair_coefs(cwa[bp], kc, q);
-                        acc = fma2(pair_expand_dot(tab, swa[bp], q, x2, xm2), code_scale_pair(ka.cd, bp, kc), acc);
-                    } else {
-                        u64 q[3];
-                        pair_coefs3(cwa[bp], kc, q);
-                        acc = fma2(pair_expand_dot3(tab, swa[bp], q, x2, xm2), code_scale_pair3(cwa[bp], kc), acc);
-                    }
-                    if (MODE == MODE_GU && PF == 4) {
-                        u64 q[4];
-                        pair_coefs(cwb[bp], kc, q);
-                        accu = fma2(pair_expand_dot(tab, swb[bp], q, x2, xm2), code_scale_pair(kb.cd, bp, kc), accu);
-                    } else if (MODE == MODE_GU) {
-                        u64 q[3];
-                        pair_coefs3(cwb[bp], kc, q);
-                        accu = fma2(pair_expand_dot3(tab, swb[bp], q, x2, xm2), code_scale_pair3(cwb[bp], kc), accu);
-                    }
-                }
-            }
-            const float s = group_sum(pair_total(acc), lpr) * sca;
-            float su = 0.0f;
-            if (MODE == MODE_GU) su = group_sum(pair_total(accu), lpr) * scb;
-            if (ok && jc == 0) store_out<MODE>(a, pair, r, s, su);
-            ka = na;
-            if (MODE == MODE_GU) kb = nb;
-        }
+        auto store = [&](int rr, float s, float su) { store_out<MODE>(a, pair, rr, s, su); };
+        if constexpr (MULTI) pair_items<MODE, PF>(tab, kc, wa, wb, pair_sx, part, sh, a.R, s_lo, s_hi, ka, kb, store);
+        else pair_rows<MODE, PF>(tab, kc, wa, wb, pair_sx, sh.lpr_log2, a.R, s_lo, s_hi, ka, kb, store);
     }
 }
 
@@ -380,46 +451,18 @@ __device__ __forceinline__ bool step_wait(const unsigned* counter, unsigned targ
     return false;
 }
 
-// A pair's inputs from memory that other blocks of this grid have written: the loads bypass the non-coherent path.
-__device__ __forceinline__ void stage_pair_inputs_cg(const float* xrow, int j, int bp, ulonglong2* sx, ulonglong2* sm) {
-    float x[16], xm[8];
-    const float4* xp = (const float4*) (xrow + (size_t) j * 64 + bp * 16);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float4 t = __ldcg(xp + i);
-        x[4 * i] = t.x * NSL_XSCALE; x[4 * i + 1] = t.y * NSL_XSCALE; x[4 * i + 2] = t.z * NSL_XSCALE; x[4 * i + 3] = t.w * NSL_XSCALE;
-    }
-    block_offsets(x, xm);
-    block_offsets(x + 8, xm + 4);
-#pragma unroll
-    for (int cq = 0; cq < 4; ++cq) {
-        ulonglong2 t;
-        t.x = pack2(x[2 * cq], x[8 + 2 * cq]);
-        t.y = pack2(x[2 * cq + 1], x[8 + 2 * cq + 1]);
-        sx[(bp * 4 + cq) * 32 + j] = t;
-    }
-#pragma unroll
-    for (int pq = 0; pq < 2; ++pq) {
-        ulonglong2 t;
-        t.x = pack2(xm[2 * pq], xm[4 + 2 * pq]);
-        t.y = pack2(xm[2 * pq + 1], xm[4 + 2 * pq + 1]);
-        sm[(bp * 2 + pq) * 32 + j] = t;
-    }
-}
-
 struct StepShared {
     StreamTab tab;
     int32_t r_ind[256];
     float r_wt[256];
-    __align__(16) ulonglong2 sx[4 * 4 * 32];
-    __align__(16) ulonglong2 sm[4 * 2 * 32];
+    __align__(16) ulonglong2 sx[32 * CX];
     int abort;
 };
 
 // One phase: MODE_GU (x -> A, signals ready[pair]) or MODE_ROUND (A -> D, waits for ready[pair], signals done[token]).
 template <int MODE>
 __device__ __forceinline__ void step_phase(const StepParams& p, const KConst& kc, StepShared& sh, int P, int lpr_log2, unsigned rs_gu) {
-    const int K = MODE == MODE_GU ? p.d : p.ff, R = MODE == MODE_GU ? p.ff : p.d;
+    const int R = MODE == MODE_GU ? p.ff : p.d;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
     const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
@@ -451,54 +494,14 @@ __device__ __forceinline__ void step_phase(const StepParams& p, const KConst& kc
         __syncthreads();   // the previous pair's inputs are no longer read; the wait's outcome is known
         if (sh.abort) return;
         if (threadIdx.x < lpr * 4) {
-            const int j = threadIdx.x & (lpr - 1), bp = threadIdx.x >> lpr_log2;
-            if (MODE == MODE_GU) {
-                MvParams ax = {};
-                ax.x = p.x;
-                ax.xs = p.xs;
-                stage_pair_inputs(ax, pair / p.top_k, j, bp, sh.sx, sh.sm);
-            } else stage_pair_inputs_cg(p.A + (size_t) pair * p.ff, j, bp, sh.sx, sh.sm);
+            float x[16];
+            if (MODE == MODE_GU) stage_load(p.x + (size_t) (pair / p.top_k) * p.xs, 0, threadIdx.x >> 2, threadIdx.x & 3, x);
+            else stage_load<true>(p.A + (size_t) pair * p.ff, 0, threadIdx.x >> 2, threadIdx.x & 3, x);
+            stage_store<4>(x, threadIdx.x >> 2, threadIdx.x & 3, sh.sx);
         }
         __syncthreads();
-        const float sca = slice_scale(wa.eb), scb = slice_scale(wb.eb);
-        for (; st < s_hi; st += MV_WARPS, r += MV_WARPS * rpw) {
-            const bool ok = r < R;
-            const int rn = r + MV_WARPS * rpw;
-            Chunk na, nb;
-            if (st + MV_WARPS < s_hi && rn < R) {
-                na = load_chunk<4>(wa, (size_t) rn * lpr + jc);
-                if (MODE == MODE_GU) nb = load_chunk<4>(wb, (size_t) rn * lpr + jc);
-            }
-            u64 acc = 0ull, accu = 0ull;
-            if (ok) {
-                const uint32_t swa[4] = {ka.s.x, ka.s.y, ka.s.z, ka.s.w}, cwa[4] = {ka.c.x, ka.c.y, ka.c.z, ka.c.w};
-                const uint32_t swb[4] = {kb.s.x, kb.s.y, kb.s.z, kb.s.w}, cwb[4] = {kb.c.x, kb.c.y, kb.c.z, kb.c.w};
-#pragma unroll
-                for (int bp = 0; bp < 4; ++bp) {
-                    u64 x2[8], xm2[4];
-#pragma unroll
-                    for (int cq = 0; cq < 4; ++cq) { const ulonglong2 t = sh.sx[(bp * 4 + cq) * 32 + jc]; x2[2 * cq] = t.x; x2[2 * cq + 1] = t.y; }
-#pragma unroll
-                    for (int pq = 0; pq < 2; ++pq) { const ulonglong2 t = sh.sm[(bp * 2 + pq) * 32 + jc]; xm2[2 * pq] = t.x; xm2[2 * pq + 1] = t.y; }
-                    {
-                        u64 q[4];
-                        pair_coefs(cwa[bp], kc, q);
-                        acc = fma2(pair_expand_dot(sh.tab, swa[bp], q, x2, xm2), code_scale_pair(ka.cd, bp, kc), acc);
-                    }
-                    if (MODE == MODE_GU) {
-                        u64 q[4];
-                        pair_coefs(cwb[bp], kc, q);
-                        accu = fma2(pair_expand_dot(sh.tab, swb[bp], q, x2, xm2), code_scale_pair(kb.cd, bp, kc), accu);
-                    }
-                }
-            }
-            const float s = group_sum(pair_total(acc), lpr) * sca;
-            float su = 0.0f;
-            if (MODE == MODE_GU) su = group_sum(pair_total(accu), lpr) * scb;
-            if (ok && jc == 0) store_out<MODE>(a, pair, r, s, su);
-            ka = na;
-            if (MODE == MODE_GU) kb = nb;
-        }
+        pair_rows<MODE, 4>(sh.tab, kc, wa, wb, sh.sx, lpr_log2, R, s_lo, s_hi, ka, kb,
+                                  [&](int rr, float s, float su) { store_out<MODE>(a, pair, rr, s, su); });
         // this block's row steps of the pair are stored: publish their number
         __threadfence();
         __syncthreads();
@@ -562,101 +565,70 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_step_kernel(StepParams p, KC
 // the same order as when it is alone, so a pair's result does not depend on its partners).  The work is the sequence of
 // (unit, row step) items, an item of a unit with n pairs weighing GRP_W[n]; blocks take contiguous equal shares of the
 // weighted sequence, inside a unit the block's warps take its row steps round-robin, a row step being the 32 /
-// lanes-per-row rows a warp expands at once.  A unit's inputs sit in shared memory as the f32x2 operands of pair_dot,
+// lanes-per-row rows a warp expands at once.  A unit's inputs sit in shared memory as the f32x2 operands of pair_expand_dot,
 // laid out [pair][block pair][operand pair][lane] so that a warp's 16-byte loads are conflict-free.
-//
-// Optionally the block first ROUTES: with logits given, warp t picks token t's top-k experts (route.cuh) and the pair
-// list is the T * top_k (token, expert) pairs; block 0 also stores ids and weights for the kernels that follow.
-#ifndef NSL_GRP_NT
-#define NSL_GRP_NT 2
-#endif
-constexpr int GRP_NT = NSL_GRP_NT;                         // pairs that share one expansion at most
+constexpr int GRP_NT = 2;                         // pairs that share one expansion at most
 constexpr int GRP_MAX_PAIRS = 1024;               // pairs a block can sort; longer lists run ungrouped
 constexpr int GRP_SMALL = 128;                    // lists up to this length are ranked by counting (no sorting network)
-#ifndef NSL_GRP_W2
-#define NSL_GRP_W2 12
-#define NSL_GRP_W3 18
-#define NSL_GRP_W4 23
-#endif
-#ifndef NSL_GRP_MINB
-#define NSL_GRP_MINB 2
-#endif
-__device__ constexpr int GRP_W[5] = {0, 8, NSL_GRP_W2, NSL_GRP_W3, NSL_GRP_W4};   // relative cost of a row step for a unit of n pairs
-constexpr int GRP_SX = 4 * 4 * 32, GRP_SS = 4 * 32;               // entries of one pair's inputs (ulonglong2) / block sums (u64)
+__device__ constexpr int GRP_W[5] = {0, 8, 12, 18, 23};   // relative cost of a row step for a unit of n pairs
+constexpr int GRP_SX = 32 * CX;                    // one pair's staged inputs
 
 struct GrpShared {
     StreamTab tab;
     uint32_t key[GRP_MAX_PAIRS];                  // sorted (slice << 10 | pair)
     int32_t prefix[GRP_MAX_PAIRS + 1];            // weight of the units that start before sorted position i
     uint32_t tmp[GRP_SMALL];                      // short lists: unsorted keys, then unit weights
-    int32_t r_ind[256];                           // the fused router's picks
-    float r_wt[256];
     __align__(16) ulonglong2 sx[GRP_NT][GRP_SX];
-    __align__(16) u64 ss[GRP_NT][GRP_SS];
 };
 
 
-// One row step of one matrix for NT pairs: four block pairs expanded once each, dotted with every pair's inputs.
-// The state-value pairs of weights 4H .. 4H+3 of two adjacent blocks (half of pair_states): v[4 (c - 4H) + p].
+// The state-value pairs of weights 4H .. 4H+3 of two adjacent blocks (half of a pair's): v[4 (c - 4H) + p].
 template <int H>
-__device__ __forceinline__ void half_states(uint32_t a0, uint32_t a1, uint32_t g0, uint32_t g1, u64* v) {
+__device__ __forceinline__ void half_states(const Words& wa, const Words& wb, u64* v) {
 #define NSL_VH(C)                                                                                \
     {                                                                                            \
-        const uint32_t y0 = weight_word<4 * H + C>(a0, g0), y1 = weight_word<4 * H + C>(a1, g1);  \
-        v[4 * C + 0] = pack2(state_value<0>(y0), state_value<0>(y1));                            \
-        v[4 * C + 1] = pack2(state_value<1>(y0), state_value<1>(y1));                            \
-        v[4 * C + 2] = pack2(state_value<2>(y0), state_value<2>(y1));                            \
-        v[4 * C + 3] = pack2(state_value<3>(y0), state_value<3>(y1));                            \
+        constexpr int B = state_bit<4, C>(), W = 2 * H + C / 2;                                  \
+        v[4 * C + 0] = pack2(state_at<B, 0>(wa.w[W]), state_at<B, 0>(wb.w[W]));                  \
+        v[4 * C + 1] = pack2(state_at<B, 1>(wa.w[W]), state_at<B, 1>(wb.w[W]));                  \
+        v[4 * C + 2] = pack2(state_at<B, 2>(wa.w[W]), state_at<B, 2>(wb.w[W]));                  \
+        v[4 * C + 3] = pack2(state_at<B, 3>(wa.w[W]), state_at<B, 3>(wb.w[W]));                  \
     }
     NSL_VH(0) NSL_VH(1) NSL_VH(2) NSL_VH(3)
 #undef NSL_VH
 }
-
+// One half of a block pair (weights 4H .. 4H+3) against every pair's inputs.
+template <int NT, int H>
+__device__ __forceinline__ void unit_half(const Words& wa, const Words& wb, int bp, const ulonglong2* const* cx, u64 (*d)[4]) {
+    u64 v[16];
+    half_states<H>(wa, wb, v);
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+#pragma unroll
+        for (int cq = 0; cq < 2; ++cq) {
+            const ulonglong2 u = cx[t][bp * 4 + 2 * H + cq];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) d[t][p] = fma2(u.x, v[8 * cq + p], d[t][p]);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) d[t][p] = fma2(u.y, v[8 * cq + 4 + p], d[t][p]);
+        }
+    }
+}
 // One row step of one matrix for NT pairs: each block pair is expanded once, half of its weights at a time (so that only
 // 16 state-value pairs are held while every pair's inputs pass), and dotted with every pair's inputs.  Per pair the
-// operations and their order are those of pair_dot.
+// operations and their order are those of pair_expand_dot.
 template <int NT>
-__device__ __forceinline__ void unit_chunk(const StreamTab& tab, const KConst& kc, const Chunk& k, const ulonglong2 (*sx)[GRP_SX],
-                                           const u64 (*ss)[GRP_SS], int jc, u64* acc) {
+__device__ __forceinline__ void unit_chunk(const StreamTab& tab, const KConst& kc, const Chunk& k, const ulonglong2* const* cx, u64* acc) {
     const uint32_t sw[4] = {k.s.x, k.s.y, k.s.z, k.s.w}, cw[4] = {k.c.x, k.c.y, k.c.z, k.c.w};
 #pragma unroll
     for (int bp = 0; bp < 4; ++bp) {
-        const uint32_t g0 = tab.lo[__byte_perm(sw[bp], 0, 0x4440)] ^ tab.hi[__byte_perm(sw[bp], 0, 0x4441)];
-        const uint32_t g1 = tab.lo[__byte_perm(sw[bp], 0, 0x4442)] ^ tab.hi[__byte_perm(sw[bp], 0, 0x4443)];
-        const uint32_t a0 = __byte_perm(sw[bp], g0, 0x5410), a1 = __byte_perm(sw[bp], g1, 0x5432);
+        uint32_t g0, g1;
+        pair_stream(tab, sw[bp], g0, g1);
+        const Words wa = window_words<4, 0>(sw[bp], g0), wb = window_words<4, 1>(sw[bp], g1);
         u64 d[NT][4];
 #pragma unroll
-        for (int t = 0; t < NT; ++t) offsets_from_sum(ss[t][bp * 32 + jc], d[t]);
-        {
-            u64 v[16];
-            half_states<0>(a0, a1, g0, g1, v);
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-#pragma unroll
-                for (int cq = 0; cq < 2; ++cq) {
-                    const ulonglong2 u = sx[t][(bp * 4 + cq) * 32 + jc];
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) d[t][p] = fma2(u.x, v[8 * cq + p], d[t][p]);
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) d[t][p] = fma2(u.y, v[8 * cq + 4 + p], d[t][p]);
-                }
-            }
-        }
-        {
-            u64 v[16];
-            half_states<1>(a0, a1, g0, g1, v);
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-#pragma unroll
-                for (int cq = 0; cq < 2; ++cq) {
-                    const ulonglong2 u = sx[t][(bp * 4 + 2 + cq) * 32 + jc];
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) d[t][p] = fma2(u.x, v[8 * cq + p], d[t][p]);
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) d[t][p] = fma2(u.y, v[8 * cq + 4 + p], d[t][p]);
-                }
-            }
-        }
+        for (int t = 0; t < NT; ++t) offsets_from_sum(staged_sum(cx[t], bp), d[t]);
+        unit_half<NT, 0>(wa, wb, bp, cx, d);
+        unit_half<NT, 1>(wa, wb, bp, cx, d);
         u64 q[4];
         pair_coefs(cw[bp], kc, q);
         const u64 e2 = code_scale_pair(k.cd, bp, kc);
@@ -687,7 +659,18 @@ __device__ __noinline__ void unit_rows(UnitArgs ua, Chunk ka, Chunk kb) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
     const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
-    const float sca = slice_scale(ua.eba), scb = slice_scale(ua.ebb);
+    if (NT == 1) {      // one pair: the pair kernel's loop
+        WSlice wa = {}, wb = {};
+        wa.p[0] = ua.sa; wa.p[1] = ua.ca; wa.p[3] = ua.da; wa.eb = ua.eba;
+        wb.p[0] = ua.sb; wb.p[1] = ua.cb; wb.p[3] = ua.db; wb.eb = ua.ebb;
+        pair_rows<MODE, 4>(sh.tab, kc, wa, wb, sh.sx[0], lpr_log2, ua.R, s_lo, s_hi, ka, kb,
+                                  [&](int r, float s, float su) { store_unit<MODE>(ua, ua.pid[0], r, s, su); });
+        return;
+    }
+    const float sca = slice_scale(ua.eba + 4), scb = slice_scale(ua.ebb + 4);
+    const ulonglong2* cx[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) cx[t] = sh.sx[t] + jc * CX;
     int st = s_lo + warp, r = st * rpw + ro;
     for (; st < s_hi; st += MV_WARPS, r += MV_WARPS * rpw) {
         const bool ok = r < ua.R;
@@ -696,49 +679,18 @@ __device__ __noinline__ void unit_rows(UnitArgs ua, Chunk ka, Chunk kb) {
         u64 acc[NT], accu[NT];
 #pragma unroll
         for (int t = 0; t < NT; ++t) acc[t] = accu[t] = 0ull;
-        if (NT == 1) {      // one pair: the pair kernel's loop (its inputs are read once per block pair for both matrices)
-            Chunk na, nb;
-            if (more) {   // the next step's streams fly during this step's expansion
-                na = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) rn * lpr + jc);
-                if (MODE == MODE_GU) nb = load_chunk3(ua.sb, ua.cb, ua.db, (size_t) rn * lpr + jc);
-            }
-            if (ok) {
-                const uint32_t swa[4] = {ka.s.x, ka.s.y, ka.s.z, ka.s.w}, cwa[4] = {ka.c.x, ka.c.y, ka.c.z, ka.c.w};
-                const uint32_t swb[4] = {kb.s.x, kb.s.y, kb.s.z, kb.s.w}, cwb[4] = {kb.c.x, kb.c.y, kb.c.z, kb.c.w};
-#pragma unroll
-                for (int bp = 0; bp < 4; ++bp) {
-                    u64 x2[8], xm2[4];
-#pragma unroll
-                    for (int cq = 0; cq < 4; ++cq) { const ulonglong2 u = sh.sx[0][(bp * 4 + cq) * 32 + jc]; x2[2 * cq] = u.x; x2[2 * cq + 1] = u.y; }
-                    offsets_from_sum(sh.ss[0][bp * 32 + jc], xm2);
-                    {
-                        u64 q[4];
-                        pair_coefs(cwa[bp], kc, q);
-                        acc[0] = fma2(pair_expand_dot(sh.tab, swa[bp], q, x2, xm2), code_scale_pair(ka.cd, bp, kc), acc[0]);
-                    }
-                    if (MODE == MODE_GU) {
-                        u64 q[4];
-                        pair_coefs(cwb[bp], kc, q);
-                        accu[0] = fma2(pair_expand_dot(sh.tab, swb[bp], q, x2, xm2), code_scale_pair(kb.cd, bp, kc), accu[0]);
-                    }
-                }
-            }
+        // a matrix's streams for the next step are requested as soon as this step has used them up, into the registers they
+        // leave free, so no second set of stream registers is held
+        if (MODE == MODE_GU) {
+            if (ok) unit_chunk<NT>(sh.tab, kc, ka, cx, acc);
+            if (more) ka = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) rn * lpr + jc);
+            if (ok) unit_chunk<NT>(sh.tab, kc, kb, cx, accu);
+            if (more) kb = load_chunk3(ua.sb, ua.cb, ua.db, (size_t) rn * lpr + jc);
+        } else {      // one matrix: its next streams are requested before this step's expansion (a second set of registers)
+            Chunk na;
+            if (more) na = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) rn * lpr + jc);
+            if (ok) unit_chunk<NT>(sh.tab, kc, ka, cx, acc);
             ka = na;
-            if (MODE == MODE_GU) kb = nb;
-        } else {
-            // several pairs (or one matrix): a matrix's streams for the next step are requested as soon as this step has
-            // used them up, into the registers they leave free, so no second set of stream registers is held
-            if (MODE == MODE_GU) {
-                if (ok) unit_chunk<NT>(sh.tab, kc, ka, sh.sx, sh.ss, jc, acc);
-                if (more) ka = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) rn * lpr + jc);
-                if (ok) unit_chunk<NT>(sh.tab, kc, kb, sh.sx, sh.ss, jc, accu);
-                if (more) kb = load_chunk3(ua.sb, ua.cb, ua.db, (size_t) rn * lpr + jc);
-            } else {      // one matrix: its next streams are requested before this step's expansion (a second set of registers)
-                Chunk na;
-                if (more) na = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) rn * lpr + jc);
-                if (ok) unit_chunk<NT>(sh.tab, kc, ka, sh.sx, sh.ss, jc, acc);
-                ka = na;
-            }
         }
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
@@ -785,7 +737,7 @@ __device__ __forceinline__ void block_exclusive_scan(int32_t* a, int n) {
 
 
 template <int MODE>
-__global__ void __launch_bounds__(MV_THREADS, NSL_GRP_MINB) mv_grp_kernel(MvParams a, KConst kc, int lpr_log2, RouteFuse rf) {
+__global__ void __launch_bounds__(MV_THREADS, 2) mv_grp_kernel(MvParams a, KConst kc, int lpr_log2) {
     extern __shared__ __align__(16) unsigned char grp_smem[];
     GrpShared& sh = *reinterpret_cast<GrpShared*>(grp_smem);
     load_stream_tab(sh.tab, a.G, threadIdx.x, MV_THREADS);
@@ -795,31 +747,13 @@ __global__ void __launch_bounds__(MV_THREADS, NSL_GRP_MINB) mv_grp_kernel(MvPara
     const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
     const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
     int P = a.count ? min(*a.count, a.P) : a.P;
-    if (rf.logits) {          // the router: one warp per token, every block the same picks
-        if (warp < rf.T) {
-            const float* l = rf.logits + (size_t) warp * rf.ld;
-            if (rf.n_exp <= 128) route_row<4>(rf.n_exp, rf.top_k, l, lane, sh.r_ind + warp * rf.top_k, sh.r_wt + warp * rf.top_k);
-            else if (rf.n_exp <= 512) route_row<16>(rf.n_exp, rf.top_k, l, lane, sh.r_ind + warp * rf.top_k, sh.r_wt + warp * rf.top_k);
-            else route_row<32>(rf.n_exp, rf.top_k, l, lane, sh.r_ind + warp * rf.top_k, sh.r_wt + warp * rf.top_k);
-        }
-        P = rf.T * rf.top_k;
-        __syncthreads();
-        if (blockIdx.x == 0 && (int) threadIdx.x < P) {
-            rf.ind_out[threadIdx.x] = sh.r_ind[threadIdx.x];
-            rf.wt_out[threadIdx.x] = sh.r_wt[threadIdx.x];
-        }
-    }
     if (P <= 0) return;
     const int rs = (a.R + rpw - 1) / rpw;             // row steps per unit
-#ifdef NSL_GRP_FORCE_PLAIN
-    const bool grouped = false;
-#else
     const bool grouped = P <= GRP_MAX_PAIRS;
-#endif
     long long total;
     if (grouped) {
         const bool small = P <= GRP_SMALL;
-        auto slice_of = [&](int i) { return rf.logits ? sh.r_ind[i] : (a.sel ? a.sel[i] : 0); };
+        auto slice_of = [&](int i) { return a.sel ? a.sel[i] : 0; };
         if (small) {      // every thread ranks one key among all: two barriers instead of a sorting network's dozens
             const int i = threadIdx.x;
             uint32_t mine = 0xFFFFFFFFu;
@@ -897,7 +831,7 @@ __global__ void __launch_bounds__(MV_THREADS, NSL_GRP_MINB) mv_grp_kernel(MvPara
 #pragma unroll
             for (int t = 0; t < GRP_NT; ++t) pid[t] = (int) (sh.key[u + (t < n ? t : 0)] & 1023u);
             slice = (int) (sh.key[u] >> 10);
-        } else slice = rf.logits ? sh.r_ind[u] : (a.sel ? a.sel[u] : 0);
+        } else slice = a.sel ? a.sel[u] : 0;
         const int s_lo = u == u_first ? s_first : 0, s_hi = u == u_last ? s_last : rs;
         if (s_lo < s_hi) {
             // Two chains of dependent loads start here and run side by side: pair -> input row -> inputs (this thread's share of
@@ -907,7 +841,7 @@ __global__ void __launch_bounds__(MV_THREADS, NSL_GRP_MINB) mv_grp_kernel(MvPara
             int e0 = threadIdx.x, t0 = e0 / per, rem0 = e0 - t0 * per;
             if (e0 < n_stage) {
                 const int p = grouped ? (int) (sh.key[u + t0] & 1023u) : u;
-                stage_load(a, a.xrow ? a.xrow[p] : p / a.xdiv, rem0 & (lpr - 1), rem0 >> lpr_log2, xin);
+                stage_load(input_row(a, a.xrow ? a.xrow[p] : p / a.xdiv), a.xbf16, rem0 >> 2, rem0 & 3, xin);
             }
             const WSlice wa = a.ws ? a.ws[slice] : a.w0;
             WSlice wb = wa;
@@ -920,12 +854,12 @@ __global__ void __launch_bounds__(MV_THREADS, NSL_GRP_MINB) mv_grp_kernel(MvPara
             }
             if (staged) __syncthreads();   // the previous unit's inputs are no longer read
             staged = true;
-            if (e0 < n_stage) stage_store(xin, rem0 & (lpr - 1), rem0 >> lpr_log2, sh.sx[t0], sh.ss[t0]);
+            if (e0 < n_stage) stage_store<4>(xin, rem0 >> 2, rem0 & 3, sh.sx[t0]);
             for (int i = threadIdx.x + MV_THREADS; i < n_stage; i += MV_THREADS) {      // units of more than two pairs
                 const int t = i / per, rem = i - t * per;
                 const int p = grouped ? (int) (sh.key[u + t] & 1023u) : u;
-                stage_load(a, a.xrow ? a.xrow[p] : p / a.xdiv, rem & (lpr - 1), rem >> lpr_log2, xin);
-                stage_store(xin, rem & (lpr - 1), rem >> lpr_log2, sh.sx[t], sh.ss[t]);
+                stage_load(input_row(a, a.xrow ? a.xrow[p] : p / a.xdiv), a.xbf16, rem >> 2, rem & 3, xin);
+                stage_store<4>(xin, rem >> 2, rem & 3, sh.sx[t]);
             }
             __syncthreads();
             UnitArgs ua;
@@ -944,108 +878,95 @@ __global__ void __launch_bounds__(MV_THREADS, NSL_GRP_MINB) mv_grp_kernel(MvPara
     }
 }
 
-// ---- inputs in shared memory: NT tokens share each expansion (dense verify rows), or rows longer than 32 chunks ------
-// Dense: the P = NT tokens are staged once per block and the rows are split over every warp of the grid.  Gather
-// (NT = 1): blocks are dealt to pairs and stage their pair's input row.
-// Shared layout, per token (K * 6 bytes): the f32x2 operands of pair_dot as 16-byte units, inputs
-// [block pair in chunk 0..3][operand pair 0..3][chunk], then centring constants [0..3][0..1][chunk]: the lanes of a warp
-// hold consecutive chunks, so their 16-byte loads are consecutive (no bank conflicts).
-template <int MODE, int NT>
-__global__ void __launch_bounds__(MV_THREADS, 1) mv_smemx_kernel(MvParams a, KConst kc, int lpr_log2, int dense) {
-    extern __shared__ __align__(16) float smem_f[];
+// ---- dense products: NT rows of inputs share each expansion ---------------------------------------------------------------
+// The weights of a block pair are formed once (weight form) and multiplied into every row of inputs; the inputs of all rows
+// sit in shared memory.  Every number of rows uses the same form, so a row's bits do not depend on the others.  The row steps
+// are dealt to the warps of the grid block by block, so a small matrix still spreads over the SMs.
+// Bound: as the pair kernel for one row (0.93 clk a block and SM in a loop without streams); a further row adds 4 packed
+// multiply-adds a block and its share of the input loads (16 bytes a lane for two weights of two blocks: with 32 lanes a row
+// 0.25 clk a block of the shared-memory pipe, half of that with 16).
+template <int PF, int NT, int C>
+__device__ __forceinline__ void dense_two_weights(const Words& wa, const Words& wb, const u64* q, const ulonglong2* const* cx, int bp, u64* d) {
+    const u64 w0 = pair_weight<PF, 2 * C>(wa, wb, q), w1 = pair_weight<PF, 2 * C + 1>(wa, wb, q);
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        const ulonglong2 u = cx[t][bp * 4 + C];
+        d[t] = fma2(u.x, w0, d[t]);
+        d[t] = fma2(u.y, w1, d[t]);
+    }
+}
+
+template <int PF, int NT>
+__global__ void __launch_bounds__(MV_THREADS, 2) mv_dense_kernel(MvParams a, KConst kc, RowShape sh) {
+    extern __shared__ __align__(16) ulonglong2 dense_sx[];
     __shared__ StreamTab tab;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lpr = 1 << sh.lpr_log2, rpw = 32 >> sh.lpr_log2, passes = 1 << (sh.lv - sh.lpr_log2);
+    const int jc = lane & (lpr - 1), ro = lane >> sh.lpr_log2, ch = sh.ch;
+    const int steps = (a.R + rpw - 1) / rpw, stride = (int) gridDim.x * MV_WARPS;
+    int st = warp * (int) gridDim.x + (int) blockIdx.x, r = st * rpw + ro, base = 0, pass = 0;
+    Chunk k;
+    if (st < steps && r < a.R && jc < ch) k = load_chunk<PF>(a.w0, (size_t) r * ch + jc);      // weights never change: requested before the wait
     load_stream_tab(tab, a.G, threadIdx.x, MV_THREADS);
     grid_dependents_go();
     grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
-    const int K = a.K, nbp = K / 16, ch = K / 64;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
-    const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
-    const int cpp = dense ? (int) gridDim.x : ((int) gridDim.x / a.P > 0 ? (int) gridDim.x / a.P : 1);
-    const long long nvc = dense ? (long long) gridDim.x : (long long) a.P * cpp;
-    for (long long vc = blockIdx.x; vc < nvc; vc += gridDim.x) {
-        const int pair = dense ? 0 : (int) (vc / cpp), ci = dense ? (int) blockIdx.x : (int) (vc % cpp);
-        const int slice = a.sel ? a.sel[pair] : 0;
-        const WSlice wa = a.ws ? a.ws[slice] : a.w0;
-        WSlice wb = wa;
-        if (MODE == MODE_GU) wb = a.wu[slice];
-        __syncthreads();   // the previous pair's inputs are no longer read
-        for (int i = threadIdx.x; i < NT * nbp; i += MV_THREADS) {
-            const int t = i / nbp, bp = i % nbp;
-            const float* xp = a.x + (size_t) (dense ? t : pair / a.xdiv) * a.xs + 16 * bp;
-            float x[16], xm[8];
+    for (int i = threadIdx.x; i < NT * ch * 4; i += MV_THREADS) {
+        const int t = i / (ch * 4), e = i - t * (ch * 4);
+        float x[16];
+        stage_load(a.x + (size_t) t * a.xs, 0, e >> 2, e & 3, x);
+        stage_store<PF>(x, e >> 2, e & 3, dense_sx + (size_t) t * ch * CX);
+    }
+    __syncthreads();
+    const float sc = slice_scale(a.w0.eb + (8 - PF));
+    u64 acc[NT];
+    float stk[NT][3];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float4 v4 = __ldg((const float4*) xp + j);
-                x[4 * j] = v4.x * NSL_XSCALE; x[4 * j + 1] = v4.y * NSL_XSCALE; x[4 * j + 2] = v4.z * NSL_XSCALE; x[4 * j + 3] = v4.w * NSL_XSCALE;
-            }
-            block_offsets(x, xm);
-            block_offsets(x + 8, xm + 4);
-            ulonglong2* tok = (ulonglong2*) smem_f + (size_t) t * ch * 24;
-            const int jch = bp >> 2, b4 = bp & 3;
+    for (int t = 0; t < NT; ++t) acc[t] = 0ull;
+    while (st < steps) {
+        int sn = st, rn = r, bn = base + 32, pn = pass;
+        if (bn >= ch) {
+            if (pass + 1 < passes) { pn = pass + 1; bn = pass_offset(pn, sh.lv); }      // (possibly a pass without chunks: zeros)
+            else { sn = st + stride; rn = r + stride * rpw; bn = 0; pn = 0; }
+        }
+        Chunk n;
+        if (sn < steps && rn < a.R && bn + jc < ch) n = load_chunk<PF>(a.w0, (uint32_t) (rn * ch + bn + jc));
+        const bool ok = r < a.R;
+        if (ok && base + jc < ch) {
+            const ulonglong2* cx[NT];
 #pragma unroll
-            for (int cq = 0; cq < 4; ++cq) {
-                ulonglong2 v2;
-                v2.x = pack2(x[2 * cq], x[8 + 2 * cq]);
-                v2.y = pack2(x[2 * cq + 1], x[8 + 2 * cq + 1]);
-                tok[(b4 * 4 + cq) * ch + jch] = v2;
-            }
+            for (int t = 0; t < NT; ++t) cx[t] = dense_sx + (size_t) (t * ch + base + jc) * CX;
+            const uint32_t sw[4] = {k.s.x, k.s.y, k.s.z, k.s.w}, cw[4] = {k.c.x, k.c.y, k.c.z, k.c.w};
 #pragma unroll
-            for (int pq = 0; pq < 2; ++pq) {
-                ulonglong2 v2;
-                v2.x = pack2(xm[2 * pq], xm[4 + 2 * pq]);
-                v2.y = pack2(xm[2 * pq + 1], xm[4 + 2 * pq + 1]);
-                tok[16 * ch + (b4 * 2 + pq) * ch + jch] = v2;
+            for (int bp = 0; bp < 4; ++bp) {
+                uint32_t g0, g1;
+                pair_stream(tab, sw[bp], g0, g1);
+                const Words wa = window_words<PF, 0>(sw[bp], g0), wb = window_words<PF, 1>(sw[bp], g1);
+                u64 q[4], d[NT];
+                if (PF == 4) pair_coefs(cw[bp], kc, q); else pair_coefs3(cw[bp], kc, q);
+                const u64 kq = pair_centre<PF>(q), e2 = PF == 4 ? code_scale_pair(k.cd, bp, kc) : code_scale_pair3(cw[bp], kc);
+#pragma unroll
+                for (int t = 0; t < NT; ++t) d[t] = mul2(kq, staged_sum(cx[t], bp));
+                dense_two_weights<PF, NT, 0>(wa, wb, q, cx, bp, d);
+                dense_two_weights<PF, NT, 1>(wa, wb, q, cx, bp, d);
+                dense_two_weights<PF, NT, 2>(wa, wb, q, cx, bp, d);
+                dense_two_weights<PF, NT, 3>(wa, wb, q, cx, bp, d);
+#pragma unroll
+                for (int t = 0; t < NT; ++t) acc[t] = fma2(d[t], e2, acc[t]);
             }
         }
-        __syncthreads();
-        const float sca = slice_scale(wa.eb), scb = slice_scale(wb.eb);
-        const int wi = ci * MV_WARPS + warp, step = cpp * MV_WARPS * rpw;
-        for (int rbase = wi * rpw; rbase < a.R; rbase += step) {
-            const int r = rbase + ro;
-            const bool ok = r < a.R;
-            u64 s2[NT], su2[NT];
-#pragma unroll
-            for (int t = 0; t < NT; ++t) s2[t] = su2[t] = 0ull;
-            if (ok) {
-                for (int j = jc; j < ch; j += lpr) {
-                    const Chunk ka = load_chunk(wa, (size_t) r * ch + j);
-                    Chunk kb = ka;
-                    if (MODE == MODE_GU) kb = load_chunk(wb, (size_t) r * ch + j);
-#pragma unroll
-                    for (int half = 0; half < (MODE == MODE_GU ? 2 : 1); ++half) {
-                        const Chunk& k = half ? kb : ka;
-                        const uint32_t sw[4] = {k.s.x, k.s.y, k.s.z, k.s.w}, cw[4] = {k.c.x, k.c.y, k.c.z, k.c.w};
-#pragma unroll
-                        for (int bp = 0; bp < 4; ++bp) {
-                            u64 v[32], q[4];
-                            pair_states(tab, sw[bp], v);
-                            pair_coefs(cw[bp], kc, q);
-                            const u64 e2 = code_scale_pair(k.cd, bp, kc);
-#pragma unroll
-                            for (int t = 0; t < NT; ++t) {
-                                u64 x2[8], xm2[4];
-                                const ulonglong2* tok = (const ulonglong2*) smem_f + (size_t) t * ch * 24;
-#pragma unroll
-                                for (int c = 0; c < 4; ++c) { const ulonglong2 u = tok[(bp * 4 + c) * ch + j]; x2[2 * c] = u.x; x2[2 * c + 1] = u.y; }
-#pragma unroll
-                                for (int p = 0; p < 2; ++p) { const ulonglong2 u = tok[16 * ch + (bp * 2 + p) * ch + j]; xm2[2 * p] = u.x; xm2[2 * p + 1] = u.y; }
-                                const u64 d = pair_dot(v, q, x2, xm2);
-                                if (half) su2[t] = fma2(d, e2, su2[t]);
-                                else s2[t] = fma2(d, e2, s2[t]);
-                            }
-                        }
-                    }
-                }
-            }
+        if (pn != pass || sn != st) {      // the pass's last chunk
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-                const float st = group_sum(pair_total(s2[t]), lpr) * sca;
-                float sut = 0.0f;
-                if (MODE == MODE_GU) sut = group_sum(pair_total(su2[t]), lpr) * scb;
-                if (ok && jc == 0) store_out<MODE>(a, dense ? t : pair, r, st, sut);
+                float s = tree_push(stk[t], pass, pair_total(acc[t]));
+                acc[t] = 0ull;
+                if (sn != st) {      // and the row's
+                    s = group_sum(s, lpr) * sc;
+                    if (ok && jc == 0) store_out<MODE_ROUND>(a, t, r, s, 0.0f);
+                }
             }
         }
+        k = n;
+        st = sn; r = rn; base = bn; pass = pn;
     }
 }
 
@@ -1150,28 +1071,95 @@ static void allow_smem(K kernel, bool* done, size_t bytes) {      // once per de
     }
 }
 
-template <int MODE, int NT>
-static void launch_smemx(cudaStream_t s, const MvParams& a, int lpr_log2, int dense, int grid, size_t smem) {
+// How many lanes a row gets: the fewest chunk slots that a warp spends on its share, the rows dealt to all warps of the grid.
+// Rows of 2^j <= 32 chunks keep a lane a chunk: its loop is the shorter one (config 1 at 8 rows: 132 us a step, 135.5 with 16
+// lanes a row).
+static RowShape row_shape(int ch, long long rows, int warps) {
+    int lv = 0;
+    while ((1 << lv) < (ch < 32 ? ch : 32)) ++lv;
+    RowShape best = {ch, lv, lv, 1};
+    if (ch == 1 << lv) return best;
+    double best_cost = 0.0;
+    for (int l = lv; l >= 0 && l >= lv - 3; --l) {
+        int slots = 0;      // chunk rounds of a row step
+        for (int p = 0; p < (1 << (lv - l)); ++p) {
+            const int off = pass_offset(p, lv);
+            slots += off < ch ? (ch - off + 31) / 32 : 0;
+        }
+        const long long steps = (rows * (1 << l) + 31) / 32;
+        const double cost = (double) ((steps + warps - 1) / warps) * (slots + 0.4);      // 0.4: a step's shuffles and stores
+        if (l == lv || cost < best_cost) { best.lpr_log2 = l; best_cost = cost; }
+    }
+    return best;
+}
+
+template <int MODE, int PF, bool MULTI>
+static void launch_pair_v(cudaStream_t s, const MvParams& a, RowShape sh, const RouteFuse& rf, size_t smem) {
     static bool attr_set[16];
-    allow_smem(mv_smemx_kernel<MODE, NT>, attr_set, (size_t) max_smem_optin() - 4096);
-    launch(mv_smemx_kernel<MODE, NT>, grid, MV_THREADS, smem, s, a, kconst(), lpr_log2, dense);
+    if (smem > 40 * 1024) allow_smem(mv_pair_kernel<MODE, PF, MULTI>, attr_set, (size_t) max_smem_optin() - 8192);
+    launch(mv_pair_kernel<MODE, PF, MULTI>, sm_count() * 2, MV_THREADS, smem, s, a, kconst(), sh, rf);
+}
+static size_t staged_bytes(int ch) { return (size_t) ch * CX * 16; }
+// Rows that are not 2^j <= 32 chunks: groups of 8, 4 or 2 lanes, whichever leaves the fewest lane slots empty (fewer lanes read
+// shorter runs of the streams: they have to save a twentieth).  A function of the row's length alone, so a row's bits do not
+// depend on the list it is part of.
+static RowShape item_shape(int ch) {
+    RowShape best = {ch, 0, 0, ch};
+    double best_cost = 1e30;
+    for (int l = 3; l >= 1; --l) {
+        const int groups = (ch + (1 << l) - 1) >> l;
+        const double cost = (double) (groups << l) / ch + 0.05 * (3 - l);
+        if (cost < best_cost && part_steps(groups, l, 2) >= 1) { best.lpr_log2 = l; best.groups = groups; best_cost = cost; }
+    }
+    return best;
+}
+template <int MODE, int PF>
+static void launch_pair(cudaStream_t s, const MvParams& a, const RouteFuse& rf) {
+    const int ch = a.K / 64;
+    if (ch <= 32 && (ch & (ch - 1)) == 0) launch_pair_v<MODE, PF, false>(s, a, RowShape{ch, log2_floor(ch), 0, 1}, rf, staged_bytes(ch));
+    else launch_pair_v<MODE, PF, true>(s, a, item_shape(ch), rf, staged_bytes(ch));
+    count_launch();
 }
 
 // Lists of more than GRP_MIN_PAIRS pairs go to the grouped kernel (one expansion per distinct slice, up to GRP_NT pairs a
 // unit): its plan and its costlier second pair pay once a good share of the pairs meet on a slice -- an expert-parallel
 // rank's list or all of a 64-row batch; a decode step's 8 .. 64 pairs over 128 experts run faster pair by pair.
 constexpr int GRP_MIN_PAIRS = 64;
-static int g_grp_min_pairs = GRP_MIN_PAIRS;
 
 template <int MODE>
-static void launch_grp(cudaStream_t s, const MvParams& a, int lpr_log2, const RouteFuse& rf) {
-    if (a.P <= g_grp_min_pairs || rf.logits) {
-        launch(mv_pair_kernel<MODE, 4>, sm_count() * 2, MV_THREADS, 0, s, a, kconst(), lpr_log2, rf);
-        return;
-    }
+static void launch_grp(cudaStream_t s, const MvParams& a, int lpr_log2) {
     static bool attr_set[16];
     allow_smem(mv_grp_kernel<MODE>, attr_set, sizeof(GrpShared));
-    launch(mv_grp_kernel<MODE>, sm_count() * NSL_GRP_MINB, MV_THREADS, sizeof(GrpShared), s, a, kconst(), lpr_log2, rf);
+    launch(mv_grp_kernel<MODE>, sm_count() * 2, MV_THREADS, sizeof(GrpShared), s, a, kconst(), lpr_log2);
+    count_launch();
+}
+
+template <int PF, int NT>
+static void launch_dense_v(cudaStream_t s, const MvParams& a, size_t smem) {
+    static bool attr_set[16];
+    if (smem > 40 * 1024) allow_smem(mv_dense_kernel<PF, NT>, attr_set, (size_t) max_smem_optin() - 8192);
+    const int bps = smem > 100 * 1024 ? 1 : 2;
+    const RowShape sh = row_shape(a.K / 64, a.R, sm_count() * bps * MV_WARPS);
+    const int steps = (a.R * (1 << sh.lpr_log2) + 31) / 32;
+    launch(mv_dense_kernel<PF, NT>, steps < sm_count() * bps ? steps : sm_count() * bps, MV_THREADS, smem, s, a, kconst(), sh);
+    count_launch();
+}
+// T rows on one slice; more rows than their inputs fit shared memory go in two launches (a row's bits do not depend on the rest).
+template <int PF>
+static void launch_dense(cudaStream_t s, MvParams a, int T) {
+    const size_t one = staged_bytes(a.K / 64), room = (size_t) max_smem_optin() - 8192;
+    while (T > 0) {
+        int n = T;
+        while (n > 1 && n * one > room) n = (n + 1) / 2;
+        switch (n) {
+#define NSL_CASE(N) case N: launch_dense_v<PF, N>(s, a, N * one); break;
+            NSL_CASE(1) NSL_CASE(2) NSL_CASE(3) NSL_CASE(4) NSL_CASE(5) NSL_CASE(6) NSL_CASE(7) NSL_CASE(8)
+#undef NSL_CASE
+        }
+        a.x += (size_t) n * a.xs;
+        a.y += (size_t) n * a.ys;
+        T -= n;
+    }
 }
 
 // The streams of a slice given by value (a dense call) can be checked on the host; slices in a device table are the
@@ -1180,59 +1168,34 @@ static bool slice_aligned(const WSlice& w) {
     return aligned16(w.p[0]) && aligned16(w.p[1]) && ((uintptr_t) w.p[3] & 3u) == 0;
 }
 
-template <int MODE>
+// PF = 4: SEED4P4; 3: SEED4.  The chunked kernels read whole chunks with 16-byte loads: rows of inputs and (checked where
+// the slice is on the host) the streams must be aligned for that, and one row of inputs must fit shared memory; anything else
+// goes to the any-shape kernel.
+template <int MODE, int PF>
 static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse& rf = RouteFuse{}) {
     if (a.R <= 0 || a.P <= 0 || T <= 0) return;
     if (a.K <= 0 || a.K % 8) { set_error("seed mat-vec: K = %d is not a multiple of 8", a.K); return; }
     if (T > MV_MAXT) { set_error("seed mat-vec: %d tokens, at most %d", T, MV_MAXT); return; }
-    const int dense = a.sel == NULL && rf.logits == NULL, sms = sm_count();
+    const bool dense = a.sel == NULL && rf.logits == NULL;
     const int ch = a.K / 64;
-    // The chunked kernels read whole chunks with 16-byte loads: rows of inputs and (checked where the slice is on the
-    // host) the streams must be aligned for that; anything else goes to the any-shape kernel.
-    const bool chunked = a.K % 64 == 0 && aligned16(a.x) && a.xs % (a.xbf16 ? 8 : 4) == 0 && (a.ws != NULL || slice_aligned(a.w0));
-    const bool pow2 = ch > 0 && (ch & (ch - 1)) == 0;
-    if ((a.xrow || a.count || a.xbf16 || rf.logits) && !(chunked && pow2 && ch <= 32 && T == 1)) {
-        set_error("seed mat-vec: the routed / row-index / device-count / bf16-input forms need K = 64 * 2^j <= 2048 and aligned rows (K = %d)", a.K);
-        return;
-    }
-    if (chunked && T == 1 && pow2 && ch <= 32) {
-        launch_grp<MODE>(s, a, log2_floor(ch), rf);
-        count_launch();
-        return;
-    }
-    const size_t smem = (size_t) (dense ? T : 1) * a.K * 6;   // inputs [K] and centring constants [K/2] per token
-    if (chunked && smem <= (size_t) max_smem_optin() - 4096) {
-        const int lpr_log2 = log2_floor(ch < 32 ? ch : 32);
-        if constexpr (MODE == MODE_GU) launch_smemx<MODE, 1>(s, a, lpr_log2, dense, sms, smem);
-        else switch (dense ? T : 1) {
-#define NSL_CASE(N) case N: launch_smemx<MODE, N>(s, a, lpr_log2, dense, sms, smem); break;
-            NSL_CASE(1) NSL_CASE(2) NSL_CASE(3) NSL_CASE(4) NSL_CASE(5) NSL_CASE(6) NSL_CASE(7) NSL_CASE(8)
-#undef NSL_CASE
+    const bool chunked = a.K % 64 == 0 && aligned16(a.x) && a.xs % (a.xbf16 ? 8 : 4) == 0 && (a.ws != NULL || slice_aligned(a.w0)) &&
+                         staged_bytes(ch) <= (size_t) max_smem_optin() - 8192;
+    if (!chunked) {
+        if (a.xrow || a.count || a.xbf16 || rf.logits) {
+            set_error("seed mat-vec: the routed / row-index / device-count / bf16-input forms need K a multiple of 64 and aligned rows (K = %d)", a.K);
+            return;
         }
+        launch(mv_generic_kernel<MODE, PF>, sm_count() * 2, MV_THREADS, 0, s, a, kconst(), dense ? T : 1);
         count_launch();
         return;
     }
-    launch(mv_generic_kernel<MODE, 4>, sms * 2, MV_THREADS, 0, s, a, kconst(), dense ? T : 1);
-    count_launch();
-}
-
-// P = 3 (SEED4): the pair kernel for rows of 64 * 2^j <= 2048 weights -- the routed experts' gathers, and a dense call as T
-// "pairs" on the one slice (token t reads input row t and writes output row t; every token expands the rows itself, so a
-// token's result cannot depend on the others) -- the any-shape kernel for everything else.
-template <int MODE>
-static void launch_mv3(cudaStream_t s, const MvParams& a, int T) {
-    if (a.R <= 0 || a.P <= 0 || T <= 0) return;
-    if (a.K <= 0 || a.K % 8) { set_error("seed mat-vec: K = %d is not a multiple of 8", a.K); return; }
-    if (T > MV_MAXT) { set_error("seed mat-vec: %d tokens, at most %d", T, MV_MAXT); return; }
-    const int ch = a.K / 64;
-    const bool chunked = a.K % 64 == 0 && aligned16(a.x) && a.xs % 4 == 0 && (a.ws != NULL || (aligned16(a.w0.p[0]) && aligned16(a.w0.p[1])));
-    if (chunked && ch > 0 && (ch & (ch - 1)) == 0 && ch <= 32) {
-        launch(mv_pair_kernel<MODE, 3>, sm_count() * 2, MV_THREADS, 0, s, a, kconst(), log2_floor(ch), RouteFuse{});
-        count_launch();
-        return;
+    if constexpr (MODE == MODE_ROUND) {
+        if (dense) { launch_dense<PF>(s, a, T); return; }
     }
-    launch(mv_generic_kernel<MODE, 3>, sm_count() * 2, MV_THREADS, 0, s, a, kconst(), a.sel ? 1 : T);
-    count_launch();
+    if constexpr (PF == 4) {
+        if (a.P > GRP_MIN_PAIRS && !rf.logits && ch <= 32 && (ch & (ch - 1)) == 0) { launch_grp<MODE>(s, a, log2_floor(ch)); return; }
+    }
+    launch_pair<MODE, PF>(s, a, rf);
 }
 
 // The decode step in one launch; false (nothing launched) when a size is outside what the pair kernel serves.
@@ -1271,37 +1234,37 @@ void kc_mv(cudaStream_t s, int fmt, WSlice w, int K, int R, const float* x, int 
     }
     if (!seed_fmt(fmt, "kc_mv")) return;
     MvParams a = {NULL, NULL, w, NULL, x, y, G, K, R, T, 1, xs, ys, add, 0, NULL, NULL, 0};
-    if (fmt == MF_SEED4) launch_mv3<MODE_ROUND>(s, a, T);
-    else launch_mv<MODE_ROUND>(s, a, T);
+    if (fmt == MF_SEED4) launch_mv<MODE_ROUND, 3>(s, a, T);
+    else launch_mv<MODE_ROUND, 4>(s, a, T);
 }
 
 void kc_mv_sel(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys,
                const int32_t* sel, int P, int xdiv, const uint32_t* G) {
     if (!seed_fmt(fmt, "kc_mv_sel")) return;
     MvParams a = {ws, NULL, WSlice{}, sel, x, y, G, K, R, P, xdiv, xs, ys, 0, 0, NULL, NULL, 0};
-    if (fmt == MF_SEED4) launch_mv3<MODE_ROUND>(s, a, 1);
-    else launch_mv<MODE_ROUND>(s, a, 1);
+    if (fmt == MF_SEED4) launch_mv<MODE_ROUND, 3>(s, a, 1);
+    else launch_mv<MODE_ROUND, 4>(s, a, 1);
 }
 
 void kc_mv_gu(cudaStream_t s, int fmt, const WSlice* wg, const WSlice* wu, int K, int R, const float* x, int xs, float* out,
               int ys, const int32_t* sel, int P, int xdiv, const uint32_t* G) {
     if (!seed_fmt(fmt, "kc_mv_gu")) return;
     MvParams a = {wg, wu, WSlice{}, sel, x, out, G, K, R, P, xdiv, xs, ys, 0, 0, NULL, NULL, 0};
-    if (fmt == MF_SEED4) launch_mv3<MODE_GU>(s, a, 1);
-    else launch_mv<MODE_GU>(s, a, 1);
+    if (fmt == MF_SEED4) launch_mv<MODE_GU, 3>(s, a, 1);
+    else launch_mv<MODE_GU, 4>(s, a, 1);
 }
 
 void nsl_mv_raw(cudaStream_t s, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys,
                 const int32_t* sel, int P, int xdiv, const uint32_t* G) {
     MvParams a = {sel ? ws : NULL, NULL, WSlice{}, sel, x, y, G, K, R, P, xdiv > 0 ? xdiv : 1, xs, ys, 0, 1, NULL, NULL, 0};
     if (!sel) a.w0 = *ws;   // dense: ws is a host pointer to the one slice
-    launch_mv<MODE_ROUND>(s, a, sel ? 1 : P);
+    launch_mv<MODE_ROUND, 4>(s, a, sel ? 1 : P);
 }
 
 void nsl_mv_gu_raw(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K, int R, const float* x, int xs, float* out,
                    int ys, const int32_t* sel, int P, int xdiv, const uint32_t* G) {
     MvParams a = {wg, wu, WSlice{}, sel, x, out, G, K, R, P, xdiv, xs, ys, 0, 1, NULL, NULL, 0};
-    launch_mv<MODE_GU>(s, a, 1);
+    launch_mv<MODE_GU, 4>(s, a, 1);
 }
 
 // kc_mv_gu with the router folded into its prologue: T <= MV_MAXT rows of logits -> ind / wt [T][top_k] and
@@ -1316,7 +1279,7 @@ void nsl_mv_gu_routed(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K,
     }
     MvParams a = {wg, wu, WSlice{}, NULL, x, out, G, K, R, T * top_k, top_k, xs, ys, 0, raw, NULL, NULL, 0};
     const RouteFuse rf = {logits, ld, n_exp, top_k, T, ind, wt};
-    launch_mv<MODE_GU>(s, a, 1, rf);
+    launch_mv<MODE_GU, 4>(s, a, 1, rf);
 }
 
 // The whole decode step of an expert layer (router, gate + up + SwiGLU, down, combine) as one launch: 1 = launched, 0 = a
@@ -1339,12 +1302,12 @@ void nsl_mv_gu_rows(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K, i
                     float* out, int ys, const int32_t* sel, const int32_t* xrow, int max_pairs, const int32_t* count,
                     int raw, const uint32_t* G) {
     MvParams a = {wg, wu, WSlice{}, sel, (const float*) x, out, G, K, R, max_pairs, 1, xs, ys, 0, raw, xrow, count, x_bf16};
-    launch_mv<MODE_GU>(s, a, 1);
+    launch_mv<MODE_GU, 4>(s, a, 1);
 }
 void nsl_mv_sel_rows(cudaStream_t s, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys,
                      const int32_t* sel, int max_pairs, const int32_t* count, int raw, const uint32_t* G) {
     MvParams a = {ws, NULL, WSlice{}, sel, x, y, G, K, R, max_pairs, 1, xs, ys, 0, raw, NULL, count, 0};
-    launch_mv<MODE_ROUND>(s, a, 1);
+    launch_mv<MODE_ROUND, 4>(s, a, 1);
 }
 
 

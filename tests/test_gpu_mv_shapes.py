@@ -1,0 +1,65 @@
+"""The mat-vec kernels at row lengths around their cuts: rows of whole 64-weight chunks that are not a power of two (groups of
+lanes with and without idle ones, more groups than warps, rows longer than 32 chunks), row counts that end inside a step, both
+seed formats; gathers, gate+up with the router in front, dense calls of 1..8 rows.  The oracle's double-precision sums and the
+bounds of the other mat-vec tests (one bf16 unit plus 64 x 1.2e-7 x sum|w x|)."""
+import numpy as np
+import pytest
+
+from oracle import binding as B
+
+pytestmark = pytest.mark.gpu
+F32B = 64 * 1.2e-7
+
+
+def matrices(p, n, R, K, seed):
+    from nanoseedlm_b200 import kernels
+    if p == 4:
+        mats = [B.Matrix(R, K, seed + s, eb=-20 - s % 3) for s in range(n)]
+        return [B.decode_rows_f32(m).astype(np.float64) for m in mats], kernels.SeedWeight.from_matrices(mats)
+    mats = [B.Matrix3(R, K, seed + s, eb=-20 - s % 3) for s in range(n)]
+    return [B.decode3_rows_f32(m).astype(np.float64) for m in mats], kernels.SeedWeight3(mats)
+
+
+def check(got, W, x, extra=1.0):
+    ref = B.bfr((W @ x).astype(np.float32)).astype(np.float64)
+    assert (np.abs(got - ref) <= np.abs(ref) / 128 + extra * F32B * (np.abs(W) @ np.abs(x)) + 1e-30).all()
+
+
+@pytest.mark.parametrize("p", [4, 3])
+@pytest.mark.parametrize("K,R", [(64 * 3, 5), (64 * 7, 66), (64 * 11, 37), (64 * 24, 130), (64 * 33, 9), (64 * 45, 33), (64 * 96, 21)])
+def test_any_number_of_chunks(p, K, R):
+    from nanoseedlm_b200 import kernels
+    W, w = matrices(p, 3, R, K, K + R)
+    U, u = matrices(p, 3, R, K, 7 * K + R)
+    x = B.bfr(np.random.default_rng(K).standard_normal((8, K)).astype(np.float32))
+    sel = np.array([2, 0, 1, 1, 2, 0, 1], np.int32)
+    mv_sel, mv_gu, mv = (kernels.kt_mv_sel, kernels.kt_mv_gu, kernels.kt_mv) if p == 4 else (kernels.kt_mv3_sel, kernels.kt_mv3_gu, kernels.kt_mv3)
+    y, a = mv_sel(w, sel, 1, x[:7]), mv_gu(w, u, sel, 1, x[:7])
+    for i, e in enumerate(sel):
+        check(y[i], W[e], x[i].astype(np.float64))
+        g, h = (B.bfr((M[e] @ x[i].astype(np.float64)).astype(np.float32)).astype(np.float64) for M in (W, U))
+        silu = g / (1 + np.exp(-g))
+        assert (np.abs(a[i] - silu * h) <= (np.abs(h) * (np.abs(g) + 1) + np.abs(silu * h)) / 64 + 1e-6).all()
+    assert np.array_equal(mv_sel(w, sel[3:4], 1, x[3:4])[0], y[3])      # a pair alone: the same bits
+    first = None
+    for T in (1, 2, 5, 8):
+        d = mv(w, x[:T], T)
+        for t in range(T):
+            check(d[t], W[0], x[t].astype(np.float64))
+        first = d[0] if first is None else first
+        assert np.array_equal(d[0], first)
+
+
+@pytest.mark.parametrize("K,R,T", [(64 * 24, 88, 5), (64 * 6, 64, 8), (64 * 45, 40, 1)])
+def test_router_in_front_at_any_number_of_chunks(K, R, T):
+    from nanoseedlm_b200 import kernels
+    E, k = 20, 3
+    _, w = matrices(4, E, R, K, 11)
+    _, u = matrices(4, E, R, K, 500)
+    rng = np.random.default_rng(R)
+    x = B.bfr(rng.standard_normal((T, K)).astype(np.float32))
+    logits = rng.standard_normal((T, E)).astype(np.float32)
+    a, ind, wt = kernels.kt_mv_gu_routed(w, u, logits, k, x)
+    rind, rwt = B.route(logits, k)
+    assert np.array_equal(ind, rind) and np.allclose(wt, rwt, rtol=1e-6)
+    assert np.array_equal(a, kernels.kt_mv_gu(w, u, ind.ravel(), k, x))
