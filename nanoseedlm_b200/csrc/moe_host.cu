@@ -8,6 +8,11 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "seed_mma.cuh"
+
+namespace nsl {
+void launch_combine_packed(cudaStream_t s, int d, int k, const uint16_t* D, const float* wt, float* out, int T);
+}
 
 extern "C" {
 
@@ -117,15 +122,22 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
         const int mt = P / MMT_BN + m->n_exp;
         nsl_route(s, m->n_exp, k, logits, m->n_exp, m->ind, m->wt, T);
         kc_bucket(s, m->ind, P, m->n_exp, m->perm, m->tiles, m->ntiles);
-        // The rows are packed to bf16 once (every row tile of every expert reads them), the up projection is launched as
-        // a dependent of the gate projection it does not depend on (its blocks fill the gate grid's last wave), and the
-        // SwiGLU results (bf16 values) go to the down projection packed.  (SwiGLU in the up GEMM's epilogue measured
-        // 27 us slower a layer.)
-        kc_pack_input_bf16(s, x, m->xp, (size_t) T * d);
+        kc_pack_input_bf16(s, x, m->xp, (size_t) T * d);      // once: every row tile of every expert reads them
+        if (!nsl::seed_gemm_exact() && d % 64 == 0 && ff % 64 == 0) {
+            // gate, up and SwiGLU in one launch, results as packed bf16 (they are bf16 values); the down projections' rows stay packed too.
+            // Few rows an expert: the kernel that keeps the weights in registers; many: one expansion for up to 384 rows.
+            const int avg = P / m->n_exp;
+            uint16_t* const D = (uint16_t*) m->Dx;
+            nsl::MmParams g = {m->wg, WSlice{}, m->xp, m->Ap, m->perm, m->tiles, m->ntiles, m->G, d, ff, 0, d, ff, k, 0, 1, 1, m->wu, 1,
+                               avg >= 96 && nsl::gemm_shares_tiles(mt) ? m->ntiles + 1 : NULL};
+            nsl::MmParams w = {m->wd, WSlice{}, m->Ap, D, m->perm, m->tiles, m->ntiles, m->G, ff, d, 0, ff, d, 1, 0, 1, 1, NULL, 1, g.offs};
+            if (avg < 12) { nsl::launch_seed_mma(s, MF_SEED4P4, g, mt); nsl::launch_seed_mma(s, MF_SEED4P4, w, mt); }
+            else { nsl::launch_gemm_gu(s, g, mt); nsl::launch_gemm(s, MF_SEED4P4, "nsl_moe_forward", w, mt); }
+            nsl::launch_combine_packed(s, d, k, D, m->wt, out, T);
+            return 0;
+        }
         kc_mm_grouped_packed(s, MF_SEED4P4, m->wg, d, ff, m->xp, d, m->Gb, ff, k, m->perm, m->tiles, m->ntiles, mt, m->G);
-        nsl::tl_mm_overlap = true;
         kc_mm_grouped_packed(s, MF_SEED4P4, m->wu, d, ff, m->xp, d, m->A, ff, k, m->perm, m->tiles, m->ntiles, mt, m->G);
-        nsl::tl_mm_overlap = false;
         nsl_swiglu_packed(s, m->Gb, m->A, m->Ap, P * ff);
         kc_mm_grouped_packed(s, MF_SEED4P4, m->wd, ff, d, m->Ap, ff, m->Dx, d, 1, m->perm, m->tiles, m->ntiles, mt, m->G);
         kq4_moe_combine(s, d, k, m->Dx, m->wt, NULL, NULL, 0, out, T);

@@ -54,6 +54,34 @@ __global__ void q4_combine_kernel(int d, int k, const float* __restrict__ D, con
     out[(size_t) t * d + i] = a;
 }
 
+// The same without a shared expert over packed bf16 rows (d a multiple of 8: 16 bytes of each of the k rows a thread).
+__global__ void __launch_bounds__(256) combine_packed_kernel(int d8, int k, const uint4* __restrict__ D, const float* __restrict__ wt,
+                                                             float4* __restrict__ out, int n) {
+    grid_dependents_go();
+    grid_dependency_wait();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const int t = i / d8, c = i - t * d8;
+    float a[8] = {};
+    for (int j = 0; j < k; ++j) {
+        const float w = __ldg(wt + t * k + j);
+        const uint4 v = __ldg(D + ((size_t) t * k + j) * d8 + c);
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            a[2 * q] += w * __uint_as_float(u[q] << 16);
+            a[2 * q + 1] += w * __uint_as_float(u[q] & 0xFFFF0000u);
+        }
+    }
+    out[2 * (size_t) i] = make_float4(a[0], a[1], a[2], a[3]);
+    out[2 * (size_t) i + 1] = make_float4(a[4], a[5], a[6], a[7]);
+}
+void launch_combine_packed(cudaStream_t s, int d, int k, const uint16_t* D, const float* wt, float* out, int T) {
+    const int n = T * (d / 8);
+    launch(combine_packed_kernel, (unsigned) (n + 255) / 256, 256, 0, s, d / 8, k, (const uint4*) D, wt, (float4*) out, n);
+    count_launch();
+}
+
 // x = bf16(x + bf16(bf16(sum_j bf16(D_j bf16(w_j))) + shared))
 __global__ void moe_combine_kernel(const float* __restrict__ D, const float* __restrict__ w, const float* __restrict__ shared,
                                    float* __restrict__ x, int d, int k) {

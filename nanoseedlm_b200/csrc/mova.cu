@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256) heads_deq_kernel(WSlice W, KConst kc, con
         const int h = (int) (gidx / (size_t) nb / (size_t) O);
         const uint32_t sb = stream_bits(tab, seed);
         float wv[8];
-        block_weights(seed | (sb << 16), sb, cw, exact_scale45(__ldg(head_bias + h) + code), kc, wv);
+        block_weights(seed | (sb << 16), sb, cw, exact_scale<42>(__ldg(head_bias + h) + code), kc, wv);
         out[gidx] = make_uint4(bf16x2_bits(wv[0], wv[1]), bf16x2_bits(wv[2], wv[3]), bf16x2_bits(wv[4], wv[5]),
                                bf16x2_bits(wv[6], wv[7]));
     }

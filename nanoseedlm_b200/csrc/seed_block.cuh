@@ -21,7 +21,9 @@
 // the 32 multiply-adds of each block issue as 32 packed operations per block pair.
 #pragma once
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 namespace nsl {
 
@@ -49,23 +51,27 @@ __device__ __forceinline__ uint32_t stream_bits(const StreamTab& t, uint32_t see
 // or constant-bank operands).  Coefficient p becomes an exact float by placing nibble ^ 8 under an exponent chosen so
 // that the nibble's low bit has the wanted weight, then subtracting the offset:
 //   dot form   q'_p = q_p 2^(65-p):  exponent field 215 - 5p, offset 2^(88-5p) + 2^(68-p)
-//   exact form q"_p = q_p 2^(100-p): exponent field 250 - 5p, offset 2^(123-5p) + 2^(103-p)
+//   exact form q"_p = q_p 2^(103-p): exponent field 253 - 5p, offset 2^(126-5p) + 2^(106-p)
 struct KConst {
     uint32_t cxor[4];
     float coff[4];
     uint32_t cxor_x[4];
     float coff_x[4];
     uint32_t cor;       // 112 << 23: 2^(code - 15) from a code placed at bits 23..26
+    unsigned long long coff_x2[4], two2;      // packed pairs: coff_x and 2 (operands from constant memory)
 };
 inline KConst kconst() {
     KConst k;
     for (int p = 0; p < 4; ++p) {
         k.cxor[p] = ((uint32_t) (215 - 5 * p) << 23) | (8u << (4 * p));
         k.coff[p] = -(ldexpf(1.0f, 88 - 5 * p) + ldexpf(1.0f, 68 - p));
-        k.cxor_x[p] = ((uint32_t) (250 - 5 * p) << 23) | (8u << (4 * p));
-        k.coff_x[p] = -(ldexpf(1.0f, 123 - 5 * p) + ldexpf(1.0f, 103 - p));
+        k.cxor_x[p] = ((uint32_t) (253 - 5 * p) << 23) | (8u << (4 * p));
+        k.coff_x[p] = -(ldexpf(1.0f, 126 - 5 * p) + ldexpf(1.0f, 106 - p));
     }
     k.cor = 112u << 23;
+    auto both = [](float v) { uint32_t u; memcpy(&u, &v, 4); return ((unsigned long long) u << 32) | u; };
+    for (int p = 0; p < 4; ++p) k.coff_x2[p] = both(k.coff_x[p]);
+    k.two2 = both(2.0f);
     return k;
 }
 #define NSL_XSCALE 18446744073709551616.0f   // 2^64: the mat-vec kernels' input scaling
@@ -186,17 +192,17 @@ __device__ __forceinline__ float states_dot(const float* v, const float* q, cons
     }
     return fmaf(q[3], d3, fmaf(q[2], d2, fmaf(q[1], d1, q[0] * d0)));
 }
-// Exact form: the eight weights bit for bit.  With q"_p = q_p 2^(100-p) every product q"_p v_cp is the integer
-// q_p state in units of 2^-45 and every partial sum is exact in f32; adding kq = -2^-30 sum_p q_p (the centring)
-// leaves isum_c 2^-45 exactly, and one multiply by sc45 = fl(R32 2^e) * 2^45 is the spec's single rounding.
-__device__ __forceinline__ void block_weights(uint32_t a, uint32_t g, uint32_t cw, float sc45, const KConst& k, float* w) {
+// Exact form: the eight weights bit for bit.  With q"_p = q_p 2^(103-p) every product q"_p v_cp is the integer
+// q_p state in units of 2^-42 and every partial sum is exact in f32; adding kq = -2^-27 sum_p q_p (the centring)
+// leaves isum_c 2^-42 exactly, and one multiply by sc = fl(R32 2^e) * 2^42 (exact_scale<42>) is the spec's single rounding.
+__device__ __forceinline__ void block_weights(uint32_t a, uint32_t g, uint32_t cw, float sc, const KConst& k, float* w) {
     float v[32], q[4];
     block_states(a, g, v);
     q[0] = coef_raw<0>(cw, k.cxor_x[0]) + k.coff_x[0];
     q[1] = coef_raw<1>(cw, k.cxor_x[1]) + k.coff_x[1];
     q[2] = coef_raw<2>(cw, k.cxor_x[2]) + k.coff_x[2];
     q[3] = coef_raw<3>(cw, k.cxor_x[3]) + k.coff_x[3];
-    // -2^(p-130) q"_p = -2^-30 q_p; the four constants are subnormal or tiny but exact
+    // -2^(p-130) q"_p = -2^-27 q_p; the four constants are subnormal or tiny but exact
     const float kq = __fmaf_rn(q[3], -5.877471754111438e-39f,
                                __fmaf_rn(q[2], -2.938735877055719e-39f,
                                          __fmaf_rn(q[1], -1.4693679385278594e-39f, __fmul_rn(q[0], -7.346839692639297e-40f))));
@@ -204,12 +210,13 @@ __device__ __forceinline__ void block_weights(uint32_t a, uint32_t g, uint32_t c
     for (int c = 0; c < 8; ++c) {
         const float t = __fmaf_rn(q[3], v[4 * c + 3],
                                   __fmaf_rn(q[2], v[4 * c + 2], __fmaf_rn(q[1], v[4 * c + 1], __fmul_rn(q[0], v[4 * c]))));
-        w[c] = __fmul_rn(__fadd_rn(t, kq), sc45);
+        w[c] = __fmul_rn(__fadd_rn(t, kq), sc);
     }
 }
-// fl(R32 2^e) * 2^45 from exponent bits.
-__device__ __forceinline__ float exact_scale45(int e) {
-    return __uint_as_float(__float_as_uint(1.0f / 32767.0f) + ((uint32_t) (e + 45) << 23));
+// fl(R32 2^e) * 2^UNIT from exponent bits.
+template <int UNIT>
+__device__ __forceinline__ float exact_scale(int e) {
+    return __uint_as_float(__float_as_uint(1.0f / 32767.0f) + ((uint32_t) (e + UNIT) << 23));
 }
 
 // ---- P = 3 blocks (format SEED4: nslm/lfsr.h:82-124) ----------------------------------------------------------------------
@@ -255,8 +262,8 @@ __device__ __forceinline__ float states_dot3(const float* v, const float* q, con
     }
     return fmaf(q[2], d2, fmaf(q[1], d1, q[0] * d0));
 }
-// The eight weights bit for bit: q"_p = q_p 2^(99-p), products in units of 2^-46, sc46 = fl(R32 2^e) * 2^46.
-__device__ __forceinline__ void block_weights3(uint32_t a, uint32_t g, uint32_t nib, float sc46, const KConst& k, float* w) {
+// The eight weights bit for bit: q"_p = q_p 2^(102-p), products in units of 2^-43, sc = fl(R32 2^e) * 2^43.
+__device__ __forceinline__ void block_weights3(uint32_t a, uint32_t g, uint32_t nib, float sc, const KConst& k, float* w) {
     float q[3];
     q[0] = coef_raw<1>(nib, k.cxor_x[1]) + k.coff_x[1];
     q[1] = coef_raw<2>(nib, k.cxor_x[2]) + k.coff_x[2];
@@ -267,7 +274,7 @@ __device__ __forceinline__ void block_weights3(uint32_t a, uint32_t g, uint32_t 
     {                                                                                                                                     \
         const uint32_t y = weight_word3<C>(a, g);                                                                                         \
         const float t = __fmaf_rn(q[2], state_value<2>(y), __fmaf_rn(q[1], state_value<1>(y), __fmul_rn(q[0], state_value<0>(y))));      \
-        w[C] = __fmul_rn(__fadd_rn(t, kq), sc46);                                                                                         \
+        w[C] = __fmul_rn(__fadd_rn(t, kq), sc);                                                                                           \
     }
     NSL_WX3(0) NSL_WX3(1) NSL_WX3(2) NSL_WX3(3) NSL_WX3(4) NSL_WX3(5) NSL_WX3(6) NSL_WX3(7)
 #undef NSL_WX3
@@ -436,31 +443,44 @@ __device__ __forceinline__ u64 code_scale_pair3(uint32_t nw, const KConst& k) {
     return and_or_pair<0x07800000u>(nw * (1u << 23), nw * (1u << 7), k.cor);      // bits 0-3 and 16-19 to bits 23-26
 }
 
-// Exact form for two adjacent blocks at once (the GEMM's weight tiles): w2[c] = {weight c of the even block, of the odd
-// block}, bit for bit as block_weights gives them.  sc2 = {exact_scale45 of the even block, of the odd block}.
-__device__ __forceinline__ void pair_weights(const StreamTab& tab, uint32_t sw, uint32_t cw, u64 sc2, const KConst& k, u64* w2) {
+// Exact form for two adjacent blocks at once (the GEMMs' weights): w2[c] = {weight c of the even block, of the odd block}, bit
+// for bit as block_weights (P = 3: block_weights3) gives them.  Weight c's products are integers in units of
+// 2^(start bit - UNIT): the centring and the scale of a start bit are powers of two times those of bit 0.
+// e2 = {2^(code - 15) of the even block, of the odd block} (code_scale_pair), base = exact_base<P>(the slice's eb).
+template <int P>
+__device__ __forceinline__ float exact_base(int eb) { return exact_scale<P == 4 ? 46 : 47>(eb + 15); }
+__device__ __forceinline__ u64 same2(float v) { return pack2(v, v); }
+template <int P>
+__device__ __forceinline__ void pair_weights(const StreamTab& tab, uint32_t sw, uint32_t cw, u64 e2, float base, const KConst& k, u64* w2) {
     u64 q[4];
-    const uint32_t g0 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4440)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4441));
-    const uint32_t g1 = lut_word(tab.lo, __byte_perm(sw, 0, 0x4442)) ^ lut_word(tab.hi, __byte_perm(sw, 0, 0x4443));
-    const uint32_t a0 = __byte_perm(sw, g0, 0x5410), a1 = __byte_perm(sw, g1, 0x5432);
+    uint32_t g0, g1;
+    pair_stream(tab, sw, g0, g1);
+    const Words wa = window_words<P, 0>(sw, g0), wb = window_words<P, 1>(sw, g1);
     const uint32_t c1 = cw >> 16;
-    q[0] = add2(and_xor_pair<0x000Fu>(cw, c1, k.cxor_x[0]), pack2(k.coff_x[0], k.coff_x[0]));
-    q[1] = add2(and_xor_pair<0x00F0u>(cw, c1, k.cxor_x[1]), pack2(k.coff_x[1], k.coff_x[1]));
-    q[2] = add2(and_xor_pair<0x0F00u>(cw, c1, k.cxor_x[2]), pack2(k.coff_x[2], k.coff_x[2]));
-    q[3] = add2(and_xor_pair<0xF000u>(cw, c1, k.cxor_x[3]), pack2(k.coff_x[3], k.coff_x[3]));
-    const u64 kq = fma2(q[3], pack2(-5.877471754111438e-39f, -5.877471754111438e-39f),
-                        fma2(q[2], pack2(-2.938735877055719e-39f, -2.938735877055719e-39f),
-                             fma2(q[1], pack2(-1.4693679385278594e-39f, -1.4693679385278594e-39f),
-                                  mul2(q[0], pack2(-7.346839692639297e-40f, -7.346839692639297e-40f)))));
-    // weight by weight (its shifts and ANDs, then its multiply-adds: the two pipes alternate in program order); the centring
-    // term first: every partial sum stays an exact integer multiple of 2^-45 below 2^24
-#define NSL_WX(C)                                                                                               \
-    {                                                                                                           \
-        const uint32_t y0 = weight_word<C>(a0, g0), y1 = weight_word<C>(a1, g1);                                \
-        w2[C] = mul2(fma2(q[3], pack2(state_value<3>(y0), state_value<3>(y1)),                                  \
-                          fma2(q[2], pack2(state_value<2>(y0), state_value<2>(y1)),                             \
-                               fma2(q[1], pack2(state_value<1>(y0), state_value<1>(y1)),                        \
-                                    fma2(q[0], pack2(state_value<0>(y0), state_value<0>(y1)), kq)))), sc2);     \
+    if (P == 4) {
+        q[0] = add2(and_xor_pair<0x000Fu>(cw, c1, k.cxor_x[0]), k.coff_x2[0]);
+        q[1] = add2(and_xor_pair<0x00F0u>(cw, c1, k.cxor_x[1]), k.coff_x2[1]);
+        q[2] = add2(and_xor_pair<0x0F00u>(cw, c1, k.cxor_x[2]), k.coff_x2[2]);
+        q[3] = add2(and_xor_pair<0xF000u>(cw, c1, k.cxor_x[3]), k.coff_x2[3]);
+    } else {
+        q[0] = add2(and_xor_pair<0x00F0u>(cw, c1, k.cxor_x[1]), k.coff_x2[1]);
+        q[1] = add2(and_xor_pair<0x0F00u>(cw, c1, k.cxor_x[2]), k.coff_x2[2]);
+        q[2] = add2(and_xor_pair<0xF000u>(cw, c1, k.cxor_x[3]), k.coff_x2[3]);
+    }
+    // the centring, sum_p -2^(p-134) q"_p for start bit 0, by doubling: few constants, they occupy register pairs
+    u64 h = P == 4 ? fma2(q[P - 1], k.two2, q[2]) : q[2];
+    h = fma2(fma2(h, k.two2, q[1]), k.two2, q[0]);
+    // weight by weight (its ANDs, then its multiply-adds: the two pipes alternate in program order); the centring term first:
+    // every partial sum stays an exact integer multiple of the unit below 2^24
+#define NSL_WX(C)                                                                                                            \
+    {                                                                                                                        \
+        constexpr int B = state_bit<P, C>(), W = word_of<P, C>();                                                            \
+        u64 t = fma2(q[0], pack2(state_at<B, 0>(wa.w[W]), state_at<B, 0>(wb.w[W])),                                          \
+                     mul2(h, same2(-4.591774807899561e-41f * (float) (1 << B))));                                            \
+        t = fma2(q[1], pack2(state_at<B, 1>(wa.w[W]), state_at<B, 1>(wb.w[W])), t);                                          \
+        t = fma2(q[2], pack2(state_at<B, 2>(wa.w[W]), state_at<B, 2>(wb.w[W])), t);                                          \
+        if (P == 4) t = fma2(q[P - 1], pack2(state_at<B, P - 1>(wa.w[W]), state_at<B, P - 1>(wb.w[W])), t);                  \
+        w2[C] = mul2(t, mul2(e2, same2(base * (1.0f / (float) (1 << B)))));                                                  \
     }
     NSL_WX(0) NSL_WX(1) NSL_WX(2) NSL_WX(3) NSL_WX(4) NSL_WX(5) NSL_WX(6) NSL_WX(7)
 #undef NSL_WX

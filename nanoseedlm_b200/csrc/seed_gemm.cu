@@ -2,19 +2,27 @@
 // Replaces the SEED4P4 paths of the reference's k_mm / k_mm3 / k_mm_packed and their grouped forms
 // (engine/kernels_moe.cu:405-525, 2354-2395), which stage one 64 x 32 weight tile per K step for mma.sync.
 //
-// Y[n][r] = sum_k W[r][k] X[n][k] for a tile of 128 weight rows x up to 128 tokens (one entry of the tile table: one
-// expert's run of pairs, or 128 consecutive tokens of a dense call).
+// Y[n][r] = sum_k W[r][k] X[n][k] for a unit of 128 weight rows x up to 128 rows of inputs (one entry of the tile table: one
+// expert's run of pairs, or 128 consecutive rows of a dense call), or up to 384 of one expert or dense call.
 //
-// One block = 8 producer warps + 1 MMA warp.  Per K step of 64 the producers regenerate the 128 x 64 weight tile from
-// its seeds (one 8-weight block per 16-byte row chunk, written bf16 in the 128-byte swizzled K-major layout the MMA
-// reads) and convert the tokens' inputs to the same layout; one elected thread issues tcgen05.mma (M 128, N = the
-// tile's pair count rounded up to 16, K 16, bf16 x bf16 -> f32 in TMEM) and commits the stage back to the producers
-// through an mbarrier.  Three stages of shared memory overlap the expansion of step k+1, k+2 with the MMAs of step k.
-// The expansion is the cost (about a hundred integer/FP operations per 8 weights against 2 x 8 x N flops of tensor
-// work), so a weight tile is expanded once per tile entry and serves all of its tokens; the tensor pipe idles most of
-// the time by construction.  The accumulator is read back with tcgen05.ld by the producer warps (TMEM lane = weight
-// row, column = token), rounded as the reference's store_y does and written so that a warp stores 32 consecutive rows
-// of one token.
+// The expansion is the cost (82 instructions per 8 weights, 0.96 clk a block of weights and SM alone in a loop, against
+// 2 x 8 x N flops of tensor work), so the weights are written where the MMA reads them with the fewest instructions: tensor
+// memory.  A producer thread owns one row (its tensor memory lane) and the 64 weights of a K step: 8 blocks from one 16-byte load
+// of seeds, one of coefficient words and 4 bytes of codes, converted to bf16 pairs and stored by two tcgen05.st; no address
+// arithmetic, no swizzle, no proxy fence.  The four warps of a warpgroup make a step; the warpgroups take the steps in turn, so
+// a step waits for one warp of each scheduler (eight warps a step left the producers waiting for one another a third of the
+// time).  The inputs (B operand) come through shared memory (128-byte swizzle), fetched by loader warps; one elected thread
+// issues tcgen05.mma (M 128, K 16, N = the tile's count rounded up to 16) and commits the stage back through an mbarrier.
+// Blocks are persistent: the stream table, the tensor memory and the barriers are set up once.
+//   TT = 1, packed inputs: 8 producer warps, two blocks an SM (256 of the 512 columns each).
+//   otherwise: 16 producer warps, one block an SM.  TT = 3: up to three tiles of an expert share one expansion, which a prompt of
+//   thousands of rows needs (each tile expands its expert's weights again).
+// The accumulator is read back with tcgen05.ld by the producer warps (lane = weight row, column = row of inputs), rounded as the
+// reference's store_y does and written so that a warp stores 32 consecutive rows of one row of outputs.  Units that fill at most
+// half of the accumulator columns alternate between the halves, and their results are read back after the next unit's first
+// step has been produced, when the MMAs are done.
+// Gate + up + SwiGLU (GU): lane 2 i holds row i of the gate matrix, lane 2 i + 1 of the up matrix, so both sums meet in
+// neighbouring lanes and the result leaves as packed bf16: no f32 intermediates, no third kernel.
 //
 // Weight precision: default, seed weights rounded to bf16 (one term); kc_seed_gemm_f32(1), three bf16 terms whose sum is
 // the f32 weight exactly (three MMAs per step), as the reference's two modes (engine/kernels_moe.cu:405-412).
@@ -23,25 +31,30 @@
 // TMEM and returns.
 #include "common.cuh"
 #include "seed_block.cuh"
+#include "seed_mma.cuh"
 
 namespace nsl {
 
-constexpr int GM_BM = 128, GM_BN = 128, GM_BK = 64, GM_STAGES = 3;
-constexpr int GM_PRODUCERS = 256, GM_THREADS = GM_PRODUCERS + 32;
-constexpr int GM_TILE_BYTES = GM_BM * GM_BK * 2;   // 16 KB: one bf16 operand tile
-constexpr uint32_t GM_WAIT_LIMIT = 1u << 22;
-
-struct MmParams {
-    const WSlice* ws;        // grouped: device table; dense: NULL
-    WSlice w0;
-    const void* X;           // f32, or packed bf16
-    float* Y;
-    const int32_t* perm;
-    const MmTile* tiles;
-    const int32_t* ntiles;   // device tile count, or NULL
-    const uint32_t* G;
-    int* status;             // device status word (0 = ok)
-    int K, R, T, xs, ys, xdiv, add, grouped, packed;
+constexpr int GM_BM = 128, GM_BN = 128, GM_BK = 64, GM_STAGES = 4;
+constexpr int GM_MAX_HEADS = 2048;      // tiles of a launch whose experts' tiles share expansions (their list sits in shared memory)
+constexpr uint32_t GM_WAIT_LIMIT = 1u << 24;
+constexpr unsigned long long GM_WAIT_NS = 1000000000ull;
+// One block: PW producer warps, the MMA warp, LW loader warps.  Tensor memory: the accumulators (128 columns per tile of inputs),
+// then the stages' weights (32 columns per term: 64 k values as bf16 pairs).  f32 inputs are converted by the loaders, whose loads
+// of a whole K step are held in registers meanwhile: seven warps of them.
+// LAUNCH_REGS: registers a thread at launch (what the launch bounds leave); PREGS, LREGS: of the producers' and of the other
+// warpgroups after the split, whose sum over the block is at most what the launch gave it.
+template <int TERMS, int TT, bool F32>
+struct GmCfg {
+    static constexpr int CTAS = TERMS == 1 && TT == 1 && !F32 ? 2 : 1, PW = TERMS == 3 || CTAS == 2 ? 8 : 16, LW = F32 && TERMS == 1 ? 7 : 3;
+    static constexpr int WARPS = PW + 1 + LW, THREADS = WARPS * 32, GROUPS = PW / 4;
+    static constexpr int ACC = GM_BN * TT, A_COLS = 32 * TERMS, COLS = ACC + GM_STAGES * A_COLS <= 256 ? 256 : 512;
+    static constexpr int X_BYTES = TT * GM_BN * GM_BK * 2;      // a stage's inputs
+    static constexpr bool SPLIT = TERMS == 1;
+    static constexpr int LAUNCH_REGS = CTAS == 2 || F32 ? 80 : 96, LREGS = F32 ? 64 : 40, PREGS = F32 ? 88 : CTAS == 2 ? 96 : 104;
+    static_assert(ACC + GM_STAGES * A_COLS <= COLS && CTAS * COLS <= 512, "tensor memory");
+    static_assert(!SPLIT || PW * PREGS + (LW + 1) * LREGS <= WARPS * LAUNCH_REGS, "registers");
+    static_assert(GM_STAGES >= GROUPS, "every warpgroup owns a stage");
 };
 
 __device__ int g_mm_status;   // 0, or the code of the first bounded wait that ran out
@@ -54,24 +67,25 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Bounded wait: false after GM_WAIT_LIMIT polls (the caller records the code and stops).  Polling on purpose: the suspended
-// form (mbarrier.try_wait) saved the polls' instructions but cost 3 us per 174 us launch in wake-up latency; short sleeps
-// between a waiting producer's polls measured the same as bare polls (158.2 -> 157.5 us) and are kept for the issue slots.
-// EAGER: false for the producers' wait for a free stage: a producer that is ahead sleeps between polls from the first
-// miss on, so that its polls do not take issue slots from the warps the stage is waiting for.
-template <bool EAGER = true>
+// Bounded wait: false after GM_WAIT_NS or GM_WAIT_LIMIT attempts (the caller records the code and stops).  The suspended form: a warp that polls
+// takes issue slots from the producers (bare polls with short sleeps: 343 us a config-2 layer, this: 328; long sleeps wake too
+// late: 376).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    unsigned long long t0 = 0;
     for (uint32_t i = 0; i < GM_WAIT_LIMIT; ++i) {
-        if (mbar_test(bar, parity)) return true;
-        if (!EAGER) __nanosleep(i < 8 ? 48 : 96);
-        if ((i & 15u) == 15u && *abort_flag) return false;
-        if (EAGER && i > 64) __nanosleep(64);
+        if (mbar_try(bar, parity)) return true;
+        if ((i & 63u) == 63u) {
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (!t0) t0 = t;
+            if (*abort_flag || t - t0 > GM_WAIT_NS) return false;
+        }
     }
     return false;
 }
@@ -101,348 +115,465 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* v) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// A thread's share of one K step: 4 consecutive blocks of its row = two block pairs (seed / coefficient words packed
-// two per 32-bit word, even block low) and their 4 exponent codes (one nibble each, block j at bits 4j).  P = 3 (SEED4)
-// has no code stream: a block's code is the low nibble of its nibble word, read where the weights are formed.
-struct QuadIn { uint32_t sw[2], cw[2], codes; bool live; };
+// tcgen05.mma with the weights (A) in tensor memory and the inputs (B) in shared memory.
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+                   "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ float to_bf16(float x) { return __uint_as_float(bf16x2_bits(x, 0.0f) << 16); }      // rounded, kept as f32
 
-template <bool P3>
-__device__ __forceinline__ QuadIn load_quad(const WSlice& w, int row, int kb, int R, int NB, bool vec) {
-    QuadIn q = {{0u, 0u}, {0u, 0u}, 0u, false};
-    if (row >= R || kb >= NB) return q;
-    q.live = true;
-    const size_t g = (size_t) row * NB + kb;
-    if (vec) {   // NB % 4 == 0: the four blocks are one aligned 8-byte load per stream and two code bytes
-        const uint2 s2 = __ldg((const uint2*) ((const uint16_t*) w.p[0] + g));
-        const uint2 c2 = __ldg((const uint2*) ((const uint16_t*) w.p[1] + g));
-        q.sw[0] = s2.x; q.sw[1] = s2.y; q.cw[0] = c2.x; q.cw[1] = c2.y;
-        if (!P3) q.codes = __ldg((const uint16_t*) ((const uint8_t*) w.p[3] + (g >> 1)));
+// A thread's share of one K step: the 8 blocks (64 weights) of its row.
+struct ChunkIn { uint4 s, c; uint32_t cd; };
+
+template <bool P3, bool VEC>
+__device__ __forceinline__ ChunkIn load_row_chunk(const WSlice& w, int row, int chunk, int R, int NB) {
+    ChunkIn q = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u), 0u};      // zero coefficients: zero weights
+    if (row >= R || chunk * 8 >= NB) return q;
+    if (VEC) {      // rows of whole chunks: one aligned load per stream
+        const uint32_t i = (uint32_t) row * (uint32_t) (NB / 8) + (uint32_t) chunk;
+        q.s = __ldg((const uint4*) w.p[0] + i);
+        q.c = __ldg((const uint4*) w.p[1] + i);
+        if (!P3) q.cd = __ldg((const uint32_t*) w.p[3] + i);
     } else {
+        uint32_t sw[4] = {0u, 0u, 0u, 0u}, cw[4] = {0u, 0u, 0u, 0u};
+        const size_t g = (size_t) row * NB + chunk * 8;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (kb + j >= NB) break;   // (a missing block keeps seed 0: its weights are forced to zero below)
-            const uint32_t sd = __ldg((const uint16_t*) w.p[0] + g + j), cf = __ldg((const uint16_t*) w.p[1] + g + j);
-            const uint32_t cd = P3 ? 0u : (__ldg((const uint8_t*) w.p[3] + ((g + j) >> 1)) >> (((g + j) & 1) * 4)) & 15u;
-            q.sw[j >> 1] |= sd << (16 * (j & 1));
-            q.cw[j >> 1] |= cf << (16 * (j & 1));
-            q.codes |= cd << (4 * j);
+        for (int j = 0; j < 8; ++j) {
+            if (chunk * 8 + j >= NB) break;
+            sw[j >> 1] |= (uint32_t) __ldg((const uint16_t*) w.p[0] + g + j) << (16 * (j & 1));
+            cw[j >> 1] |= (uint32_t) __ldg((const uint16_t*) w.p[1] + g + j) << (16 * (j & 1));
+            if (!P3) q.cd |= (uint32_t) ((__ldg((const uint8_t*) w.p[3] + ((g + j) >> 1)) >> (((g + j) & 1) * 4)) & 15) << (4 * j);
         }
+        q.s = make_uint4(sw[0], sw[1], sw[2], sw[3]);
+        q.c = make_uint4(cw[0], cw[1], cw[2], cw[3]);
     }
     return q;
 }
 
-// WF: the weights' form.  0: SEED4P4 blocks; 1: stored BF16 values; 2: SEED4 (P = 3) blocks.
-// VEC: rows are whole quads of blocks (K a multiple of 32), so a thread's four blocks are one aligned load per stream and no
-// row ends inside a quad.
-template <int NT, int WF, bool VEC>
-__global__ void __launch_bounds__(GM_THREADS, 2) seed_gemm_kernel(MmParams a, KConst kc) {
-    constexpr bool BF16W = WF == 1, P3 = WF == 2;
-    // A launch that follows this one and does not depend on it (the up projection after the gate projection) may be made
-    // a programmatic dependent launch: its blocks then fill the SMs this grid's last wave leaves idle.
-    grid_dependents_go();
-    if (a.ntiles && (int) blockIdx.y >= *a.ntiles) return;
-    extern __shared__ uint8_t smem_raw[];
-    __shared__ StreamTab tab;
-    __shared__ __align__(8) uint64_t bars[2 * GM_STAGES + 1];
-    __shared__ uint32_t tmem_slot;
-    __shared__ int srow[GM_BN], drow[GM_BN];
-    __shared__ int abort_flag;
+// Where a unit of work lies: 128 rows of weights x up to TT consecutive tiles of one slice.
+struct UnitPos { WSlice wa, wb; int start, count, r0; };
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    uint8_t* smem = (uint8_t*) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
-    constexpr int STAGE_BYTES = (NT + 1) * GM_TILE_BYTES;   // NT weight tiles + the input tile
-    const uint32_t smem_base = smem_u32(smem);
-    const uint32_t bar_full = smem_u32(&bars[0]), bar_empty = smem_u32(&bars[GM_STAGES]), bar_done = smem_u32(&bars[2 * GM_STAGES]);
-
-    int start, count;
-    WSlice w;
+// heads: the tiles that start a unit (TT > 1, grouped); otherwise every tile does.
+template <int TT, bool GU>
+__device__ __forceinline__ UnitPos unit_pos(const MmParams& a, int unit, int row_tiles, const uint16_t* heads) {
+    UnitPos u;
+    const int y = unit / row_tiles, x = unit - y * row_tiles;
+    u.r0 = x * (GU ? GM_BM / 2 : GM_BM);
     if (a.grouped) {
-        const MmTile tl = a.tiles[blockIdx.y];
-        w = a.ws[tl.slice];
-        start = tl.start;
-        count = tl.count < GM_BN ? tl.count : GM_BN;
+        const MmTile tl = a.tiles[TT > 1 ? heads[y] : y];
+        u.start = tl.start;
+        u.count = TT > 1 ? min(a.offs[tl.slice + 1] - tl.start, GM_BN * TT) : min(tl.count, GM_BN);
+        u.wa = a.ws[tl.slice];
+        u.wb = GU ? a.wu[tl.slice] : u.wa;
     } else {
-        w = a.w0;
-        start = (int) blockIdx.y * GM_BN;
-        count = a.T - start < GM_BN ? a.T - start : GM_BN;
+        u.start = y * GM_BN * TT;
+        u.count = min(a.T - u.start, GM_BN * TT);
+        u.wa = a.w0;
+        u.wb = a.w0;
     }
-    if (count <= 0) return;
-    const int n_eff = (count + 15) & ~15;
-    const int r0 = (int) blockIdx.x * GM_BM;
-    const int NB = a.K / 8, KT = (a.K + GM_BK - 1) / GM_BK;
+    return u;
+}
+__device__ __forceinline__ int input_row_of(const MmParams& a, const UnitPos& u, int n) {      // rows beyond the count repeat the last one
+    const int p = u.start + min(n, u.count - 1);
+    return a.grouped ? a.perm[p] / a.xdiv : p;
+}
+// 16-byte unit uu (8 inputs) of row n of a stage: 128-byte swizzle, 16 KB a tile of 128 rows.
+__device__ __forceinline__ uint32_t input_at(uint32_t stage, int n, int uu) {
+    return stage + (uint32_t) ((n >> 7) * 16384 + (n & 127) * 128 + ((uu ^ (n & 7)) << 4));
+}
 
-    if (!BF16W) load_stream_tab(tab, a.G, tid, GM_THREADS);
-    if (tid < GM_BN) {
-        const bool ok = tid < count;
-        srow[tid] = !ok ? -1 : a.grouped ? a.perm[start + tid] / a.xdiv : start + tid;
-        drow[tid] = !ok ? -1 : a.grouped ? a.perm[start + tid] : start + tid;
-    }
-    if (tid == 0) {
-        abort_flag = 0;
-        for (int s = 0; s < GM_STAGES; ++s) {
-            mbar_init(bar_full + 8 * s, GM_PRODUCERS / 32);      // one arrival per producer warp
-            mbar_init(bar_empty + 8 * s, 1);
-        }
-        mbar_init(bar_done, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == GM_PRODUCERS / 32) {   // the MMA warp owns the TMEM allocation: 128 f32 columns x 128 lanes
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(GM_BN) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_acc = tmem_slot;
-
-    if (warp < GM_PRODUCERS / 32) {
-        // ---- producers: weight tile (thread = row, half of the 8 blocks) and input tile (thread = token, half of 64 k) --
-        const int prow = tid >> 1, half = tid & 1;
-        const int grow = r0 + prow;
-        constexpr bool vec = VEC;
-        QuadIn cur = {{0u, 0u}, {0u, 0u}, 0u, false}, nxt = cur;
-        uint4 bcur[4], bnxt[4];      // BF16 weights: this thread's 32 values of the K step, as stored
-        auto load_bf16 = [&](int kt, uint4* o) {
+// The results of a unit, by the producer warps: warp w reads the tensor memory lanes of its quarter, 16 columns at a time, the
+// warpgroups taking turns.  col: the unit's first column.
+template <bool GU, int GROUPS>
+__device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, int col, int start, int count, int r0) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lq = warp & 3, rl = lq * 32 + lane;
+    const int grow = GU ? r0 + (rl >> 1) : r0 + rl;
+    for (int c0 = (warp >> 2) * 16; c0 < count; c0 += GROUPS * 16) {
+        uint32_t v[16];
+        const int p = start + min(c0 + (lane & 15), count - 1), dst_lane = a.grouped ? a.perm[p] : p;      // lane j: column c0 + j's place
+        tmem_ld16(tmem + ((uint32_t) (lq * 32) << 16) + (uint32_t) (col + c0), v);
+        if (GU) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int k = kt * GM_BK + half * 32 + 8 * i;
-                o[i] = grow < a.R && k < a.K ? __ldg((const uint4*) ((const uint16_t*) w.p[0] + (size_t) grow * a.K + k)) : make_uint4(0u, 0u, 0u, 0u);
+            for (int j = 0; j < 8; ++j) {      // even lanes finish columns 0..7, odd lanes 8..15
+                const int jj = lane & 1 ? j + 8 : j;
+                const float lo = __uint_as_float(v[j]), hi = __uint_as_float(v[j + 8]);
+                const float from = __shfl_xor_sync(0xFFFFFFFFu, lane & 1 ? lo : hi, 1), mine = lane & 1 ? hi : lo;
+                const int dst = __shfl_sync(0xFFFFFFFFu, dst_lane, jj);
+                const float g = to_bf16(lane & 1 ? from : mine), up = to_bf16(lane & 1 ? mine : from);
+                const float r = to_bf16(g * to_bf16(1.0f / (1.0f + expf(-g)))) * up;
+                if (c0 + jj < count && grow < a.R) ((uint16_t*) a.Y)[(size_t) dst * a.ys + grow] = (uint16_t) bf16x2_bits(r, 0.0f);
             }
-        };
-        if (BF16W) load_bf16(0, bcur);
-        else cur = load_quad<P3>(w, grow, half * 4, a.R, NB, vec);
-        nxt = cur;
-        // packed inputs: this thread's 16-byte chunks of the K step's n_eff x 64 tile (chunk ci = tid + 256 i), requested one
-        // K step ahead so that they land during the expansion
-        uint4 xq[4];
-        const int nx = (n_eff * 8 + GM_PRODUCERS - 1) / GM_PRODUCERS;      // chunks per thread: 1 for tiles of up to 32 pairs
-        auto load_x = [&](int kt) {
+        } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int ci = tid + i * GM_PRODUCERS;
-                if (i < nx) xq[i] = make_uint4(0u, 0u, 0u, 0u);
-                if (i < nx && ci < n_eff * 8) {
-                    const int src = srow[ci >> 3], k = kt * GM_BK + 8 * (ci & 7);
-                    if (src >= 0 && k < a.K) xq[i] = __ldg((const uint4*) ((const uint16_t*) a.X + (size_t) src * a.xs + k));
-                }
-            }
-        };
-        // f32 inputs: the thread's first two chunks (tiles of up to 64 pairs whole) travel the same way as raw values, two
-        // float4 a chunk in the same registers (xq[2 c], xq[2 c + 1]); further chunks are loaded and converted in place
-        auto load_xf = [&](int kt) {
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const int ci = tid + c * GM_PRODUCERS;
-                xq[2 * c] = xq[2 * c + 1] = make_uint4(0u, 0u, 0u, 0u);
-                if (c < nx && ci < n_eff * 8) {
-                    const int src = srow[ci >> 3], k = kt * GM_BK + 8 * (ci & 7);
-                    if (src >= 0 && k < a.K) {
-                        const uint4* xp = (const uint4*) ((const float*) a.X + (size_t) src * a.xs + k);
-                        xq[2 * c] = __ldg(xp);
-                        xq[2 * c + 1] = __ldg(xp + 1);
-                    }
-                }
-            }
-        };
-        if (a.packed) load_x(0); else load_xf(0);
-        bool live = true;
-        for (int kt = 0; kt < KT && live; ++kt) {
-            const int s = kt % GM_STAGES;
-            if (kt + 1 < KT) {
-                if (BF16W) load_bf16(kt + 1, bnxt);
-                else nxt = load_quad<P3>(w, grow, (kt + 1) * 8 + half * 4, a.R, NB, vec);
-            }
-            if (kt >= GM_STAGES && !mbar_wait<false>(bar_empty + 8 * s, ((kt / GM_STAGES) - 1) & 1, &abort_flag)) {
-                abort_flag = 1;
-                atomicCAS(&g_mm_status, 0, 1);
-                live = false;
-                break;
-            }
-            uint8_t* stage = smem + (size_t) s * STAGE_BYTES;
-            if (BF16W) {      // stored weights: the row's four 16-byte chunks of this half, as they are
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int chunk = half * 4 + i;
-                    *(uint4*) (stage + (uint32_t) prow * 128u + (uint32_t) ((chunk ^ (prow & 7)) << 4)) = bcur[i];
-                }
-            }
-            if (a.packed) {      // this K step's inputs (requested a step ago), then the next step's request
-                uint8_t* bt = stage + (size_t) NT * GM_TILE_BYTES;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int ci = tid + i * GM_PRODUCERS, n = ci >> 3, chunk = ci & 7;
-                    if (i < nx && ci < n_eff * 8) *(uint4*) (bt + (uint32_t) n * 128u + (uint32_t) ((chunk ^ (n & 7)) << 4)) = xq[i];
-                }
-                if (kt + 1 < KT) load_x(kt + 1);
-            } else {
-                uint8_t* bt = stage + (size_t) NT * GM_TILE_BYTES;
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const int ci = tid + c * GM_PRODUCERS, n = ci >> 3, chunk = ci & 7;
-                    if (c < nx && ci < n_eff * 8) {
-                        const uint4 lo = xq[2 * c], hi = xq[2 * c + 1];
-                        *(uint4*) (bt + (uint32_t) n * 128u + (uint32_t) ((chunk ^ (n & 7)) << 4)) =
-                            make_uint4(bf16x2_bits(__uint_as_float(lo.x), __uint_as_float(lo.y)), bf16x2_bits(__uint_as_float(lo.z), __uint_as_float(lo.w)),
-                                       bf16x2_bits(__uint_as_float(hi.x), __uint_as_float(hi.y)), bf16x2_bits(__uint_as_float(hi.z), __uint_as_float(hi.w)));
-                    }
-                }
-                if (kt + 1 < KT) load_xf(kt + 1);
-            }
-            // seed weights: two block pairs, expanded side by side
-#pragma unroll
-            for (int bp = 0; bp < (BF16W ? 0 : 2); ++bp) {
-                float wa[8], wb[8];
-                if (cur.live && P3) {      // two P = 3 blocks, each bit for bit as nsl_decode3_f32 gives it
-                    const uint32_t sa = cur.sw[bp] & 0xFFFFu, sb = cur.sw[bp] >> 16, na = cur.cw[bp] & 0xFFFFu, nb = cur.cw[bp] >> 16;
-                    const uint32_t ga = stream_bits(tab, sa), gb = stream_bits(tab, sb);
-                    block_weights3(sa | (ga << 16), ga, na, exact_scale45(w.eb + (int) (na & 15u) + 1), kc, wa);
-                    block_weights3(sb | (gb << 16), gb, nb, exact_scale45(w.eb + (int) (nb & 15u) + 1), kc, wb);
-                } else if (cur.live) {
-                    const uint32_t cd = cur.codes >> (8 * bp);
-                    const u64 sc2 = pack2(exact_scale45(w.eb + (int) (cd & 15u)), exact_scale45(w.eb + (int) ((cd >> 4) & 15u)));
-                    u64 w2[8];
-                    pair_weights(tab, cur.sw[bp], cur.cw[bp], sc2, kc, w2);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) unpack2(w2[i], wa[i], wb[i]);
-                }
-                if (cur.live) {
-                    if (!vec) {   // a row whose block count is not a multiple of 4 ends inside a quad: blocks past it are zero
-                        const bool has_a = (cur.sw[bp] & 0xFFFFu) != 0u, has_b = (cur.sw[bp] >> 16) != 0u;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            if (!has_a) wa[i] = 0.0f;
-                            if (!has_b) wb[i] = 0.0f;
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) wa[i] = wb[i] = 0.0f;
-                }
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    float* wv = e ? wb : wa;
-                    const int chunk = half * 4 + 2 * bp + e;
-                    const uint32_t off = (uint32_t) prow * 128u + (uint32_t) ((chunk ^ (prow & 7)) << 4);
-#pragma unroll
-                    for (int q = 0; q < NT; ++q) {   // term q = the bf16 value of what remains (exact subtraction)
-                        const uint4 o = make_uint4(bf16x2_bits(wv[0], wv[1]), bf16x2_bits(wv[2], wv[3]),
-                                                   bf16x2_bits(wv[4], wv[5]), bf16x2_bits(wv[6], wv[7]));
-                        *(uint4*) (stage + (size_t) q * GM_TILE_BYTES + off) = o;
-                        if (q + 1 < NT) {
-                            wv[0] -= __uint_as_float(o.x << 16); wv[1] -= __uint_as_float(o.x & 0xFFFF0000u);
-                            wv[2] -= __uint_as_float(o.y << 16); wv[3] -= __uint_as_float(o.y & 0xFFFF0000u);
-                            wv[4] -= __uint_as_float(o.z << 16); wv[5] -= __uint_as_float(o.z & 0xFFFF0000u);
-                            wv[6] -= __uint_as_float(o.w << 16); wv[7] -= __uint_as_float(o.w & 0xFFFF0000u);
-                        }
-                    }
-                }
-            }
-            // f32 inputs: the n_eff x 64 tile as 16-byte chunks (8 values) dealt round-robin to the producer threads
-            if (!a.packed) {
-                uint8_t* bt = stage + (size_t) NT * GM_TILE_BYTES;
-                for (int ci = tid + 2 * GM_PRODUCERS; ci < n_eff * 8; ci += GM_PRODUCERS) {      // chunks beyond the two that were requested ahead
-                    const int n = ci >> 3, chunk = ci & 7, src = srow[n], k = kt * GM_BK + 8 * chunk;
-                    uint4 o = make_uint4(0u, 0u, 0u, 0u);
-                    if (src >= 0 && k < a.K) {
-                        const float4* xp = (const float4*) ((const float*) a.X + (size_t) src * a.xs + k);
-                        const float4 x0 = __ldg(xp), x1 = __ldg(xp + 1);
-                        o = make_uint4(bf16x2_bits(x0.x, x0.y), bf16x2_bits(x0.z, x0.w), bf16x2_bits(x1.x, x1.y),
-                                       bf16x2_bits(x1.z, x1.w));
-                    }
-                    *(uint4*) (bt + (uint32_t) n * 128u + (uint32_t) ((chunk ^ (n & 7)) << 4)) = o;
-                }
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the MMA's reads
-            __syncwarp();                                                  // the warp's 32 lanes have written and fenced:
-            if (lane == 0) mbar_arrive(bar_full + 8 * s);                  // one arrival for all of them (not 32 on one word)
-            cur = nxt;
-            if (BF16W) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) bcur[i] = bnxt[i];
-            }
-        }
-        // ---- epilogue: TMEM lane = weight row, column = token ----------------------------------------------------------
-        if (live && !mbar_wait(bar_done, 0, &abort_flag)) {
-            abort_flag = 1;
-            atomicCAS(&g_mm_status, 0, 2);
-            live = false;
-        }
-        if (live) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int lq = warp & 3, chalf = warp >> 2;
-            const int row = r0 + lq * 32 + lane;
-            for (int c0 = chalf * 64; c0 < chalf * 64 + 64 && c0 < n_eff; c0 += 16) {
-                uint32_t v[16];
-                tmem_ld16(tmem_acc + ((uint32_t) (lq * 32) << 16) + (uint32_t) c0, v);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int dst = drow[c0 + j];
-                    if (dst < 0 || row >= a.R) continue;
-                    float* yo = a.Y + (size_t) dst * a.ys + row;
-                    const float acc = __uint_as_float(v[j]);
+            for (int j = 0; j < 16; ++j) {
+                const int dst = __shfl_sync(0xFFFFFFFFu, dst_lane, j);
+                if (c0 + j >= count || grow >= a.R) continue;
+                const float acc = __uint_as_float(v[j]);
+                if (a.out_bf16) ((uint16_t*) a.Y)[(size_t) dst * a.ys + grow] = (uint16_t) bf16x2_bits(acc, 0.0f);
+                else {
+                    float* yo = (float*) a.Y + (size_t) dst * a.ys + grow;
                     *yo = a.add ? bf16_round(*yo + bf16_round(acc)) : bf16_round(acc);   // engine/kernels_moe.cu:214
                 }
             }
         }
-    } else if (lane == 0) {
-        // ---- the MMA issuer --------------------------------------------------------------------------------------------
-        const uint32_t idesc = umma_idesc(n_eff);
-        bool live = true;
-        for (int kt = 0; kt < KT; ++kt) {
-            const int s = kt % GM_STAGES;
-            if (!mbar_wait(bar_full + 8 * s, (kt / GM_STAGES) & 1, &abort_flag)) {
-                abort_flag = 1;
-                atomicCAS(&g_mm_status, 0, 3);
-                live = false;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t sa = smem_base + (uint32_t) s * STAGE_BYTES, sb = sa + NT * GM_TILE_BYTES;
-#pragma unroll
-            for (int q = 0; q < NT; ++q)
-#pragma unroll
-                for (int k4 = 0; k4 < GM_BK / 16; ++k4)
-                    umma(tmem_acc, umma_desc(sa + q * GM_TILE_BYTES + k4 * 32), umma_desc(sb + k4 * 32), idesc,
-                         (kt | q | k4) != 0);
-            umma_commit(bar_empty + 8 * s);   // the stage is free when these MMAs have read it
+    }
+}
+
+// WF: the weights' form.  0: SEED4P4 blocks; 1: stored BF16 values; 2: SEED4 (P = 3) blocks.  TERMS: bf16 terms a weight (1, or 3:
+// exact).  TT: tiles of 128 rows of inputs that share one expansion.  VEC: K a multiple of 64, streams in aligned 16-byte pieces.
+// GU: gate + up + SwiGLU; row i of the gate matrix on lane 2 i, of the up matrix on lane 2 i + 1.  F32: f32 inputs (else packed).
+template <int TERMS, int WF, int TT, bool VEC, bool GU, bool F32>
+__global__ void __launch_bounds__(GmCfg<TERMS, TT, F32>::THREADS, GmCfg<TERMS, TT, F32>::CTAS) seed_gemm_kernel(MmParams a, KConst kc) {
+    using Cfg = GmCfg<TERMS, TT, F32>;
+    constexpr bool BF16W = WF == 1, P3 = WF == 2;
+    constexpr int PW = Cfg::PW, GROUPS = Cfg::GROUPS, HALF = Cfg::ACC / 2;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ StreamTab tab;
+    __shared__ __align__(8) uint64_t bars[2 * GM_STAGES + 3];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int srow[GM_BN * TT];      // the unit's rows of inputs
+    __shared__ int abort_flag, n_heads;
+    __shared__ uint16_t heads[TT > 1 ? GM_MAX_HEADS : 1];
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t smem_base = smem_u32((uint8_t*) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023));
+    const uint32_t bar_full = smem_u32(&bars[0]), bar_empty = bar_full + 8 * GM_STAGES, bar_done = bar_empty + 8 * GM_STAGES, bar_read = bar_done + 8;
+    if (!BF16W) load_stream_tab(tab, a.G, tid, Cfg::THREADS);
+    if (tid == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < GM_STAGES; ++s) {
+            mbar_init(bar_full + 8 * s, 4 + Cfg::LW);      // one arrival per warp of the stage's warpgroup and per loader warp
+            mbar_init(bar_empty + 8 * s, 1);
         }
-        if (live) umma_commit(bar_done);
+        mbar_init(bar_done, 1);                            // a unit's MMAs are done
+        mbar_init(bar_read, PW);                           // the results in a half of the accumulators have been read
+        mbar_init(bar_read + 8, PW);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == PW) {   // the MMA warp owns the tensor memory
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(Cfg::COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    grid_dependents_go();
+    grid_dependency_wait();
+    if (TT > 1 && a.grouped && warp == 0) {      // the tiles that start a unit: every TT-th of a slice, in order
+        const int nt = a.ntiles ? *a.ntiles : a.T;
+        int n = 0;
+        for (int y0 = 0; y0 < nt; y0 += 32) {
+            const int y = y0 + lane;
+            bool head = false;
+            if (y < nt) { const MmTile tl = a.tiles[y]; head = ((tl.start - a.offs[tl.slice]) / GM_BN) % TT == 0; }
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, head);
+            if (head) heads[n + __popc(m & ((1u << lane) - 1u))] = (uint16_t) y;
+            n += __popc(m);
+        }
+        if (lane == 0) n_heads = n;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == GM_PRODUCERS / 32) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(GM_BN) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot, tmem_w = tmem + Cfg::ACC;
+    const int NB = a.K / 8, KT = (a.K + GM_BK - 1) / GM_BK, rows_u = GU ? GM_BM / 2 : GM_BM;
+    const int row_tiles = (a.R + rows_u - 1) / rows_u;
+    const int n_units = row_tiles * (a.grouped ? (TT > 1 ? n_heads : a.ntiles ? *a.ntiles : a.T) : (a.T + GM_BN * TT - 1) / (GM_BN * TT));
+    const int half_max = KT < GROUPS ? 0 : HALF;      // (a warpgroup without a step in a unit must not fall a unit behind the MMAs)
+    // Every role walks the same units and counts the same K steps (kr: its stage and the stage's phase) and units.
+    int kr0 = 0, unit_run = 0;
+    bool ok = true;
+    auto fail = [&](int code) { abort_flag = 1; atomicCAS(&g_mm_status, 0, code); ok = false; };
+
+    if (warp < PW) {
+        if (Cfg::SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::PREGS));
+        // ---- producers: thread = one row's 64 weights of a K step; warpgroup g makes the steps with kr % GROUPS = g -----------------
+        const int group = warp >> 2, lq = warp & 3, rl = lq * 32 + lane;      // rl: tensor memory lane = row of the tile
+        int p_start = 0, p_count = 0, p_r0 = 0, p_col = 0;                      // the unit whose results are still to be read
+        int small_run = 0;                                                      // units so far that filled a half
+        auto results = [&]() {      // of the pending unit, the unit_run-th
+            if (!mbar_wait(bar_done, (unit_run - 1) & 1, &abort_flag)) fail(2);
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                unit_results<GU, GROUPS>(a, tmem, p_col, p_start, p_count, p_r0);
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    if (p_count > half_max || p_col == 0) mbar_arrive(bar_read);
+                    if (p_count > half_max || p_col != 0) mbar_arrive(bar_read + 8);
+                }
+            }
+            p_count = 0;
+        };
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+            const UnitPos u = unit_pos<TT, GU>(a, unit, row_tiles, heads);
+            if (u.count <= 0) continue;
+            const WSlice w = GU && (lane & 1) ? u.wb : u.wa;
+            const int grow = GU ? u.r0 + (rl >> 1) : u.r0 + rl;
+            const float base = BF16W ? 0.0f : exact_base<P3 ? 3 : 4>(w.eb);
+            int kt = (group - kr0 % GROUPS + GROUPS) % GROUPS;
+            ChunkIn cur = {};
+            if (!BF16W && kt < KT) cur = load_row_chunk<P3, VEC>(w, grow, kt, a.R, NB);
+            for (; kt < KT && ok; kt += GROUPS) {
+                const int kr = kr0 + kt, s = kr % GM_STAGES;
+                const uint32_t ta = tmem_w + ((uint32_t) (lq * 32) << 16) + (uint32_t) (s * Cfg::A_COLS);
+                ChunkIn nxt = {};
+                if (!BF16W && kt + GROUPS < KT) nxt = load_row_chunk<P3, VEC>(w, grow, kt + GROUPS, a.R, NB);
+                const uint32_t sw[4] = {cur.s.x, cur.s.y, cur.s.z, cur.s.w}, cw[4] = {cur.c.x, cur.c.y, cur.c.z, cur.c.w};
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {      // 32 weights = 16 words
+                    uint32_t v[TERMS][16];
+                    if (BF16W) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int k = kt * GM_BK + q * 32 + 8 * i;
+                            const uint4 t = grow < a.R && k < a.K ? __ldg((const uint4*) ((const uint16_t*) w.p[0] + (size_t) grow * a.K + k)) : make_uint4(0u, 0u, 0u, 0u);
+                            v[0][4 * i] = t.x; v[0][4 * i + 1] = t.y; v[0][4 * i + 2] = t.z; v[0][4 * i + 3] = t.w;
+                        }
+                    } else {
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) {
+                            const int bp = 2 * q + b;
+                            u64 w2[8];
+                            const u64 e2 = P3 ? code_scale_pair3(cw[bp], kc) : code_scale_pair(cur.cd, bp, kc);
+                            pair_weights<P3 ? 3 : 4>(tab, sw[bp], cw[bp], e2, base, kc, w2);
+                            float wa[8], wb[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) unpack2(w2[i], wa[i], wb[i]);
+#pragma unroll
+                            for (int t = 0; t < TERMS; ++t) {      // term t = the bf16 value of what remains (exact subtraction)
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    const uint32_t o = bf16x2_bits(wa[2 * i], wa[2 * i + 1]), p = bf16x2_bits(wb[2 * i], wb[2 * i + 1]);
+                                    v[t][8 * b + i] = o;
+                                    v[t][8 * b + 4 + i] = p;
+                                    if (t + 1 < TERMS) {
+                                        wa[2 * i] -= __uint_as_float(o << 16); wa[2 * i + 1] -= __uint_as_float(o & 0xFFFF0000u);
+                                        wb[2 * i] -= __uint_as_float(p << 16); wb[2 * i + 1] -= __uint_as_float(p & 0xFFFF0000u);
+                                    }
+                                }
+                            }
+                        }
+                    }
+                    if (q == 0) {      // the stage has to be free only now: half of the step is in registers
+                        if (kr >= GM_STAGES && !mbar_wait(bar_empty + 8 * s, ((kr / GM_STAGES) - 1) & 1, &abort_flag)) fail(1);
+                        ok = __all_sync(0xFFFFFFFFu, ok);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    }
+#pragma unroll
+                    for (int t = 0; t < TERMS; ++t) tmem_st16(ta + t * 32 + q * 16, v[t]);
+                }
+                if (!ok) break;
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full + 8 * s);
+                cur = nxt;
+                if (p_count) results();      // the previous unit's, under its MMAs' last step
+            }
+            if (ok && p_count) results();      // (a unit with fewer steps than warpgroups)
+            kr0 += KT;
+            ++unit_run;
+            p_start = u.start; p_count = u.count; p_r0 = u.r0;
+            p_col = u.count <= half_max ? (small_run++ & 1) * HALF : 0;
+            if (ok && u.count > half_max) results();
+        }
+        if (ok && p_count) results();
+    } else {
+        if (Cfg::SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::LREGS));      // (one instruction for the whole warpgroup)
+        if (warp == PW) {
+            // ---- the MMA issuer --------------------------------------------------------------------------------------------------
+            if (lane == 0) {
+                const uint64_t desc0 = umma_desc(smem_base);      // + bytes / 16 for another place in the 256 KB window
+                int small_run = 0, uses[2] = {0, 0};               // units so far in each half of the accumulators
+                for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+                    const UnitPos u = unit_pos<TT, GU>(a, unit, row_tiles, heads);
+                    if (u.count <= 0) continue;
+                    const int half = u.count <= half_max ? small_run++ & 1 : 0, col = half * HALF;
+                    for (int h = 0; h < 2 && ok; ++h)
+                        if (u.count > half_max || h == half) {
+                            if (uses[h] > 0 && !mbar_wait(bar_read + 8 * h, (uses[h] - 1) & 1, &abort_flag)) fail(3);
+                            ++uses[h];
+                        }
+                    for (int kt = 0; kt < KT && ok; ++kt) {
+                        const int kr = kr0 + kt, s = kr % GM_STAGES;
+                        if (!mbar_wait(bar_full + 8 * s, (kr / GM_STAGES) & 1, &abort_flag)) { fail(3); break; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint32_t sa = tmem_w + (uint32_t) (s * Cfg::A_COLS);
+#pragma unroll 1
+                        for (int tt = 0; tt < TT && tt * GM_BN < u.count; ++tt) {
+                            const uint32_t idesc = umma_idesc((min(u.count - tt * GM_BN, GM_BN) + 15) & ~15);
+                            const uint64_t db = desc0 + (uint64_t) ((s * Cfg::X_BYTES + tt * 16384) >> 4);
+#pragma unroll
+                            for (int q = 0; q < TERMS; ++q)
+#pragma unroll
+                                for (int k16 = 0; k16 < GM_BK / 16; ++k16)
+                                    umma_ts(tmem + col + tt * GM_BN, sa + q * 32 + k16 * 8, db + (uint64_t) (k16 * 2), idesc, (kt | q | k16) != 0);
+                        }
+                        umma_commit(bar_empty + 8 * s);   // the stage is free when these MMAs have read it
+                    }
+                    if (ok) umma_commit(bar_done);
+                    kr0 += KT;
+                }
+            }
+        } else {
+            // ---- loaders: a K step's inputs -------------------------------------------------------------------------------------------
+            const int lt = tid - (PW + 1) * 32;
+            constexpr int LT = Cfg::LW * 32, RPP = LT / 8;      // threads; rows a pass
+            const int uu = lt & 7, n_lo = lt >> 3;              // this thread's 16-byte unit of the K step's 64 inputs, its first row
+            int pending = -1;                                   // packed: the stage whose copies are in flight
+            auto settle = [&]() {      // a stage's inputs are complete
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the MMA's reads
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full + 8 * pending);
+            };
+            for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+                const UnitPos u = unit_pos<TT, GU>(a, unit, row_tiles, heads);
+                if (u.count <= 0) continue;
+                const int n16 = (u.count + 15) & ~15;
+                __syncwarp();
+                for (int i = lane;; i += 32) {      // this warp's own rows: 4 w .. 4 w + 3, then every RPP on
+                    const int n = ((lt >> 5) << 2) + (i & 3) + (i >> 2) * RPP;
+                    if (n >= n16) break;
+                    srow[n] = input_row_of(a, u, n);
+                }
+                __syncwarp();
+                constexpr int FLIGHT = 5;      // F32: 16-byte results in flight a thread (5 x 28 rows: a tile)
+                float4 x[F32 ? 2 * FLIGHT : 1];
+                auto request = [&](int kt, int n0) {
+                    const int k = kt * GM_BK + 8 * uu;
+#pragma unroll
+                    for (int i = 0; i < FLIGHT; ++i) {
+                        const int n = n0 + i * RPP;
+                        x[2 * i] = x[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        if (n < n16 && k < a.K) {
+                            const float4* xp = (const float4*) ((const float*) a.X + ((size_t) srow[n] * a.xs + k));
+                            x[2 * i] = __ldg(xp);
+                            x[2 * i + 1] = __ldg(xp + 1);
+                        }
+                    }
+                };
+                if (F32) request(0, n_lo);
+                for (int kt = 0; kt < KT && ok; ++kt) {
+                    const int kr = kr0 + kt, s = kr % GM_STAGES;
+                    if (kr >= GM_STAGES && !mbar_wait(bar_empty + 8 * s, ((kr / GM_STAGES) - 1) & 1, &abort_flag)) fail(4);
+                    ok = __all_sync(0xFFFFFFFFu, ok);
+                    if (!ok) break;
+                    const uint32_t stage = smem_base + (uint32_t) (s * Cfg::X_BYTES);
+                    if (!F32) {      // copies of this step, then the arrival of the previous one's
+                        const int k = kt * GM_BK + 8 * uu;
+                        const bool in = k < a.K;
+                        const uint16_t* xk = (const uint16_t*) a.X + (in ? k : 0);
+#pragma unroll 4
+                        for (int n = n_lo; n < n16; n += RPP)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(input_at(stage, n, uu)), "l"(xk + (size_t) srow[n] * a.xs), "r"(in ? 16 : 0) : "memory");
+                        asm volatile("cp.async.commit_group;" ::: "memory");
+                        if (pending >= 0) {
+                            asm volatile("cp.async.wait_group 1;" ::: "memory");
+                            settle();
+                        }
+                        pending = s;
+                    } else {
+                        for (int n0 = n_lo;;) {
+#pragma unroll
+                            for (int i = 0; i < FLIGHT; ++i) {
+                                const int n = n0 + i * RPP;
+                                if (n < n16)
+                                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(input_at(stage, n, uu)), "r"(bf16x2_bits(x[2 * i].x, x[2 * i].y)),
+                                                 "r"(bf16x2_bits(x[2 * i].z, x[2 * i].w)), "r"(bf16x2_bits(x[2 * i + 1].x, x[2 * i + 1].y)),
+                                                 "r"(bf16x2_bits(x[2 * i + 1].z, x[2 * i + 1].w)) : "memory");
+                            }
+                            n0 += FLIGHT * RPP;
+                            const bool more = __any_sync(0xFFFFFFFFu, n0 < n16);      // (warp-uniform)
+                            if (more) request(kt, n0);
+                            else if (kt + 1 < KT) request(kt + 1, n_lo);
+                            if (!more) break;
+                        }
+                        pending = s;
+                        settle();
+                    }
+                }
+                kr0 += KT;
+            }
+            if (!F32 && pending >= 0 && ok) {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                settle();
+            }
+        }
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == PW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::COLS) : "memory");
 }
 
 bool launch_bf16_mm_skinny(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add);
 
-thread_local bool tl_mm_overlap = false;
-
 static int g_exact;   // kc_seed_gemm_f32: process-wide, as the reference's switch (engine/kernels_moe.cu:2354)
+bool seed_gemm_exact() { return g_exact != 0; }
 
-template <int NT, int WF, bool VEC>
-static void launch_gemm_v(cudaStream_t s, const MmParams& a, dim3 grid) {
-    const size_t smem = (size_t) GM_STAGES * (NT + 1) * GM_TILE_BYTES + 1024;
+template <int TERMS, int WF, int TT, bool VEC, bool GU, bool F32>
+static void launch_gemm_v(cudaStream_t s, const MmParams& a, int units) {
+    using Cfg = GmCfg<TERMS, TT, F32>;
+    const size_t smem = (size_t) GM_STAGES * Cfg::X_BYTES + 1024;
     static bool attr_set[16];
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev & 15]) {
-        cudaFuncSetAttribute(seed_gemm_kernel<NT, WF, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+        cudaFuncSetAttribute(seed_gemm_kernel<TERMS, WF, TT, VEC, GU, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
         attr_set[dev & 15] = true;
     }
-    // tl_mm_overlap: the caller says this launch reads nothing its predecessor in the stream writes
-    PdlScope pdl(tl_mm_overlap);
-    launch(seed_gemm_kernel<NT, WF, VEC>, grid, GM_THREADS, smem, s, a, kconst());
+    const int slots = sm_count() * Cfg::CTAS;
+    launch(seed_gemm_kernel<TERMS, WF, TT, VEC, GU, F32>, (unsigned) (units < slots ? units : slots), Cfg::THREADS, smem, s, a, kconst());
     count_launch();
 }
-template <int NT, int WF>
-static void launch_gemm_nt(cudaStream_t s, const MmParams& a, dim3 grid) {
-    if (WF == 1 || a.K % 32 == 0) launch_gemm_v<NT, WF, true>(s, a, grid);      // stored BF16 weights have no quads
-    else launch_gemm_v<NT, WF, false>(s, a, grid);
+// How many tiles of a dense call share an expansion: a unit takes the time of its expansion (twice that where two blocks share an
+// SM) or of its inputs' conversion (f32: nine tenths of it per tile), and the units go round the SMs.
+static int dense_tiles(const MmParams& a, int row_tiles) {
+    int best = 1;
+    double best_cost = 0.0;
+    for (int tt = 1; tt <= 3; ++tt) {
+        if (a.packed && tt == 2) continue;
+        const int units = row_tiles * ((a.T + GM_BN * tt - 1) / (GM_BN * tt)), slots = sm_count() * (a.packed && tt == 1 ? 2 : 1);
+        const double unit = a.packed ? (tt == 1 && units > sm_count() ? 2.0 : 1.0) : tt == 1 ? 1.0 : 0.9 * tt;
+        const double cost = (double) ((units + slots - 1) / slots) * unit;
+        if (tt == 1 || cost < best_cost) { best = tt; best_cost = cost; }
+    }
+    return best;
 }
+template <int WF>
+static void launch_gemm_seed(cudaStream_t s, const MmParams& a, int row_tiles, int tiles_y) {
+    const int units = row_tiles * tiles_y;
+    if (g_exact) {
+        if (a.packed) launch_gemm_v<3, WF, 1, false, false, false>(s, a, units);
+        else if (a.K % 64 == 0) launch_gemm_v<3, WF, 1, true, false, true>(s, a, units);
+        else launch_gemm_v<3, WF, 1, false, false, true>(s, a, units);
+    } else if (a.K % 64) {
+        if (a.packed) launch_gemm_v<1, WF, 1, false, false, false>(s, a, units);
+        else launch_gemm_v<1, WF, 1, false, false, true>(s, a, units);
+    } else if (a.grouped) {
+        if (!a.packed) launch_gemm_v<1, WF, 1, true, false, true>(s, a, units);
+        else if (a.offs) launch_gemm_v<1, WF, 3, true, false, false>(s, a, units);
+        else launch_gemm_v<1, WF, 1, true, false, false>(s, a, units);
+    } else {
+        const int tt = dense_tiles(a, row_tiles), u = row_tiles * ((a.T + GM_BN * tt - 1) / (GM_BN * tt));
+        if (a.packed) { if (tt == 1) launch_gemm_v<1, WF, 1, true, false, false>(s, a, u); else launch_gemm_v<1, WF, 3, true, false, false>(s, a, u); }
+        else if (tt == 1) launch_gemm_v<1, WF, 1, true, false, true>(s, a, u);
+        else if (tt == 2) launch_gemm_v<1, WF, 2, true, false, true>(s, a, u);
+        else launch_gemm_v<1, WF, 3, true, false, true>(s, a, u);
+    }
+}
+void launch_gemm_gu(cudaStream_t s, const MmParams& a, int tiles_y) {
+    const int units = (a.R + GM_BM / 2 - 1) / (GM_BM / 2) * tiles_y;
+    if (a.offs) launch_gemm_v<1, 0, 3, true, true, false>(s, a, units);
+    else launch_gemm_v<1, 0, 1, true, true, false>(s, a, units);
+}
+bool gemm_shares_tiles(int max_tiles) { return max_tiles <= GM_MAX_HEADS; }
 
-static void launch_gemm(cudaStream_t s, int fmt, const char* who, MmParams a, int tiles_y) {
+void launch_gemm(cudaStream_t s, int fmt, const char* who, MmParams a, int tiles_y) {
     if (fmt != MF_SEED4P4 && fmt != MF_SEED4 && fmt != MF_BF16) {
         set_error("%s: weight format %d is not served by this library (SEED4P4 = %d, SEED4 = %d and BF16 = %d only)", who, fmt, (int) MF_SEED4P4,
                   (int) MF_SEED4, (int) MF_BF16);
@@ -455,11 +586,15 @@ static void launch_gemm(cudaStream_t s, int fmt, const char* who, MmParams a, in
         set_error("%s: inputs must be 16-byte aligned with a row stride that is a multiple of 16 bytes", who);
         return;
     }
-    const dim3 grid((unsigned) ((a.R + GM_BM - 1) / GM_BM), (unsigned) tiles_y);
-    if (fmt == MF_BF16) launch_gemm_nt<1, 1>(s, a, grid);      // stored BF16 weights (p[0] = [R][K]): no expansion, one term
-    else if (fmt == MF_SEED4) { if (g_exact) launch_gemm_nt<3, 2>(s, a, grid); else launch_gemm_nt<1, 2>(s, a, grid); }      // P = 3
-    else if (g_exact) launch_gemm_nt<3, 0>(s, a, grid);
-    else launch_gemm_nt<1, 0>(s, a, grid);
+    if (a.grouped && !a.ntiles) a.T = tiles_y;
+    // a dense call of a few rows: the weights stay in registers (64 rows: 2 tiles there)
+    if (fmt != MF_BF16 && !g_exact && !a.grouped && a.T <= 64 && smm_serves(a.K, a.X, a.xs, a.packed)) { launch_seed_mma(s, fmt, a, tiles_y); return; }
+    const int row_tiles = (a.R + GM_BM - 1) / GM_BM;
+    if (fmt == MF_BF16) {      // stored BF16 weights (p[0] = [R][K]): no expansion, one term
+        if (a.packed) launch_gemm_v<1, 1, 1, true, false, false>(s, a, row_tiles * tiles_y);
+        else launch_gemm_v<1, 1, 1, true, false, true>(s, a, row_tiles * tiles_y);
+    } else if (fmt == MF_SEED4) launch_gemm_seed<2>(s, a, row_tiles, tiles_y);
+    else launch_gemm_seed<0>(s, a, row_tiles, tiles_y);
 }
 
 }   // namespace nsl
@@ -473,29 +608,29 @@ void kc_seed_gemm_f32(int on) { g_exact = on; }
 void kc_mm(cudaStream_t s, int fmt, WSlice w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add,
            const uint32_t* G) {
     if (fmt == MF_BF16 && launch_bf16_mm_skinny(s, w, K, R, x, xs, y, ys, T, add)) return;      // a decode batch (dense_bf16.cu)
-    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, NULL, K, R, T, xs, ys, 1, add, 0, 0};
+    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, K, R, T, xs, ys, 1, add, 0, 0, NULL, 0, NULL};
     launch_gemm(s, fmt, "kc_mm", a, (T + GM_BN - 1) / GM_BN);
 }
 void kc_mm_packed(cudaStream_t s, int fmt, WSlice w, int K, int R, const uint16_t* x, int xs, float* y, int ys, int T, int add,
                   const uint32_t* G) {
-    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, NULL, K, R, T, xs, ys, 1, add, 0, 1};
+    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, K, R, T, xs, ys, 1, add, 0, 1, NULL, 0, NULL};
     launch_gemm(s, fmt, "kc_mm_packed", a, (T + GM_BN - 1) / GM_BN);
 }
 void kc_mm_grouped(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys,
                    int xdiv, const int32_t* perm, const MmTile* tiles, int ntiles, const uint32_t* G) {
-    MmParams a = {ws, WSlice{}, x, y, perm, tiles, NULL, G, NULL, K, R, 0, xs, ys, xdiv, 0, 1, 0};
+    MmParams a = {ws, WSlice{}, x, y, perm, tiles, NULL, G, K, R, 0, xs, ys, xdiv, 0, 1, 0, NULL, 0, NULL};
     launch_gemm(s, fmt, "kc_mm_grouped", a, ntiles);
 }
 void kc_mm_grouped_dev(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys,
                        int xdiv, const int32_t* perm, const MmTile* tiles, const int32_t* ntiles, int max_tiles,
                        const uint32_t* G) {
-    MmParams a = {ws, WSlice{}, x, y, perm, tiles, ntiles, G, NULL, K, R, 0, xs, ys, xdiv, 0, 1, 0};
+    MmParams a = {ws, WSlice{}, x, y, perm, tiles, ntiles, G, K, R, 0, xs, ys, xdiv, 0, 1, 0, NULL, 0, NULL};
     launch_gemm(s, fmt, "kc_mm_grouped_dev", a, max_tiles);
 }
 void kc_mm_grouped_packed(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const uint16_t* x, int xs, float* y, int ys,
                           int xdiv, const int32_t* perm, const MmTile* tiles, const int32_t* nt, int max_tiles,
                           const uint32_t* G) {
-    MmParams a = {ws, WSlice{}, x, y, perm, tiles, nt, G, NULL, K, R, 0, xs, ys, xdiv, 0, 1, 1};
+    MmParams a = {ws, WSlice{}, x, y, perm, tiles, nt, G, K, R, 0, xs, ys, xdiv, 0, 1, 1, NULL, 0, NULL};
     launch_gemm(s, fmt, "kc_mm_grouped_packed", a, max_tiles);
 }
 

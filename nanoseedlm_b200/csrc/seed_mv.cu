@@ -56,8 +56,8 @@ constexpr KConst kconst_static() {
     for (int p = 0; p < 4; ++p) {
         k.cxor[p] = ((uint32_t) (215 - 5 * p) << 23) | (8u << (4 * p));
         k.coff[p] = -(pow2_f(88 - 5 * p) + pow2_f(68 - p));
-        k.cxor_x[p] = ((uint32_t) (250 - 5 * p) << 23) | (8u << (4 * p));
-        k.coff_x[p] = -(pow2_f(123 - 5 * p) + pow2_f(103 - p));
+        k.cxor_x[p] = ((uint32_t) (253 - 5 * p) << 23) | (8u << (4 * p));
+        k.coff_x[p] = -(pow2_f(126 - 5 * p) + pow2_f(106 - p));
     }
     k.cor = 112u << 23;
     return k;
@@ -1042,8 +1042,8 @@ __global__ void __launch_bounds__(256) decode_kernel(WSlice w, KConst kc, int K,
         const int code = P == 4 ? (((const uint8_t*) w.p[3])[gidx >> 1] >> ((gidx & 1) * 4)) & 15 : (int) (cw & 15u);
         const uint32_t g = stream_bits(tab, seed);
         float wv[8];
-        if (P == 4) block_weights(seed | (g << 16), g, cw, exact_scale45(w.eb + code), kc, wv);
-        else block_weights3(seed | (g << 16), g, cw, exact_scale45(w.eb + code + 1), kc, wv);
+        if (P == 4) block_weights(seed | (g << 16), g, cw, exact_scale<42>(w.eb + code), kc, wv);
+        else block_weights3(seed | (g << 16), g, cw, exact_scale<43>(w.eb + code), kc, wv);
         if (BF16) {
             uint4 o;
             o.x = bf16_bits(wv[0]) | ((uint32_t) bf16_bits(wv[1]) << 16);
