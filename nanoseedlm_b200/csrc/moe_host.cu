@@ -11,6 +11,7 @@
 #include "seed_mma.cuh"
 
 namespace nsl {
+void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* perm, uint16_t* y, int P, int xdiv, int d);
 void launch_combine_packed(cudaStream_t s, int d, int k, const uint16_t* D, const float* wt, float* out, int T);
 }
 
@@ -122,20 +123,38 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
         const int mt = P / MMT_BN + m->n_exp;
         nsl_route(s, m->n_exp, k, logits, m->n_exp, m->ind, m->wt, T);
         kc_bucket(s, m->ind, P, m->n_exp, m->perm, m->tiles, m->ntiles);
-        kc_pack_input_bf16(s, x, m->xp, (size_t) T * d);      // once: every row tile of every expert reads them
         if (!nsl::seed_gemm_exact() && d % 64 == 0 && ff % 64 == 0) {
-            // gate, up and SwiGLU in one launch, results as packed bf16 (they are bf16 values); the down projections' rows stay packed too.
-            // Few rows an expert: the kernel that keeps the weights in registers; many: one expansion for up to 384 rows.
+            // gate, up and SwiGLU in one launch, results as packed bf16 (they are bf16 values); the down projections' rows stay packed too
             const int avg = P / m->n_exp;
-            uint16_t* const D = (uint16_t*) m->Dx;
-            nsl::MmParams g = {m->wg, WSlice{}, m->xp, m->Ap, m->perm, m->tiles, m->ntiles, m->G, d, ff, 0, d, ff, k, 0, 1, 1, m->wu, 1,
-                               avg >= 96 && nsl::gemm_shares_tiles(mt) ? m->ntiles + 1 : NULL};
-            nsl::MmParams w = {m->wd, WSlice{}, m->Ap, D, m->perm, m->tiles, m->ntiles, m->G, ff, d, 0, ff, d, 1, 0, 1, 1, NULL, 1, g.offs};
-            if (avg < 12) { nsl::launch_seed_mma(s, MF_SEED4P4, g, mt); nsl::launch_seed_mma(s, MF_SEED4P4, w, mt); }
-            else { nsl::launch_gemm_gu(s, g, mt); nsl::launch_gemm(s, MF_SEED4P4, "nsl_moe_forward", w, mt); }
+            uint16_t* const D = (uint16_t*) m->Dx;      // packed rows take half of the f32 buffer; the sorted inputs have the other half
+            nsl::MmParams g = {m->wg, WSlice{}, m->xp, m->Ap, m->perm, m->tiles, m->ntiles, m->G, d, ff, 0, d, ff, k, 0, 1, 1, m->wu, 1, NULL, 0, 0, 0};
+            nsl::MmParams w = {m->wd, WSlice{}, m->Ap, D, m->perm, m->tiles, m->ntiles, m->G, ff, d, 0, ff, d, 1, 0, 1, 1, NULL, 1, NULL, 0, 0, 0};
+            if (avg >= 96 && nsl::gemm_shares_tiles(mt)) {
+                // many rows an expert: one expansion for up to 384 of them, whose inputs are fetched as boxes of consecutive rows, so
+                // the rows are packed in the order of the pairs by expert (4096 rows of config 1's layer: 549 -> 486 us; at 32
+                // rows an expert the copy costs what it saves)
+                uint16_t* const xs = D + (size_t) P * d;
+                nsl::launch_pack_sorted(s, x, m->perm, xs, P, k, d);
+                g.X = xs;
+                g.in_sorted = g.out_sorted = w.in_sorted = 1;
+                g.T_in = w.T_in = P;
+                g.offs = w.offs = m->ntiles + 1;
+                nsl::launch_gemm_gu(s, g, mt);
+                nsl::launch_gemm(s, MF_SEED4P4, "nsl_moe_forward", w, mt);
+            } else {
+                kc_pack_input_bf16(s, x, m->xp, (size_t) T * d);      // once: every row tile of every expert reads them
+                if (avg < 8) {      // few rows an expert: the kernel that keeps the weights in registers (at 11 rows the other is 4 % faster, at 1.3 2 % slower)
+                    nsl::launch_seed_mma(s, MF_SEED4P4, g, mt);
+                    nsl::launch_seed_mma(s, MF_SEED4P4, w, mt);
+                } else {
+                    nsl::launch_gemm_gu(s, g, mt);
+                    nsl::launch_gemm(s, MF_SEED4P4, "nsl_moe_forward", w, mt);
+                }
+            }
             nsl::launch_combine_packed(s, d, k, D, m->wt, out, T);
             return 0;
         }
+        kc_pack_input_bf16(s, x, m->xp, (size_t) T * d);
         kc_mm_grouped_packed(s, MF_SEED4P4, m->wg, d, ff, m->xp, d, m->Gb, ff, k, m->perm, m->tiles, m->ntiles, mt, m->G);
         kc_mm_grouped_packed(s, MF_SEED4P4, m->wu, d, ff, m->xp, d, m->A, ff, k, m->perm, m->tiles, m->ntiles, mt, m->G);
         nsl_swiglu_packed(s, m->Gb, m->A, m->Ap, P * ff);

@@ -107,6 +107,25 @@ __global__ void pack_bf16_kernel(const float* __restrict__ x, uint16_t* __restri
     if (blockIdx.x == 0 && threadIdx.x < (n & 7)) y[n8 * 8 + threadIdx.x] = bf16_bits(x[n8 * 8 + threadIdx.x]);
 }
 
+// Row n of y = row perm[n] / xdiv of x as packed bf16 (d a multiple of 8; a thread: 8 values).
+__global__ void __launch_bounds__(256) pack_sorted_kernel(const float4* __restrict__ x, const int32_t* __restrict__ perm, uint4* __restrict__ y, int xdiv, int d8,
+                                                          int P) {
+    grid_dependents_go();
+    grid_dependency_wait();
+    for (int row = blockIdx.x; row < P; row += gridDim.x) {
+        const float4* xp = x + (size_t) (__ldg(perm + row) / xdiv) * d8 * 2;
+        for (int c = threadIdx.x; c < d8; c += 256) {
+            const float4 a = __ldg(xp + 2 * c), b = __ldg(xp + 2 * c + 1);
+            y[(size_t) row * d8 + c] = make_uint4(bf16x2_bits(a.x, a.y), bf16x2_bits(a.z, a.w), bf16x2_bits(b.x, b.y), bf16x2_bits(b.z, b.w));
+        }
+    }
+}
+void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* perm, uint16_t* y, int P, int xdiv, int d) {
+    const int cap = sm_count() * 8;
+    launch(pack_sorted_kernel, (unsigned) (P < cap ? P : cap), 256, 0, s, (const float4*) x, perm, (uint4*) y, xdiv, d / 8, P);
+    count_launch();
+}
+
 // ---- grouping ---------------------------------------------------------------------------------------------------------
 // work (2n+3 ints): [0] tile count, [1..n+1] pair offset of each expert, [n+2..2n+2] tile offset of each expert.
 // One block: histogram by shared-memory atomics, then an inclusive scan of pairs and tiles over the experts.

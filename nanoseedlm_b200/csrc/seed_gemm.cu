@@ -18,9 +18,9 @@
 //   otherwise: 16 producer warps, one block an SM.  TT = 3: up to three tiles of an expert share one expansion, which a prompt of
 //   thousands of rows needs (each tile expands its expert's weights again).
 // The accumulator is read back with tcgen05.ld by the producer warps (lane = weight row, column = row of inputs), rounded as the
-// reference's store_y does and written so that a warp stores 32 consecutive rows of one row of outputs.  Units that fill at most
-// half of the accumulator columns alternate between the halves, and their results are read back after the next unit's first
-// step has been produced, when the MMAs are done.
+// reference's store_y does and written so that a warp stores 32 consecutive rows of one row of outputs: after each warpgroup's
+// first step of the next unit, under which the last MMAs run.  Units that fill at most half of the accumulator columns alternate
+// between the halves, so the next unit's MMAs need not wait for that.
 // Gate + up + SwiGLU (GU): lane 2 i holds row i of the gate matrix, lane 2 i + 1 of the up matrix, so both sums meet in
 // neighbouring lanes and the result leaves as packed bf16: no f32 intermediates, no third kernel.
 //
@@ -29,6 +29,8 @@
 //
 // Every wait on an mbarrier is bounded: after the limit the block records a status word, stops issuing work, frees its
 // TMEM and returns.
+#include <cuda.h>
+
 #include "common.cuh"
 #include "seed_block.cuh"
 #include "seed_mma.cuh"
@@ -39,19 +41,23 @@ constexpr int GM_BM = 128, GM_BN = 128, GM_BK = 64, GM_STAGES = 4;
 constexpr int GM_MAX_HEADS = 2048;      // tiles of a launch whose experts' tiles share expansions (their list sits in shared memory)
 constexpr uint32_t GM_WAIT_LIMIT = 1u << 24;
 constexpr unsigned long long GM_WAIT_NS = 1000000000ull;
+// How the inputs reach shared memory.  IN_LIST: packed rows picked by a list (cp.async by the loader warps); IN_F32: f32 rows,
+// converted by the loaders, whose loads of a whole K step are held in registers meanwhile; IN_TMA: packed rows that follow one
+// another (dense, or sorted by expert), by one thread.
+enum { IN_LIST = 0, IN_F32 = 1, IN_TMA = 2 };
 // One block: PW producer warps, the MMA warp, LW loader warps.  Tensor memory: the accumulators (128 columns per tile of inputs),
-// then the stages' weights (32 columns per term: 64 k values as bf16 pairs).  f32 inputs are converted by the loaders, whose loads
-// of a whole K step are held in registers meanwhile: seven warps of them.
+// then the stages' weights (32 columns per term: 64 k values as bf16 pairs).
 // LAUNCH_REGS: registers a thread at launch (what the launch bounds leave); PREGS, LREGS: of the producers' and of the other
 // warpgroups after the split, whose sum over the block is at most what the launch gave it.
-template <int TERMS, int TT, bool F32>
+template <int TERMS, int TT, int IN>
 struct GmCfg {
-    static constexpr int CTAS = TERMS == 1 && TT == 1 && !F32 ? 2 : 1, PW = TERMS == 3 || CTAS == 2 ? 8 : 16, LW = F32 && TERMS == 1 ? 7 : 3;
+    static constexpr bool F32 = IN == IN_F32;
+    static constexpr int CTAS = TERMS == 1 && TT == 1 && !F32 ? 2 : 1, PW = TERMS == 3 || CTAS == 2 ? 8 : 16, LW = TERMS == 1 && F32 ? 7 : 3;
     static constexpr int WARPS = PW + 1 + LW, THREADS = WARPS * 32, GROUPS = PW / 4;
     static constexpr int ACC = GM_BN * TT, A_COLS = 32 * TERMS, COLS = ACC + GM_STAGES * A_COLS <= 256 ? 256 : 512;
     static constexpr int X_BYTES = TT * GM_BN * GM_BK * 2;      // a stage's inputs
     static constexpr bool SPLIT = TERMS == 1;
-    static constexpr int LAUNCH_REGS = CTAS == 2 || F32 ? 80 : 96, LREGS = F32 ? 64 : 40, PREGS = F32 ? 88 : CTAS == 2 ? 96 : 104;
+    static constexpr int LAUNCH_REGS = CTAS == 1 && LW == 3 ? 96 : 80, LREGS = F32 ? 64 : 40, PREGS = F32 ? 88 : LAUNCH_REGS == 96 ? 104 : 96;
     static_assert(ACC + GM_STAGES * A_COLS <= COLS && CTAS * COLS <= 512, "tensor memory");
     static_assert(!SPLIT || PW * PREGS + (LW + 1) * LREGS <= WARPS * LAUNCH_REGS, "registers");
     static_assert(GM_STAGES >= GROUPS, "every warpgroup owns a stage");
@@ -182,43 +188,67 @@ __device__ __forceinline__ int input_row_of(const MmParams& a, const UnitPos& u,
     const int p = u.start + min(n, u.count - 1);
     return a.grouped ? a.perm[p] / a.xdiv : p;
 }
-// 16-byte unit uu (8 inputs) of row n of a stage: 128-byte swizzle, 16 KB a tile of 128 rows.
+// 16-byte unit uu (8 inputs) of row n of a stage: 128-byte swizzle.
 __device__ __forceinline__ uint32_t input_at(uint32_t stage, int n, int uu) {
-    return stage + (uint32_t) ((n >> 7) * 16384 + (n & 127) * 128 + ((uu ^ (n & 7)) << 4));
+    return stage + (uint32_t) (n * 128 + ((uu ^ (n & 7)) << 4));
+}
+
+// 1 / (1 + e^-g): the hardware's reciprocal and one Newton step (within an ulp; rounded to bf16 by the caller).
+__device__ __forceinline__ float sigmoid(float g) {
+    const float d = 1.0f + fminf(expf(-g), 1e38f);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
 
 // The results of a unit, by the producer warps: warp w reads the tensor memory lanes of its quarter, 16 columns at a time, the
-// warpgroups taking turns.  col: the unit's first column.
+// warpgroups taking turns.  col: the unit's first column.  bf16 results are turned round in 1 KB of shared memory a warp (box), so
+// that a lane stores 16 bytes of one row of outputs: with 2-byte stores straight from the registers the results of a 256-row unit
+// took 8400 clk, a quarter of its expansion.
 template <bool GU, int GROUPS>
-__device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, int col, int start, int count, int r0) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lq = warp & 3, rl = lq * 32 + lane;
-    const int grow = GU ? r0 + (rl >> 1) : r0 + rl;
+__device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, uint16_t* box, int col, int start, int count, int r0) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lq = warp & 3;
+    constexpr int ROWS = GU ? 16 : 32;      // rows of outputs' values a warp makes of its 32 lanes
+    const int row0 = r0 + lq * ROWS;
     for (int c0 = (warp >> 2) * 16; c0 < count; c0 += GROUPS * 16) {
         uint32_t v[16];
-        const int p = start + min(c0 + (lane & 15), count - 1), dst_lane = a.grouped ? a.perm[p] : p;      // lane j: column c0 + j's place
+        const int p = start + min(c0 + (lane & 15), count - 1), dst_lane = a.grouped && !a.out_sorted ? a.perm[p] : p;      // lane j: column c0 + j's place
         tmem_ld16(tmem + ((uint32_t) (lq * 32) << 16) + (uint32_t) (col + c0), v);
-        if (GU) {
+        if (GU || a.out_bf16) {      // (R and ys are multiples of 8 here)
+            if (GU) {
+                uint16_t* const at = box + (lane & 1) * 8 * ROWS + (lane >> 1);      // even lanes finish columns 0..7, odd lanes 8..15
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {      // even lanes finish columns 0..7, odd lanes 8..15
-                const int jj = lane & 1 ? j + 8 : j;
-                const float lo = __uint_as_float(v[j]), hi = __uint_as_float(v[j + 8]);
-                const float from = __shfl_xor_sync(0xFFFFFFFFu, lane & 1 ? lo : hi, 1), mine = lane & 1 ? hi : lo;
-                const int dst = __shfl_sync(0xFFFFFFFFu, dst_lane, jj);
-                const float g = to_bf16(lane & 1 ? from : mine), up = to_bf16(lane & 1 ? mine : from);
-                const float r = to_bf16(g * to_bf16(1.0f / (1.0f + expf(-g)))) * up;
-                if (c0 + jj < count && grow < a.R) ((uint16_t*) a.Y)[(size_t) dst * a.ys + grow] = (uint16_t) bf16x2_bits(r, 0.0f);
+                for (int j = 0; j < 8; ++j) {
+                    const float lo = __uint_as_float(v[j]), hi = __uint_as_float(v[j + 8]);
+                    const float from = __shfl_xor_sync(0xFFFFFFFFu, lane & 1 ? lo : hi, 1), mine = lane & 1 ? hi : lo;
+                    const float g = to_bf16(lane & 1 ? from : mine), up = to_bf16(lane & 1 ? mine : from);
+                    at[j * ROWS] = (uint16_t) bf16x2_bits(to_bf16(g * to_bf16(sigmoid(g))) * up, 0.0f);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint32_t two = bf16x2_bits(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                    box[2 * j * ROWS + lane] = (uint16_t) two;
+                    box[(2 * j + 1) * ROWS + lane] = (uint16_t) (two >> 16);
+                }
             }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < ROWS / 16; ++i) {      // the lane's 8 rows of column c
+                const int e = lane + 32 * i, c = e / (ROWS / 8), r = row0 + (e % (ROWS / 8)) * 8;
+                const int dst = __shfl_sync(0xFFFFFFFFu, dst_lane, c);
+                if (c0 + c < count && r + 8 <= a.R) *(uint4*) ((uint16_t*) a.Y + (size_t) dst * a.ys + r) = *(const uint4*) (box + e * 8);
+            }
+            __syncwarp();
         } else {
+            const int grow = row0 + lane;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 const int dst = __shfl_sync(0xFFFFFFFFu, dst_lane, j);
                 if (c0 + j >= count || grow >= a.R) continue;
                 const float acc = __uint_as_float(v[j]);
-                if (a.out_bf16) ((uint16_t*) a.Y)[(size_t) dst * a.ys + grow] = (uint16_t) bf16x2_bits(acc, 0.0f);
-                else {
-                    float* yo = (float*) a.Y + (size_t) dst * a.ys + grow;
-                    *yo = a.add ? bf16_round(*yo + bf16_round(acc)) : bf16_round(acc);   // engine/kernels_moe.cu:214
-                }
+                float* yo = (float*) a.Y + (size_t) dst * a.ys + grow;
+                *yo = a.add ? bf16_round(*yo + bf16_round(acc)) : bf16_round(acc);   // engine/kernels_moe.cu:214
             }
         }
     }
@@ -226,10 +256,11 @@ __device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, i
 
 // WF: the weights' form.  0: SEED4P4 blocks; 1: stored BF16 values; 2: SEED4 (P = 3) blocks.  TERMS: bf16 terms a weight (1, or 3:
 // exact).  TT: tiles of 128 rows of inputs that share one expansion.  VEC: K a multiple of 64, streams in aligned 16-byte pieces.
-// GU: gate + up + SwiGLU; row i of the gate matrix on lane 2 i, of the up matrix on lane 2 i + 1.  F32: f32 inputs (else packed).
-template <int TERMS, int WF, int TT, bool VEC, bool GU, bool F32>
-__global__ void __launch_bounds__(GmCfg<TERMS, TT, F32>::THREADS, GmCfg<TERMS, TT, F32>::CTAS) seed_gemm_kernel(MmParams a, KConst kc) {
-    using Cfg = GmCfg<TERMS, TT, F32>;
+// GU: gate + up + SwiGLU; row i of the gate matrix on lane 2 i, of the up matrix on lane 2 i + 1.
+template <int TERMS, int WF, int TT, bool VEC, bool GU, int IN>
+__global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT, IN>::CTAS) seed_gemm_kernel(MmParams a, KConst kc, const __grid_constant__ CUtensorMap tm) {
+    using Cfg = GmCfg<TERMS, TT, IN>;
+    constexpr bool F32 = IN == IN_F32;
     constexpr bool BF16W = WF == 1, P3 = WF == 2;
     constexpr int PW = Cfg::PW, GROUPS = Cfg::GROUPS, HALF = Cfg::ACC / 2;
     extern __shared__ uint8_t smem_raw[];
@@ -241,13 +272,14 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, F32>::THREADS, GmCfg<TERMS, T
     __shared__ uint16_t heads[TT > 1 ? GM_MAX_HEADS : 1];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint16_t* const box = (uint16_t*) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023) + GM_STAGES * Cfg::X_BYTES / 2;      // 1 KB a producer warp
     const uint32_t smem_base = smem_u32((uint8_t*) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023));
     const uint32_t bar_full = smem_u32(&bars[0]), bar_empty = bar_full + 8 * GM_STAGES, bar_done = bar_empty + 8 * GM_STAGES, bar_read = bar_done + 8;
     if (!BF16W) load_stream_tab(tab, a.G, tid, Cfg::THREADS);
     if (tid == 0) {
         abort_flag = 0;
         for (int s = 0; s < GM_STAGES; ++s) {
-            mbar_init(bar_full + 8 * s, 4 + Cfg::LW);      // one arrival per warp of the stage's warpgroup and per loader warp
+            mbar_init(bar_full + 8 * s, 4 + (IN == IN_TMA ? 1 : Cfg::LW));      // one arrival per warp of the stage's warpgroup and per loader
             mbar_init(bar_empty + 8 * s, 1);
         }
         mbar_init(bar_done, 1);                            // a unit's MMAs are done
@@ -298,7 +330,7 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, F32>::THREADS, GmCfg<TERMS, T
             ok = __all_sync(0xFFFFFFFFu, ok);
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                unit_results<GU, GROUPS>(a, tmem, p_col, p_start, p_count, p_r0);
+                unit_results<GU, GROUPS>(a, tmem, box + warp * 512, p_col, p_start, p_count, p_r0);
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {
@@ -373,14 +405,14 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, F32>::THREADS, GmCfg<TERMS, T
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_full + 8 * s);
                 cur = nxt;
-                if (p_count) results();      // the previous unit's, under its MMAs' last step
+                if (p_count) results();      // the previous unit's: its last MMAs ran under this step
             }
             if (ok && p_count) results();      // (a unit with fewer steps than warpgroups)
             kr0 += KT;
             ++unit_run;
             p_start = u.start; p_count = u.count; p_r0 = u.r0;
             p_col = u.count <= half_max ? (small_run++ & 1) * HALF : 0;
-            if (ok && u.count > half_max) results();
+            if (ok && KT < GROUPS) results();
         }
         if (ok && p_count) results();
     } else {
@@ -405,18 +437,37 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, F32>::THREADS, GmCfg<TERMS, T
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t sa = tmem_w + (uint32_t) (s * Cfg::A_COLS);
 #pragma unroll 1
-                        for (int tt = 0; tt < TT && tt * GM_BN < u.count; ++tt) {
-                            const uint32_t idesc = umma_idesc((min(u.count - tt * GM_BN, GM_BN) + 15) & ~15);
-                            const uint64_t db = desc0 + (uint64_t) ((s * Cfg::X_BYTES + tt * 16384) >> 4);
+                        for (int n0 = 0; n0 < GM_BN * TT && n0 < u.count; n0 += 256) {      // (the tiles of a stage follow one another)
+                            const uint32_t idesc = umma_idesc((min(u.count - n0, 256) + 15) & ~15);
+                            const uint64_t db = desc0 + (uint64_t) ((s * Cfg::X_BYTES + n0 * 128) >> 4);
 #pragma unroll
                             for (int q = 0; q < TERMS; ++q)
 #pragma unroll
                                 for (int k16 = 0; k16 < GM_BK / 16; ++k16)
-                                    umma_ts(tmem + col + tt * GM_BN, sa + q * 32 + k16 * 8, db + (uint64_t) (k16 * 2), idesc, (kt | q | k16) != 0);
+                                    umma_ts(tmem + col + n0, sa + q * 32 + k16 * 8, db + (uint64_t) (k16 * 2), idesc, (kt | q | k16) != 0);
                         }
                         umma_commit(bar_empty + 8 * s);   // the stage is free when these MMAs have read it
                     }
                     if (ok) umma_commit(bar_done);
+                    kr0 += KT;
+                }
+            }
+        } else if (IN == IN_TMA) {
+            // ---- loader: one thread asks for a K step's inputs, 32 rows at a time (rows beyond the unit's belong to others) ---------------
+            if (tid == (PW + 1) * 32) {
+                for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+                    const UnitPos u = unit_pos<TT, GU>(a, unit, row_tiles, heads);
+                    if (u.count <= 0) continue;
+                    for (int kt = 0; kt < KT && ok; ++kt) {
+                        const int kr = kr0 + kt, s = kr % GM_STAGES;
+                        if (kr >= GM_STAGES && !mbar_wait(bar_empty + 8 * s, ((kr / GM_STAGES) - 1) & 1, &abort_flag)) { fail(4); break; }
+                        const uint32_t bar = bar_full + 8 * s, dst = smem_base + (uint32_t) (s * Cfg::X_BYTES);
+                        asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}"
+                                     ::"r"(bar), "r"((uint32_t) (((u.count + 31) & ~31) * GM_BK * 2)) : "memory");
+                        for (int n = 0; n < u.count; n += 32)
+                            asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                                         ::"r"(dst + n * 128), "l"(&tm), "r"(kt * GM_BK), "r"(u.start + n), "r"(bar) : "memory");
+                    }
                     kr0 += KT;
                 }
             }
@@ -515,19 +566,38 @@ bool launch_bf16_mm_skinny(cudaStream_t s, const WSlice& w, int K, int R, const 
 static int g_exact;   // kc_seed_gemm_f32: process-wide, as the reference's switch (engine/kernels_moe.cu:2354)
 bool seed_gemm_exact() { return g_exact != 0; }
 
-template <int TERMS, int WF, int TT, bool VEC, bool GU, bool F32>
+// The tensor map of packed rows that follow one another: K bf16 values a row, xs apart, boxes of 32 rows x 64 values with the 128-byte
+// swizzle; what lies beyond K or the last row arrives as zeros.
+static bool encode_inputs(CUtensorMap* tm, const MmParams& a) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                               CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* f = NULL;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = NULL;
+        return (Encode) f;
+    }();
+    const cuuint64_t dims[2] = {(cuuint64_t) a.K, (cuuint64_t) (a.grouped ? a.T_in : a.T)}, strides[1] = {(cuuint64_t) a.xs * 2};
+    const cuuint32_t box[2] = {64, 32}, step[2] = {1, 1};
+    return encode && encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a.X), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int TERMS, int WF, int TT, bool VEC, bool GU, int IN>
 static void launch_gemm_v(cudaStream_t s, const MmParams& a, int units) {
-    using Cfg = GmCfg<TERMS, TT, F32>;
-    const size_t smem = (size_t) GM_STAGES * Cfg::X_BYTES + 1024;
+    using Cfg = GmCfg<TERMS, TT, IN>;
+    const size_t smem = (size_t) GM_STAGES * Cfg::X_BYTES + Cfg::PW * 1024 + 1024;
     static bool attr_set[16];
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev & 15]) {
-        cudaFuncSetAttribute(seed_gemm_kernel<TERMS, WF, TT, VEC, GU, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+        cudaFuncSetAttribute(seed_gemm_kernel<TERMS, WF, TT, VEC, GU, IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
         attr_set[dev & 15] = true;
     }
+    CUtensorMap tm = {};
+    if (IN == IN_TMA && !encode_inputs(&tm, a)) { set_error("seed GEMM: no tensor map for packed inputs of row stride %d", a.xs); return; }
     const int slots = sm_count() * Cfg::CTAS;
-    launch(seed_gemm_kernel<TERMS, WF, TT, VEC, GU, F32>, (unsigned) (units < slots ? units : slots), Cfg::THREADS, smem, s, a, kconst());
+    launch(seed_gemm_kernel<TERMS, WF, TT, VEC, GU, IN>, (unsigned) (units < slots ? units : slots), Cfg::THREADS, smem, s, a, kconst(), tm);
     count_launch();
 }
 // How many tiles of a dense call share an expansion: a unit takes the time of its expansion (twice that where two blocks share an
@@ -548,28 +618,28 @@ template <int WF>
 static void launch_gemm_seed(cudaStream_t s, const MmParams& a, int row_tiles, int tiles_y) {
     const int units = row_tiles * tiles_y;
     if (g_exact) {
-        if (a.packed) launch_gemm_v<3, WF, 1, false, false, false>(s, a, units);
-        else if (a.K % 64 == 0) launch_gemm_v<3, WF, 1, true, false, true>(s, a, units);
-        else launch_gemm_v<3, WF, 1, false, false, true>(s, a, units);
+        if (a.packed) launch_gemm_v<3, WF, 1, false, false, IN_LIST>(s, a, units);
+        else if (a.K % 64 == 0) launch_gemm_v<3, WF, 1, true, false, IN_F32>(s, a, units);
+        else launch_gemm_v<3, WF, 1, false, false, IN_F32>(s, a, units);
     } else if (a.K % 64) {
-        if (a.packed) launch_gemm_v<1, WF, 1, false, false, false>(s, a, units);
-        else launch_gemm_v<1, WF, 1, false, false, true>(s, a, units);
+        if (a.packed) launch_gemm_v<1, WF, 1, false, false, IN_LIST>(s, a, units);
+        else launch_gemm_v<1, WF, 1, false, false, IN_F32>(s, a, units);
     } else if (a.grouped) {
-        if (!a.packed) launch_gemm_v<1, WF, 1, true, false, true>(s, a, units);
-        else if (a.offs) launch_gemm_v<1, WF, 3, true, false, false>(s, a, units);
-        else launch_gemm_v<1, WF, 1, true, false, false>(s, a, units);
+        if (!a.packed) launch_gemm_v<1, WF, 1, true, false, IN_F32>(s, a, units);
+        else if (a.in_sorted && a.offs) launch_gemm_v<1, WF, 3, true, false, IN_TMA>(s, a, units);
+        else launch_gemm_v<1, WF, 1, true, false, IN_LIST>(s, a, units);
     } else {
         const int tt = dense_tiles(a, row_tiles), u = row_tiles * ((a.T + GM_BN * tt - 1) / (GM_BN * tt));
-        if (a.packed) { if (tt == 1) launch_gemm_v<1, WF, 1, true, false, false>(s, a, u); else launch_gemm_v<1, WF, 3, true, false, false>(s, a, u); }
-        else if (tt == 1) launch_gemm_v<1, WF, 1, true, false, true>(s, a, u);
-        else if (tt == 2) launch_gemm_v<1, WF, 2, true, false, true>(s, a, u);
-        else launch_gemm_v<1, WF, 3, true, false, true>(s, a, u);
+        if (a.packed) { if (tt == 1) launch_gemm_v<1, WF, 1, true, false, IN_TMA>(s, a, u); else launch_gemm_v<1, WF, 3, true, false, IN_TMA>(s, a, u); }
+        else if (tt == 1) launch_gemm_v<1, WF, 1, true, false, IN_F32>(s, a, u);
+        else if (tt == 2) launch_gemm_v<1, WF, 2, true, false, IN_F32>(s, a, u);
+        else launch_gemm_v<1, WF, 3, true, false, IN_F32>(s, a, u);
     }
 }
 void launch_gemm_gu(cudaStream_t s, const MmParams& a, int tiles_y) {
     const int units = (a.R + GM_BM / 2 - 1) / (GM_BM / 2) * tiles_y;
-    if (a.offs) launch_gemm_v<1, 0, 3, true, true, false>(s, a, units);
-    else launch_gemm_v<1, 0, 1, true, true, false>(s, a, units);
+    if (a.offs) launch_gemm_v<1, 0, 3, true, true, IN_TMA>(s, a, units);
+    else launch_gemm_v<1, 0, 1, true, true, IN_LIST>(s, a, units);
 }
 bool gemm_shares_tiles(int max_tiles) { return max_tiles <= GM_MAX_HEADS; }
 
@@ -591,8 +661,8 @@ void launch_gemm(cudaStream_t s, int fmt, const char* who, MmParams a, int tiles
     if (fmt != MF_BF16 && !g_exact && !a.grouped && a.T <= 64 && smm_serves(a.K, a.X, a.xs, a.packed)) { launch_seed_mma(s, fmt, a, tiles_y); return; }
     const int row_tiles = (a.R + GM_BM - 1) / GM_BM;
     if (fmt == MF_BF16) {      // stored BF16 weights (p[0] = [R][K]): no expansion, one term
-        if (a.packed) launch_gemm_v<1, 1, 1, true, false, false>(s, a, row_tiles * tiles_y);
-        else launch_gemm_v<1, 1, 1, true, false, true>(s, a, row_tiles * tiles_y);
+        if (a.packed) launch_gemm_v<1, 1, 1, true, false, IN_LIST>(s, a, row_tiles * tiles_y);
+        else launch_gemm_v<1, 1, 1, true, false, IN_F32>(s, a, row_tiles * tiles_y);
     } else if (fmt == MF_SEED4) launch_gemm_seed<2>(s, a, row_tiles, tiles_y);
     else launch_gemm_seed<0>(s, a, row_tiles, tiles_y);
 }
@@ -608,29 +678,29 @@ void kc_seed_gemm_f32(int on) { g_exact = on; }
 void kc_mm(cudaStream_t s, int fmt, WSlice w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add,
            const uint32_t* G) {
     if (fmt == MF_BF16 && launch_bf16_mm_skinny(s, w, K, R, x, xs, y, ys, T, add)) return;      // a decode batch (dense_bf16.cu)
-    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, K, R, T, xs, ys, 1, add, 0, 0, NULL, 0, NULL};
+    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, K, R, T, xs, ys, 1, add, 0, 0, NULL, 0, NULL, 0, 0, 0};
     launch_gemm(s, fmt, "kc_mm", a, (T + GM_BN - 1) / GM_BN);
 }
 void kc_mm_packed(cudaStream_t s, int fmt, WSlice w, int K, int R, const uint16_t* x, int xs, float* y, int ys, int T, int add,
                   const uint32_t* G) {
-    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, K, R, T, xs, ys, 1, add, 0, 1, NULL, 0, NULL};
+    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, K, R, T, xs, ys, 1, add, 0, 1, NULL, 0, NULL, 0, 0, 0};
     launch_gemm(s, fmt, "kc_mm_packed", a, (T + GM_BN - 1) / GM_BN);
 }
 void kc_mm_grouped(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys,
                    int xdiv, const int32_t* perm, const MmTile* tiles, int ntiles, const uint32_t* G) {
-    MmParams a = {ws, WSlice{}, x, y, perm, tiles, NULL, G, K, R, 0, xs, ys, xdiv, 0, 1, 0, NULL, 0, NULL};
+    MmParams a = {ws, WSlice{}, x, y, perm, tiles, NULL, G, K, R, 0, xs, ys, xdiv, 0, 1, 0, NULL, 0, NULL, 0, 0, 0};
     launch_gemm(s, fmt, "kc_mm_grouped", a, ntiles);
 }
 void kc_mm_grouped_dev(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys,
                        int xdiv, const int32_t* perm, const MmTile* tiles, const int32_t* ntiles, int max_tiles,
                        const uint32_t* G) {
-    MmParams a = {ws, WSlice{}, x, y, perm, tiles, ntiles, G, K, R, 0, xs, ys, xdiv, 0, 1, 0, NULL, 0, NULL};
+    MmParams a = {ws, WSlice{}, x, y, perm, tiles, ntiles, G, K, R, 0, xs, ys, xdiv, 0, 1, 0, NULL, 0, NULL, 0, 0, 0};
     launch_gemm(s, fmt, "kc_mm_grouped_dev", a, max_tiles);
 }
 void kc_mm_grouped_packed(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const uint16_t* x, int xs, float* y, int ys,
                           int xdiv, const int32_t* perm, const MmTile* tiles, const int32_t* nt, int max_tiles,
                           const uint32_t* G) {
-    MmParams a = {ws, WSlice{}, x, y, perm, tiles, nt, G, K, R, 0, xs, ys, xdiv, 0, 1, 1, NULL, 0, NULL};
+    MmParams a = {ws, WSlice{}, x, y, perm, tiles, nt, G, K, R, 0, xs, ys, xdiv, 0, 1, 1, NULL, 0, NULL, 0, 0, 0};
     launch_gemm(s, fmt, "kc_mm_grouped_packed", a, max_tiles);
 }
 

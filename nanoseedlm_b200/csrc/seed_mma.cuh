@@ -16,11 +16,12 @@ struct MmParams {
     int K, R, T, xs, ys, xdiv, add, grouped, packed;      // T: dense rows; grouped without a device count: the number of tiles
     const WSlice* wu;        // gate + up + SwiGLU (SEED4P4, grouped): the up table (ws: the gate's), Y = packed bf16 [pair][R]
     int out_bf16;
-    const int32_t* offs;     // grouped: the slices' first pairs (kc_bucket's work), or NULL; given: up to three tiles of a slice share an expansion
+    const int32_t* offs;     // grouped: the slices' first pairs (kc_bucket's work), or NULL; given (with in_sorted): up to three tiles of a slice share an expansion
+    int in_sorted, out_sorted, T_in;      // grouped, packed: row n of the inputs (of the outputs) belongs to pair perm[n]; T_in: rows of inputs
 };
 
 bool seed_gemm_exact();      // kc_seed_gemm_f32's switch
-// Gate + up + SwiGLU of a grouped prompt (packed inputs, K a multiple of 64); the GEMM; whether MmParams.offs may be given.
+// Gate + up + SwiGLU of a grouped prompt (packed inputs, sorted where offs is given; K a multiple of 64); the GEMM; whether MmParams.offs may be given.
 void launch_gemm_gu(cudaStream_t s, const MmParams& a, int tiles_y);
 void launch_gemm(cudaStream_t s, int fmt, const char* who, MmParams a, int tiles_y);
 bool gemm_shares_tiles(int max_tiles);
