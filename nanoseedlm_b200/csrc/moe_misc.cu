@@ -10,13 +10,16 @@
 
 namespace nsl {
 
+__device__ __forceinline__ bool aligned16_dev(const void* p) { return ((unsigned long long) p & 15ull) == 0; }
+
 // ---- router ------------------------------------------------------------------------------------------------------------
 // One warp per row (route_row in route.cuh).
 template <int PER>                   // experts per lane held in registers: E <= 32 * PER
 __global__ void __launch_bounds__(128) route_kernel(int E, int k, const float* __restrict__ logits, int ld,
                                                     int32_t* __restrict__ ind, float* __restrict__ wt, int T) {
     const int lane = threadIdx.x & 31, t = blockIdx.x * 4 + (threadIdx.x >> 5);
-    grid_dependents_go();   // a dependent launch of the next kernel may bring its blocks in as these retire
+    grid_dependency_wait();
+    grid_dependents_go();   // only now: the next kernel's blocks would otherwise sit on the SMs the previous one still needs
     if (t >= T) return;
     route_row<PER>(E, k, logits + (size_t) t * ld, lane, ind + (size_t) t * k, wt + (size_t) t * k);
 }
@@ -57,21 +60,31 @@ __global__ void q4_combine_kernel(int d, int k, const float* __restrict__ D, con
 // The same without a shared expert over packed bf16 rows (d a multiple of 8: 16 bytes of each of the k rows a thread).
 __global__ void __launch_bounds__(256) combine_packed_kernel(int d8, int k, const uint4* __restrict__ D, const float* __restrict__ wt,
                                                              float4* __restrict__ out, int n) {
-    grid_dependents_go();
     grid_dependency_wait();
+    grid_dependents_go();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
     const int t = i / d8, c = i - t * d8;
     float a[8] = {};
-    for (int j = 0; j < k; ++j) {
-        const float w = __ldg(wt + t * k + j);
-        const uint4 v = __ldg(D + ((size_t) t * k + j) * d8 + c);
-        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+    for (int j0 = 0; j0 < k; j0 += 8) {      // eight rows requested side by side, added in order
+        uint4 v[8];
+        float w[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            a[2 * q] += w * __uint_as_float(u[q] << 16);
-            a[2 * q + 1] += w * __uint_as_float(u[q] & 0xFFFF0000u);
-        }
+        for (int q = 0; q < 8; ++q)
+            if (j0 + q < k) {
+                v[q] = __ldg(D + ((size_t) t * k + j0 + q) * d8 + c);
+                w[q] = __ldg(wt + t * k + j0 + q);
+            }
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (j0 + q < k) {
+                const uint32_t u[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    a[2 * e] += w[q] * __uint_as_float(u[e] << 16);
+                    a[2 * e + 1] += w[q] * __uint_as_float(u[e] & 0xFFFF0000u);
+                }
+            }
     }
     out[2 * (size_t) i] = make_float4(a[0], a[1], a[2], a[3]);
     out[2 * (size_t) i + 1] = make_float4(a[4], a[5], a[6], a[7]);
@@ -94,6 +107,8 @@ __global__ void moe_combine_kernel(const float* __restrict__ D, const float* __r
 }
 
 __global__ void pack_bf16_kernel(const float* __restrict__ x, uint16_t* __restrict__ y, size_t n) {
+    grid_dependency_wait();
+    grid_dependents_go();
     const size_t n8 = n / 8;
     for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t) gridDim.x * blockDim.x) {
         const float4 a = ((const float4*) x)[2 * i], b = ((const float4*) x)[2 * i + 1];
@@ -110,8 +125,8 @@ __global__ void pack_bf16_kernel(const float* __restrict__ x, uint16_t* __restri
 // Row n of y = row perm[n] / xdiv of x as packed bf16 (d a multiple of 8; a thread: 8 values).
 __global__ void __launch_bounds__(256) pack_sorted_kernel(const float4* __restrict__ x, const int32_t* __restrict__ perm, uint4* __restrict__ y, int xdiv, int d8,
                                                           int P) {
-    grid_dependents_go();
     grid_dependency_wait();
+    grid_dependents_go();
     for (int row = blockIdx.x; row < P; row += gridDim.x) {
         const float4* xp = x + (size_t) (__ldg(perm + row) / xdiv) * d8 * 2;
         for (int c = threadIdx.x; c < d8; c += 256) {
@@ -128,71 +143,95 @@ void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* perm, uin
 
 // ---- grouping ---------------------------------------------------------------------------------------------------------
 // work (2n+3 ints): [0] tile count, [1..n+1] pair offset of each expert, [n+2..2n+2] tile offset of each expert.
-// One block: histogram by shared-memory atomics, then an inclusive scan of pairs and tiles over the experts.
+// One block: histogram by shared-memory atomics, then an exclusive scan of pairs and tiles over the experts (both in one 64-bit
+// word, by warp shuffles: two barriers).
 __global__ void __launch_bounds__(1024) bucket_count_kernel(const int32_t* __restrict__ inds, int count, int n,
                                                             int32_t* __restrict__ work) {
     __shared__ int cnt[BUCKET_MAX_EXPERTS];
-    __shared__ int psum[BUCKET_MAX_EXPERTS], tsum[BUCKET_MAX_EXPERTS];
-    const int tid = threadIdx.x;
+    __shared__ unsigned long long wsum[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     cnt[tid] = 0;
+    grid_dependency_wait();
+    grid_dependents_go();
     __syncthreads();
-    for (int i = tid; i < count; i += 1024) {
-        const int e = inds[i];
-        if (e >= 0 && e < n) atomicAdd(&cnt[e], 1);
-    }
+    auto add = [&](int e) { if (e >= 0 && e < n) atomicAdd(&cnt[e], 1); };
+    const int n4 = aligned16_dev(inds) ? count / 4 : 0;
+    for (int i = tid; i < n4; i += 1024) { const int4 e = ((const int4*) inds)[i]; add(e.x); add(e.y); add(e.z); add(e.w); }
+    for (int i = n4 * 4 + tid; i < count; i += 1024) add(inds[i]);
     __syncthreads();
-    const int c = tid < n ? cnt[tid] : 0;
-    psum[tid] = c;
-    tsum[tid] = (c + MMT_BN - 1) / MMT_BN;
+    const int c = tid < n ? cnt[tid] : 0, tl = (c + MMT_BN - 1) / MMT_BN;
+    const unsigned long long mine = ((unsigned long long) tl << 32) | (unsigned) c;
+    unsigned long long inc = mine;
+    for (int o = 1; o < 32; o <<= 1) { const unsigned long long v = __shfl_up_sync(FULL, inc, o); if (lane >= o) inc += v; }
+    if (lane == 31) wsum[w] = inc;
     __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {   // Hillis-Steele inclusive scan
-        const int pv = tid >= o ? psum[tid - o] : 0, tv = tid >= o ? tsum[tid - o] : 0;
-        __syncthreads();
-        psum[tid] += pv;
-        tsum[tid] += tv;
-        __syncthreads();
-    }
+    const unsigned long long ws = wsum[lane];      // every warp scans the 32 warp sums itself
+    unsigned long long wi = ws;
+    for (int o = 1; o < 32; o <<= 1) { const unsigned long long v = __shfl_up_sync(FULL, wi, o); if (lane >= o) wi += v; }
+    const unsigned long long before = __shfl_sync(FULL, wi - ws, w) + inc - mine, all = __shfl_sync(FULL, wi, 31);
     if (tid < n) {
-        work[1 + tid] = psum[tid] - c;
-        work[2 + n + tid] = tsum[tid] - (c + MMT_BN - 1) / MMT_BN;
+        work[1 + tid] = (int) (unsigned) before;
+        work[2 + n + tid] = (int) (before >> 32);
     }
-    if (tid == n - 1 || (n == 0 && tid == 0)) {
-        work[1 + n] = n ? psum[tid] : 0;
-        work[2 + 2 * n] = n ? tsum[tid] : 0;
-        work[0] = n ? tsum[tid] : 0;
+    if (tid == 0) {
+        work[1 + n] = (int) (unsigned) all;
+        work[2 + 2 * n] = work[0] = (int) (all >> 32);
     }
 }
-// One block per expert.  Each warp owns a contiguous range of the pair list: it counts its matches, the block scans the
-// 32 counts, then each warp writes its matches in order (a ballot prefix), so perm is ascending within the expert.
+// One block per expert.  Each warp owns a contiguous range of the pair list (a multiple of 128, four entries a lane): it counts its
+// matches, the block scans the 32 counts, then each warp writes its matches in order (ballot prefixes), so perm is ascending
+// within the expert.
 __global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* __restrict__ inds, int count,
                                                             const int32_t* __restrict__ work, int32_t* __restrict__ perm,
                                                             MmTile* __restrict__ tiles) {
     __shared__ int wcount[32];
     const int e = blockIdx.x, n = gridDim.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    grid_dependency_wait();
+    grid_dependents_go();
     const int begin = work[1 + e], total = work[2 + e] - begin;
-    if (total > 0) {
-        const int per = ((count + 31) / 32 + 31) & ~31;   // pairs per warp, a multiple of 32
-        const int lo = w * per, hi = lo + per < count ? lo + per : count;
-        int mine = 0;
-        for (int i = lo + lane; i - lane < hi; i += 32) {
-            const bool f = i < hi && inds[i] == e;
-            mine += __popc(__ballot_sync(FULL, f));
+    if (total <= 0) return;
+    const bool vec = aligned16_dev(inds);
+    const int per = ((count + 31) / 32 + 127) & ~127;
+    const int lo = w * per, hi = lo + per < count ? lo + per : count;
+    auto four = [&](int i, bool* f) {      // the lane's entries i .. i + 3
+        if (vec && i + 3 < hi) {
+            const int4 v = __ldg((const int4*) (inds + i));
+            f[0] = v.x == e; f[1] = v.y == e; f[2] = v.z == e; f[3] = v.w == e;
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) f[q] = i + q < hi && __ldg(inds + i + q) == e;
         }
-        if (lane == 0) wcount[w] = mine;
-        __syncthreads();
-        int at = begin;
-        for (int q = 0; q < w; ++q) at += wcount[q];
-        for (int i = lo + lane; i - lane < hi; i += 32) {
-            const bool f = i < hi && inds[i] == e;
-            const uint32_t m = __ballot_sync(FULL, f);
-            if (f) perm[at + __popc(m & ((1u << lane) - 1u))] = i;
-            at += __popc(m);
+    };
+    int mine = 0;
+    for (int i = lo + 4 * lane; i - 4 * lane < hi; i += 128) {
+        bool f[4];
+        four(i, f);
+        mine += (int) f[0] + (int) f[1] + (int) f[2] + (int) f[3];
+    }
+    mine = __reduce_add_sync(FULL, mine);
+    if (lane == 0) wcount[w] = mine;
+    __syncthreads();
+    if (mine) {
+        int at = begin + __reduce_add_sync(FULL, lane < w ? wcount[lane] : 0);
+        const uint32_t below = (1u << lane) - 1u;
+        for (int i = lo + 4 * lane; i - 4 * lane < hi; i += 128) {
+            bool f[4];
+            four(i, f);
+            if (!__any_sync(FULL, f[0] || f[1] || f[2] || f[3])) continue;
+            uint32_t m[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) m[q] = __ballot_sync(FULL, f[q]);
+            int pos = at + __popc(m[0] & below) + __popc(m[1] & below) + __popc(m[2] & below) + __popc(m[3] & below);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (f[q]) perm[pos++] = i + q;
+            at += __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
         }
-        const int t0 = work[2 + n + e];
-        for (int t = tid; t * MMT_BN < total; t += 1024) {
-            MmTile tl = {e, begin + t * MMT_BN, total - t * MMT_BN < MMT_BN ? total - t * MMT_BN : MMT_BN, 0};
-            tiles[t0 + t] = tl;
-        }
+    }
+    const int t0 = work[2 + n + e];
+    for (int t = tid; t * MMT_BN < total; t += 1024) {
+        MmTile tl = {e, begin + t * MMT_BN, total - t * MMT_BN < MMT_BN ? total - t * MMT_BN : MMT_BN, 0};
+        tiles[t0 + t] = tl;
     }
 }
 
@@ -372,6 +411,8 @@ constexpr int BUCKET_SCRATCH_INTS = 2 * BUCKET_MAX_EXPERTS + 3;
 static __device__ __align__(256) int32_t g_bucket_scratch[BUCKET_SCRATCH_INTS];
 
 __global__ void bucket_publish_kernel(const int32_t* __restrict__ work, int32_t* __restrict__ ntiles_out) {
+    grid_dependency_wait();
+    grid_dependents_go();
     if (threadIdx.x == 0 && blockIdx.x == 0) ntiles_out[0] = work[0];
 }
 
@@ -403,9 +444,9 @@ void nsl_route(cudaStream_t s, int n_exp, int top_k, const float* logits, int ld
         return;
     }
     const dim3 grid((unsigned) (T + 3) / 4);
-    if (n_exp <= 128) route_kernel<4><<<grid, 128, 0, s>>>(n_exp, top_k, logits, ld, ind, wt, T);
-    else if (n_exp <= 512) route_kernel<16><<<grid, 128, 0, s>>>(n_exp, top_k, logits, ld, ind, wt, T);
-    else route_kernel<32><<<grid, 128, 0, s>>>(n_exp, top_k, logits, ld, ind, wt, T);
+    if (n_exp <= 128) launch(route_kernel<4>, grid, 128, 0, s, n_exp, top_k, logits, ld, ind, wt, T);
+    else if (n_exp <= 512) launch(route_kernel<16>, grid, 128, 0, s, n_exp, top_k, logits, ld, ind, wt, T);
+    else launch(route_kernel<32>, grid, 128, 0, s, n_exp, top_k, logits, ld, ind, wt, T);
     count_launch();
 }
 void kq4_route_ld(cudaStream_t s, const void* cfg, const float* logits, int ld, int32_t* ind, float* wt, int T) {
@@ -447,14 +488,14 @@ void kc_moe_combine(cudaStream_t s, const float* D, const float* w, const float*
 void kc_pack_input_bf16(cudaStream_t s, const float* x, uint16_t* y, size_t n) {
     if (!n) return;
     const size_t blocks = (n / 8 + 255) / 256 + 1;
-    pack_bf16_kernel<<<(unsigned) (blocks < (size_t) sm_count() * 16 ? blocks : (size_t) sm_count() * 16), 256, 0, s>>>(x, y, n);
+    launch(pack_bf16_kernel, (unsigned) (blocks < (size_t) sm_count() * 16 ? blocks : (size_t) sm_count() * 16), 256, 0, s, x, y, n);
     count_launch();
 }
 
 void kc_bucket(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles) {
     if (n < 1 || n > BUCKET_MAX_EXPERTS) { set_error("kc_bucket: %d experts, at most %d", n, BUCKET_MAX_EXPERTS); return; }
-    bucket_count_kernel<<<1, 1024, 0, s>>>(inds, count, n, ntiles);
-    bucket_place_kernel<<<(unsigned) n, 1024, 0, s>>>(inds, count, ntiles, perm, tiles);
+    launch(bucket_count_kernel, 1, 1024, 0, s, inds, count, n, ntiles);
+    launch(bucket_place_kernel, (unsigned) n, 1024, 0, s, inds, count, (const int32_t*) ntiles, perm, tiles);
     count_launch(2);
 }
 
@@ -466,9 +507,9 @@ void nsl_bucket_noalloc(cudaStream_t s, const int32_t* inds, int count, int n, i
     int32_t* work = bucket_scratch_ptr();
     if (!work) return;
     // every entry the placement reads is rewritten by the count kernel, so nothing has to be cleared between calls
-    bucket_count_kernel<<<1, 1024, 0, s>>>(inds, count, n, work);
-    bucket_place_kernel<<<(unsigned) n, 1024, 0, s>>>(inds, count, work, perm, tiles);
-    bucket_publish_kernel<<<1, 32, 0, s>>>(work, ntiles_out);
+    launch(bucket_count_kernel, 1, 1024, 0, s, inds, count, n, work);
+    launch(bucket_place_kernel, (unsigned) n, 1024, 0, s, inds, count, (const int32_t*) work, perm, tiles);
+    launch(bucket_publish_kernel, 1, 32, 0, s, (const int32_t*) work, ntiles_out);
     count_launch(3);
 }
 
