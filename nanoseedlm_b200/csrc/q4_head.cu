@@ -331,8 +331,8 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
     constexpr int ROW = Q4Ring<4>::ROW, STAGE = Q4Ring<4>::STAGE;
     constexpr int G = 4 * WARPS, KB = 128 * WARPS;      // groups and bytes of codes per row (K = 256 x WARPS)
     extern __shared__ __align__(16) uint32_t q4_smem[];
-    float* part = (float*) q4_smem;                                              // [2][WARPS][32][4]
-    uint32_t* xb = q4_smem + 2 * WARPS * 128;
+    float* part = (float*) q4_smem;                                              // [2 buffers][2 tiles][WARPS][32][4]
+    uint32_t* xb = q4_smem + 4 * WARPS * 128;
     float* xsum = (float*) (xb + (size_t) G * 256);
     // the rings take the place of the staged inputs once those sit in the warps' registers
     unsigned char* ring = (unsigned char*) xb + (size_t) (threadIdx.x >> 5) * NST * STAGE;
@@ -425,51 +425,56 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
 #pragma unroll
     for (int i = 0; i < NST - 1; ++i) issue();
 
+    // Two tiles an iteration: one barrier and one reduction of 256 outputs (a thread each) for both.
     int stage = 0;
-    for (int idx = 0; idx < my_tiles; ++idx) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
-        __syncwarp();
-        const int tile = blockIdx.x + idx * gridDim.x;
-        const unsigned char* st = ring + (size_t) stage * STAGE;
-        stage = stage + 1 == NST ? 0 : stage + 1;
-        const unsigned char* row0 = st + rr * ROW, *row1 = st + (rr + 8) * ROW;
-        const uint4 t0 = *(const uint4*) (row0 + 128), t2 = *(const uint4*) (row1 + 128);      // {4 scales, 4 biases}
-        const uint32_t sa0[2] = {t0.x, t0.y}, ba0[2] = {t0.z, t0.w}, sa1[2] = {t2.x, t2.y}, ba1[2] = {t2.z, t2.w};
-        float out[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int idx = 0; idx < my_tiles; idx += 2) {
+        float* pb = part + (size_t) ((idx >> 1) & 1) * 2 * WARPS * 128;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int sh = (j & 1) * 16;
-            const uint2 w0 = *(const uint2*) (row0 + j * 32 + q * 8), w1 = *(const uint2*) (row1 + j * 32 + q * 8);
-            uint32_t a0[8], a1[8];
-            unpack8(w0.x, a0); unpack8(w0.y, a0 + 4);
-            unpack8(w1.x, a1); unpack8(w1.y, a1 + 4);
-            float c[4];
-            const uint32_t f0[4] = {a0[0], a1[0], a0[4], a1[4]}, f1[4] = {a0[1], a1[1], a0[5], a1[5]};
-            const uint32_t f2[4] = {a0[2], a1[2], a0[6], a1[6]}, f3[4] = {a0[3], a1[3], a0[7], a1[7]};
-            mma_bf16_16x8x16_first(c, f0, breg[j][0], breg[j][1]);
-            mma_bf16_16x8x16(c, f1, breg[j][2], breg[j][3]);
-            mma_bf16_16x8x16(c, f2, breg[j][4], breg[j][5]);
-            mma_bf16_16x8x16(c, f3, breg[j][6], breg[j][7]);
-            const float s0 = bf16_to_f32((uint16_t) (sa0[j >> 1] >> sh)), s1 = bf16_to_f32((uint16_t) (sa1[j >> 1] >> sh));
-            const float e0 = fmaf(8.0f, s0, bf16_to_f32((uint16_t) (ba0[j >> 1] >> sh)));
-            const float e1 = fmaf(8.0f, s1, bf16_to_f32((uint16_t) (ba1[j >> 1] >> sh)));
-            out[0] = fmaf(s0, c[0], fmaf(e0, xg[j][0], out[0]));
-            out[1] = fmaf(s0, c[1], fmaf(e0, xg[j][1], out[1]));
-            out[2] = fmaf(s1, c[2], fmaf(e1, xg[j][0], out[2]));
-            out[3] = fmaf(s1, c[3], fmaf(e1, xg[j][1], out[3]));
+        for (int h = 0; h < 2; ++h) {
+            if (idx + h >= my_tiles) break;
+            asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
+            __syncwarp();
+            const unsigned char* st = ring + (size_t) stage * STAGE;
+            stage = stage + 1 == NST ? 0 : stage + 1;
+            const unsigned char* row0 = st + rr * ROW, *row1 = st + (rr + 8) * ROW;
+            const uint4 t0 = *(const uint4*) (row0 + 128), t2 = *(const uint4*) (row1 + 128);      // {4 scales, 4 biases}
+            const uint32_t sa0[2] = {t0.x, t0.y}, ba0[2] = {t0.z, t0.w}, sa1[2] = {t2.x, t2.y}, ba1[2] = {t2.z, t2.w};
+            float out[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint2 w0 = *(const uint2*) (row0 + j * 32 + q * 8), w1 = *(const uint2*) (row1 + j * 32 + q * 8);
+                uint32_t a0[8], a1[8];
+                unpack8(w0.x, a0); unpack8(w0.y, a0 + 4);
+                unpack8(w1.x, a1); unpack8(w1.y, a1 + 4);
+                float c[4];
+                const uint32_t f0[4] = {a0[0], a1[0], a0[4], a1[4]}, f1[4] = {a0[1], a1[1], a0[5], a1[5]};
+                const uint32_t f2[4] = {a0[2], a1[2], a0[6], a1[6]}, f3[4] = {a0[3], a1[3], a0[7], a1[7]};
+                mma_bf16_16x8x16_first(c, f0, breg[j][0], breg[j][1]);
+                mma_bf16_16x8x16(c, f1, breg[j][2], breg[j][3]);
+                mma_bf16_16x8x16(c, f2, breg[j][4], breg[j][5]);
+                mma_bf16_16x8x16(c, f3, breg[j][6], breg[j][7]);
+                // scale and bias j: the high halves need no shift, only a mask
+                auto val = [&](const uint32_t* v) { return __uint_as_float(j & 1 ? v[j >> 1] & 0xFFFF0000u : v[j >> 1] << 16); };
+                const float s0 = val(sa0), s1 = val(sa1), e0 = fmaf(8.0f, s0, val(ba0)), e1 = fmaf(8.0f, s1, val(ba1));
+                out[0] = fmaf(s0, c[0], fmaf(e0, xg[j][0], out[0]));
+                out[1] = fmaf(s0, c[1], fmaf(e0, xg[j][1], out[1]));
+                out[2] = fmaf(s1, c[2], fmaf(e1, xg[j][0], out[2]));
+                out[3] = fmaf(s1, c[3], fmaf(e1, xg[j][1], out[3]));
+            }
+            __syncwarp();
+            issue();
+            *(float4*) (pb + h * WARPS * 128 + (warp * 32 + lane) * 4) = make_float4(out[0], out[1], out[2], out[3]);
         }
-        __syncwarp();
-        issue();
-        float* pb = part + (size_t) (idx & 1) * WARPS * 128;
-        *(float4*) (pb + (warp * 32 + lane) * 4) = make_float4(out[0], out[1], out[2], out[3]);
-        __syncthreads();      // the block's partial sums of this tile are in; the other buffer is free for the next tile
-        // the tile's 128 outputs (32 lane slots x 4) are shared out over the warps; each is the warps' sum in warp order
-        for (int e = warp * 32 + lane; e < 128; e += 32 * WARPS) {
-            float acc = pb[e];
+        __syncthreads();      // the block's partial sums of these tiles are in; the other buffer is free for the next ones
+        for (int e = threadIdx.x; e < 256; e += 32 * WARPS) {      // each output is the warps' sum in warp order
+            const int h = e >> 7, o = e & 127;
+            if (idx + h >= my_tiles) break;
+            const float* ps = pb + h * WARPS * 128 + o;
+            float acc = ps[0];
 #pragma unroll
-            for (int w = 1; w < WARPS; ++w) acc += pb[w * 128 + e];
-            const int sl = e >> 2, i = e & 3;      // the lane slot (rr, q) and its output i
-            const int row = tile * 16 + (sl >> 2) + (i >> 1) * 8, t = 2 * (sl & 3) + (i & 1);
+            for (int w = 1; w < WARPS; ++w) acc += ps[w * 128];
+            const int sl = o >> 2, i = o & 3;      // the lane slot (rr, q) and its output i
+            const int row = (blockIdx.x + (idx + h) * gridDim.x) * 16 + (sl >> 2) + (i >> 1) * 8, t = 2 * (sl & 3) + (i & 1);
             if (row < R && t < T) {
                 float* yo = y + (size_t) t * ys + row;
                 *yo = add ? bf16_round(*yo + bf16_round(acc)) : bf16_round(acc);
@@ -507,48 +512,104 @@ static void launch_q4_ring(cudaStream_t s, size_t total, int blocks, const WSlic
            (const uint16_t*) w.p[1], (const uint16_t*) w.p[2], K, R, x, xs, y, ys, T, add);
 }
 
-// Greedy arg-max of each row (ties: the lowest id) and, optionally, its softmax probability 1 / sum exp(l - max).
-__global__ void __launch_bounds__(1024) argmax_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, float* __restrict__ prob,
-                                                      int V) {
-    __shared__ float bv[32];
-    __shared__ int bi[32];
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const float* l = logits + (size_t) blockIdx.x * V;
+// Greedy arg-max of each row (ties: the lowest id) and, optionally, its softmax probability 1 / sum exp(l - max).  A row is shared by
+// a cluster of ARG_CTAS blocks, whose candidates meet in the first one's shared memory: one block a row left the chip idle
+// (15.6 us for 8 rows of 151936, a load's latency per 1024 values).
+constexpr int ARG_CTAS = 8, ARG_T = 512;
+
+__device__ __forceinline__ void arg_better(float& v, int& i, float v2, int i2) {
+    if (v2 > v || (v2 == v && i2 < i)) { v = v2; i = i2; }
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of a variable of this block's in block `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t) __cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+
+__global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax_kernel(const float* __restrict__ logits, int32_t* __restrict__ out,
+                                                                                       float* __restrict__ prob, int V) {
+    __shared__ float bv[ARG_T / 32];
+    __shared__ int bi[ARG_T / 32];
+    __shared__ float cv[ARG_CTAS], cs[ARG_CTAS];      // in the first block: the blocks' candidates, their sums
+    __shared__ int ci[ARG_CTAS];
+    __shared__ float row_max;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, rank = blockIdx.x;      // (the grid's x is one cluster)
+    grid_dependents_go();
+    grid_dependency_wait();
+    const float* l = logits + (size_t) blockIdx.y * V;
+    // this block's share: whole 16-byte pieces of the row after its misaligned head, which the first block takes with the tail
+    const int head = min(V, (int) ((4 - (((size_t) (uintptr_t) l >> 2) & 3)) & 3)), n4 = (V - head) / 4;
+    const int lo = (int) ((long long) n4 * rank / ARG_CTAS), hi = (int) ((long long) n4 * (rank + 1) / ARG_CTAS);
+    const float4* l4 = (const float4*) (l + head);
     float best = -INFINITY;
     int idx = 0x7FFFFFFF;
-    for (int i = tid; i < V; i += 1024) {
-        const float v = l[i];
-        if (v > best) { best = v; idx = i; }      // ascending i: the first of equal values stays
+    for (int i = lo + tid; i < hi; i += 4 * ARG_T) {
+        float4 v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (i + q * ARG_T < hi) v[q] = __ldg(l4 + i + q * ARG_T);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (i + q * ARG_T < hi) {      // ascending ids: the first of equal values stays
+                const int e = head + 4 * (i + q * ARG_T);
+                if (v[q].x > best) { best = v[q].x; idx = e; }
+                if (v[q].y > best) { best = v[q].y; idx = e + 1; }
+                if (v[q].z > best) { best = v[q].z; idx = e + 2; }
+                if (v[q].w > best) { best = v[q].w; idx = e + 3; }
+            }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const float b2 = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-        const int i2 = __shfl_xor_sync(0xFFFFFFFFu, idx, o);
-        if (b2 > best || (b2 == best && i2 < idx)) { best = b2; idx = i2; }
-    }
+    const int rest = head + 4 * n4, odd = tid < head ? tid : rest + (tid - head);      // the head's ids, then the tail's
+    if (rank == 0 && odd < V && (tid < head || odd >= rest)) arg_better(best, idx, l[odd], odd);
+    auto block_best = [&]() {
+        for (int o = 16; o > 0; o >>= 1) arg_better(best, idx, __shfl_xor_sync(0xFFFFFFFFu, best, o), __shfl_xor_sync(0xFFFFFFFFu, idx, o));
+    };
+    block_best();
     if (lane == 0) { bv[w] = best; bi[w] = idx; }
     __syncthreads();
     if (w == 0) {
-        best = bv[lane]; idx = bi[lane];
-        for (int o = 16; o > 0; o >>= 1) {
-            const float b2 = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-            const int i2 = __shfl_xor_sync(0xFFFFFFFFu, idx, o);
-            if (b2 > best || (b2 == best && i2 < idx)) { best = b2; idx = i2; }
+        best = lane < ARG_T / 32 ? bv[lane] : -INFINITY;
+        idx = lane < ARG_T / 32 ? bi[lane] : 0x7FFFFFFF;
+        block_best();
+        if (lane == 0) {
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr(&cv[rank], 0)), "f"(best) : "memory");
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(&ci[rank], 0)), "r"(idx) : "memory");
         }
-        if (lane == 0) { out[blockIdx.x] = idx == 0x7FFFFFFF ? 0 : idx; bv[0] = best; }
+    }
+    cluster_sync();
+    if (rank == 0 && w == 0) {
+        best = lane < ARG_CTAS ? cv[lane] : -INFINITY;
+        idx = lane < ARG_CTAS ? ci[lane] : 0x7FFFFFFF;
+        block_best();
+        if (lane == 0) out[blockIdx.y] = idx == 0x7FFFFFFF ? 0 : idx;
+        if (prob && lane < ARG_CTAS) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr(&row_max, lane)), "f"(best) : "memory");
     }
     if (!prob) return;
-    __syncthreads();
-    const float mx = bv[0];
+    cluster_sync();
+    const float mx = row_max;
     float s = 0.0f;
-    for (int i = tid; i < V; i += 1024) s += expf(l[i] - mx);
+    for (int i = lo + tid; i < hi; i += ARG_T) {
+        const float4 v = __ldg(l4 + i);
+        s += (expf(v.x - mx) + expf(v.y - mx)) + (expf(v.z - mx) + expf(v.w - mx));
+    }
+    if (rank == 0 && odd < V && (tid < head || odd >= rest)) s += expf(l[odd] - mx);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    __syncthreads();      // every thread has read bv[0]
+    __syncthreads();      // bv is free again
     if (lane == 0) bv[w] = s;
     __syncthreads();
     if (tid == 0) {
         float tot = 0.0f;
-        for (int i = 0; i < 32; ++i) tot += bv[i];
-        prob[blockIdx.x] = 1.0f / tot;
+        for (int i = 0; i < ARG_T / 32; ++i) tot += bv[i];
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr(&cs[rank], 0)), "f"(tot) : "memory");
+    }
+    cluster_sync();
+    if (rank == 0 && tid == 0) {
+        float tot = 0.0f;
+        for (int i = 0; i < ARG_CTAS; ++i) tot += cs[i];
+        prob[blockIdx.y] = 1.0f / tot;
     }
 }
 
@@ -578,7 +639,7 @@ bool launch_q4_mv(cudaStream_t s, const WSlice& w, int K, int R, const float* x,
         // 8 warps and 6 stages, 49.2 us with two blocks of 4 stages)
         const int warps = K / 256, bps = 16 / warps;
         const size_t rings = (size_t) warps * 4 * Q4Ring<4>::STAGE;
-        const size_t total = (size_t) 2 * warps * 512 + (rings > smem ? rings : smem);
+        const size_t total = (size_t) 4 * warps * 512 + (rings > smem ? rings : smem);
         const int blocks = tiles < bps * sm_count() ? tiles : bps * sm_count();
         if (warps == 4) launch_q4_ksplit<4, 4, 4>(s, total, blocks, w, K, R, x, xs, y, ys, T, add);
         else if (warps == 8) launch_q4_ksplit<8, 4, 2>(s, total, blocks, w, K, R, x, xs, y, ys, T, add);
@@ -618,7 +679,10 @@ extern "C" {
 
 void kc_argmax_p(cudaStream_t s, const float* logits, int32_t* out, float* prob, int V, int n) {
     if (V < 1 || n < 1) return;
-    argmax_kernel<<<(unsigned) n, 1024, 0, s>>>(logits, out, prob, V);
+    for (int n0 = 0; n0 < n; n0 += 65535) {
+        const int m = n - n0 < 65535 ? n - n0 : 65535;
+        launch(argmax_kernel, dim3(ARG_CTAS, (unsigned) m), ARG_T, 0, s, logits + (size_t) n0 * V, out + n0, prob ? prob + n0 : (float*) NULL, V);
+    }
     count_launch();
 }
 
