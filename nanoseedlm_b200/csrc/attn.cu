@@ -35,7 +35,8 @@ constexpr int ATT_KROW = 272;      // bytes of a staged K row (256 + 16: ldmatri
 // banks); at the end the warps' states are merged through the same shared memory.
 constexpr int ATT_MMA_WARPS = 4, ATT_VROW = 272, ATT_MT = 16, ATT_SLOT = ATT_MT * (ATT_KROW + ATT_VROW);
 constexpr int ATT_MAX_ROWS = 1024;      // rows of a step in the balanced form (the reference's rows x splits <= 1024)
-static_assert(2 * ATT_SLOT >= ATT_MAX_GROUP * 130 * 4, "a warp's ring holds its final state");
+constexpr int ATT_Q8_STATE = ATT_MAX_GROUP * 130 * 4;      // bytes of a warp's final state
+static_assert(2 * ATT_SLOT >= ATT_Q8_STATE, "a warp's ring holds its final state");
 static_assert(32 * ATT_MMA_WARPS == ATT_HD && ATT_MMA_WARPS == 4, "the merge gives a thread one dim; ring_sync numbers four rings");
 
 __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
@@ -90,41 +91,16 @@ __device__ __forceinline__ void attn_fill_slot(unsigned char* slot, const KvView
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned) __cvta_generic_to_shared(p); }
 
 // ---- the 8-bit cache (KV_Q8: int8 codes, one f32 scale per row and KV head; engine/kernels_cuda.h:58-59) ------------------
-// A warp's ring holds the raw rows of two steps (16 K rows and 16 V rows of 128 bytes, then their 32 scales); before a step
-// is used its rows are expanded into the one BF16 slot the products read: bf16(code * scale), the value the reference's
-// kernels read (engine/kernels_moe.cu:807-824).
-constexpr int ATT_RAW_V = ATT_MT * ATT_HD, ATT_RAW_SCALES = 2 * ATT_RAW_V, ATT_RAW = ATT_RAW_SCALES + 2 * ATT_MT * 4;
-static_assert(ATT_SLOT + 2 * ATT_RAW <= 2 * ATT_SLOT, "the BF16 slot and two raw slots fit a two-slot ring");
-
-__device__ __forceinline__ void attn_cp4s(unsigned smem, const void* gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem), "l"(gmem) : "memory");
-}
+// A value is bf16(code * scale), what the reference's kernels read (engine/kernels_moe.cu:807-824).
 __device__ __forceinline__ const KvSeg& kv_seg_of(const KvView& kv, int abs_pos, int& row) {
     const bool first = abs_pos < kv.nv;
     row = first ? abs_pos : abs_pos - kv.nv;
     return first ? kv.a : kv.b;
 }
-// The step at key p, raw: 256 pieces of 16 bytes (8 rounds of 32) and 32 scales.
-// Always one cp.async group.
-__device__ __forceinline__ void attn_fill_raw(unsigned char* raw, const KvView& kv, int n_kv, int kvh, int kv0, int p, int p1, int lane) {
-    if (p < p1) {
-        const unsigned base = smem_u32(raw);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int id = i * 32 + lane, is_v = id >> 7, r = (id >> 3) & 15, piece = id & 7;
-            int row;
-            const KvSeg& sg = kv_seg_of(kv, kv0 + min(p + r, p1 - 1), row);
-            attn_cp16s(base + is_v * ATT_RAW_V + r * ATT_HD + piece * 16,
-                       (const unsigned char*) (is_v ? sg.v : sg.k) + ((size_t) row * n_kv + kvh) * ATT_HD + piece * 16);
-        }
-        {
-            const int is_v = lane >> 4, r = lane & 15;
-            int row;
-            const KvSeg& sg = kv_seg_of(kv, kv0 + min(p + r, p1 - 1), row);
-            attn_cp4s(base + ATT_RAW_SCALES + lane * 4, (is_v ? sg.vs : sg.ks) + (size_t) row * n_kv + kvh);
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+__device__ __forceinline__ uint4 ld_stream(const void* p) {      // read once
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
 }
 // The four codes of a word times the row's scale, as two bf16 pairs: byte ^ 0x80 under the exponent of 2^23 is the float
 // 2^23 + 128 + code, one packed subtraction gives the code exactly, one packed product is rounded as the reference's: 11
@@ -139,20 +115,13 @@ __device__ __forceinline__ uint2 q8_four(uint32_t u, u64 s2) {
     unpack2(b, b0, b1);
     return make_uint2(pack_bf16x2(a0, a1), pack_bf16x2(b0, b1));
 }
-// Raw rows -> the BF16 slot (rows 272 bytes apart, K then V).
-__device__ __forceinline__ void attn_expand_raw(unsigned char* slot, const unsigned char* raw, int lane) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int id = i * 32 + lane, is_v = id >> 7, r = (id >> 3) & 15, piece = id & 7;
-        const uint4 u = *(const uint4*) (raw + is_v * ATT_RAW_V + r * ATT_HD + piece * 16);
-        const float sc = *(const float*) (raw + ATT_RAW_SCALES + (is_v * ATT_MT + r) * 4);
-        const u64 s2 = pack2(sc, sc);
-        const uint2 x0 = q8_four(u.x, s2), x1 = q8_four(u.y, s2), x2 = q8_four(u.z, s2), x3 = q8_four(u.w, s2);
-        const uint4 lo = make_uint4(x0.x, x0.y, x1.x, x1.y), hi = make_uint4(x2.x, x2.y, x3.x, x3.y);
-        uint4* dst = (uint4*) (slot + is_v * ATT_MT * ATT_KROW + r * ATT_KROW + piece * 32);
-        dst[0] = lo;
-        dst[1] = hi;
-    }
+// Bytes i of two words times their rows' scales, as a bf16 pair.
+__device__ __forceinline__ uint32_t q8_two(uint32_t x0, uint32_t x1, int i, u64 s2) {      // x: codes ^ 0x80
+    const uint32_t sel = 0x7440u | (uint32_t) i;
+    const u64 a = mul2(add2(pack2(__uint_as_float(__byte_perm(x0, 0x4B000000u, sel)), __uint_as_float(__byte_perm(x1, 0x4B000000u, sel))), pack2(-8388736.0f, -8388736.0f)), s2);
+    float lo, hi;
+    unpack2(a, lo, hi);
+    return pack_bf16x2(lo, hi);
 }
 
 __device__ __forceinline__ void ldsm_x4(uint32_t* r, const unsigned char* p) {
@@ -169,6 +138,105 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {      // an 8 x
     return r;
 }
 
+// One step's scores (two accumulation chains, s and s2) into the running maxima, sums and accumulators, and the weights as the B
+// fragments of the value product, in two bf16 terms.  v0, v1: whether the lane's keys r0 and r0 + 8 exist.
+template <int NT>
+__device__ __forceinline__ void attn_softmax(float (*s)[4], float (*s2)[4], float scale2, bool v0, bool v1, float (*m)[2], float (*l)[2], float (*ot)[8][4],
+                                             uint32_t (*ph)[2], uint32_t (*pl)[2]) {
+    constexpr int DT = 8;
+    // softmax in the base-2 domain: x = score * scale * log2(e); keys r0 (elements 0, 1) and r0 + 8 (2, 3)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        s[nt][0] = v0 ? (s[nt][0] + s2[nt][0]) * scale2 : -INFINITY; s[nt][1] = v0 ? (s[nt][1] + s2[nt][1]) * scale2 : -INFINITY;
+        s[nt][2] = v1 ? (s[nt][2] + s2[nt][2]) * scale2 : -INFINITY; s[nt][3] = v1 ? (s[nt][3] + s2[nt][3]) * scale2 : -INFINITY;
+        float mxa = fmaxf(s[nt][0], s[nt][2]), mxb = fmaxf(s[nt][1], s[nt][3]);
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) {
+            mxa = fmaxf(mxa, __shfl_xor_sync(0xFFFFFFFFu, mxa, off));
+            mxb = fmaxf(mxb, __shfl_xor_sync(0xFFFFFFFFu, mxb, off));
+        }
+        mxa = fmaxf(mxa, m[nt][0]); mxb = fmaxf(mxb, m[nt][1]);      // finite: a step's first key is always valid
+        const float cora = ex2_approx(m[nt][0] - mxa), corb = ex2_approx(m[nt][1] - mxb);
+        m[nt][0] = mxa; m[nt][1] = mxb;
+        s[nt][0] = ex2_approx(s[nt][0] - mxa); s[nt][2] = ex2_approx(s[nt][2] - mxa);
+        s[nt][1] = ex2_approx(s[nt][1] - mxb); s[nt][3] = ex2_approx(s[nt][3] - mxb);
+        l[nt][0] = fmaf(l[nt][0], cora, s[nt][0] + s[nt][2]);
+        l[nt][1] = fmaf(l[nt][1], corb, s[nt][1] + s[nt][3]);
+        if (cora != 1.0f || corb != 1.0f) {      // the running maxima rarely move after a range's first steps
+#pragma unroll
+            for (int i = 0; i < DT; ++i) { ot[nt][i][0] *= cora; ot[nt][i][1] *= corb; ot[nt][i][2] *= cora; ot[nt][i][3] *= corb; }
+        }
+        // the weights as two bf16 terms, hi + lo (16 significant bits): one bf16 term alone moves an output by up to a third
+        // of its own bf16 unit, which after the two roundings of the gate shows as two-unit differences
+        const uint32_t h01 = pack_bf16x2(s[nt][0], s[nt][1]), h23 = pack_bf16x2(s[nt][2], s[nt][3]);
+        const uint32_t l01 = pack_bf16x2(s[nt][0] - bf_lo(h01), s[nt][1] - bf_hi(h01));
+        const uint32_t l23 = pack_bf16x2(s[nt][2] - bf_lo(h23), s[nt][3] - bf_hi(h23));
+        ph[nt][0] = movmatrix_trans(h01); ph[nt][1] = movmatrix_trans(h23);
+        pl[nt][0] = movmatrix_trans(l01); pl[nt][1] = movmatrix_trans(l23);
+    }
+}
+
+// The warps' states (m in base-2 units, l, O^T) through shared memory, STAGE bytes a warp, merged into the group's partials at pp.
+// PAIRED: rows r0 and r0 + 8 of value tile i are dims 16 r0 + 2 i and + 1; otherwise 16 i + r0 and + 8.
+template <int NT, bool PAIRED>
+__device__ __forceinline__ void attn_merge(unsigned char* att_smem, int STAGE, int group, float (*m)[2], float (*l)[2], float (*ot)[8][4], float* pp, size_t head_stride) {
+    constexpr int DT = 8;
+    const int lane = threadIdx.x & 31, q4 = lane & 3, r0 = lane >> 2;
+    float* mine = (float*) (att_smem + (size_t) (threadIdx.x >> 5) * STAGE);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) {
+            l[nt][0] += __shfl_xor_sync(0xFFFFFFFFu, l[nt][0], off);
+            l[nt][1] += __shfl_xor_sync(0xFFFFFFFFu, l[nt][1], off);
+        }
+        float* ha = mine + (8 * nt + 2 * q4) * 130, *hb = ha + 130;
+        if (r0 == 0) {
+            ha[0] = m[nt][0] * 0.69314718055994531f; ha[1] = l[nt][0];
+            hb[0] = m[nt][1] * 0.69314718055994531f; hb[1] = l[nt][1];
+        }
+#pragma unroll
+        for (int i = 0; i < DT; ++i) {
+            if (PAIRED) {
+                *(float2*) (ha + 2 + 16 * r0 + 2 * i) = make_float2(ot[nt][i][0], ot[nt][i][2]);
+                *(float2*) (hb + 2 + 16 * r0 + 2 * i) = make_float2(ot[nt][i][1], ot[nt][i][3]);
+            } else {
+                const int d = 2 + 16 * i + r0;
+                ha[d] = ot[nt][i][0]; hb[d] = ot[nt][i][1]; ha[d + 8] = ot[nt][i][2]; hb[d + 8] = ot[nt][i][3];
+            }
+        }
+    }
+    __syncthreads();
+    // merge the rings' states.  A head's four weights exp(m_ring - max) are the same for all 128 dims: thread h computes
+    // them once (and the head's m and l), then thread d handles dim d of every head.
+    __shared__ float merge_c[ATT_MMA_WARPS][ATT_MAX_GROUP], merge_m[ATT_MAX_GROUP], merge_l[ATT_MAX_GROUP];
+    if (threadIdx.x < group) {
+        const int h = threadIdx.x;
+        float mm = -INFINITY;
+        for (int w = 0; w < ATT_MMA_WARPS; ++w) mm = fmaxf(mm, ((const float*) (att_smem + (size_t) w * STAGE))[h * 130]);
+        float ll = 0.0f;
+        for (int w = 0; w < ATT_MMA_WARPS; ++w) {
+            const float* st = (const float*) (att_smem + (size_t) w * STAGE) + h * 130;
+            const float c = st[0] == -INFINITY ? 0.0f : expf(st[0] - mm);      // a ring without keys: weight 0 (its l and acc are 0)
+            merge_c[w][h] = c;
+            ll = fmaf(st[1], c, ll);
+        }
+        merge_m[h] = mm;
+        merge_l[h] = ll;
+    }
+    __syncthreads();
+    const int d = threadIdx.x;
+    for (int h = 0; h < group; ++h) {
+        float acc = 0.0f;
+#pragma unroll
+        for (int w = 0; w < ATT_MMA_WARPS; ++w) acc = fmaf(((const float*) (att_smem + (size_t) w * STAGE))[h * 130 + 2 + d], merge_c[w][h], acc);
+        float* ph = pp + h * head_stride;
+        if (d == 0) { ph[0] = merge_m[h]; ph[1] = merge_l[h]; }
+        ph[2 + d] = acc;
+    }
+    __syncthreads();
+}
+
 // Keys [p0, p1) of row t's cache for the query heads of KV head kvh, by the whole block: the warps take the steps of 16 keys
 // in turn, merge their states and write the group's partials (m, l, acc[128]) at pp, pp + head_stride, ...
 // NSLOT = slots of a warp's ring (steps in flight + the one in use); NT = tiles of 8 heads (1: groups of <= 8; 2: <= 16).
@@ -178,27 +246,17 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {      // an 8 x
 //                                                          as bf16 pairs, transposed across the warp by movmatrix
 // A lane holds keys r0 and r0 + 8 of heads 2 q4 and 2 q4 + 1 of each tile: the maxima and sums of a head run over the 8
 // lanes of equal q4.  Ends with the block in step (shared memory reusable).
-// SRC: how the rows come.  ATT_SRC_ASYNC: BF16 rows by cp.async; ATT_SRC_Q8: the 8-bit cache (one BF16 slot and two raw slots).
-enum { ATT_SRC_ASYNC = 0, ATT_SRC_Q8 = 2 };
-template <int NSLOT, int NT, int SRC>
-__device__ __forceinline__ void attn_keys(const AttnArgs& a, const float* __restrict__ q, const KvView& kv, int t, int kvh, int kv0,
+template <int NSLOT, int NT>
+__device__ __forceinline__ void attn_keys_bf16(const AttnArgs& a, const float* __restrict__ q, const KvView& kv, int t, int kvh, int kv0,
                                           int p0, int p1, unsigned char* att_smem, float* pp, size_t head_stride) {
     constexpr int STAGE = NSLOT * ATT_SLOT, STRIDE = ATT_MMA_WARPS * ATT_MT;
     const int lane = threadIdx.x & 31, ring_id = threadIdx.x >> 5, q4 = lane & 3, r0 = lane >> 2;
     const int group = a.n_head / a.n_kv;
     unsigned char* stage = att_smem + (size_t) ring_id * STAGE;
-    constexpr bool Q8 = SRC == ATT_SRC_Q8;
     constexpr int DT = 8;      // tiles of 16 dims of the value product
-    static_assert(!Q8 || NSLOT == 2, "the 8-bit cache's ring has two raw slots");
-    unsigned char* raw = stage + ATT_SLOT;      // Q8: the two raw slots behind the BF16 slot
     int p = p0 + ring_id * ATT_MT;
-    if (Q8) {
-        attn_fill_raw(raw, kv, a.n_kv, kvh, kv0, p, p1, lane);
-    } else {
 #pragma unroll
-        for (int i = 0; i < NSLOT - 1; ++i)
-            attn_fill_slot(stage + i * ATT_SLOT, kv, a.n_kv, kvh, kv0, p + i * STRIDE, p1, lane);
-    }
+    for (int i = 0; i < NSLOT - 1; ++i) attn_fill_slot(stage + i * ATT_SLOT, kv, a.n_kv, kvh, kv0, p + i * STRIDE, p1, lane);
     // Q^T as the B fragments of the 8 steps over the 128 dims: column r0 of a tile = head 8 nt + r0 (zero beyond the group);
     // the first rows of K and V fly meanwhile
     uint32_t qb[NT][8][2];
@@ -232,18 +290,10 @@ __device__ __forceinline__ void attn_keys(const AttnArgs& a, const float* __rest
     int cur = 0, nxt = NSLOT - 1;      // the slot in use; the slot the step NSLOT - 1 ahead goes to (its reads ended with the
                                        // previous step's closing ring_sync)
     for (; p < p1; p += STRIDE) {
-        if (Q8) {
-            attn_fill_raw(raw + nxt * ATT_RAW, kv, a.n_kv, kvh, kv0, p + STRIDE, p1, lane);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncwarp();
-            // the BF16 slot's reads ended with the previous step's closing ring_sync
-            attn_expand_raw(stage, raw + cur * ATT_RAW, lane);
-        } else {
-            attn_fill_slot(stage + nxt * ATT_SLOT, kv, a.n_kv, kvh, kv0, p + (NSLOT - 1) * STRIDE, p1, lane);
-            asm volatile("cp.async.wait_group %0;" ::"n"(NSLOT - 1) : "memory");
-        }
+        attn_fill_slot(stage + nxt * ATT_SLOT, kv, a.n_kv, kvh, kv0, p + (NSLOT - 1) * STRIDE, p1, lane);
+        asm volatile("cp.async.wait_group %0;" ::"n"(NSLOT - 1) : "memory");
         __syncwarp();
-        const unsigned char* slot = Q8 ? stage : stage + cur * ATT_SLOT;
+        const unsigned char* slot = stage + cur * ATT_SLOT;
         nxt = cur;
         cur = cur + 1 == NSLOT ? 0 : cur + 1;
         // scores: two accumulation chains a tile (even and odd dim steps)
@@ -257,38 +307,8 @@ __device__ __forceinline__ void attn_keys(const AttnArgs& a, const float* __rest
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) mma_bf16((j & 1) ? s2[nt] : s[nt], ka, qb[nt][j][0], qb[nt][j][1]);
         }
-        // softmax in the base-2 domain: x = score * scale * log2(e); keys r0 (elements 0, 1) and r0 + 8 (2, 3)
-        const bool v0 = p + r0 < p1, v1 = p + r0 + 8 < p1;
         uint32_t ph[NT][2], pl[NT][2];
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            s[nt][0] = v0 ? (s[nt][0] + s2[nt][0]) * scale2 : -INFINITY; s[nt][1] = v0 ? (s[nt][1] + s2[nt][1]) * scale2 : -INFINITY;
-            s[nt][2] = v1 ? (s[nt][2] + s2[nt][2]) * scale2 : -INFINITY; s[nt][3] = v1 ? (s[nt][3] + s2[nt][3]) * scale2 : -INFINITY;
-            float mxa = fmaxf(s[nt][0], s[nt][2]), mxb = fmaxf(s[nt][1], s[nt][3]);
-#pragma unroll
-            for (int off = 4; off < 32; off <<= 1) {
-                mxa = fmaxf(mxa, __shfl_xor_sync(0xFFFFFFFFu, mxa, off));
-                mxb = fmaxf(mxb, __shfl_xor_sync(0xFFFFFFFFu, mxb, off));
-            }
-            mxa = fmaxf(mxa, m[nt][0]); mxb = fmaxf(mxb, m[nt][1]);      // finite: a step's first key is always valid
-            const float cora = ex2_approx(m[nt][0] - mxa), corb = ex2_approx(m[nt][1] - mxb);
-            m[nt][0] = mxa; m[nt][1] = mxb;
-            s[nt][0] = ex2_approx(s[nt][0] - mxa); s[nt][2] = ex2_approx(s[nt][2] - mxa);
-            s[nt][1] = ex2_approx(s[nt][1] - mxb); s[nt][3] = ex2_approx(s[nt][3] - mxb);
-            l[nt][0] = fmaf(l[nt][0], cora, s[nt][0] + s[nt][2]);
-            l[nt][1] = fmaf(l[nt][1], corb, s[nt][1] + s[nt][3]);
-            if (cora != 1.0f || corb != 1.0f) {      // the running maxima rarely move after a range's first steps
-#pragma unroll
-                for (int i = 0; i < DT; ++i) { ot[nt][i][0] *= cora; ot[nt][i][1] *= corb; ot[nt][i][2] *= cora; ot[nt][i][3] *= corb; }
-            }
-            // the weights as two bf16 terms, hi + lo (16 significant bits): one bf16 term alone moves an output by up to a third
-            // of its own bf16 unit, which after the two roundings of the gate shows as two-unit differences
-            const uint32_t h01 = pack_bf16x2(s[nt][0], s[nt][1]), h23 = pack_bf16x2(s[nt][2], s[nt][3]);
-            const uint32_t l01 = pack_bf16x2(s[nt][0] - bf_lo(h01), s[nt][1] - bf_hi(h01));
-            const uint32_t l23 = pack_bf16x2(s[nt][2] - bf_lo(h23), s[nt][3] - bf_hi(h23));
-            ph[nt][0] = movmatrix_trans(h01); ph[nt][1] = movmatrix_trans(h23);
-            pl[nt][0] = movmatrix_trans(l01); pl[nt][1] = movmatrix_trans(l23);
-        }
+        attn_softmax<NT>(s, s2, scale2, p + r0 < p1, p + r0 + 8 < p1, m, l, ot, ph, pl);
         // values: this warp's tiles of 16 dims
 #pragma unroll
         for (int i = 0; i < DT; ++i) {
@@ -303,56 +323,117 @@ __device__ __forceinline__ void attn_keys(const AttnArgs& a, const float* __rest
         __syncwarp();      // this slot's reads are done before a later step refills it
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");      // only empty groups are left
-    // the ring's state into the ring: [16 heads][130] = m (natural units; -inf stays -inf), l, acc (each warp its dims)
     __syncwarp();
-    float* mine = (float*) stage;
+    attn_merge<NT, false>(att_smem, STAGE, group, m, l, ot, pp, head_stride);
+}
+
+// The same over the 8-bit cache, whose rows go from global memory to the fragments without shared memory: a fragment's order along
+// the contraction and the value product's order of dims are free, and the codes are picked one by one anyway.
+//   S^T: lane (r0, q4) owns bytes 16 q4 .. + 15 of both halves of key rows r0 and r0 + 8: word w of them is the A fragment of one
+//        MMA (dims 64 c + 16 q4 + 4 w .. + 3), the queries' B fragments are loaded in that order.
+//   O^T: lane (r0, q4) owns bytes 16 r0 .. + 15 of key rows 2 q4, 2 q4 + 1, 2 q4 + 8, 2 q4 + 9: byte pairs of two rows are the
+//        fragments, value tile i has dims 16 r0 + 2 i (row r0) and + 1 (row r0 + 8).
+// The next step's K rows are requested when this step's are in fragments, V rows likewise.  (Staged through shared memory and
+// expanded there a step took 4500 clk of latency: 26.7 us for 24 rows of 2500..5000 keys, 2 KV heads, 22 % of the HBM peak.)
+template <int NT>
+__device__ __forceinline__ void attn_keys_q8(const AttnArgs& a, const float* __restrict__ q, const KvView& kv, int t, int kvh, int kv0, int p0, int p1,
+                                             unsigned char* att_smem, float* pp, size_t head_stride) {
+    constexpr int STRIDE = ATT_MMA_WARPS * ATT_MT;
+    const int lane = threadIdx.x & 31, q4 = lane & 3, r0 = lane >> 2, group = a.n_head / a.n_kv;
+    uint4 kr[2][2], vr[4];      // [row][half]; [row]
+    float ks[2], vs[4];
+    auto load_k = [&](int p) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            int row;
+            const KvSeg& sg = kv_seg_of(kv, kv0 + min(p + r0 + 8 * i, p1 - 1), row);
+            const size_t at = (size_t) row * a.n_kv + kvh;
+            const unsigned char* src = (const unsigned char*) sg.k + at * ATT_HD + 16 * q4;
+            kr[i][0] = ld_stream(src);
+            kr[i][1] = ld_stream(src + 64);
+            ks[i] = __ldg(sg.ks + at);
+        }
+    };
+    auto load_v = [&](int p) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            int row;
+            const KvSeg& sg = kv_seg_of(kv, kv0 + min(p + 2 * q4 + (i & 1) + (i >> 1) * 8, p1 - 1), row);
+            const size_t at = (size_t) row * a.n_kv + kvh;
+            vr[i] = ld_stream((const unsigned char*) sg.v + at * ATT_HD + 16 * r0);
+            vs[i] = __ldg(sg.vs + at);
+        }
+    };
+    int p = p0 + (int) (threadIdx.x >> 5) * ATT_MT;
+    if (p < p1) { load_k(p); load_v(p); }
+    uint32_t qb[NT][8][2];      // column r0 of a tile = head 8 nt + r0 (zero beyond the group)
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
+        const int head = 8 * nt + r0;
+        const float* qh = q + ((size_t) t * a.n_head + kvh * group + head) * ATT_HD;
 #pragma unroll
-        for (int off = 4; off < 32; off <<= 1) {
-            l[nt][0] += __shfl_xor_sync(0xFFFFFFFFu, l[nt][0], off);
-            l[nt][1] += __shfl_xor_sync(0xFFFFFFFFu, l[nt][1], off);
-        }
-        float* ha = mine + (8 * nt + 2 * q4) * 130, *hb = ha + 130;
-        if (r0 == 0) {
-            ha[0] = m[nt][0] * 0.69314718055994531f; ha[1] = l[nt][0];
-            hb[0] = m[nt][1] * 0.69314718055994531f; hb[1] = l[nt][1];
-        }
-#pragma unroll
-        for (int i = 0; i < DT; ++i) {
-            const int d = 2 + 16 * i + r0;
-            ha[d] = ot[nt][i][0]; hb[d] = ot[nt][i][1]; ha[d + 8] = ot[nt][i][2]; hb[d + 8] = ot[nt][i][3];
+        for (int j = 0; j < 8; ++j) {
+            const float4 x = head < group ? *(const float4*) (qh + 64 * (j >> 2) + 16 * q4 + 4 * (j & 3)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            qb[nt][j][0] = pack_bf16x2(x.x, x.y);
+            qb[nt][j][1] = pack_bf16x2(x.z, x.w);
         }
     }
-    __syncthreads();
-    // merge the rings' states.  A head's four weights exp(m_ring - max) are the same for all 128 dims: thread h computes
-    // them once (and the head's m and l), then thread d handles dim d of every head.
-    __shared__ float merge_c[ATT_MMA_WARPS][ATT_MAX_GROUP], merge_m[ATT_MAX_GROUP], merge_l[ATT_MAX_GROUP];
-    if (threadIdx.x < group) {
-        const int h = threadIdx.x;
-        float mm = -INFINITY;
-        for (int w = 0; w < ATT_MMA_WARPS; ++w) mm = fmaxf(mm, ((const float*) (att_smem + (size_t) w * STAGE))[h * 130]);
-        float ll = 0.0f;
-        for (int w = 0; w < ATT_MMA_WARPS; ++w) {
-            const float* st = (const float*) (att_smem + (size_t) w * STAGE) + h * 130;
-            const float c = st[0] == -INFINITY ? 0.0f : expf(st[0] - mm);      // a ring without keys: weight 0 (its l and acc are 0)
-            merge_c[w][h] = c;
-            ll = fmaf(st[1], c, ll);
-        }
-        merge_m[h] = mm;
-        merge_l[h] = ll;
-    }
-    __syncthreads();
-    const int d = threadIdx.x;
-    for (int h = 0; h < group; ++h) {
-        float acc = 0.0f;
+    float m[NT][2], l[NT][2], ot[NT][8][4];
 #pragma unroll
-        for (int w = 0; w < ATT_MMA_WARPS; ++w) acc = fmaf(((const float*) (att_smem + (size_t) w * STAGE))[h * 130 + 2 + d], merge_c[w][h], acc);
-        float* ph = pp + h * head_stride;
-        if (d == 0) { ph[0] = merge_m[h]; ph[1] = merge_l[h]; }
-        ph[2 + d] = acc;
+    for (int nt = 0; nt < NT; ++nt) {
+        m[nt][0] = m[nt][1] = -INFINITY;
+        l[nt][0] = l[nt][1] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ot[nt][i][0] = ot[nt][i][1] = ot[nt][i][2] = ot[nt][i][3] = 0.0f;
     }
-    __syncthreads();
+    const float scale2 = a.scale * 1.4426950408889634f;
+    for (; p < p1; p += STRIDE) {
+        float s[NT][4], s2[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = s2[nt][0] = s2[nt][1] = s2[nt][2] = s2[nt][3] = 0.0f;
+        const u64 ka = pack2(ks[0], ks[0]), kb = pack2(ks[1], ks[1]);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const uint32_t wa[4] = {kr[0][c].x, kr[0][c].y, kr[0][c].z, kr[0][c].w}, wb[4] = {kr[1][c].x, kr[1][c].y, kr[1][c].z, kr[1][c].w};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const uint2 fa = q8_four(wa[w], ka), fb = q8_four(wb[w], kb);
+                const uint32_t f[4] = {fa.x, fb.x, fa.y, fb.y};
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) mma_bf16((w & 1) ? s2[nt] : s[nt], f, qb[nt][4 * c + w][0], qb[nt][4 * c + w][1]);
+            }
+        }
+        if (p + STRIDE < p1) load_k(p + STRIDE);
+        uint32_t ph[NT][2], pl[NT][2];
+        attn_softmax<NT>(s, s2, scale2, p + r0 < p1, p + r0 + 8 < p1, m, l, ot, ph, pl);
+        const u64 va = pack2(vs[0], vs[1]), vb = pack2(vs[2], vs[3]);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            uint32_t x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = (w == 0 ? vr[i].x : w == 1 ? vr[i].y : w == 2 ? vr[i].z : vr[i].w) ^ 0x80808080u;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t f[4] = {q8_two(x[0], x[1], 2 * h, va), q8_two(x[0], x[1], 2 * h + 1, va), q8_two(x[2], x[3], 2 * h, vb), q8_two(x[2], x[3], 2 * h + 1, vb)};
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    mma_bf16(ot[nt][2 * w + h], f, ph[nt][0], ph[nt][1]);
+                    mma_bf16(ot[nt][2 * w + h], f, pl[nt][0], pl[nt][1]);
+                }
+            }
+        }
+        if (p + STRIDE < p1) load_v(p + STRIDE);
+    }
+    attn_merge<NT, true>(att_smem, ATT_Q8_STATE, group, m, l, ot, pp, head_stride);
+}
+
+// SRC: the cache's form.
+enum { ATT_SRC_BF16 = 0, ATT_SRC_Q8 = 2 };
+template <int NSLOT, int NT, int SRC>
+__device__ __forceinline__ void attn_keys(const AttnArgs& a, const float* __restrict__ q, const KvView& kv, int t, int kvh, int kv0, int p0, int p1,
+                                          unsigned char* att_smem, float* pp, size_t head_stride) {
+    if (SRC == ATT_SRC_Q8) attn_keys_q8<NT>(a, q, kv, t, kvh, kv0, p0, p1, att_smem, pp, head_stride);
+    else attn_keys_bf16<NSLOT, NT>(a, q, kv, t, kvh, kv0, p0, p1, att_smem, pp, head_stride);
 }
 
 // One block per (split, KV head, row): the split's keys as the reference cuts them.
@@ -430,7 +511,7 @@ __device__ __forceinline__ AttnPlan attn_plan(const RowInfo* __restrict__ ri, in
 }
 
 template <int NSLOT, int NT, int SRC>
-__global__ void __launch_bounds__(32 * ATT_MMA_WARPS, NT == 2 && SRC == ATT_SRC_Q8 ? 2 : 3)      // three blocks an SM: <= 168 / 85 registers
+__global__ void __launch_bounds__(32 * ATT_MMA_WARPS, 3)      // (8-bit cache, four blocks of 128 registers: 26.2 us where three take 25.7)
 attn_flat_mma_kernel(AttnArgs a, const float* __restrict__ q, KvView kv, const RowInfo* __restrict__ ri, float* __restrict__ part, int T) {
     extern __shared__ __align__(16) unsigned char att_smem[];
     __shared__ int pre[ATT_MAX_ROWS + 1];
@@ -538,7 +619,7 @@ static int attn_sm_count() {
 template <int NT, int SRC>
 static void launch_attn_flat(cudaStream_t s, int n_blocks, const AttnArgs& a, const float* q, const KvView& kv, const RowInfo* ri, float* part, int T) {
     static bool done[16];
-    constexpr int SMEM = ATT_MMA_WARPS * 2 * ATT_SLOT;
+    constexpr int SMEM = ATT_MMA_WARPS * (SRC == ATT_SRC_Q8 ? ATT_Q8_STATE : 2 * ATT_SLOT);
     attn_smem_attr(attn_flat_mma_kernel<2, NT, SRC>, SMEM, done);
     launch(attn_flat_mma_kernel<2, NT, SRC>, dim3((unsigned) n_blocks), 32 * ATT_MMA_WARPS, (size_t) SMEM, s, a, q, kv, ri, part, T);
 }
@@ -546,7 +627,7 @@ static void launch_attn_flat(cudaStream_t s, int n_blocks, const AttnArgs& a, co
 template <int NT, int SRC>
 static void launch_attn_split(cudaStream_t s, const AttnArgs& a, const float* q, const KvView& kv, const RowInfo* ri, float* part, int T) {
     static bool done[16];
-    constexpr int SMEM = ATT_MMA_WARPS * 2 * ATT_SLOT;
+    constexpr int SMEM = ATT_MMA_WARPS * (SRC == ATT_SRC_Q8 ? ATT_Q8_STATE : 2 * ATT_SLOT);
     attn_smem_attr(attn_split_mma_kernel<2, NT, SRC>, SMEM, done);
     launch(attn_split_mma_kernel<2, NT, SRC>, dim3((unsigned) a.n_splits, (unsigned) a.n_kv, (unsigned) T), 32 * ATT_MMA_WARPS, (size_t) SMEM, s,
            a, q, kv, ri, part);
@@ -577,16 +658,16 @@ void kc_attn(cudaStream_t s, AttnArgs a, const float* q, KvView kv, const RowInf
     const bool flat = !g_attn_invariant && a.n_splits >= 3 && a.chunk > 0 && T <= ATT_MAX_ROWS;
     int n_blocks = 0;
     if (flat) {
-        n_blocks = 3 * attn_sm_count();      // three blocks with two-slot rings (70 KB of shared memory) fit an SM
+        n_blocks = 3 * attn_sm_count();      // as many as fit (BF16: two-slot rings, 70 KB of shared memory a block; 168 registers)
         if (q8 && group <= 8) launch_attn_flat<1, ATT_SRC_Q8>(s, n_blocks, a, q, kv, ri, part, T);
         else if (q8) launch_attn_flat<2, ATT_SRC_Q8>(s, n_blocks, a, q, kv, ri, part, T);
-        else if (group <= 8) launch_attn_flat<1, ATT_SRC_ASYNC>(s, n_blocks, a, q, kv, ri, part, T);
-        else launch_attn_flat<2, ATT_SRC_ASYNC>(s, n_blocks, a, q, kv, ri, part, T);
+        else if (group <= 8) launch_attn_flat<1, ATT_SRC_BF16>(s, n_blocks, a, q, kv, ri, part, T);
+        else launch_attn_flat<2, ATT_SRC_BF16>(s, n_blocks, a, q, kv, ri, part, T);
     } else {
         if (q8 && group <= 8) launch_attn_split<1, ATT_SRC_Q8>(s, a, q, kv, ri, part, T);
         else if (q8) launch_attn_split<2, ATT_SRC_Q8>(s, a, q, kv, ri, part, T);
-        else if (group <= 8) launch_attn_split<1, ATT_SRC_ASYNC>(s, a, q, kv, ri, part, T);
-        else launch_attn_split<2, ATT_SRC_ASYNC>(s, a, q, kv, ri, part, T);
+        else if (group <= 8) launch_attn_split<1, ATT_SRC_BF16>(s, a, q, kv, ri, part, T);
+        else launch_attn_split<2, ATT_SRC_BF16>(s, a, q, kv, ri, part, T);
     }
     PdlScope chain(true);      // the reduction's blocks come in while the first pass drains
     launch(attn_reduce_kernel, dim3((unsigned) a.n_head, (unsigned) T), ATT_HD, 0, s, a, (const float*) part, g, o, ri, T, n_blocks);
