@@ -71,8 +71,8 @@ struct UnitArgs {
     int eba, ebb;
     float* y;
     int ys, R, raw, add;
-    int pid[4];                           // the unit's pairs (output rows)
-    int s_lo, s_hi, lpr_log2;
+    int pid[2];                           // the unit's pairs (output rows)
+    int st, s_hi, lpr_log2, buf;          // the warp's first step; which of the two staged units this is
 };
 __device__ __forceinline__ Chunk load_chunk3(const uint4* s, const uint4* c, const uint32_t* d, size_t chunk_index) {
     Chunk k;
@@ -231,36 +231,91 @@ __device__ __forceinline__ void chunk_dots(const StreamTab& tab, const KConst& k
     }
 }
 
-// The row steps [s_lo, s_hi) of one pair that fall to this warp (every MV_WARPS-th), for rows of 2^j <= 32 chunks: a step = the
-// 32 / lpr rows a warp expands at once, a lane owning one chunk of its row.  ka / kb: the first step's streams, requested by
-// the caller before the inputs were staged; the next ones are requested before the current ones are expanded.
+// Butterfly sums of N values over the lpr lanes of a row (distance lpr / 2 first), each finished by lpr / N lanes only: at the first
+// distances a lane sends the values it will not finish and keeps the others.  Returns the sum of value jc / (lpr / N), bit for
+// bit what a whole butterfly gives, for 5 (N = 2) or 6 (N = 4) shuffles at 32 lanes instead of 5 N.
+template <int N>
+__device__ __forceinline__ float split_sum(const float* v, int lpr, int jc) {
+    int o = lpr >> 1;
+    float a[2] = {v[0], v[1]};
+    if (N == 4) {
+        const bool up = jc & o;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float keep = up ? v[N - 2 + i] : v[i], send = up ? v[i] : v[N - 2 + i];
+            a[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, o);
+        }
+        o >>= 1;
+    }
+    const bool up = jc & o;
+    float m = (up ? a[1] : a[0]) + __shfl_xor_sync(0xFFFFFFFFu, up ? a[0] : a[1], o);
+    for (o >>= 1; o > 0; o >>= 1) m += __shfl_xor_sync(0xFFFFFFFFu, m, o);
+    return m;
+}
+
+// Rows of 2^j = 2 .. 32 chunks: a row step = the 32 / lpr rows a warp expands at once, a lane owning one chunk of its row; the
+// steps [s_lo, s_hi) of a pair go to the block's warps in turn.  A warp takes two rows of streams at a time against the same
+// inputs (an ITEM): a row of the gate and of the up matrix, or two of its steps of the one matrix.
+template <int MODE>
+struct RowItem {
+    static constexpr int STEPS = MODE == MODE_GU ? 1 : 2;      // row steps of the warp an item takes
+};
+// An item's streams: its first step st, row r.
+template <int MODE, int PF>
+__device__ __forceinline__ void load_item(const WSlice& wa, const WSlice& wb, int st, int r, int s_hi, int R, int lpr_log2, int jc, Chunk& ka, Chunk& kb) {
+    const int S = MV_WARPS * (32 >> lpr_log2);
+    if (st < s_hi && r < R) {
+        ka = load_chunk<PF>(wa, (size_t) ((r << lpr_log2) + jc));
+        if (MODE == MODE_GU) kb = load_chunk<PF>(wb, (size_t) ((r << lpr_log2) + jc));
+    }
+    if (MODE != MODE_GU && st + MV_WARPS < s_hi && r + S < R) kb = load_chunk<PF>(wa, (size_t) (((r + S) << lpr_log2) + jc));
+}
+// The items of one pair that fall to this warp, whose first step is st.  ka / kb: the first item's streams, requested by the caller before the inputs were
+// staged; the next ones are requested before the current ones are expanded.  The sums stay in the lanes that finish them until
+// every lane has one: SwiGLU, rounding and stores then run once for lpr / 2 items (once an item, with one lane in work, they
+// and the reductions took 17 of 90 instructions a block).
 // store(r, s, su): row r's sum (and the up matrix's).
 template <int MODE, int PF, typename Store>
 __device__ __forceinline__ void pair_rows(const StreamTab& tab, const KConst& kc, const WSlice& wa, const WSlice& wb, const ulonglong2* sx,
-                                          int lpr_log2, int R, int s_lo, int s_hi, Chunk ka, Chunk kb, Store store) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
-    const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
+                                          int lpr_log2, int R, int st, int s_hi, Chunk ka, Chunk kb, Store store) {
+    constexpr int STEPS = RowItem<MODE>::STEPS;
+    const int lane = threadIdx.x & 31;
+    const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2, S = MV_WARPS * rpw, h = lpr >> 1;
+    const int jc = lane & (lpr - 1), slot = jc & (h - 1);
+    const bool upper = jc & h;
     const float sca = slice_scale(wa.eb + (8 - PF)), scb = slice_scale(wb.eb + (8 - PF));      // P = 3 products are half as large
     const ulonglong2* cx = sx + jc * CX;
-    int st = s_lo + warp, r = st * rpw + ro;
-    for (; st < s_hi; st += MV_WARPS, r += MV_WARPS * rpw) {
-        const bool ok = r < R;
-        const int rn = r + MV_WARPS * rpw;
-        Chunk na, nb;
-        if (st + MV_WARPS < s_hi && rn < R) {
-            na = load_chunk<PF>(wa, (size_t) rn * lpr + jc);
-            if (MODE == MODE_GU) nb = load_chunk<PF>(wb, (size_t) rn * lpr + jc);
+    int r = st * rpw + (lane >> lpr_log2), cnt = 0;
+    float keep = 0.0f;
+    auto flush = [&](int st0, int r0) {      // the kept items' results; st0, r0: the first one's
+        if (MODE == MODE_GU) {
+            const float su = __shfl_xor_sync(0xFFFFFFFFu, keep, h);
+            const int row = r0 + slot * S;
+            if (!upper && slot < cnt && row < R) store(row, keep * sca, su * scb);
+        } else {
+            const int e = 2 * slot + (upper ? 1 : 0), row = r0 + e * S;
+            if (slot < cnt && st0 + e * MV_WARPS < s_hi && row < R) store(row, keep * sca, 0.0f);
         }
-        u64 acc = 0ull, accu = 0ull;
-        if (ok) chunk_dots<MODE, PF>(tab, kc, ka, kb, cx, acc, accu);
-        const float s = group_sum(pair_total(acc), lpr) * sca;
-        float su = 0.0f;
-        if (MODE == MODE_GU) su = group_sum(pair_total(accu), lpr) * scb;
-        if (ok && jc == 0) store(r, s, su);
+    };
+    for (; st < s_hi; st += STEPS * MV_WARPS, r += STEPS * S) {
+        Chunk na, nb;
+        load_item<MODE, PF>(wa, wb, st + STEPS * MV_WARPS, r + STEPS * S, s_hi, R, lpr_log2, jc, na, nb);
+        u64 acc[2] = {0ull, 0ull};
+        if (r < R) {
+            if (MODE == MODE_GU || st + MV_WARPS < s_hi) chunk_dots<MODE_GU, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);
+            else chunk_dots<MODE_ROUND, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);
+        }
+        const float v[2] = {pair_total(acc[0]), pair_total(acc[1])};
+        const float mine = split_sum<2>(v, lpr, jc);
+        if (slot == cnt) keep = mine;
+        if (++cnt == h) {
+            flush(st - (h - 1) * STEPS * MV_WARPS, r - (h - 1) * STEPS * S);
+            cnt = 0;
+        }
         ka = na;
-        if (MODE == MODE_GU) kb = nb;
+        kb = nb;
     }
+    if (cnt) flush(st - cnt * STEPS * MV_WARPS, r - cnt * STEPS * S);
 }
 
 // The same for rows of any number of chunks: a row is cut into groups of lpr chunks, an ITEM is one group of the 32 / lpr rows of
@@ -363,6 +418,16 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_pair_kernel(MvParams a, KCon
     const long long begin = (long long) blockIdx.x * total / gridDim.x, end = (long long) (blockIdx.x + 1) * total / gridDim.x;
     if (begin >= end) return;
     const int p_first = (int) (begin / rs), p_last = (int) ((end - 1) / rs);
+    auto stage = [&](int pair, int buf) {
+        const void* row = input_row(a, a.xrow ? a.xrow[pair] : pair / a.xdiv);
+        ulonglong2* sx = pair_sx + (size_t) buf * ch * CX;
+        for (int i = threadIdx.x; i < ch * 4; i += MV_THREADS) {
+            float x[16];
+            stage_load(row, a.xbf16, i >> 2, i & 3, x);
+            stage_store<PF>(x, i >> 2, i & 3, sx);
+        }
+    };
+    int turn = 0;      // steps of the block so far: the warps' round-robin goes on from one pair to the next
     for (int pair = p_first; pair <= p_last; ++pair) {
         const int s_lo = pair == p_first ? (int) (begin - (long long) pair * rs) : 0;
         const int s_hi = pair == p_last ? (int) (end - (long long) pair * rs) : rs;
@@ -371,24 +436,27 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_pair_kernel(MvParams a, KCon
         WSlice wb = wa;
         if (MODE == MODE_GU) wb = a.wu[slice];
         // this warp's first streams are requested before the inputs are staged: their DRAM latency runs under it
-        const int st = s_lo + (MULTI ? warp / sh.groups : warp), r = st * rpw + (lane >> sh.lpr_log2);
+        const int st = s_lo + (MULTI ? warp / sh.groups : (warp - turn) & (MV_WARPS - 1)), r = st * rpw + (lane >> sh.lpr_log2);
         const int jc = (lane & (lpr - 1)) + (MULTI ? warp % sh.groups * lpr : 0);
         Chunk ka, kb;
-        if (st < s_hi && r < a.R && (!MULTI || jc < ch)) {
+        if (!MULTI) load_item<MODE, PF>(wa, wb, st, r, s_hi, a.R, sh.lpr_log2, jc, ka, kb);
+        else if (st < s_hi && r < a.R && jc < ch) {
             ka = load_chunk<PF>(wa, (size_t) r * ch + jc);
             if (MODE == MODE_GU) kb = load_chunk<PF>(wb, (size_t) r * ch + jc);
         }
-        if (pair != p_first) __syncthreads();   // the previous pair's inputs are no longer read
-        const void* row = input_row(a, a.xrow ? a.xrow[pair] : pair / a.xdiv);
-        for (int i = threadIdx.x; i < ch * 4; i += MV_THREADS) {
-            float x[16];
-            stage_load(row, a.xbf16, i >> 2, i & 3, x);
-            stage_store<PF>(x, i >> 2, i & 3, pair_sx);
+        // inputs of two pairs at a time (a share of a short list has no more): a warp that is done with the first goes on to the
+        // second by itself
+        const int buf = MULTI ? 0 : (pair - p_first) & 1;
+        if (buf == 0) {
+            if (pair != p_first) __syncthreads();   // the previous pairs' inputs are no longer read
+            stage(pair, 0);
+            if (!MULTI && pair < p_last) stage(pair + 1, 1);
+            __syncthreads();   // inputs staged (and, for the block's first pair, the stream table loaded)
         }
-        __syncthreads();   // inputs staged (and, for the block's first pair, the stream table loaded)
         auto store = [&](int rr, float s, float su) { store_out<MODE>(a, pair, rr, s, su); };
         if constexpr (MULTI) pair_items<MODE, PF>(tab, kc, wa, wb, pair_sx, part, sh, a.R, s_lo, s_hi, ka, kb, store);
-        else pair_rows<MODE, PF>(tab, kc, wa, wb, pair_sx, sh.lpr_log2, a.R, s_lo, s_hi, ka, kb, store);
+        else pair_rows<MODE, PF>(tab, kc, wa, wb, pair_sx + (size_t) buf * ch * CX, sh.lpr_log2, a.R, st, s_hi, ka, kb, store);
+        turn += s_hi - s_lo;
     }
 }
 
@@ -486,10 +554,7 @@ __device__ __forceinline__ void step_phase(const StepParams& p, const KConst& kc
         int st = s_lo + warp;
         int r = st * rpw + ro;
         Chunk ka, kb;
-        if (st < s_hi && r < R) {      // the streams do not depend on other blocks: requested before any wait
-            ka = load_chunk<4>(wa, (size_t) r * lpr + jc);
-            if (MODE == MODE_GU) kb = load_chunk<4>(wb, (size_t) r * lpr + jc);
-        }
+        load_item<MODE, 4>(wa, wb, st, r, s_hi, R, lpr_log2, jc, ka, kb);      // the streams do not depend on other blocks: requested before any wait
         if (MODE == MODE_ROUND && threadIdx.x == 0 && !step_wait(p.sy.ready + pair, rs_gu, p.sy.status)) sh.abort = 1;
         __syncthreads();   // the previous pair's inputs are no longer read; the wait's outcome is known
         if (sh.abort) return;
@@ -500,7 +565,7 @@ __device__ __forceinline__ void step_phase(const StepParams& p, const KConst& kc
             stage_store<4>(x, threadIdx.x >> 2, threadIdx.x & 3, sh.sx);
         }
         __syncthreads();
-        pair_rows<MODE, 4>(sh.tab, kc, wa, wb, sh.sx, lpr_log2, R, s_lo, s_hi, ka, kb,
+        pair_rows<MODE, 4>(sh.tab, kc, wa, wb, sh.sx, lpr_log2, R, st, s_hi, ka, kb,
                                   [&](int rr, float s, float su) { store_out<MODE>(a, pair, rr, s, su); });
         // this block's row steps of the pair are stored: publish their number
         __threadfence();
@@ -578,7 +643,7 @@ struct GrpShared {
     uint32_t key[GRP_MAX_PAIRS];                  // sorted (slice << 10 | pair)
     int32_t prefix[GRP_MAX_PAIRS + 1];            // weight of the units that start before sorted position i
     uint32_t tmp[GRP_SMALL];                      // short lists: unsorted keys, then unit weights
-    __align__(16) ulonglong2 sx[GRP_NT][GRP_SX];
+    __align__(16) ulonglong2 sx[2 * GRP_NT][GRP_SX];      // two units
 };
 
 
@@ -655,51 +720,59 @@ __device__ __noinline__ void unit_rows(UnitArgs ua, Chunk ka, Chunk kb) {
     extern __shared__ __align__(16) unsigned char grp_smem[];
     const GrpShared& sh = *reinterpret_cast<const GrpShared*>(grp_smem);
     const KConst& kc = c_kc;
-    const int s_lo = ua.s_lo, s_hi = ua.s_hi, lpr_log2 = ua.lpr_log2;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int s_hi = ua.s_hi, lpr_log2 = ua.lpr_log2;
+    const int lane = threadIdx.x & 31;
     const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
+    const ulonglong2 (*sx)[GRP_SX] = sh.sx + ua.buf * GRP_NT;
     const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
     if (NT == 1) {      // one pair: the pair kernel's loop
         WSlice wa = {}, wb = {};
         wa.p[0] = ua.sa; wa.p[1] = ua.ca; wa.p[3] = ua.da; wa.eb = ua.eba;
         wb.p[0] = ua.sb; wb.p[1] = ua.cb; wb.p[3] = ua.db; wb.eb = ua.ebb;
-        pair_rows<MODE, 4>(sh.tab, kc, wa, wb, sh.sx[0], lpr_log2, ua.R, s_lo, s_hi, ka, kb,
+        pair_rows<MODE, 4>(sh.tab, kc, wa, wb, sx[0], lpr_log2, ua.R, ua.st, s_hi, ka, kb,
                                   [&](int r, float s, float su) { store_unit<MODE>(ua, ua.pid[0], r, s, su); });
         return;
     }
-    const float sca = slice_scale(ua.eba + 4), scb = slice_scale(ua.ebb + 4);
+    // two pairs: each item's four sums (pair 0: A, B; pair 1: A, B) end in a quarter of the row's lanes each
+    static_assert(NT <= 2, "units of one or two pairs");
+    constexpr int STEPS = RowItem<MODE>::STEPS;
+    const float sca = slice_scale(ua.eba + 4), scb = slice_scale((MODE == MODE_GU ? ua.ebb : ua.eba) + 4);
     const ulonglong2* cx[NT];
 #pragma unroll
-    for (int t = 0; t < NT; ++t) cx[t] = sh.sx[t] + jc * CX;
-    int st = s_lo + warp, r = st * rpw + ro;
-    for (; st < s_hi; st += MV_WARPS, r += MV_WARPS * rpw) {
-        const bool ok = r < ua.R;
-        const int rn = r + MV_WARPS * rpw;
-        const bool more = st + MV_WARPS < s_hi && rn < ua.R;
-        u64 acc[NT], accu[NT];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) acc[t] = accu[t] = 0ull;
-        // a matrix's streams for the next step are requested as soon as this step has used them up, into the registers they
-        // leave free, so no second set of stream registers is held
+    for (int t = 0; t < NT; ++t) cx[t] = sx[t] + jc * CX;
+    const int S = MV_WARPS * rpw, h = lpr >> 2, slot = jc & (h - 1), part = jc >> (lpr_log2 - 2);
+    const int pid = part & 2 ? ua.pid[1] : ua.pid[0];
+    int st = ua.st, r = st * rpw + ro, cnt = 0;
+    float keep = 0.0f;
+    auto flush = [&](int st0, int r0) {
         if (MODE == MODE_GU) {
-            if (ok) unit_chunk<NT>(sh.tab, kc, ka, cx, acc);
-            if (more) ka = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) rn * lpr + jc);
-            if (ok) unit_chunk<NT>(sh.tab, kc, kb, cx, accu);
-            if (more) kb = load_chunk3(ua.sb, ua.cb, ua.db, (size_t) rn * lpr + jc);
-        } else {      // one matrix: its next streams are requested before this step's expansion (a second set of registers)
-            Chunk na;
-            if (more) na = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) rn * lpr + jc);
-            if (ok) unit_chunk<NT>(sh.tab, kc, ka, cx, acc);
-            ka = na;
+            const float su = __shfl_xor_sync(0xFFFFFFFFu, keep, h);
+            const int row = r0 + slot * S;
+            if (!(part & 1) && slot < cnt && row < ua.R) store_unit<MODE>(ua, pid, row, keep * sca, su * scb);
+        } else {
+            const int e = 2 * slot + (part & 1), row = r0 + e * S;
+            if (slot < cnt && st0 + e * MV_WARPS < s_hi && row < ua.R) store_unit<MODE>(ua, pid, row, keep * sca, 0.0f);
         }
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            const float s = group_sum(pair_total(acc[t]), lpr) * sca;
-            float su = 0.0f;
-            if (MODE == MODE_GU) su = group_sum(pair_total(accu[t]), lpr) * scb;
-            if (ok && jc == 0) store_unit<MODE>(ua, ua.pid[t], r, s, su);
+    };
+    for (; st < s_hi; st += STEPS * MV_WARPS, r += STEPS * S) {
+        // the next item's streams are requested as soon as this item's have been used up, into the registers they leave free
+        u64 acc[2] = {0ull, 0ull}, accb[2] = {0ull, 0ull};
+        const bool ok = r < ua.R, okb = ok && (MODE == MODE_GU || st + MV_WARPS < s_hi);
+        const int sn = st + STEPS * MV_WARPS, rn = r + STEPS * S;
+        if (ok) unit_chunk<NT>(sh.tab, kc, ka, cx, acc);
+        if (sn < s_hi && rn < ua.R) ka = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) ((rn << lpr_log2) + jc));
+        if (okb) unit_chunk<NT>(sh.tab, kc, kb, cx, accb);
+        if (MODE == MODE_GU) { if (sn < s_hi && rn < ua.R) kb = load_chunk3(ua.sb, ua.cb, ua.db, (size_t) ((rn << lpr_log2) + jc)); }
+        else if (sn + MV_WARPS < s_hi && rn + S < ua.R) kb = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) (((rn + S) << lpr_log2) + jc));
+        const float v[4] = {pair_total(acc[0]), pair_total(accb[0]), pair_total(acc[1]), pair_total(accb[1])};
+        const float mine = split_sum<4>(v, lpr, jc);
+        if (slot == cnt) keep = mine;
+        if (++cnt == h) {
+            flush(st - (h - 1) * STEPS * MV_WARPS, r - (h - 1) * STEPS * S);
+            cnt = 0;
         }
     }
+    if (cnt) flush(st - cnt * STEPS * MV_WARPS, r - cnt * STEPS * S);
 }
 
 // Ascending bitonic sort of n (a power of two) keys in shared memory by the whole block.
@@ -820,60 +893,46 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_grp_kernel(MvParams a, KCons
     int u_first, s_first, u_last, s_last;
     locate(begin, u_first, s_first);
     if (end >= total) { u_last = P; s_last = 0; } else locate(end, u_last, s_last);
-    bool staged = false;
-    for (int u = u_first; u <= u_last && u < P;) {
-        int n = 1, pid[GRP_NT], slice = 0;
-#pragma unroll
-        for (int t = 0; t < GRP_NT; ++t) pid[t] = u;
-        if (grouped) {
-            const int w = sh.prefix[u + 1] - sh.prefix[u];
-            n = w == GRP_W[1] ? 1 : w == GRP_W[2] ? 2 : w == GRP_W[3] ? 3 : 4;
-#pragma unroll
-            for (int t = 0; t < GRP_NT; ++t) pid[t] = (int) (sh.key[u + (t < n ? t : 0)] & 1023u);
-            slice = (int) (sh.key[u] >> 10);
-        } else slice = a.sel ? a.sel[u] : 0;
-        const int s_lo = u == u_first ? s_first : 0, s_hi = u == u_last ? s_last : rs;
-        if (s_lo < s_hi) {
-            // Two chains of dependent loads start here and run side by side: pair -> input row -> inputs (this thread's share of
-            // the staging, held in registers), and slice -> stream addresses -> this warp's first streams.
-            const int per = lpr * 4, n_stage = n * per;
-            float xin[16];
-            int e0 = threadIdx.x, t0 = e0 / per, rem0 = e0 - t0 * per;
-            if (e0 < n_stage) {
-                const int p = grouped ? (int) (sh.key[u + t0] & 1023u) : u;
-                stage_load(input_row(a, a.xrow ? a.xrow[p] : p / a.xdiv), a.xbf16, rem0 >> 2, rem0 & 3, xin);
-            }
-            const WSlice wa = a.ws ? a.ws[slice] : a.w0;
-            WSlice wb = wa;
-            if (MODE == MODE_GU) wb = a.wu[slice];
-            const int st0 = s_lo + warp, r0 = st0 * rpw + ro;
-            Chunk ka, kb;
-            if (st0 < s_hi && r0 < a.R) {
-                ka = load_chunk(wa, (size_t) r0 * lpr + jc);
-                if (MODE == MODE_GU) kb = load_chunk(wb, (size_t) r0 * lpr + jc);
-            }
-            if (staged) __syncthreads();   // the previous unit's inputs are no longer read
-            staged = true;
-            if (e0 < n_stage) stage_store<4>(xin, rem0 >> 2, rem0 & 3, sh.sx[t0]);
-            for (int i = threadIdx.x + MV_THREADS; i < n_stage; i += MV_THREADS) {      // units of more than two pairs
-                const int t = i / per, rem = i - t * per;
-                const int p = grouped ? (int) (sh.key[u + t] & 1023u) : u;
-                stage_load(input_row(a, a.xrow ? a.xrow[p] : p / a.xdiv), a.xbf16, rem >> 2, rem & 3, xin);
-                stage_store<4>(xin, rem >> 2, rem & 3, sh.sx[t]);
-            }
-            __syncthreads();
-            UnitArgs ua;
-            ua.sa = (const uint4*) wa.p[0]; ua.ca = (const uint4*) wa.p[1]; ua.da = (const uint32_t*) wa.p[3]; ua.eba = wa.eb;
-            ua.sb = (const uint4*) wb.p[0]; ua.cb = (const uint4*) wb.p[1]; ua.db = (const uint32_t*) wb.p[3]; ua.ebb = wb.eb;
-            ua.y = a.y; ua.ys = a.ys; ua.R = a.R; ua.raw = a.raw; ua.add = a.add;
-#pragma unroll
-            for (int t = 0; t < 4; ++t) ua.pid[t] = pid[t < GRP_NT ? t : 0];
-            ua.s_lo = s_lo; ua.s_hi = s_hi; ua.lpr_log2 = lpr_log2;
-            if (GRP_NT >= 4 && n == 4) unit_rows<MODE, GRP_NT >= 4 ? 4 : 1>(ua, ka, kb);
-            else if (GRP_NT >= 3 && n == 3) unit_rows<MODE, GRP_NT >= 3 ? 3 : 1>(ua, ka, kb);
-            else if (GRP_NT >= 2 && n == 2) unit_rows<MODE, GRP_NT >= 2 ? 2 : 1>(ua, ka, kb);
-            else unit_rows<MODE, 1>(ua, ka, kb);
+    auto unit_size = [&](int u) { return grouped && sh.prefix[u + 1] - sh.prefix[u] != GRP_W[1] ? 2 : 1; };
+    auto pair_of = [&](int u, int t) { return grouped ? (int) (sh.key[u + t] & 1023u) : u; };
+    const int per = lpr * 4;
+    auto stage_unit = [&](int u, int n, int buf) {      // the inputs of unit u's n pairs
+        for (int i = threadIdx.x; i < n * per; i += MV_THREADS) {
+            const int t = i >= per, rem = i - (t ? per : 0), p = pair_of(u, t);
+            float x[16];
+            stage_load(input_row(a, a.xrow ? a.xrow[p] : p / a.xdiv), a.xbf16, rem >> 2, rem & 3, x);
+            stage_store<4>(x, rem >> 2, rem & 3, sh.sx[buf * GRP_NT + t]);
         }
+    };
+    int turn = 0, buf = 0;      // steps of the block so far (the warps' round-robin goes on from unit to unit); units are staged two at a time
+    if (u_first < P && s_first >= rs) { u_first += unit_size(u_first); s_first = 0; }
+    for (int u = u_first; u < P && (u < u_last || (u == u_last && s_last > 0));) {
+        const int n = unit_size(u), slice = grouped ? (int) (sh.key[u] >> 10) : (a.sel ? a.sel[u] : 0);
+        const int s_lo = u == u_first ? s_first : 0, s_hi = u == u_last ? s_last : rs;
+        const WSlice wa = a.ws ? a.ws[slice] : a.w0;
+        WSlice wb = wa;
+        if (MODE == MODE_GU) wb = a.wu[slice];
+        const int st0 = s_lo + ((warp - turn) & (MV_WARPS - 1)), r0 = st0 * rpw + ro;
+        Chunk ka, kb;
+        load_item<MODE, 4>(wa, wb, st0, r0, s_hi, a.R, lpr_log2, jc, ka, kb);      // under the staging
+        if (buf == 0) {
+            if (turn) __syncthreads();   // the previous units' inputs are no longer read
+            stage_unit(u, n, 0);
+            const int un = u + n;
+            if (un < P && (un < u_last || (un == u_last && s_last > 0))) stage_unit(un, unit_size(un), 1);
+            __syncthreads();
+        }
+        UnitArgs ua;
+        ua.sa = (const uint4*) wa.p[0]; ua.ca = (const uint4*) wa.p[1]; ua.da = (const uint32_t*) wa.p[3]; ua.eba = wa.eb;
+        ua.sb = (const uint4*) wb.p[0]; ua.cb = (const uint4*) wb.p[1]; ua.db = (const uint32_t*) wb.p[3]; ua.ebb = wb.eb;
+        ua.y = a.y; ua.ys = a.ys; ua.R = a.R; ua.raw = a.raw; ua.add = a.add;
+        ua.pid[0] = pair_of(u, 0);
+        ua.pid[1] = pair_of(u, n - 1);
+        ua.st = st0; ua.s_hi = s_hi; ua.lpr_log2 = lpr_log2; ua.buf = buf;
+        if (n == 2) unit_rows<MODE, 2>(ua, ka, kb);
+        else unit_rows<MODE, 1>(ua, ka, kb);
+        turn += s_hi - s_lo;
+        buf ^= 1;
         u += n;
     }
 }
@@ -1116,7 +1175,7 @@ static RowShape item_shape(int ch) {
 template <int MODE, int PF>
 static void launch_pair(cudaStream_t s, const MvParams& a, const RouteFuse& rf) {
     const int ch = a.K / 64;
-    if (ch <= 32 && (ch & (ch - 1)) == 0) launch_pair_v<MODE, PF, false>(s, a, RowShape{ch, log2_floor(ch), 0, 1}, rf, staged_bytes(ch));
+    if (ch >= 2 && ch <= 32 && (ch & (ch - 1)) == 0) launch_pair_v<MODE, PF, false>(s, a, RowShape{ch, log2_floor(ch), 0, 1}, rf, 2 * staged_bytes(ch));
     else launch_pair_v<MODE, PF, true>(s, a, item_shape(ch), rf, staged_bytes(ch));
     count_launch();
 }
@@ -1193,7 +1252,7 @@ static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse&
         if (dense) { launch_dense<PF>(s, a, T); return; }
     }
     if constexpr (PF == 4) {
-        if (a.P > GRP_MIN_PAIRS && !rf.logits && ch <= 32 && (ch & (ch - 1)) == 0) { launch_grp<MODE>(s, a, log2_floor(ch)); return; }
+        if (a.P > GRP_MIN_PAIRS && !rf.logits && ch >= 4 && ch <= 32 && (ch & (ch - 1)) == 0) { launch_grp<MODE>(s, a, log2_floor(ch)); return; }
     }
     launch_pair<MODE, PF>(s, a, rf);
 }
@@ -1202,7 +1261,7 @@ static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse&
 static bool launch_mv_step(cudaStream_t s, const StepParams& p) {
     const int cd = p.d / 64, cf = p.ff / 64;
     if (p.T < 1 || p.T > MV_MAXT || p.top_k < 1 || p.top_k > 32 || p.T * p.top_k > 256 || p.n_exp < p.top_k || p.n_exp > 32 * ROUTE_PER_LANE) return false;
-    if (p.d % 64 || p.ff % 64 || cd < 1 || cf < 1 || (cd & (cd - 1)) || (cf & (cf - 1)) || cd > 32 || cf > 32) return false;
+    if (p.d % 64 || p.ff % 64 || cd < 2 || cf < 2 || (cd & (cd - 1)) || (cf & (cf - 1)) || cd > 32 || cf > 32) return false;
     if (!aligned16(p.x) || p.xs % 4 || !aligned16(p.A) || !aligned16(p.D)) return false;
     launch(mv_step_kernel, sm_count() * 2, MV_THREADS, 0, s, p, kconst(), log2_floor(cd), log2_floor(cf));
     count_launch();
