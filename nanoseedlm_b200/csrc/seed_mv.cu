@@ -375,21 +375,172 @@ __device__ __forceinline__ void pair_items(const StreamTab& tab, const KConst& k
     }
 }
 
-// ---- one expansion per pair, inputs in shared memory, two blocks of 8 warps per SM ----------------------------------------
-// Any row of whole chunks.  The pair's inputs sit in shared memory; a thread fits in 128 registers and 16 warps per SM hide
-// the logic pipe's latencies.  The work is the pair-major sequence of row steps (pair_rows); blocks take contiguous equal
-// shares of it, inside a pair the block's warps take its steps round-robin.
+// The router in a kernel's prologue: warp t picks token t's top-k experts; block 0 also stores ids and weights for the kernels that
+// follow.  Ends with a barrier.
+__device__ __forceinline__ void route_prologue(const RouteFuse& rf, int32_t* r_ind, float* r_wt) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < rf.T) {
+        const float* l = rf.logits + (size_t) warp * rf.ld;
+        if (rf.n_exp <= 128) route_row<4>(rf.n_exp, rf.top_k, l, lane, r_ind + warp * rf.top_k, r_wt + warp * rf.top_k);
+        else if (rf.n_exp <= 512) route_row<16>(rf.n_exp, rf.top_k, l, lane, r_ind + warp * rf.top_k, r_wt + warp * rf.top_k);
+        else route_row<32>(rf.n_exp, rf.top_k, l, lane, r_ind + warp * rf.top_k, r_wt + warp * rf.top_k);
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && (int) threadIdx.x < rf.T * rf.top_k) {
+        rf.ind_out[threadIdx.x] = r_ind[threadIdx.x];
+        rf.wt_out[threadIdx.x] = r_wt[threadIdx.x];
+    }
+}
+
+// ---- one expansion per pair, inputs in shared memory, one block of 16 warps per SM -----------------------------------------
+// Rows of 2 .. 32 chunks (a power of two).  The work is the pair-major sequence of items (RowItem); blocks take contiguous equal
+// shares of it, and a block's warps fetch its items one by one from a counter in shared memory: the schedulers favour some warps,
+// and with items dealt in advance the favoured ones left the others alone for the last third of the launch (13.5 of 16 warps
+// active on average).  Inputs, stream addresses and scales of up to PAIR_WIN pairs are staged at a time.
 // Bound: the logic pipe (38 LOP3 + 4 PRMT + 2 SHF a block of 8 weights) together with the register file's read ports (a packed
 // multiply-add reads three register pairs, three cycles alone, 2.4 with one of them shared by neighbours): the arithmetic
-// alone runs at 0.875 clk a block and SM (256 threads x 2 blocks, a loop without streams).
+// alone runs at 0.875 clk a block and SM (16 warps, a loop without streams).
 // Optionally the block first ROUTES: with logits given, warp t picks token t's top-k experts (route.cuh) and the pair
-// list is the T * top_k (token, expert) pairs; block 0 also stores ids and weights for the kernels that follow.
+// list is the T * top_k (token, expert) pairs.
 // PF: coefficients per block.  4: SEED4P4; 3: SEED4 (24 states, the nibble word).
-template <int MODE, int PF, bool MULTI>
-__global__ void __launch_bounds__(MV_THREADS, 2) mv_pair_kernel(MvParams a, KConst kc, RowShape sh, RouteFuse rf) {
+constexpr int PAIR_WARPS = 16, PAIR_THREADS = 32 * PAIR_WARPS, PAIR_WIN = 8;
+
+struct PairDesc {      // what an item needs of its pair
+    const void *sa, *ca, *da, *sb, *cb, *db;
+    float sca, scb;
+    int pair, pad;
+};
+
+template <int MODE, int PF>
+__global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KConst kc, int lpr_log2, int win, RouteFuse rf) {
+    extern __shared__ __align__(16) ulonglong2 pair_sx[];      // [win][lpr * CX]
+    __shared__ StreamTab tab;
+    __shared__ int32_t r_ind[256];   // the fused router's picks
+    __shared__ float r_wt[256];
+    __shared__ PairDesc desc[PAIR_WIN];
+    __shared__ int next_item;
+    constexpr int STEPS = RowItem<MODE>::STEPS;
+    load_stream_tab(tab, a.G, threadIdx.x, PAIR_THREADS);
+    grid_dependents_go();
+    grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2, h = lpr >> 1;
+    const int jc = lane & (lpr - 1), ro = lane >> lpr_log2, slot = jc & (h - 1);
+    const bool upper = jc & h;
+    int P = a.count ? min(*a.count, a.P) : a.P;
+    if (rf.logits) {
+        route_prologue(rf, r_ind, r_wt);
+        P = rf.T * rf.top_k;
+    }
+    const int rs = (a.R + rpw - 1) / rpw, ips = (rs + STEPS - 1) / STEPS;      // row steps, items of a pair
+    const long long total = (long long) P * ips;
+    const long long begin = (long long) blockIdx.x * total / gridDim.x, end = (long long) (blockIdx.x + 1) * total / gridDim.x;
+    if (begin >= end) return;
+    const float inv = 1.0f / (float) ips;
+    const ulonglong2* const cx0 = pair_sx + jc * CX;
+    for (int p0 = (int) (begin / ips); (long long) p0 * ips < end; p0 += win) {
+        // items of this window, counted from pair p0's first: [lo, hi)
+        const int lo = (int) (begin - (long long) p0 * ips > 0 ? begin - (long long) p0 * ips : 0);
+        const int hi = (int) (end - (long long) p0 * ips < (long long) win * ips ? end - (long long) p0 * ips : (long long) win * ips);
+        const int np = (hi + ips - 1) / ips;
+        __syncthreads();      // the previous window is no longer read
+        if ((int) threadIdx.x < np) {
+            const int pair = p0 + threadIdx.x, slice = rf.logits ? r_ind[pair] : (a.sel ? a.sel[pair] : 0);
+            const WSlice wa = a.ws ? a.ws[slice] : a.w0;
+            PairDesc d = {wa.p[0], wa.p[1], wa.p[3], NULL, NULL, NULL, slice_scale(wa.eb + (8 - PF)), 0.0f, pair, 0};      // P = 3 products are half as large
+            if (MODE == MODE_GU) {
+                const WSlice wb = a.wu[slice];
+                d.sb = wb.p[0]; d.cb = wb.p[1]; d.db = wb.p[3];
+                d.scb = slice_scale(wb.eb + (8 - PF));
+            }
+            desc[threadIdx.x] = d;
+        }
+        if (threadIdx.x == PAIR_THREADS - 1) next_item = lo + PAIR_WARPS;
+        for (int i = threadIdx.x; i < np * lpr * 4; i += PAIR_THREADS) {
+            const int t = i >> (lpr_log2 + 2), e = i - (t << (lpr_log2 + 2)), pair = p0 + t;
+            float x[16];
+            stage_load(input_row(a, a.xrow ? a.xrow[pair] : pair / a.xdiv), a.xbf16, e >> 2, e & 3, x);
+            stage_store<PF>(x, e >> 2, e & 3, pair_sx + (size_t) t * lpr * CX);
+        }
+        __syncthreads();      // (and, the first time, the stream table is loaded)
+        auto locate = [&](int it, int& t, int& r) {      // item -> its pair in the window, this lane's first row
+            t = (int) ((float) it * inv);
+            if (t * ips > it) --t;
+            if ((t + 1) * ips <= it) ++t;
+            r = (it - t * ips) * (STEPS * rpw) + ro;
+        };
+        auto load = [&](int it, Chunk& ka, Chunk& kb) {
+            int t, r;
+            locate(it, t, r);
+            if (it >= hi || r >= a.R) return;
+            const PairDesc& d = desc[t];
+            const uint32_t at = (uint32_t) ((r << lpr_log2) + jc);
+            ka.s = __ldg((const uint4*) d.sa + at);
+            ka.c = __ldg((const uint4*) d.ca + at);
+            if (PF == 4) ka.cd = __ldg((const uint32_t*) d.da + at);
+            if (MODE == MODE_GU) {
+                kb.s = __ldg((const uint4*) d.sb + at);
+                kb.c = __ldg((const uint4*) d.cb + at);
+                if (PF == 4) kb.cd = __ldg((const uint32_t*) d.db + at);
+            } else if (r + rpw < a.R) {
+                kb.s = __ldg((const uint4*) d.sa + at + 32);      // the next row step: 32 chunks on
+                kb.c = __ldg((const uint4*) d.ca + at + 32);
+                if (PF == 4) kb.cd = __ldg((const uint32_t*) d.da + at + 32);
+            }
+        };
+        // The sums stay in the lanes that finish them until every lane has one: SwiGLU, rounding and stores then run once for
+        // lpr / 2 items (once an item, with one lane in work, they and the reductions took 17 of 90 instructions a block).
+        float keep = 0.0f;
+        int kept = -1, cnt = 0;      // kept: the item's number
+        auto flush = [&]() {
+            int t, r;
+            locate(kept < 0 ? lo : kept, t, r);
+            const PairDesc& d = desc[t];
+            if (MODE == MODE_GU) {
+                const float su = __shfl_xor_sync(0xFFFFFFFFu, keep, h);
+                if (!upper && kept >= 0 && r < a.R) store_out<MODE>(a, d.pair, r, keep * d.sca, su * d.scb);
+            } else {
+                r += upper ? rpw : 0;
+                if (kept >= 0 && r < a.R) store_out<MODE>(a, d.pair, r, keep * d.sca, 0.0f);
+            }
+            kept = -1;
+            cnt = 0;
+        };
+        int it = lo + warp;
+        Chunk ka, kb;
+        load(it, ka, kb);
+        while (it < hi) {
+            int nx = 0;
+            if (lane == 0) nx = atomicAdd(&next_item, 1);
+            nx = __shfl_sync(0xFFFFFFFFu, nx, 0);
+            Chunk na, nb;
+            load(nx, na, nb);
+            int t, r;
+            locate(it, t, r);
+            u64 acc[2] = {0ull, 0ull};
+            if (r < a.R) {
+                const ulonglong2* cx = cx0 + t * (lpr * CX);
+                if (MODE == MODE_GU || (it - t * ips + 1) * STEPS <= rs) chunk_dots<MODE_GU, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);
+                else chunk_dots<MODE_ROUND, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);      // (a pair's last, single step)
+            }
+            const float v[2] = {pair_total(acc[0]), pair_total(acc[1])};
+            const float mine = split_sum<2>(v, lpr, jc);
+            if (slot == cnt) { keep = mine; kept = it; }
+            if (++cnt == h) flush();
+            it = nx;
+            ka = na;
+            kb = nb;
+        }
+        if (cnt) flush();
+    }
+}
+
+// ---- the same for rows of any number of chunks (pair_items), two blocks of 8 warps per SM -----------------------------------
+template <int MODE, int PF>
+__global__ void __launch_bounds__(MV_THREADS, 2) mv_items_kernel(MvParams a, KConst kc, RowShape sh, RouteFuse rf) {
     extern __shared__ __align__(16) ulonglong2 pair_sx[];
     __shared__ StreamTab tab;
-    __shared__ float part[MULTI ? PART_FLOATS : 1];
+    __shared__ float part[PART_FLOATS];
     __shared__ int32_t r_ind[256];   // the fused router's picks
     __shared__ float r_wt[256];
     load_stream_tab(tab, a.G, threadIdx.x, MV_THREADS);
@@ -397,37 +548,17 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_pair_kernel(MvParams a, KCon
     grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lpr = 1 << sh.lpr_log2, rpw = 32 >> sh.lpr_log2;
-    const int ch = MULTI ? sh.ch : lpr;
+    const int ch = sh.ch;
     int P = a.count ? min(*a.count, a.P) : a.P;
-    if (rf.logits) {          // the router: one warp per token, every block the same picks; block 0 stores them
-        if (warp < rf.T) {
-            const float* l = rf.logits + (size_t) warp * rf.ld;
-            if (rf.n_exp <= 128) route_row<4>(rf.n_exp, rf.top_k, l, lane, r_ind + warp * rf.top_k, r_wt + warp * rf.top_k);
-            else if (rf.n_exp <= 512) route_row<16>(rf.n_exp, rf.top_k, l, lane, r_ind + warp * rf.top_k, r_wt + warp * rf.top_k);
-            else route_row<32>(rf.n_exp, rf.top_k, l, lane, r_ind + warp * rf.top_k, r_wt + warp * rf.top_k);
-        }
+    if (rf.logits) {
+        route_prologue(rf, r_ind, r_wt);
         P = rf.T * rf.top_k;
-        __syncthreads();
-        if (blockIdx.x == 0 && (int) threadIdx.x < P) {
-            rf.ind_out[threadIdx.x] = r_ind[threadIdx.x];
-            rf.wt_out[threadIdx.x] = r_wt[threadIdx.x];
-        }
     }
     const int rs = (a.R + rpw - 1) / rpw;
     const long long total = (long long) P * rs;
     const long long begin = (long long) blockIdx.x * total / gridDim.x, end = (long long) (blockIdx.x + 1) * total / gridDim.x;
     if (begin >= end) return;
     const int p_first = (int) (begin / rs), p_last = (int) ((end - 1) / rs);
-    auto stage = [&](int pair, int buf) {
-        const void* row = input_row(a, a.xrow ? a.xrow[pair] : pair / a.xdiv);
-        ulonglong2* sx = pair_sx + (size_t) buf * ch * CX;
-        for (int i = threadIdx.x; i < ch * 4; i += MV_THREADS) {
-            float x[16];
-            stage_load(row, a.xbf16, i >> 2, i & 3, x);
-            stage_store<PF>(x, i >> 2, i & 3, sx);
-        }
-    };
-    int turn = 0;      // steps of the block so far: the warps' round-robin goes on from one pair to the next
     for (int pair = p_first; pair <= p_last; ++pair) {
         const int s_lo = pair == p_first ? (int) (begin - (long long) pair * rs) : 0;
         const int s_hi = pair == p_last ? (int) (end - (long long) pair * rs) : rs;
@@ -436,27 +567,22 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_pair_kernel(MvParams a, KCon
         WSlice wb = wa;
         if (MODE == MODE_GU) wb = a.wu[slice];
         // this warp's first streams are requested before the inputs are staged: their DRAM latency runs under it
-        const int st = s_lo + (MULTI ? warp / sh.groups : (warp - turn) & (MV_WARPS - 1)), r = st * rpw + (lane >> sh.lpr_log2);
-        const int jc = (lane & (lpr - 1)) + (MULTI ? warp % sh.groups * lpr : 0);
+        const int st = s_lo + warp / sh.groups, r = st * rpw + (lane >> sh.lpr_log2), jc = (lane & (lpr - 1)) + warp % sh.groups * lpr;
         Chunk ka, kb;
-        if (!MULTI) load_item<MODE, PF>(wa, wb, st, r, s_hi, a.R, sh.lpr_log2, jc, ka, kb);
-        else if (st < s_hi && r < a.R && jc < ch) {
+        if (st < s_hi && r < a.R && jc < ch) {
             ka = load_chunk<PF>(wa, (size_t) r * ch + jc);
             if (MODE == MODE_GU) kb = load_chunk<PF>(wb, (size_t) r * ch + jc);
         }
-        // inputs of two pairs at a time (a share of a short list has no more): a warp that is done with the first goes on to the
-        // second by itself
-        const int buf = MULTI ? 0 : (pair - p_first) & 1;
-        if (buf == 0) {
-            if (pair != p_first) __syncthreads();   // the previous pairs' inputs are no longer read
-            stage(pair, 0);
-            if (!MULTI && pair < p_last) stage(pair + 1, 1);
-            __syncthreads();   // inputs staged (and, for the block's first pair, the stream table loaded)
+        if (pair != p_first) __syncthreads();   // the previous pair's inputs are no longer read
+        const void* row = input_row(a, a.xrow ? a.xrow[pair] : pair / a.xdiv);
+        for (int i = threadIdx.x; i < ch * 4; i += MV_THREADS) {
+            float x[16];
+            stage_load(row, a.xbf16, i >> 2, i & 3, x);
+            stage_store<PF>(x, i >> 2, i & 3, pair_sx);
         }
-        auto store = [&](int rr, float s, float su) { store_out<MODE>(a, pair, rr, s, su); };
-        if constexpr (MULTI) pair_items<MODE, PF>(tab, kc, wa, wb, pair_sx, part, sh, a.R, s_lo, s_hi, ka, kb, store);
-        else pair_rows<MODE, PF>(tab, kc, wa, wb, pair_sx + (size_t) buf * ch * CX, sh.lpr_log2, a.R, st, s_hi, ka, kb, store);
-        turn += s_hi - s_lo;
+        __syncthreads();   // inputs staged (and, for the block's first pair, the stream table loaded)
+        pair_items<MODE, PF>(tab, kc, wa, wb, pair_sx, part, sh, a.R, s_lo, s_hi, ka, kb,
+                             [&](int rr, float s, float su) { store_out<MODE>(a, pair, rr, s, su); });
     }
 }
 
@@ -1152,12 +1278,6 @@ static RowShape row_shape(int ch, long long rows, int warps) {
     return best;
 }
 
-template <int MODE, int PF, bool MULTI>
-static void launch_pair_v(cudaStream_t s, const MvParams& a, RowShape sh, const RouteFuse& rf, size_t smem) {
-    static bool attr_set[16];
-    if (smem > 40 * 1024) allow_smem(mv_pair_kernel<MODE, PF, MULTI>, attr_set, (size_t) max_smem_optin() - 8192);
-    launch(mv_pair_kernel<MODE, PF, MULTI>, sm_count() * 2, MV_THREADS, smem, s, a, kconst(), sh, rf);
-}
 static size_t staged_bytes(int ch) { return (size_t) ch * CX * 16; }
 // Rows that are not 2^j <= 32 chunks: groups of 8, 4 or 2 lanes, whichever leaves the fewest lane slots empty (fewer lanes read
 // shorter runs of the streams: they have to save a twentieth).  A function of the row's length alone, so a row's bits do not
@@ -1174,9 +1294,20 @@ static RowShape item_shape(int ch) {
 }
 template <int MODE, int PF>
 static void launch_pair(cudaStream_t s, const MvParams& a, const RouteFuse& rf) {
-    const int ch = a.K / 64;
-    if (ch >= 2 && ch <= 32 && (ch & (ch - 1)) == 0) launch_pair_v<MODE, PF, false>(s, a, RowShape{ch, log2_floor(ch), 0, 1}, rf, 2 * staged_bytes(ch));
-    else launch_pair_v<MODE, PF, true>(s, a, item_shape(ch), rf, staged_bytes(ch));
+    const int ch = a.K / 64, sms = sm_count();
+    static bool attr_set[16], attr_set_items[16];
+    if (ch >= 2 && ch <= 32 && (ch & (ch - 1)) == 0) {
+        const int lpr_log2 = log2_floor(ch);
+        int win = a.P / sms + 2;      // a share's pairs, whole or in part
+        if (win > PAIR_WIN) win = PAIR_WIN;
+        if (win > a.P) win = a.P;
+        allow_smem(mv_pair_kernel<MODE, PF>, attr_set, (size_t) PAIR_WIN * 32 * CX * 16);
+        launch(mv_pair_kernel<MODE, PF>, sms, PAIR_THREADS, win * staged_bytes(ch), s, a, kconst(), lpr_log2, win, rf);
+    } else {
+        const size_t smem = staged_bytes(ch);
+        if (smem > 40 * 1024) allow_smem(mv_items_kernel<MODE, PF>, attr_set_items, (size_t) max_smem_optin() - 10240);
+        launch(mv_items_kernel<MODE, PF>, sms * 2, MV_THREADS, smem, s, a, kconst(), item_shape(ch), rf);
+    }
     count_launch();
 }
 
@@ -1238,7 +1369,7 @@ static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse&
     const bool dense = a.sel == NULL && rf.logits == NULL;
     const int ch = a.K / 64;
     const bool chunked = a.K % 64 == 0 && aligned16(a.x) && a.xs % (a.xbf16 ? 8 : 4) == 0 && (a.ws != NULL || slice_aligned(a.w0)) &&
-                         staged_bytes(ch) <= (size_t) max_smem_optin() - 8192;
+                         staged_bytes(ch) <= (size_t) max_smem_optin() - 10240;
     if (!chunked) {
         if (a.xrow || a.count || a.xbf16 || rf.logits) {
             set_error("seed mat-vec: the routed / row-index / device-count / bf16-input forms need K a multiple of 64 and aligned rows (K = %d)", a.K);
