@@ -64,15 +64,11 @@ constexpr KConst kconst_static() {
 }
 __constant__ KConst c_kc = kconst_static();
 
-// What a unit's row loop needs, by value (it runs in a function of its own: see unit_rows).
-struct UnitArgs {
-    const uint4 *sa, *ca, *sb, *cb;      // seeds and coefficient words of the (gate or only) matrix and of the up matrix
-    const uint32_t *da, *db;              // their exponent codes
-    int eba, ebb;
+// What the loop over the units' items needs, by value (it runs in a function of its own: see unit_items).
+struct UnitCall {
     float* y;
     int ys, R, raw, add;
-    int pid[2];                           // the unit's pairs (output rows)
-    int st, s_hi, lpr_log2, buf;          // the warp's first step; which of the two staged units this is
+    int lpr_log2, items;      // items of the window's units of this size
 };
 __device__ __forceinline__ Chunk load_chunk3(const uint4* s, const uint4* c, const uint32_t* d, size_t chunk_index) {
     Chunk k;
@@ -755,21 +751,33 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_step_kernel(StepParams p, KC
 // a unit's rows are expanded once for all its pairs (the logic-pipe work is shared; each pair keeps its own sums, formed in
 // the same order as when it is alone, so a pair's result does not depend on its partners).  The work is the sequence of
 // (unit, row step) items, an item of a unit with n pairs weighing GRP_W[n]; blocks take contiguous equal shares of the
-// weighted sequence, inside a unit the block's warps take its row steps round-robin, a row step being the 32 /
-// lanes-per-row rows a warp expands at once.  A unit's inputs sit in shared memory as the f32x2 operands of pair_expand_dot,
-// laid out [pair][block pair][operand pair][lane] so that a warp's 16-byte loads are conflict-free.
+// weighted sequence.  A block stages the inputs of as many of its units as GRP_SLOTS pairs are; its 16 warps then fetch the
+// items (RowItem) of the two-pair units and after them those of the single ones one by one, as in the pair kernel.
 constexpr int GRP_NT = 2;                         // pairs that share one expansion at most
 constexpr int GRP_MAX_PAIRS = 1024;               // pairs a block can sort; longer lists run ungrouped
 constexpr int GRP_SMALL = 128;                    // lists up to this length are ranked by counting (no sorting network)
-__device__ constexpr int GRP_W[5] = {0, 8, 12, 18, 23};   // relative cost of a row step for a unit of n pairs
+__device__ constexpr int GRP_W[GRP_NT + 1] = {0, 8, 12};   // relative cost of a row step for a unit of n pairs
 constexpr int GRP_SX = 32 * CX;                    // one pair's staged inputs
+constexpr int GRP_SLOTS = 12;                     // pairs staged at a time (a share of the longest sorted list is 7 and two parts)
+constexpr int GRP_WARPS = 16, GRP_THREADS = 32 * GRP_WARPS;
 
+struct GrpUnit {      // what an item needs of its unit
+    const uint4 *sa, *ca, *sb, *cb;
+    const uint32_t *da, *db;
+    float sca, scb;
+    int pid[2];                                    // its pairs
+    int slot, s_lo, s_hi;                          // its first pair's staged inputs; the block's row steps of it
+};
 struct GrpShared {
     StreamTab tab;
     uint32_t key[GRP_MAX_PAIRS];                  // sorted (slice << 10 | pair)
     int32_t prefix[GRP_MAX_PAIRS + 1];            // weight of the units that start before sorted position i
     uint32_t tmp[GRP_SMALL];                      // short lists: unsorted keys, then unit weights
-    __align__(16) ulonglong2 sx[2 * GRP_NT][GRP_SX];      // two units
+    GrpUnit unit[GRP_NT][GRP_SLOTS];              // the window's units of 1, 2 pairs ...
+    int start[GRP_NT][32];                        // ... their first items (beyond the last unit: never reached)
+    int next[GRP_NT];                             // the next item to fetch
+    int slot_pair[GRP_SLOTS];
+    __align__(16) ulonglong2 sx[GRP_SLOTS][GRP_SX];
 };
 
 
@@ -829,83 +837,110 @@ __device__ __forceinline__ void unit_chunk(const StreamTab& tab, const KConst& k
     }
 }
 
-// The row steps [s_lo, s_hi) of a unit of NT pairs that fall to this warp.  ka / kb: the streams of its first step,
-// requested by the caller before the unit's inputs were staged.
 template <int MODE>
-__device__ __forceinline__ void store_unit(const UnitArgs& ua, int pair, int r, float s, float su) {
-    float* yo = ua.y + (size_t) pair * ua.ys + r;
-    if (MODE == MODE_GU) *yo = ua.raw ? (s / (1.0f + expf(-s))) * su : bf16_round(silu_bf(bf16_round(s)) * bf16_round(su));
-    else if (ua.raw) *yo = s;
-    else *yo = ua.add ? bf16_round(*yo + bf16_round(s)) : bf16_round(s);   // engine/kernels_moe.cu:214
+__device__ __forceinline__ void store_unit(const UnitCall& uc, int pair, int r, float s, float su) {
+    float* yo = uc.y + (size_t) pair * uc.ys + r;
+    if (MODE == MODE_GU) *yo = uc.raw ? (s / (1.0f + expf(-s))) * su : bf16_round(silu_bf(bf16_round(s)) * bf16_round(su));
+    else if (uc.raw) *yo = s;
+    else *yo = uc.add ? bf16_round(*yo + bf16_round(s)) : bf16_round(s);   // engine/kernels_moe.cu:214
 }
 
+// The items of the window's units of NT pairs, fetched one by one by the block's warps.
 template <int MODE, int NT>
-__device__ __noinline__ void unit_rows(UnitArgs ua, Chunk ka, Chunk kb) {
+__device__ __noinline__ void unit_items(UnitCall uc) {
     // Not inlined on purpose: each unit size gets a register allocation of its own (inlined into one body, the larger
-    // sizes' pressure spilled the single-pair loop too).  Shared memory and the constants are reached by name.
+    // size's pressure spilled the single-pair loop too).  Shared memory and the constants are reached by name.
+    static_assert(NT == 1 || NT == 2, "units of one or two pairs");
     extern __shared__ __align__(16) unsigned char grp_smem[];
-    const GrpShared& sh = *reinterpret_cast<const GrpShared*>(grp_smem);
+    GrpShared& sh = *reinterpret_cast<GrpShared*>(grp_smem);
     const KConst& kc = c_kc;
-    const int s_hi = ua.s_hi, lpr_log2 = ua.lpr_log2;
-    const int lane = threadIdx.x & 31;
-    const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
-    const ulonglong2 (*sx)[GRP_SX] = sh.sx + ua.buf * GRP_NT;
-    const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
-    if (NT == 1) {      // one pair: the pair kernel's loop
-        WSlice wa = {}, wb = {};
-        wa.p[0] = ua.sa; wa.p[1] = ua.ca; wa.p[3] = ua.da; wa.eb = ua.eba;
-        wb.p[0] = ua.sb; wb.p[1] = ua.cb; wb.p[3] = ua.db; wb.eb = ua.ebb;
-        pair_rows<MODE, 4>(sh.tab, kc, wa, wb, sx[0], lpr_log2, ua.R, ua.st, s_hi, ka, kb,
-                                  [&](int r, float s, float su) { store_unit<MODE>(ua, ua.pid[0], r, s, su); });
-        return;
-    }
-    // two pairs: each item's four sums (pair 0: A, B; pair 1: A, B) end in a quarter of the row's lanes each
-    static_assert(NT <= 2, "units of one or two pairs");
     constexpr int STEPS = RowItem<MODE>::STEPS;
-    const float sca = slice_scale(ua.eba + 4), scb = slice_scale((MODE == MODE_GU ? ua.ebb : ua.eba) + 4);
-    const ulonglong2* cx[NT];
-#pragma unroll
-    for (int t = 0; t < NT; ++t) cx[t] = sx[t] + jc * CX;
-    const int S = MV_WARPS * rpw, h = lpr >> 2, slot = jc & (h - 1), part = jc >> (lpr_log2 - 2);
-    const int pid = part & 2 ? ua.pid[1] : ua.pid[0];
-    int st = ua.st, r = st * rpw + ro, cnt = 0;
+    const int lane = threadIdx.x & 31, lpr_log2 = uc.lpr_log2;
+    const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
+    const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
+    // an item's 2 NT sums (pair by pair: A, B) end in lpr / (2 NT) = h lanes of the row each, and stay there until each has one
+    const int h = lpr / (2 * NT), slot = jc & (h - 1), part = jc / h;
+    const int my_start = sh.start[NT - 1][lane];
+    auto fetch = [&]() {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(&sh.next[NT - 1], 1);
+        return __shfl_sync(0xFFFFFFFFu, i, 0);
+    };
+    int u, st;      // the current item's unit and first row step
+    auto locate = [&](int it) {
+        u = __popc(__ballot_sync(0xFFFFFFFFu, my_start <= it)) - 1;
+        st = sh.unit[NT - 1][u].s_lo + (it - __shfl_sync(0xFFFFFFFFu, my_start, u)) * STEPS;
+    };
+    auto load_a = [&](Chunk& k, const GrpUnit& d, int r) {
+        if (r < uc.R) k = load_chunk3(d.sa, d.ca, d.da, (size_t) ((r << lpr_log2) + jc));
+    };
+    auto load_b = [&](Chunk& k, const GrpUnit& d, int s, int r) {
+        if (MODE == MODE_GU) { if (r < uc.R) k = load_chunk3(d.sb, d.cb, d.db, (size_t) ((r << lpr_log2) + jc)); }
+        else if (s + 1 < d.s_hi && r + rpw < uc.R) k = load_chunk3(d.sa, d.ca, d.da, (size_t) ((r << lpr_log2) + jc + 32));
+    };
     float keep = 0.0f;
-    auto flush = [&](int st0, int r0) {
+    int kept_u = 0, kept_r = 0, cnt = 0;
+    auto flush = [&]() {
+        const GrpUnit& d = sh.unit[NT - 1][kept_u];
+        const int pid = part & 2 ? d.pid[1] : d.pid[0];
         if (MODE == MODE_GU) {
             const float su = __shfl_xor_sync(0xFFFFFFFFu, keep, h);
-            const int row = r0 + slot * S;
-            if (!(part & 1) && slot < cnt && row < ua.R) store_unit<MODE>(ua, pid, row, keep * sca, su * scb);
+            if (!(part & 1) && slot < cnt && kept_r < uc.R) store_unit<MODE>(uc, pid, kept_r, keep * d.sca, su * d.scb);
         } else {
-            const int e = 2 * slot + (part & 1), row = r0 + e * S;
-            if (slot < cnt && st0 + e * MV_WARPS < s_hi && row < ua.R) store_unit<MODE>(ua, pid, row, keep * sca, 0.0f);
+            const int r = kept_r + (part & 1 ? rpw : 0);
+            if (slot < cnt && r < min(d.s_hi * rpw, uc.R)) store_unit<MODE>(uc, pid, r, keep * d.sca, 0.0f);
         }
+        cnt = 0;
     };
-    for (; st < s_hi; st += STEPS * MV_WARPS, r += STEPS * S) {
-        // the next item's streams are requested as soon as this item's have been used up, into the registers they leave free
-        u64 acc[2] = {0ull, 0ull}, accb[2] = {0ull, 0ull};
-        const bool ok = r < ua.R, okb = ok && (MODE == MODE_GU || st + MV_WARPS < s_hi);
-        const int sn = st + STEPS * MV_WARPS, rn = r + STEPS * S;
-        if (ok) unit_chunk<NT>(sh.tab, kc, ka, cx, acc);
-        if (sn < s_hi && rn < ua.R) ka = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) ((rn << lpr_log2) + jc));
-        if (okb) unit_chunk<NT>(sh.tab, kc, kb, cx, accb);
-        if (MODE == MODE_GU) { if (sn < s_hi && rn < ua.R) kb = load_chunk3(ua.sb, ua.cb, ua.db, (size_t) ((rn << lpr_log2) + jc)); }
-        else if (sn + MV_WARPS < s_hi && rn + S < ua.R) kb = load_chunk3(ua.sa, ua.ca, ua.da, (size_t) (((rn + S) << lpr_log2) + jc));
-        const float v[4] = {pair_total(acc[0]), pair_total(accb[0]), pair_total(acc[1]), pair_total(accb[1])};
-        const float mine = split_sum<4>(v, lpr, jc);
-        if (slot == cnt) keep = mine;
-        if (++cnt == h) {
-            flush(st - (h - 1) * STEPS * MV_WARPS, r - (h - 1) * STEPS * S);
-            cnt = 0;
+    int it = fetch();
+    if (it >= uc.items) return;
+    Chunk ka, kb;
+    locate(it);
+    load_a(ka, sh.unit[NT - 1][u], st * rpw + ro);
+    load_b(kb, sh.unit[NT - 1][u], st, st * rpw + ro);
+    for (;;) {
+        const int nx = fetch(), u0 = u, r = st * rpw + ro;
+        const GrpUnit& d = sh.unit[NT - 1][u];
+        const bool ok = r < uc.R, okb = ok && (MODE == MODE_GU || st + 1 < d.s_hi);
+        const ulonglong2* const cx = sh.sx[d.slot] + jc * CX;
+        const bool more = nx < uc.items;
+        if (more) locate(nx);
+        const GrpUnit& dn = sh.unit[NT - 1][u];
+        const int rn = st * rpw + ro;
+        float mine;
+        if (NT == 1) {
+            Chunk na, nb;
+            if (more) { load_a(na, dn, rn); load_b(nb, dn, st, rn); }
+            u64 acc[2] = {0ull, 0ull};
+            if (okb) chunk_dots<MODE_GU, 4>(sh.tab, kc, ka, kb, cx, acc[0], acc[1]);
+            else if (ok) chunk_dots<MODE_ROUND, 4>(sh.tab, kc, ka, kb, cx, acc[0], acc[1]);
+            ka = na;
+            kb = nb;
+            const float v[2] = {pair_total(acc[0]), pair_total(acc[1])};
+            mine = split_sum<2>(v, lpr, jc);
+        } else {
+            // the next item's streams are requested as soon as this item's have been used up, into the registers they leave free
+            const ulonglong2* const cx2[2] = {cx, cx + GRP_SX};
+            u64 acc[2] = {0ull, 0ull}, accb[2] = {0ull, 0ull};
+            if (ok) unit_chunk<2>(sh.tab, kc, ka, cx2, acc);
+            if (more) load_a(ka, dn, rn);
+            if (okb) unit_chunk<2>(sh.tab, kc, kb, cx2, accb);
+            if (more) load_b(kb, dn, st, rn);
+            const float v[4] = {pair_total(acc[0]), pair_total(accb[0]), pair_total(acc[1]), pair_total(accb[1])};
+            mine = split_sum<4>(v, lpr, jc);
         }
+        if (slot == cnt) { keep = mine; kept_u = u0; kept_r = r; }
+        if (++cnt == h) flush();
+        if (!more) break;
     }
-    if (cnt) flush(st - cnt * STEPS * MV_WARPS, r - cnt * STEPS * S);
+    if (cnt) flush();
 }
 
 // Ascending bitonic sort of n (a power of two) keys in shared memory by the whole block.
 __device__ __forceinline__ void block_sort(uint32_t* key, int n) {
     for (int k = 2; k <= n; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < n; i += MV_THREADS) {
+            for (int i = threadIdx.x; i < n; i += GRP_THREADS) {
                 const int o = i ^ j;
                 if (o > i) {
                     const uint32_t x = key[i], y = key[o];
@@ -918,9 +953,9 @@ __device__ __forceinline__ void block_sort(uint32_t* key, int n) {
 
 // In-place exclusive prefix sum of a[0..n) by the whole block, a[n] = the total (n <= GRP_MAX_PAIRS).
 __device__ __forceinline__ void block_exclusive_scan(int32_t* a, int n) {
-    __shared__ int wtot[MV_WARPS];
+    __shared__ int wtot[GRP_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int per = (n + MV_THREADS - 1) / MV_THREADS, lo = threadIdx.x * per;      // a contiguous run per thread
+    const int per = (n + GRP_THREADS - 1) / GRP_THREADS, lo = threadIdx.x * per;      // a contiguous run per thread
     int sum = 0;
     for (int i = lo; i < lo + per && i < n; ++i) sum += a[i];
     int inc = sum;
@@ -930,21 +965,19 @@ __device__ __forceinline__ void block_exclusive_scan(int32_t* a, int n) {
     int base = inc - sum;
     for (int w = 0; w < warp; ++w) base += wtot[w];
     for (int i = lo; i < lo + per && i < n; ++i) { const int v = a[i]; a[i] = base; base += v; }
-    if (threadIdx.x == MV_THREADS - 1) { int t = 0; for (int w = 0; w < MV_WARPS; ++w) t += wtot[w]; a[n] = t; }
+    if (threadIdx.x == GRP_THREADS - 1) { int t = 0; for (int w = 0; w < GRP_WARPS; ++w) t += wtot[w]; a[n] = t; }
     __syncthreads();
 }
 
 
 template <int MODE>
-__global__ void __launch_bounds__(MV_THREADS, 2) mv_grp_kernel(MvParams a, KConst kc, int lpr_log2) {
+__global__ void __launch_bounds__(GRP_THREADS, 1) mv_grp_kernel(MvParams a, KConst kc, int lpr_log2) {
     extern __shared__ __align__(16) unsigned char grp_smem[];
     GrpShared& sh = *reinterpret_cast<GrpShared*>(grp_smem);
-    load_stream_tab(sh.tab, a.G, threadIdx.x, MV_THREADS);
+    load_stream_tab(sh.tab, a.G, threadIdx.x, GRP_THREADS);
     grid_dependents_go();
     grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
-    const int jc = lane & (lpr - 1), ro = lane >> lpr_log2;
     int P = a.count ? min(*a.count, a.P) : a.P;
     if (P <= 0) return;
     const int rs = (a.R + rpw - 1) / rpw;             // row steps per unit
@@ -975,12 +1008,12 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_grp_kernel(MvParams a, KCons
         } else {
             int n = 32;
             while (n < P) n <<= 1;
-            for (int i = threadIdx.x; i < n; i += MV_THREADS) sh.key[i] = i < P ? ((uint32_t) slice_of(i) << 10) | (uint32_t) i : 0xFFFFFFFFu;
+            for (int i = threadIdx.x; i < n; i += GRP_THREADS) sh.key[i] = i < P ? ((uint32_t) slice_of(i) << 10) | (uint32_t) i : 0xFFFFFFFFu;
             __syncthreads();
             block_sort(sh.key, n);
         }
         // a sorted position starts a unit when it is a multiple of GRP_NT pairs into its slice's run
-        for (int i = threadIdx.x; i < P; i += MV_THREADS) {
+        for (int i = threadIdx.x; i < P; i += GRP_THREADS) {
             const uint32_t first = sh.key[i] & ~1023u;          // the smallest key of this slice
             int lo = 0, hi = i;                                  // lower bound of `first`
             while (lo < hi) { const int mid = (lo + hi) >> 1; if (sh.key[mid] < first) lo = mid + 1; else hi = mid; }
@@ -994,7 +1027,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_grp_kernel(MvParams a, KCons
         }
         __syncthreads();
         if (small) {
-            for (int i = threadIdx.x; i <= P; i += MV_THREADS) {
+            for (int i = threadIdx.x; i <= P; i += GRP_THREADS) {
                 int before = 0;
                 for (int j = 0; j < i; ++j) before += (int) sh.tmp[j];
                 sh.prefix[i] = before;
@@ -1021,45 +1054,56 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_grp_kernel(MvParams a, KCons
     if (end >= total) { u_last = P; s_last = 0; } else locate(end, u_last, s_last);
     auto unit_size = [&](int u) { return grouped && sh.prefix[u + 1] - sh.prefix[u] != GRP_W[1] ? 2 : 1; };
     auto pair_of = [&](int u, int t) { return grouped ? (int) (sh.key[u + t] & 1023u) : u; };
-    const int per = lpr * 4;
-    auto stage_unit = [&](int u, int n, int buf) {      // the inputs of unit u's n pairs
-        for (int i = threadIdx.x; i < n * per; i += MV_THREADS) {
-            const int t = i >= per, rem = i - (t ? per : 0), p = pair_of(u, t);
-            float x[16];
-            stage_load(input_row(a, a.xrow ? a.xrow[p] : p / a.xdiv), a.xbf16, rem >> 2, rem & 3, x);
-            stage_store<4>(x, rem >> 2, rem & 3, sh.sx[buf * GRP_NT + t]);
-        }
-    };
-    int turn = 0, buf = 0;      // steps of the block so far (the warps' round-robin goes on from unit to unit); units are staged two at a time
     if (u_first < P && s_first >= rs) { u_first += unit_size(u_first); s_first = 0; }
-    for (int u = u_first; u < P && (u < u_last || (u == u_last && s_last > 0));) {
-        const int n = unit_size(u), slice = grouped ? (int) (sh.key[u] >> 10) : (a.sel ? a.sel[u] : 0);
-        const int s_lo = u == u_first ? s_first : 0, s_hi = u == u_last ? s_last : rs;
-        const WSlice wa = a.ws ? a.ws[slice] : a.w0;
-        WSlice wb = wa;
-        if (MODE == MODE_GU) wb = a.wu[slice];
-        const int st0 = s_lo + ((warp - turn) & (MV_WARPS - 1)), r0 = st0 * rpw + ro;
-        Chunk ka, kb;
-        load_item<MODE, 4>(wa, wb, st0, r0, s_hi, a.R, lpr_log2, jc, ka, kb);      // under the staging
-        if (buf == 0) {
-            if (turn) __syncthreads();   // the previous units' inputs are no longer read
-            stage_unit(u, n, 0);
-            const int un = u + n;
-            if (un < P && (un < u_last || (un == u_last && s_last > 0))) stage_unit(un, unit_size(un), 1);
-            __syncthreads();
+    constexpr int STEPS = RowItem<MODE>::STEPS;
+    auto mine = [&](int u) { return u < P && (u < u_last || (u == u_last && s_last > 0)); };
+    for (int u = u_first; mine(u);) {
+        if (u != u_first) __syncthreads();      // the previous window is no longer read
+        if (threadIdx.x < 32 * GRP_NT) sh.start[threadIdx.x >> 5][threadIdx.x & 31] = 0x7FFFFFFF;
+        __syncthreads();
+        int slots = 0, units[GRP_NT] = {0, 0}, items[GRP_NT] = {0, 0};
+        for (; mine(u); ) {
+            const int n = unit_size(u), s_lo = u == u_first ? s_first : 0, s_hi = u == u_last ? s_last : rs;
+            if (slots + n > GRP_SLOTS) break;
+            const int at = n == 2 ? units[1] : units[0];
+            if ((int) threadIdx.x == 32 * slots) {      // one warp a unit: the slices' table entries arrive side by side
+                const int slice = grouped ? (int) (sh.key[u] >> 10) : (a.sel ? a.sel[u] : 0);
+                GrpUnit d;
+                const WSlice wa = a.ws ? a.ws[slice] : a.w0;
+                d.sa = (const uint4*) wa.p[0]; d.ca = (const uint4*) wa.p[1]; d.da = (const uint32_t*) wa.p[3];
+                d.sca = d.scb = slice_scale(wa.eb + 4);
+                d.sb = d.cb = NULL;
+                d.db = NULL;
+                if (MODE == MODE_GU) {
+                    const WSlice wb = a.wu[slice];
+                    d.sb = (const uint4*) wb.p[0]; d.cb = (const uint4*) wb.p[1]; d.db = (const uint32_t*) wb.p[3];
+                    d.scb = slice_scale(wb.eb + 4);
+                }
+                d.pid[0] = sh.slot_pair[slots] = pair_of(u, 0);
+                d.pid[1] = pair_of(u, n - 1);
+                if (n == 2) sh.slot_pair[slots + 1] = d.pid[1];
+                d.slot = slots; d.s_lo = s_lo; d.s_hi = s_hi;
+                sh.unit[n - 1][at] = d;
+                sh.start[n - 1][at] = n == 2 ? items[1] : items[0];
+            }
+            const int more = (s_hi - s_lo + STEPS - 1) / STEPS;
+            if (n == 2) { ++units[1]; items[1] += more; } else { ++units[0]; items[0] += more; }
+            slots += n;
+            u += n;
         }
-        UnitArgs ua;
-        ua.sa = (const uint4*) wa.p[0]; ua.ca = (const uint4*) wa.p[1]; ua.da = (const uint32_t*) wa.p[3]; ua.eba = wa.eb;
-        ua.sb = (const uint4*) wb.p[0]; ua.cb = (const uint4*) wb.p[1]; ua.db = (const uint32_t*) wb.p[3]; ua.ebb = wb.eb;
-        ua.y = a.y; ua.ys = a.ys; ua.R = a.R; ua.raw = a.raw; ua.add = a.add;
-        ua.pid[0] = pair_of(u, 0);
-        ua.pid[1] = pair_of(u, n - 1);
-        ua.st = st0; ua.s_hi = s_hi; ua.lpr_log2 = lpr_log2; ua.buf = buf;
-        if (n == 2) unit_rows<MODE, 2>(ua, ka, kb);
-        else unit_rows<MODE, 1>(ua, ka, kb);
-        turn += s_hi - s_lo;
-        buf ^= 1;
-        u += n;
+        if (threadIdx.x < GRP_NT) sh.next[threadIdx.x] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < slots * lpr * 4; i += GRP_THREADS) {
+            const int t = i >> (lpr_log2 + 2), e = i & (lpr * 4 - 1), p = sh.slot_pair[t];
+            float x[16];
+            stage_load(input_row(a, a.xrow ? a.xrow[p] : p / a.xdiv), a.xbf16, e >> 2, e & 3, x);
+            stage_store<4>(x, e >> 2, e & 3, sh.sx[t]);
+        }
+        __syncthreads();
+        UnitCall uc = {a.y, a.ys, a.R, a.raw, a.add, lpr_log2, items[1]};
+        if (items[1]) unit_items<MODE, 2>(uc);
+        uc.items = items[0];
+        if (items[0]) unit_items<MODE, 1>(uc);
     }
 }
 
@@ -1320,7 +1364,7 @@ template <int MODE>
 static void launch_grp(cudaStream_t s, const MvParams& a, int lpr_log2) {
     static bool attr_set[16];
     allow_smem(mv_grp_kernel<MODE>, attr_set, sizeof(GrpShared));
-    launch(mv_grp_kernel<MODE>, sm_count() * 2, MV_THREADS, sizeof(GrpShared), s, a, kconst(), lpr_log2);
+    launch(mv_grp_kernel<MODE>, sm_count(), GRP_THREADS, sizeof(GrpShared), s, a, kconst(), lpr_log2);
     count_launch();
 }
 
