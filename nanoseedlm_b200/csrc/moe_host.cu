@@ -145,8 +145,8 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
             } else {
                 kc_pack_input_bf16(s, x, m->xp, (size_t) T * d);      // once: every row tile of every expert reads them
                 if (avg < 8) {      // few rows an expert: the kernel that keeps the weights in registers (at 11 rows the other is 4 % faster, at 1.3 2 % slower)
-                    nsl::launch_seed_mma(s, MF_SEED4P4, g, mt);
-                    nsl::launch_seed_mma(s, MF_SEED4P4, w, mt);
+                    nsl::launch_seed_mma_grouped(s, g);
+                    nsl::launch_seed_mma_grouped(s, w);
                 } else {
                     nsl::launch_gemm_gu(s, g, mt);
                     nsl::launch_gemm(s, MF_SEED4P4, "nsl_moe_forward", w, mt);

@@ -658,7 +658,7 @@ void launch_gemm(cudaStream_t s, int fmt, const char* who, MmParams a, int tiles
     }
     if (a.grouped && !a.ntiles) a.T = tiles_y;
     // a dense call of a few rows: the weights stay in registers (64 rows: 2 tiles there)
-    if (fmt != MF_BF16 && !g_exact && !a.grouped && a.T <= 64 && smm_serves(a.K, a.X, a.xs, a.packed)) { launch_seed_mma(s, fmt, a, tiles_y); return; }
+    if (fmt != MF_BF16 && !g_exact && !a.grouped && a.T <= 64 && smm_serves(a.K, a.X, a.xs, a.packed)) { launch_seed_mma(s, fmt, a); return; }
     const int row_tiles = (a.R + GM_BM - 1) / GM_BM;
     if (fmt == MF_BF16) {      // stored BF16 weights (p[0] = [R][K]): no expansion, one term
         if (a.packed) launch_gemm_v<1, 1, 1, true, false, IN_LIST>(s, a, row_tiles * tiles_y);

@@ -81,19 +81,20 @@ struct SmmShared {
 };
 
 // One pass: up to 8 NT rows of inputs for this block's rows of weights.
-template <int NT, int P, bool GU>
-__device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, SmmShared& sh, unsigned char* xs, const WSlice& wa, const WSlice& wb, int r0) {
+template <int NT, int P>
+__device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, SmmShared& sh, unsigned char* xs, int r0) {
     const MmParams& a = sp.m;
     const int kw = sp.kw, rw = sp.rw;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int kg = warp / rw, rg = warp - kg * rw;             // the warp's share of K and of the block's rows
     const int ch = a.K / 64, nss = (ch + 3) / 4, iters = (nss + kw - 1) / kw;
-    const int rowA = GU ? r0 + rg * 8 + g : r0 + rg * 16 + g, rowB = GU ? rowA : rowA + 8;
+    const int rowA = r0 + rg * 16 + g, rowB = rowA + 8;
+    const WSlice& w = a.w0;
     const bool okA = rowA < a.R, okB = rowB < a.R;
     constexpr int SS_BYTES = NT * 8 * 512;
     const int per = sp.per * (sp.rows / 8) / NT;      // a buffer holds more steps of fewer rows
     const uint32_t buf_bytes = (uint32_t) (per * kw * SS_BYTES);
-    const float baseA = exact_base<P>(wa.eb), baseB = exact_base<P>(GU ? wb.eb : wa.eb);
+    const float base = exact_base<P>(w.eb);
     float acc[NT][4];
 #pragma unroll
     for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
@@ -130,8 +131,8 @@ __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, 
     auto chunk_ok = [&](int it) { return it < iters && (it * kw + kg) * 4 + t < ch; };
     auto load = [&](int it, MmaChunk& ca, MmaChunk& cb) {      // (a chunk that is not there stays zero: zero coefficients, zero weights)
         const int c = (it * kw + kg) * 4 + t;
-        if (okA) ca = load_mma_chunk<P>(wa, (uint32_t) (rowA * ch + c));
-        if (okB) cb = load_mma_chunk<P>(GU ? wb : wa, (uint32_t) (rowB * ch + c));
+        if (okA) ca = load_mma_chunk<P>(w, (uint32_t) (rowA * ch + c));
+        if (okB) cb = load_mma_chunk<P>(w, (uint32_t) (rowB * ch + c));
     };
     MmaChunk ca = {}, cb = {};
     if (chunk_ok(0)) load(0, ca, cb);
@@ -155,8 +156,8 @@ __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, 
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj) {
                 uint32_t fa[8], fb[8];
-                pair_fragments<P>(sh.tab, sA[jj], cA[jj], P == 4 ? code_scale_pair(ca.cd, jj, kc) : code_scale_pair3(cA[jj], kc), baseA, kc, fa);
-                pair_fragments<P>(sh.tab, sB[jj], cB[jj], P == 4 ? code_scale_pair(cb.cd, jj, kc) : code_scale_pair3(cB[jj], kc), baseB, kc, fb);
+                pair_fragments<P>(sh.tab, sA[jj], cA[jj], P == 4 ? code_scale_pair(ca.cd, jj, kc) : code_scale_pair3(cA[jj], kc), base, kc, fa);
+                pair_fragments<P>(sh.tab, sB[jj], cB[jj], P == 4 ? code_scale_pair(cb.cd, jj, kc) : code_scale_pair3(cB[jj], kc), base, kc, fb);
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const uint32_t at = xb ^ (uint32_t) ((2 * jj + e) << 4);
@@ -203,10 +204,7 @@ __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, 
             const int dst = sh.drow[8 * i + 2 * t + e];
             const float va = acc[i][e], vb = acc[i][2 + e];
             if (dst < 0) continue;
-            if (GU) {
-                const float v = bf16_round(silu_round(bf16_round(va)) * bf16_round(vb));
-                if (okA) ((uint16_t*) a.Y)[(size_t) dst * a.ys + rowA] = (uint16_t) (__float_as_uint(v) >> 16);
-            } else if (a.out_bf16) {
+            if (a.out_bf16) {
                 uint16_t* y = (uint16_t*) a.Y + (size_t) dst * a.ys;
                 if (okA) y[rowA] = bf16_bits(va);
                 if (okB) y[rowB] = bf16_bits(vb);
@@ -219,7 +217,7 @@ __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, 
     }
 }
 
-template <int P, bool GU>
+template <int P>
 __global__ void __launch_bounds__(SMM_THREADS, 2) seed_mma_kernel(SmmParams sp, KConst kc) {
     extern __shared__ __align__(128) unsigned char smm_smem[];
     __shared__ SmmShared sh;
@@ -228,47 +226,213 @@ __global__ void __launch_bounds__(SMM_THREADS, 2) seed_mma_kernel(SmmParams sp, 
     load_stream_tab(sh.tab, a.G, tid, SMM_THREADS);
     grid_dependents_go();
     grid_dependency_wait();
-    if (a.grouped && a.ntiles && (int) blockIdx.y >= *a.ntiles) return;
-    int start, total;
-    WSlice wa, wb;
-    if (a.grouped) {
-        const MmTile tl = a.tiles[blockIdx.y];
-        wa = a.ws[tl.slice];
-        wb = GU ? a.wu[tl.slice] : wa;
-        start = tl.start;
-        total = tl.count < MMT_BN ? tl.count : MMT_BN;
-    } else {
-        wa = a.w0;
-        wb = wa;
-        start = (int) blockIdx.y * SMM_TILE;
-        total = min(a.T - start, SMM_TILE);
+    const int start = (int) blockIdx.y * SMM_TILE, count = min(a.T - start, SMM_TILE), r0 = (int) blockIdx.x * sp.rw * 16;
+    if (tid < SMM_TILE) {
+        const int d = tid >= count ? -1 : start + tid;
+        sh.soff[tid] = d < 0 ? -1 : (int) ((long long) d * a.xs / (a.packed ? 8 : 4));
+        sh.drow[tid] = d;
     }
-    const int r0 = (int) blockIdx.x * sp.rw * (GU ? 8 : 16);
-    for (int n0 = 0; n0 < total; n0 += SMM_TILE) {      // (a tile of more rows is expanded again: rare where this kernel is chosen)
-        const int count = min(SMM_TILE, total - n0);
-        __syncthreads();
-        if (tid < SMM_TILE) {
-            const int p = start + n0 + tid, d = tid >= count ? -1 : a.grouped ? a.perm[p] : p;
-            sh.soff[tid] = d < 0 ? -1 : (int) ((long long) (a.grouped ? d / a.xdiv : d) * a.xs / (a.packed ? 8 : 4));
-            sh.drow[tid] = d;
-        }
-        __syncthreads();
-        if (count <= 8) smm_pass<1, P, GU>(sp, kc, sh, smm_smem, wa, wb, r0);
-        else if (count <= 16) smm_pass<2, P, GU>(sp, kc, sh, smm_smem, wa, wb, r0);
-        else smm_pass<4, P, GU>(sp, kc, sh, smm_smem, wa, wb, r0);
-    }
+    __syncthreads();
+    if (count <= 8) smm_pass<1, P>(sp, kc, sh, smm_smem, r0);
+    else if (count <= 16) smm_pass<2, P>(sp, kc, sh, smm_smem, r0);
+    else smm_pass<4, P>(sp, kc, sh, smm_smem, r0);
 }
 
-template <int P, bool GU>
+template <int P>
 static void launch_smm_v(cudaStream_t s, const SmmParams& a, dim3 grid, size_t smem) {
     static bool done[16];
     int dev = 0;
     cudaGetDevice(&dev);
     if (!done[dev & 15]) {
-        cudaFuncSetAttribute(seed_mma_kernel<P, GU>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 8192);
+        cudaFuncSetAttribute(seed_mma_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 8192);
         done[dev & 15] = true;
     }
-    launch(seed_mma_kernel<P, GU>, grid, SMM_THREADS, smem, s, a, kconst());
+    launch(seed_mma_kernel<P>, grid, SMM_THREADS, smem, s, a, kconst());
+    count_launch();
+}
+
+// ---- grouped: few rows an expert ---------------------------------------------------------------------------------------------
+// An ITEM is 16 rows of weights of one tile, the whole of K, and belongs to one warp; nothing is shared between warps, so there is
+// no barrier.  One block of 16 warps an SM; block b's items come in runs of SMG_RUN: runs b, b + grid, ... of the tile-major
+// sequence, so that a tile of many rows is spread over many blocks, and its warps fetch them one by one from a counter (a warp
+// that the scheduler favours takes more).  The inputs are read through L1 straight into the B fragments: 16 bytes a lane, the
+// tile's few rows stay there while its items last.  What the next item needs (its slices' table entries, its pairs) is
+// copied into shared memory two steps before the end of the current one, and its first streams are requested in the last step.
+// With blocks of 8 warps a tile's 64 or 128 rows, their inputs staged in shared memory, a block's slowest warp and its
+// start-up (table entries, pairs, inputs, first streams, one after the other) took a fifth of the time.
+constexpr int SMG_WARPS = 16, SMG_THREADS = 32 * SMG_WARPS, SMG_RUN = 8;
+
+struct __align__(16) SmgItem {
+    int slice, start, count, r0;      // its tile, its first row of weights
+    WSlice wa, wb;
+    int perm[SMM_TILE];      // the first SMM_TILE pairs
+};
+struct SmgShared {
+    StreamTab tab;
+    SmgItem item[SMG_WARPS][2];
+    int next;
+};
+
+// One pass of an item: up to 8 NT rows of inputs.  ca / cb: the first step's streams; on return what last() has requested.
+template <int NT, bool GU, typename Step, typename Last>
+__device__ __forceinline__ void smg_pass(const MmParams& a, const KConst& kc, const StreamTab& tab, const SmgItem& d, int count,
+                                         MmaChunk& ca, MmaChunk& cb, Step step, Last last) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int ch = a.K / 64, nss = (ch + 3) / 4;
+    const float baseA = exact_base<4>(d.wa.eb), baseB = GU ? exact_base<4>(d.wb.eb) : baseA;
+    const uint16_t* x[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) x[i] = (const uint16_t*) a.X + (size_t) (d.perm[8 * i + g < count ? 8 * i + g : 0] / a.xdiv) * a.xs;      // (a row that is not there: any, its sums are dropped)
+    float acc[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+    for (int it = 0; it < nss; ++it) {
+        const int c = min(it * 4 + t, ch - 1);
+        const uint32_t sA[4] = {ca.s.x, ca.s.y, ca.s.z, ca.s.w}, cA[4] = {ca.c.x, ca.c.y, ca.c.z, ca.c.w}, cdA = ca.cd;
+        const uint32_t sB[4] = {cb.s.x, cb.s.y, cb.s.z, cb.s.w}, cB[4] = {cb.c.x, cb.c.y, cb.c.z, cb.c.w}, cdB = cb.cd;
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+            if (jj == 3) {      // the next streams, into the registers that these leave free: a quarter of a step ahead is enough
+                if (it + 1 < nss) step(it, ca, cb);
+                else last(ca, cb);
+            }
+            constexpr int AHEAD = NT <= 2 ? 2 : 1;      // steps whose inputs are requested before the expansion
+            uint4 xv[AHEAD][NT];
+#pragma unroll
+            for (int e = 0; e < AHEAD; ++e)
+#pragma unroll
+                for (int i = 0; i < NT; ++i) xv[e][i] = __ldg((const uint4*) (x[i] + c * 64) + 2 * jj + e);
+            uint32_t fa[8], fb[8];
+            pair_fragments<4>(tab, sA[jj], cA[jj], code_scale_pair(cdA, jj, kc), baseA, kc, fa);
+            pair_fragments<4>(tab, sB[jj], cB[jj], code_scale_pair(cdB, jj, kc), baseB, kc, fb);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (AHEAD == 1 && e == 1) {
+#pragma unroll
+                    for (int i = 0; i < NT; ++i) xv[0][i] = __ldg((const uint4*) (x[i] + c * 64) + 2 * jj + 1);
+                }
+#pragma unroll
+                for (int i = 0; i < NT; ++i) {
+                    const uint4 v = xv[AHEAD == 1 ? 0 : e][i];
+                    mma16816(acc[i], fa[4 * e], fb[4 * e], fa[4 * e + 1], fb[4 * e + 1], v.x, v.y);
+                    mma16816(acc[i], fa[4 * e + 2], fb[4 * e + 2], fa[4 * e + 3], fb[4 * e + 3], v.z, v.w);
+                }
+            }
+        }
+    }
+    // lane (g, t): rows 8 i + 2 t and + 1 of the inputs (elements 0, 1 of weight row A; 2, 3 of row B)
+    const int rowA = d.r0 + g, rowB = rowA + 8;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int n = 8 * i + 2 * t + e;
+            const float va = acc[i][e], vb = acc[i][2 + e];
+            if (n >= count) continue;
+            uint16_t* y = (uint16_t*) a.Y + (size_t) d.perm[n] * a.ys;
+            if (GU) {
+                const float v = bf16_round(silu_round(bf16_round(va)) * bf16_round(vb));
+                if (rowA < a.R) y[rowA] = (uint16_t) (__float_as_uint(v) >> 16);
+            } else {
+                if (rowA < a.R) y[rowA] = bf16_bits(va);
+                if (rowB < a.R) y[rowB] = bf16_bits(vb);
+            }
+        }
+    }
+}
+
+template <bool GU>
+__global__ void __launch_bounds__(SMG_THREADS, 1) seed_mma_grouped_kernel(MmParams a, KConst kc) {
+    __shared__ SmgShared sh;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    constexpr int ROWS = GU ? 8 : 16;
+    load_stream_tab(sh.tab, a.G, tid, SMG_THREADS);
+    if (tid == 0) sh.next = 0;
+    grid_dependents_go();
+    grid_dependency_wait();
+    __syncthreads();
+    const int ch = a.K / 64, nss = (ch + 3) / 4;
+    const int groups = (a.R + ROWS - 1) / ROWS, rpt = (groups + SMG_RUN - 1) / SMG_RUN, runs = *a.ntiles * rpt;      // runs a tile, in all
+    auto fetch = [&](int buf) {      // the warp's next item, into one of its two places
+        for (;;) {
+            int i = 0;
+            if (lane == 0) i = atomicAdd(&sh.next, 1);
+            i = __shfl_sync(0xFFFFFFFFu, i, 0);
+            const int run = i / SMG_RUN * (int) gridDim.x + (int) blockIdx.x;
+            if (run >= runs) return false;
+            const int tile = run / rpt, grp = (run - tile * rpt) * SMG_RUN + i % SMG_RUN;
+            if (grp >= groups) continue;
+            if (lane == 0) {
+                const int4 tl = __ldg((const int4*) a.tiles + tile);
+                *(int4*) &sh.item[warp][buf] = make_int4(tl.x, tl.y, min(tl.z, MMT_BN), grp * ROWS);
+            }
+            __syncwarp();
+            return true;
+        }
+    };
+    auto describe = [&](int buf) {      // requests its table entries and pairs
+        SmgItem& d = sh.item[warp][buf];
+        const int words = (int) sizeof(WSlice) / 8, w = lane & 15;
+        if (w < words && (GU || lane < 16)) {
+            const WSlice* from = (lane < 16 ? a.ws : a.wu) + d.slice;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t) __cvta_generic_to_shared(lane < 16 ? &d.wa : &d.wb) + w * 8), "l"((const char*) from + w * 8) : "memory");
+        }
+        if (lane < d.count) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t) __cvta_generic_to_shared(d.perm + lane)), "l"(a.perm + d.start + lane) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto described = [&]() {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+    };
+    auto load = [&](const SmgItem& d, int it, MmaChunk& ca, MmaChunk& cb) {      // (rows that are not there: the last one, its sums are dropped)
+        const int c = it * 4 + t, cc = min(c, ch - 1), rowA = min(d.r0 + g, a.R - 1), rowB = GU ? rowA : min(d.r0 + g + 8, a.R - 1);
+        ca = load_mma_chunk<4>(d.wa, (uint32_t) (rowA * ch + cc));
+        cb = load_mma_chunk<4>(GU ? d.wb : d.wa, (uint32_t) (rowB * ch + cc));
+        if (it * 4 + 4 > ch && c >= ch) ca = cb = MmaChunk{};      // a chunk that is not there: zero coefficients, zero weights
+    };
+    int buf = 0;
+    if (!fetch(0)) return;
+    MmaChunk ca, cb;
+    describe(0);
+    described();
+    load(sh.item[warp][0], 0, ca, cb);
+    for (;;) {
+        const bool next = fetch(buf ^ 1);
+        SmgItem& d = sh.item[warp][buf];
+        for (int n0 = 0; n0 < d.count; n0 += SMM_TILE) {      // (a tile of more rows is expanded again: rare where this kernel is chosen)
+            const int count = min(d.count - n0, SMM_TILE);
+            if (n0) {
+                __syncwarp();
+                if (lane < count) d.perm[lane] = a.perm[d.start + n0 + lane];
+                __syncwarp();
+            }
+            const bool more = n0 + SMM_TILE < d.count, ahead = !more && next;
+            auto step = [&](int it, MmaChunk& na, MmaChunk& nb) {
+                if (it == nss - 2 && ahead) describe(buf ^ 1);
+                load(d, it + 1, na, nb);
+            };
+            auto last = [&](MmaChunk& na, MmaChunk& nb) {
+                if (more) load(d, 0, na, nb);
+                else if (next) {
+                    if (nss == 1) describe(buf ^ 1);
+                    described();
+                    load(sh.item[warp][buf ^ 1], 0, na, nb);
+                }
+            };
+            if (count <= 8) smg_pass<1, GU>(a, kc, sh.tab, d, count, ca, cb, step, last);
+            else if (count <= 16) smg_pass<2, GU>(a, kc, sh.tab, d, count, ca, cb, step, last);
+            else smg_pass<4, GU>(a, kc, sh.tab, d, count, ca, cb, step, last);
+        }
+        if (!next) break;
+        buf ^= 1;
+        __syncwarp();      // the place that the item after the next one goes to is no longer read
+    }
+}
+
+void launch_seed_mma_grouped(cudaStream_t s, const MmParams& m) {
+    if (m.R <= 0) return;
+    if (m.wu) launch(seed_mma_grouped_kernel<true>, sm_count(), SMG_THREADS, 0, s, m, kconst());
+    else launch(seed_mma_grouped_kernel<false>, sm_count(), SMG_THREADS, 0, s, m, kconst());
     count_launch();
 }
 
@@ -276,20 +440,16 @@ bool smm_serves(int K, const void* X, int xs, int packed) {
     return K >= 64 && K % 64 == 0 && aligned16(X) && xs % (packed ? 8 : 4) == 0;
 }
 
-void launch_seed_mma(cudaStream_t s, int fmt, const MmParams& m, int tiles_y) {
-    if (tiles_y <= 0 || m.R <= 0) return;
-    const bool gu = m.wu != NULL;
+void launch_seed_mma(cudaStream_t s, int fmt, const MmParams& m) {
+    if (m.T <= 0 || m.R <= 0) return;
     SmmParams a = {m, SMM_WARPS, 1, 1, 2, SMM_TILE};
-    if (!m.grouped) {
-        // A dense product of a few rows: 16 rows of weights a warp leave most SMs idle on a matrix of a few thousand rows, so
-        // the block's warps share K until the blocks fill the SMs (a function of the matrix alone).
-        while (a.kw < 8 && (m.R + 16 * SMM_WARPS / a.kw - 1) / (16 * SMM_WARPS / a.kw) < sm_count() * 3 / 4 && m.K >= SMM_SS * 2 * a.kw) a.kw *= 2;
-        a.rw = SMM_WARPS / a.kw;
-        tiles_y = (m.T + SMM_TILE - 1) / SMM_TILE;
-    }
+    // 16 rows of weights a warp leave most SMs idle on a matrix of a few thousand rows, so the block's warps share K until the
+    // blocks fill the SMs (a function of the matrix alone).
+    while (a.kw < 8 && (m.R + 16 * SMM_WARPS / a.kw - 1) / (16 * SMM_WARPS / a.kw) < sm_count() * 3 / 4 && m.K >= SMM_SS * 2 * a.kw) a.kw *= 2;
+    a.rw = SMM_WARPS / a.kw;
     // All of K in one buffer where two blocks of that size fit an SM, else two buffers of 48 KB, else (K shared by many warps) one
     // step at a time.  The sizes are those of the most rows a tile may have; fewer rows make a buffer hold more steps.
-    a.rows = m.grouped || m.T > 16 ? 32 : m.T > 8 ? 16 : 8;
+    a.rows = m.T > 16 ? 32 : m.T > 8 ? 16 : 8;
     const size_t step = (size_t) a.kw * a.rows * 512, room = 96 * 1024;
     const int iters = (m.K + SMM_SS * a.kw - 1) / (SMM_SS * a.kw);
     if ((size_t) iters * step <= room) { a.per = iters; a.bufs = 1; }
@@ -298,11 +458,10 @@ void launch_seed_mma(cudaStream_t s, int fmt, const MmParams& m, int tiles_y) {
     size_t smem = (size_t) a.bufs * a.per * step;
     const size_t red = (size_t) (a.kw - 1) * a.rw * (a.rows / 8) * 512;
     if (red > smem) smem = red;
-    const int wrows = a.rw * (gu ? 8 : 16);
-    const dim3 grid((unsigned) ((m.R + wrows - 1) / wrows), (unsigned) tiles_y);
-    if (fmt == MF_SEED4) launch_smm_v<3, false>(s, a, grid, smem);
-    else if (gu) launch_smm_v<4, true>(s, a, grid, smem);
-    else launch_smm_v<4, false>(s, a, grid, smem);
+    const int wrows = a.rw * 16;
+    const dim3 grid((unsigned) ((m.R + wrows - 1) / wrows), (unsigned) ((m.T + SMM_TILE - 1) / SMM_TILE));
+    if (fmt == MF_SEED4) launch_smm_v<3>(s, a, grid, smem);
+    else launch_smm_v<4>(s, a, grid, smem);
 }
 
 }   // namespace nsl
