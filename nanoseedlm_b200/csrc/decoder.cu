@@ -10,6 +10,8 @@
 #include "common.cuh"
 #include "../../include/nslm_decoder.h"
 
+namespace nsl { bool launch_q4_mv(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add); }      // q4_head.cu
+
 extern "C" {
 // declared in nslm_kernels.h / nslm_ep.h; the routed form of the gate+up mat-vec
 void nsl_mv_gu_routed(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K, int R, const float* x, int xs, float* a, int ys,
@@ -222,10 +224,7 @@ int nsl_decoder_step(NslDecoder* m, cudaStream_t s, const int32_t* ids, const Ro
         nsl_residual_add(s, m->x, m->br, (size_t) T * d);
     }
     kc_gnorm(s, d, c.eps, m->x, m->norm_out, m->h, T);
-    for (int t0 = 0; t0 < T; t0 += MV_MAXT) {
-        const int n = T - t0 < MV_MAXT ? T - t0 : MV_MAXT;
-        kc_mv(s, MF_Q4, m->head, d, c.vocab, m->h + (size_t) t0 * d, d, m->lm + (size_t) t0 * c.vocab, c.vocab, n, 0, NULL);
-    }
+    nsl::launch_q4_mv(s, m->head, d, c.vocab, m->h, d, m->lm, c.vocab, T, 0);
     kc_argmax(s, m->lm, next, c.vocab, T);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -323,7 +323,10 @@ __global__ void __launch_bounds__(32 * WARPS, 1) q4_mv_ring_kernel(const uint32_
 // partial sums meet in shared memory (8 KB per tile), where they are added in warp order.  K = 256 x WARPS.
 // BPS blocks share an SM (16 warps in all): a block's barrier per tile then overlaps another block's work.  Shared
 // memory: the partial sums, then the staged inputs, whose place the rings take once every warp holds its fragments.
-template <int WARPS, int NST, int BPS>
+// NT: tiles of 8 tokens that share an unpacking; the grid's y counts groups of 8 NT tokens, whose blocks stream the same rows at
+// about the same time, so that memory sees them once.  (32 tokens in four launches of 8: 196 us for 151936 x 2048.)  A token's
+// operations and their order do not depend on NT.
+template <int WARPS, int NST, int BPS, int NT>
 __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uint32_t* __restrict__ codes, const uint16_t* __restrict__ S,
                                                                      const uint16_t* __restrict__ B, int K, int R,
                                                                      const float* __restrict__ x, int xs, float* __restrict__ y,
@@ -331,9 +334,14 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
     constexpr int ROW = Q4Ring<4>::ROW, STAGE = Q4Ring<4>::STAGE;
     constexpr int G = 4 * WARPS, KB = 128 * WARPS;      // groups and bytes of codes per row (K = 256 x WARPS)
     extern __shared__ __align__(16) uint32_t q4_smem[];
-    float* part = (float*) q4_smem;                                              // [2 buffers][2 tiles][WARPS][32][4]
+    constexpr int TPI = 2 / NT;      // tiles of 16 rows an iteration: 256 outputs
+    float* part = (float*) q4_smem;                                              // [2 buffers][TPI][NT][WARPS][32][4]
+    const int tok0 = blockIdx.y * 8 * NT;
+    x += (size_t) tok0 * xs;
+    y += (size_t) tok0 * ys;
+    T -= tok0;
     uint32_t* xb = q4_smem + 4 * WARPS * 128;
-    float* xsum = (float*) (xb + (size_t) G * 256);
+    float* xsum = (float*) (xb + (size_t) NT * G * 256);
     // the rings take the place of the staged inputs once those sit in the warps' registers
     unsigned char* ring = (unsigned char*) xb + (size_t) (threadIdx.x >> 5) * NST * STAGE;
     grid_dependents_go();
@@ -376,8 +384,8 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
         nstage = nstage + 1 == NST ? 0 : nstage + 1;
     };
     const bool vec = (xs & 3) == 0 && aligned16_dev(x);
-    for (int i = threadIdx.x; i < G * 32; i += 32 * WARPS) {
-        const int g = i >> 5, sq = (i >> 3) & 3, n = i & 7;
+    for (int i = threadIdx.x; i < NT * G * 32; i += 32 * WARPS) {      // (token tile, group, quarter, token)
+        const int g = (i >> 5) % G, sq = (i >> 3) & 3, n = (i & 7) + i / (G * 32) * 8;
         uint32_t* dst = xb + (size_t) i * 8;
         float v[16];
         if (n < T) {
@@ -406,31 +414,33 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
         }
         psum += __shfl_xor_sync(0xFFFFFFFFu, psum, 8);
         psum += __shfl_xor_sync(0xFFFFFFFFu, psum, 16);
-        if (sq == 0) xsum[g * 8 + n] = psum;
+        if (sq == 0) xsum[(i >> 5) * 8 + (i & 7)] = psum;
     }
     __syncthreads();
     // this warp's four groups of inputs: fragments and sums, in registers for the whole kernel
-    uint32_t breg[4][8];
-    float xg[4][2];
+    uint32_t breg[NT][4][8];
+    float xg[NT][4][2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int g = warp * 4 + j;
-        const uint4 lo = *(const uint4*) (xb + ((size_t) (g * 4 + q) * 8 + rr) * 8), hi = *(const uint4*) (xb + ((size_t) (g * 4 + q) * 8 + rr) * 8 + 4);
-        breg[j][0] = lo.x; breg[j][1] = lo.y; breg[j][2] = lo.z; breg[j][3] = lo.w;
-        breg[j][4] = hi.x; breg[j][5] = hi.y; breg[j][6] = hi.z; breg[j][7] = hi.w;
-        xg[j][0] = xsum[g * 8 + 2 * q];
-        xg[j][1] = xsum[g * 8 + 2 * q + 1];
-    }
+    for (int tt = 0; tt < NT; ++tt)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int g = tt * G + warp * 4 + j;
+            const uint4 lo = *(const uint4*) (xb + ((size_t) (g * 4 + q) * 8 + rr) * 8), hi = *(const uint4*) (xb + ((size_t) (g * 4 + q) * 8 + rr) * 8 + 4);
+            breg[tt][j][0] = lo.x; breg[tt][j][1] = lo.y; breg[tt][j][2] = lo.z; breg[tt][j][3] = lo.w;
+            breg[tt][j][4] = hi.x; breg[tt][j][5] = hi.y; breg[tt][j][6] = hi.z; breg[tt][j][7] = hi.w;
+            xg[tt][j][0] = xsum[g * 8 + 2 * q];
+            xg[tt][j][1] = xsum[g * 8 + 2 * q + 1];
+        }
     __syncthreads();      // every warp has its inputs: their place is the rings' now
 #pragma unroll
     for (int i = 0; i < NST - 1; ++i) issue();
 
-    // Two tiles an iteration: one barrier and one reduction of 256 outputs (a thread each) for both.
-    int stage = 0;
-    for (int idx = 0; idx < my_tiles; idx += 2) {
-        float* pb = part + (size_t) ((idx >> 1) & 1) * 2 * WARPS * 128;
+    // 256 outputs an iteration: one barrier and one reduction (a thread each) for all of them.
+    int stage = 0, pbuf = 0;
+    for (int idx = 0; idx < my_tiles; idx += TPI, pbuf ^= 1) {
+        float* pb = part + (size_t) pbuf * 2 * WARPS * 128;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < TPI; ++h) {
             if (idx + h >= my_tiles) break;
             asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
             __syncwarp();
@@ -439,42 +449,49 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
             const unsigned char* row0 = st + rr * ROW, *row1 = st + (rr + 8) * ROW;
             const uint4 t0 = *(const uint4*) (row0 + 128), t2 = *(const uint4*) (row1 + 128);      // {4 scales, 4 biases}
             const uint32_t sa0[2] = {t0.x, t0.y}, ba0[2] = {t0.z, t0.w}, sa1[2] = {t2.x, t2.y}, ba1[2] = {t2.z, t2.w};
-            float out[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            float out[NT][4];
+#pragma unroll
+            for (int tt = 0; tt < NT; ++tt) out[tt][0] = out[tt][1] = out[tt][2] = out[tt][3] = 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const uint2 w0 = *(const uint2*) (row0 + j * 32 + q * 8), w1 = *(const uint2*) (row1 + j * 32 + q * 8);
                 uint32_t a0[8], a1[8];
                 unpack8(w0.x, a0); unpack8(w0.y, a0 + 4);
                 unpack8(w1.x, a1); unpack8(w1.y, a1 + 4);
-                float c[4];
                 const uint32_t f0[4] = {a0[0], a1[0], a0[4], a1[4]}, f1[4] = {a0[1], a1[1], a0[5], a1[5]};
                 const uint32_t f2[4] = {a0[2], a1[2], a0[6], a1[6]}, f3[4] = {a0[3], a1[3], a0[7], a1[7]};
-                mma_bf16_16x8x16_first(c, f0, breg[j][0], breg[j][1]);
-                mma_bf16_16x8x16(c, f1, breg[j][2], breg[j][3]);
-                mma_bf16_16x8x16(c, f2, breg[j][4], breg[j][5]);
-                mma_bf16_16x8x16(c, f3, breg[j][6], breg[j][7]);
                 // scale and bias j: the high halves need no shift, only a mask
                 auto val = [&](const uint32_t* v) { return __uint_as_float(j & 1 ? v[j >> 1] & 0xFFFF0000u : v[j >> 1] << 16); };
                 const float s0 = val(sa0), s1 = val(sa1), e0 = fmaf(8.0f, s0, val(ba0)), e1 = fmaf(8.0f, s1, val(ba1));
-                out[0] = fmaf(s0, c[0], fmaf(e0, xg[j][0], out[0]));
-                out[1] = fmaf(s0, c[1], fmaf(e0, xg[j][1], out[1]));
-                out[2] = fmaf(s1, c[2], fmaf(e1, xg[j][0], out[2]));
-                out[3] = fmaf(s1, c[3], fmaf(e1, xg[j][1], out[3]));
+#pragma unroll
+                for (int tt = 0; tt < NT; ++tt) {
+                    float c[4];
+                    mma_bf16_16x8x16_first(c, f0, breg[tt][j][0], breg[tt][j][1]);
+                    mma_bf16_16x8x16(c, f1, breg[tt][j][2], breg[tt][j][3]);
+                    mma_bf16_16x8x16(c, f2, breg[tt][j][4], breg[tt][j][5]);
+                    mma_bf16_16x8x16(c, f3, breg[tt][j][6], breg[tt][j][7]);
+                    out[tt][0] = fmaf(s0, c[0], fmaf(e0, xg[tt][j][0], out[tt][0]));
+                    out[tt][1] = fmaf(s0, c[1], fmaf(e0, xg[tt][j][1], out[tt][1]));
+                    out[tt][2] = fmaf(s1, c[2], fmaf(e1, xg[tt][j][0], out[tt][2]));
+                    out[tt][3] = fmaf(s1, c[3], fmaf(e1, xg[tt][j][1], out[tt][3]));
+                }
             }
             __syncwarp();
             issue();
-            *(float4*) (pb + h * WARPS * 128 + (warp * 32 + lane) * 4) = make_float4(out[0], out[1], out[2], out[3]);
+#pragma unroll
+            for (int tt = 0; tt < NT; ++tt)
+                *(float4*) (pb + (h * NT + tt) * WARPS * 128 + (warp * 32 + lane) * 4) = make_float4(out[tt][0], out[tt][1], out[tt][2], out[tt][3]);
         }
         __syncthreads();      // the block's partial sums of these tiles are in; the other buffer is free for the next ones
         for (int e = threadIdx.x; e < 256; e += 32 * WARPS) {      // each output is the warps' sum in warp order
-            const int h = e >> 7, o = e & 127;
-            if (idx + h >= my_tiles) break;
+            const int h = e >> 7, o = e & 127, tile = idx + h / NT;      // (h: tile of rows, tile of tokens)
+            if (tile >= my_tiles) break;
             const float* ps = pb + h * WARPS * 128 + o;
             float acc = ps[0];
 #pragma unroll
             for (int w = 1; w < WARPS; ++w) acc += ps[w * 128];
             const int sl = o >> 2, i = o & 3;      // the lane slot (rr, q) and its output i
-            const int row = (blockIdx.x + (idx + h) * gridDim.x) * 16 + (sl >> 2) + (i >> 1) * 8, t = 2 * (sl & 3) + (i & 1);
+            const int row = (blockIdx.x + tile * gridDim.x) * 16 + (sl >> 2) + (i >> 1) * 8, t = h % NT * 8 + 2 * (sl & 3) + (i & 1);
             if (row < R && t < T) {
                 float* yo = y + (size_t) t * ys + row;
                 *yo = add ? bf16_round(*yo + bf16_round(acc)) : bf16_round(acc);
@@ -484,18 +501,34 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-template <int WARPS, int NST, int BPS>
-static void launch_q4_ksplit(cudaStream_t s, size_t total, int blocks, const WSlice& w, int K, int R, const float* x, int xs, float* y,
+template <int WARPS, int NST, int BPS, int NT>
+static void launch_q4_ksplit_v(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y,
                              int ys, int T, int add) {
+    // 16 warps an SM in blocks of K / 256 warps, four stages per warp in the place of the staged inputs: with two
+    // blocks an SM one block's barrier per tile overlaps the other's work (151936 x 2048: 51.9 us with one block of
+    // 8 warps and 6 stages, 49.2 us with two blocks of 4 stages)
+    const size_t staged = (size_t) NT * (K / Q4_GROUP) * (4 * 8 * 8 * 4 + 8 * 4), rings = (size_t) WARPS * NST * Q4Ring<4>::STAGE;
+    const size_t total = (size_t) 4 * WARPS * 512 + (rings > staged ? rings : staged);
+    const int tiles = (R + 15) / 16, groups = (T + 8 * NT - 1) / (8 * NT);
+    int blocks = BPS * sm_count() / groups;
+    if (blocks < 1) blocks = 1;
+    if (blocks > tiles) blocks = tiles;
     static bool attr_set[16];
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev & 15]) {
-        cudaFuncSetAttribute(q4_mv_ksplit_kernel<WARPS, NST, BPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 1024);
+        cudaFuncSetAttribute(q4_mv_ksplit_kernel<WARPS, NST, BPS, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 1024);
         attr_set[dev & 15] = true;
     }
-    launch(q4_mv_ksplit_kernel<WARPS, NST, BPS>, (unsigned) blocks, 32 * WARPS, total, s, (const uint32_t*) w.p[0], (const uint16_t*) w.p[1],
+    launch(q4_mv_ksplit_kernel<WARPS, NST, BPS, NT>, dim3((unsigned) blocks, (unsigned) groups), 32 * WARPS, total, s, (const uint32_t*) w.p[0], (const uint16_t*) w.p[1],
            (const uint16_t*) w.p[2], K, R, x, xs, y, ys, T, add);
+    count_launch();
+}
+// K = 256 x WARPS.  Up to 8 tokens: one tile of them; more: two share an unpacking.
+template <int WARPS, int NST, int BPS>
+static void launch_q4_ksplit(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add) {
+    if (T <= 8) launch_q4_ksplit_v<WARPS, NST, BPS, 1>(s, w, K, R, x, xs, y, ys, T, add);
+    else launch_q4_ksplit_v<WARPS, NST, BPS, 2>(s, w, K, R, x, xs, y, ys, T, add);
 }
 
 template <int NST, int WARPS, int GPP>
@@ -613,10 +646,11 @@ __global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax
     }
 }
 
-// Called by kc_mv for fmt == MF_Q4.  Returns false (with the error recorded) when the shape is not served.
+// kc_mv for fmt == MF_Q4, and the decoder's head for any number of tokens.  Returns false (with the error recorded) when the shape
+// is not served.
 bool launch_q4_mv(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add) {
-    if (K < Q4_GROUP || K % Q4_GROUP || R < 1 || T < 1 || T > MV_MAXT || (w.gs != 0 && w.gs != 6)) {
-        set_error("kc_mv (Q4): K = %d must be a multiple of 64, 1..%d tokens, groups of 64 (gs %d)", K, (int) MV_MAXT, w.gs);
+    if (K < Q4_GROUP || K % Q4_GROUP || R < 1 || T < 1 || (w.gs != 0 && w.gs != 6)) {
+        set_error("kc_mv (Q4): K = %d must be a multiple of 64, at least one token, groups of 64 (gs %d)", K, w.gs);
         return false;
     }
     if (((uintptr_t) w.p[0] & 7u) || !aligned16(w.p[1]) || !aligned16(w.p[2])) {
@@ -634,19 +668,13 @@ bool launch_q4_mv(cudaStream_t s, const WSlice& w, int K, int R, const float* x,
     }
     const size_t budget = (size_t) max_smem_optin() - 1024;
     if (aligned16(w.p[0]) && (K == 1024 || K == 2048 || K == 4096)) {      // K split over the block's warps
-        // 16 warps an SM in blocks of K / 256 warps, four stages per warp in the place of the staged inputs: with two
-        // blocks an SM one block's barrier per tile overlaps the other's work (151936 x 2048: 51.9 us with one block of
-        // 8 warps and 6 stages, 49.2 us with two blocks of 4 stages)
-        const int warps = K / 256, bps = 16 / warps;
-        const size_t rings = (size_t) warps * 4 * Q4Ring<4>::STAGE;
-        const size_t total = (size_t) 4 * warps * 512 + (rings > smem ? rings : smem);
-        const int blocks = tiles < bps * sm_count() ? tiles : bps * sm_count();
-        if (warps == 4) launch_q4_ksplit<4, 4, 4>(s, total, blocks, w, K, R, x, xs, y, ys, T, add);
-        else if (warps == 8) launch_q4_ksplit<8, 4, 2>(s, total, blocks, w, K, R, x, xs, y, ys, T, add);
-        else launch_q4_ksplit<16, 4, 1>(s, total, blocks, w, K, R, x, xs, y, ys, T, add);
-        count_launch();
+        if (K == 1024) launch_q4_ksplit<4, 4, 4>(s, w, K, R, x, xs, y, ys, T, add);
+        else if (K == 2048) launch_q4_ksplit<8, 4, 2>(s, w, K, R, x, xs, y, ys, T, add);
+        else launch_q4_ksplit<16, 4, 1>(s, w, K, R, x, xs, y, ys, T, add);
         return true;
     }
+    for (; T > MV_MAXT; T -= MV_MAXT, x += (size_t) MV_MAXT * xs, y += (size_t) MV_MAXT * ys)      // the other kernels hold 8 tokens
+        launch_q4_mv(s, w, K, R, x, xs, y, ys, MV_MAXT, add);
     if (K % 512 == 0 && aligned16(w.p[0]) && smem + (size_t) 8 * 2 * Q4Ring<8>::STAGE <= budget) {      // streams through shared memory
         // 8 warps with three passes of eight groups in flight each (measured faster than 16 warps with three passes of four:
         // 66.9 against 77.2 us on the 151936 x 2048 head), or 8 warps with one pass in flight when shared memory is short

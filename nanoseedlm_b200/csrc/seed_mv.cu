@@ -1461,7 +1461,11 @@ extern "C" {
 
 void kc_mv(cudaStream_t s, int fmt, WSlice w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add,
            const uint32_t* G) {
-    if (fmt == MF_Q4) { launch_q4_mv(s, w, K, R, x, xs, y, ys, T, add); return; }   // the LM head's affine int4 (q4_head.cu)
+    if (fmt == MF_Q4) {      // the LM head's affine int4 (q4_head.cu)
+        if (T > MV_MAXT) set_error("kc_mv (Q4): %d tokens, at most %d", T, (int) MV_MAXT);
+        else launch_q4_mv(s, w, K, R, x, xs, y, ys, T, add);
+        return;
+    }
     if (fmt == MF_BF16) {      // stored BF16 weights (dense_bf16.cu): the tensor-core kernel where its shape rules allow, else a warp per row
         if (!launch_bf16_mm_skinny(s, w, K, R, x, xs, y, ys, T, add)) launch_bf16_mv(s, w, K, R, x, xs, y, ys, T, add);
         return;

@@ -276,3 +276,29 @@ def test_decoder_step_of_more_rows_than_a_mat_vec_takes(oracle):
     n = nxt.cpu().numpy()
     assert ((n >= 0) & (n < c["vocab"])).all()
     dec.close()
+
+
+@pytest.mark.parametrize("d,T", [(1024, 9), (2048, 17), (2048, 32), (4096, 25), (512, 9)])
+def test_head_of_more_rows_than_a_mat_vec_takes(oracle, d, T):
+    """The LM head of a large step against kc_mv (eight rows at a time) on the same normalised rows: the same bits (512: the
+    kernels without a form of their own for more rows; 17, 25: a group of rows that is not full)."""
+    import torch
+    from nanoseedlm_b200 import decoder, lib as L
+    c = dict(CFG, n_layer=1, d=d, vocab=5000)
+    cfg = decoder.make_cfg(max_rows=T, eps=EPS, theta=THETA, **c)
+    dec = decoder.random_decoder(cfg, seed=5)
+    nxt = torch.full((T,), -1, dtype=torch.int32, device="cuda")
+    dec.step(torch.arange(T, dtype=torch.int32, device="cuda"), decoder.row_info([0] * T, [t * c["ctx"] for t in range(T)]), T, nxt)
+    h = dec.hidden(T).contiguous()
+    hn, want = torch.empty_like(h), torch.empty((T, c["vocab"]), device="cuda")
+    lib = L.load()
+    norm_out, codes, sc, bi = dec.keep[-4:]
+    head = L.WSlice()
+    head.p[0], head.p[1], head.p[2] = codes.data_ptr(), sc.data_ptr(), bi.data_ptr()
+    lib.kc_gnorm(None, d, EPS, h.data_ptr(), norm_out.data_ptr(), hn.data_ptr(), T)
+    for t in range(0, T, 8):
+        lib.kc_mv(None, L.MF_Q4, head, d, c["vocab"], hn[t:].data_ptr(), d, want[t:].data_ptr(), c["vocab"], min(8, T - t), 0, None)
+    torch.cuda.synchronize()
+    L.check()
+    assert torch.equal(dec.logits(T).view(T, -1), want)
+    dec.close()
