@@ -42,7 +42,24 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Up to three matrices of one width applied to the same rows of inputs in one launch (the attention's q, k, v; the shared expert's
+// gate and up): a block works on one of them, matrix m has the blocks first[m] .. first[m + 1] - 1.
+constexpr int DENSE_SET = 3;
+struct DenseSet {
+    int n;
+    int first[DENSE_SET + 1];
+    WSlice w[DENSE_SET];
+    int R[DENSE_SET];
+    float* y[DENSE_SET];      // [T][R]
+};
+
 #ifdef __CUDACC__
+__device__ __forceinline__ int set_member(const DenseSet& set, int block) {
+    int m = 0;
+#pragma unroll
+    for (int i = 1; i < DENSE_SET; ++i) m += i < set.n && block >= set.first[i];
+    return m;
+}
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif

@@ -10,7 +10,13 @@
 #include "common.cuh"
 #include "../../include/nslm_decoder.h"
 
-namespace nsl { bool launch_q4_mv(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add); }      // q4_head.cu
+namespace nsl {
+bool launch_q4_mv(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add);      // q4_head.cu
+bool launch_bf16_set(cudaStream_t s, const DenseSet& set, int K, const float* x, int T);                                         // dense_bf16.cu
+bool launch_seed_set(cudaStream_t s, DenseSet set, int K, const float* x, int T, const uint32_t* G);                             // seed_mv.cu
+void launch_combine_residual_gnorm(cudaStream_t s, int d, int k, const float* D, const float* wt, const float* sh, const float* sg, int sgld, float* x,
+                                   float eps, const uint16_t* w, float* y, int T);                                               // moe_misc.cu
+}
 
 extern "C" {
 // declared in nslm_kernels.h / nslm_ep.h; the routed form of the gate+up mat-vec
@@ -36,7 +42,7 @@ struct NslDecoder {
     int chunk_rows;
     std::vector<void*> dev;
     // activations of a step
-    float *x, *h, *q, *k, *v, *o, *logits, *wt, *A, *Dx, *As, *Gs, *Us, *sh, *br, *moe, *part, *lm, *inv, *ones, *wsel;
+    float *x, *h, *q, *k, *v, *o, *logits, *wt, *A, *Dx, *As, *Gs, *Us, *sh, *moe, *part, *lm, *inv, *ones, *wsel;
     int32_t *ind, *zero_sel, *sel, *xrow, *tok_off, *count;
     WSlice* shared_tab;      // device: per layer the shared expert's gate and up as one-entry tables
     std::vector<uint16_t*> kc, vc;
@@ -96,7 +102,7 @@ NslDecoder* nsl_decoder_create(const NslDecoderCfg* cfg, const NslDecoderLayer* 
 #define DEC_I(field, count) ok = ok && (m->field = (int32_t*) dec_alloc(m, 4 * (size_t) (count))) != NULL
     DEC_F(x, T * d); DEC_F(h, T * d); DEC_F(q, T * HQ); DEC_F(k, T * HK); DEC_F(v, T * HK); DEC_F(o, T * HQ);
     DEC_F(logits, T * (c.n_exp + 1)); DEC_F(wt, T * c.top_k); DEC_F(A, P * c.ff_exp); DEC_F(Dx, P * d);
-    DEC_F(As, T * c.ff_shared); DEC_F(Gs, T * c.ff_shared); DEC_F(Us, T * c.ff_shared); DEC_F(sh, T * d); DEC_F(br, T * d); DEC_F(moe, T * d);
+    DEC_F(As, T * c.ff_shared); DEC_F(Gs, T * c.ff_shared); DEC_F(Us, T * c.ff_shared); DEC_F(sh, T * d); DEC_F(moe, T * d);
     DEC_F(part, T * c.n_head * 32 * 130); DEC_F(lm, T * (size_t) c.vocab); DEC_F(inv, 64); DEC_F(ones, T); DEC_F(wsel, P);
     DEC_I(ind, T * c.top_k); DEC_I(zero_sel, T); DEC_I(sel, P); DEC_I(xrow, P); DEC_I(tok_off, Tall + 1); DEC_I(count, 4);
     for (int l = 0; ok && l < c.n_layer; ++l) {
@@ -145,6 +151,12 @@ static void dense(NslDecoder* m, cudaStream_t s, const WSlice& w, int K, int R, 
     else kc_mm(s, fmt, w, K, R, x, K, y, R, T, add, m->G);
 }
 
+// The same for matrices that share their inputs: one launch where the decode batch's kernels take them.
+static void dense_set(NslDecoder* m, cudaStream_t s, const nsl::DenseSet& set, int K, const float* x, int T) {
+    if (m->c.dense_bf16 ? nsl::launch_bf16_set(s, set, K, x, T) : nsl::launch_seed_set(s, set, K, x, T, m->G)) return;
+    for (int i = 0; i < set.n; ++i) dense(m, s, set.w[i], K, set.R[i], x, set.y[i], T, 0);
+}
+
 // A dense SEED4P4 matrix expanded once to BF16 [R][K] in device memory; w then points at the expansion.
 static bool expand_dense(NslDecoder* m, WSlice& w, int K, int R) {
     uint16_t* out = (uint16_t*) dec_alloc(m, 2 * (size_t) R * K);
@@ -167,16 +179,14 @@ int nsl_decoder_step(NslDecoder* m, cudaStream_t s, const int32_t* ids, const Ro
     const AttnArgs aa = {c.n_head, c.n_kv, 128, 32, 1.0f / sqrtf(128.0f)};
     nsl::PdlScope pdl(true);      // the kernels that know how wait on the device for their predecessor; the others launch as usual
     kc_embed(s, MF_BF16, m->embed, d, ids, m->x, T);
+    kc_gnorm(s, d, c.eps, m->x, m->L[0].norm_attn, m->h, T);
     for (int l = 0; l < c.n_layer; ++l) {
         const NslDecoderLayer& L = m->L[l];
         KvView kv;
         memset(&kv, 0, sizeof kv);
         kv.a.k = m->kc[l]; kv.a.v = m->vc[l]; kv.nv = c.max_rows * c.ctx; kv.fmt = KV_BF16;
         // attention
-        kc_gnorm(s, d, c.eps, m->x, L.norm_attn, m->h, T);
-        dense(m, s, L.wq, d, HQ, m->h, m->q, T, 0);
-        dense(m, s, L.wk, d, HK, m->h, m->k, T, 0);
-        dense(m, s, L.wv, d, HK, m->h, m->v, T, 0);
+        dense_set(m, s, {3, {0}, {L.wq, L.wk, L.wv}, {HQ, HK, HK}, {m->q, m->k, m->v}}, d, m->h, T);
         kc_rope_kv(s, m->q, m->k, m->v, kv, ri, m->inv, c.n_head, c.n_kv, T);
         kc_attn(s, aa, m->q, kv, ri, m->part, NULL, m->o, T);
         dense(m, s, L.wo, HQ, d, m->o, m->x, T, 1);      // x = bf16(x + bf16(Wo o))
@@ -190,13 +200,13 @@ int nsl_decoder_step(NslDecoder* m, cudaStream_t s, const int32_t* ids, const Ro
                 kc_mv_gu(m->s2, MF_SEED4P4, m->shared_tab + 2 * l, m->shared_tab + 2 * l + 1, d, fs, m->h, d, m->As, fs, m->zero_sel, T, 1, m->G);
                 kc_mv(m->s2, MF_SEED4P4, L.sd, fs, d, m->As, fs, m->sh, d, T, 0, m->G);
             } else {
-                dense(m, m->s2, L.sg, d, fs, m->h, m->Gs, T, 0);
-                dense(m, m->s2, L.su, d, fs, m->h, m->Us, T, 0);
+                dense_set(m, m->s2, {2, {0}, {L.sg, L.su}, {fs, fs}, {m->Gs, m->Us}}, d, m->h, T);
                 kc_swiglu(m->s2, m->Gs, m->Us, m->As, T * fs);
                 dense(m, m->s2, L.sd, fs, d, m->As, m->sh, T, 0);
             }
         }
         cudaEventRecord(m->ev_sh, m->s2);
+        const uint16_t* const next_norm = l + 1 < c.n_layer ? m->L[l + 1].norm_attn : m->norm_out;
         dense(m, s, L.router, d, ld, m->h, m->logits, T, 0);
         if (!m->ep) {
             const int P = T * k;
@@ -207,7 +217,7 @@ int nsl_decoder_step(NslDecoder* m, cudaStream_t s, const int32_t* ids, const Ro
             }
             kc_mv_sel(s, MF_SEED4P4, L.ed, ff, d, m->A, ff, m->Dx, d, m->ind, P, 1, m->G);
             cudaStreamWaitEvent(s, m->ev_sh, 0);
-            kq4_moe_combine(s, d, k, m->Dx, m->wt, m->sh, m->logits + c.n_exp, ld, m->br, T);
+            nsl::launch_combine_residual_gnorm(s, d, k, m->Dx, m->wt, m->sh, m->logits + c.n_exp, ld, m->x, c.eps, next_norm, m->h, T);
         } else {
             const NslEpWindow& w = m->win;
             const int P = w.n * w.t_loc * k;
@@ -219,11 +229,9 @@ int nsl_decoder_step(NslDecoder* m, cudaStream_t s, const int32_t* ids, const Ro
             nsl_ep_p2p_combine(s, w, m->Dx, m->wsel, m->tok_off, d);
             nsl_ep_p2p_reduce(s, w, d, m->moe);
             cudaStreamWaitEvent(s, m->ev_sh, 0);
-            kq4_moe_combine(s, d, 1, m->moe, m->ones, m->sh, m->logits + c.n_exp, ld, m->br, T);      // the shared expert's share + the routed sum
+            nsl::launch_combine_residual_gnorm(s, d, 1, m->moe, m->ones, m->sh, m->logits + c.n_exp, ld, m->x, c.eps, next_norm, m->h, T);      // the shared expert's share + the routed sum
         }
-        nsl_residual_add(s, m->x, m->br, (size_t) T * d);
     }
-    kc_gnorm(s, d, c.eps, m->x, m->norm_out, m->h, T);
     nsl::launch_q4_mv(s, m->head, d, c.vocab, m->h, d, m->lm, c.vocab, T, 0);
     kc_argmax(s, m->lm, next, c.vocab, T);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;

@@ -81,13 +81,18 @@ __device__ __forceinline__ void mma_bf16_16816(float* c, uint32_t a0, uint32_t a
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__global__ void __launch_bounds__(256) bf16_mm_skinny_kernel(const uint16_t* __restrict__ W, int K, int R, const float* __restrict__ x, int xs,
-                                                             float* __restrict__ y, int ys, int T, int add) {
+// The matrices of a set are sixteen-row tiles side by side.  (Three launches for q, k, v of one decoder row cost three latencies, 3 us
+// each, for 1 us of memory traffic.)
+__global__ void __launch_bounds__(256) bf16_mm_skinny_kernel(DenseSet set, int K, const float* __restrict__ x, int xs, int ys, int T, int add) {
     extern __shared__ __align__(16) unsigned char xsm[];      // 8 rows of K bf16 inputs
     __shared__ float part[8][16][9];
     grid_dependents_go();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
-    const int r0 = blockIdx.x * 16, tok0 = blockIdx.y * 8;
+    const int mat = set_member(set, (int) blockIdx.x), R = set.R[mat];
+    const int r0 = ((int) blockIdx.x - set.first[mat]) * 16, tok0 = blockIdx.y * 8;
+    const uint16_t* const W = (const uint16_t*) set.w[mat].p[0];
+    float* const y = set.y[mat];
+    if (set.n > 1) ys = R;
     const uint16_t* wa = W + (size_t) min(r0 + g, R - 1) * K + 8 * t4;
     const uint16_t* wb = W + (size_t) min(r0 + g + 8, R - 1) * K + 8 * t4;
     const int kw = K / 8, k0 = warp * kw, stride = K * 2 + 64;
@@ -137,10 +142,12 @@ __global__ void __launch_bounds__(256) bf16_mm_skinny_kernel(const uint16_t* __r
     }
 }
 
-// Serves kc_mm for stored BF16 weights when the batch is a decode batch; false: the caller runs the tile GEMM.
-bool launch_bf16_mm_skinny(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add) {
+// A decode batch's products with stored BF16 weights; false: a shape it does not serve.
+static bool launch_skinny(cudaStream_t s, const DenseSet& set, int K, const float* x, int xs, int ys, int T, int add) {
     const size_t smem = 8 * ((size_t) K * 2 + 64);
-    if (T < 1 || T > 64 || K < 256 || K % 256 || R < 1 || smem > 160 * 1024 || !aligned16(w.p[0]) || !aligned16(x) || xs % 4) return false;
+    if (T < 1 || T > 64 || K < 256 || K % 256 || smem > 160 * 1024 || !aligned16(x) || xs % 4) return false;
+    for (int m = 0; m < set.n; ++m)
+        if (set.R[m] < 1 || !aligned16(set.w[m].p[0])) return false;
     static bool done[16];
     int dev = 0;
     cudaGetDevice(&dev);
@@ -148,10 +155,16 @@ bool launch_bf16_mm_skinny(cudaStream_t s, const WSlice& w, int K, int R, const 
         cudaFuncSetAttribute(bf16_mm_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
         done[dev & 15] = true;
     }
-    launch(bf16_mm_skinny_kernel, dim3((unsigned) ((R + 15) / 16), (unsigned) ((T + 7) / 8)), 256, smem, s, (const uint16_t*) w.p[0], K, R, x, xs, y, ys,
-           T, add);
+    DenseSet a = set;
+    for (int m = 0; m < DENSE_SET; ++m) a.first[m + 1] = a.first[m] + (m < set.n ? (set.R[m] + 15) / 16 : 0);
+    launch(bf16_mm_skinny_kernel, dim3((unsigned) a.first[DENSE_SET], (unsigned) ((T + 7) / 8)), 256, smem, s, a, K, x, xs, ys, T, add);
     count_launch();
     return true;
 }
+// Serves kc_mm (and kc_mv) for stored BF16 weights when the batch is a decode batch; false: the caller runs the tile GEMM.
+bool launch_bf16_mm_skinny(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add) {
+    return launch_skinny(s, DenseSet{1, {0}, {w}, {R}, {y}}, K, x, xs, ys, T, add);
+}
+bool launch_bf16_set(cudaStream_t s, const DenseSet& set, int K, const float* x, int T) { return launch_skinny(s, set, K, x, K, 0, T, 0); }
 
 }   // namespace nsl

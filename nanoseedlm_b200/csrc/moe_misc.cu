@@ -57,6 +57,61 @@ __global__ void q4_combine_kernel(int d, int k, const float* __restrict__ D, con
     out[(size_t) t * d + i] = a;
 }
 
+// The end of a decoder layer and the start of the next: the combine above, x = bf16(x + its result) (nsl_residual_add) and y = the
+// grouped RMSNorm of x (kc_gnorm), a block a row, each value formed as those three kernels form it.  For a decode batch
+// each of them is a launch's latency and little else.
+__global__ void __launch_bounds__(256) combine_residual_gnorm_kernel(int d, int k, const float* __restrict__ D, const float* __restrict__ wt,
+                                                                     const float* __restrict__ sh, const float* __restrict__ sg, int sgld,
+                                                                     float* __restrict__ x, float eps,
+                                                                     const uint16_t* __restrict__ w, float* __restrict__ y) {
+    __shared__ float part[8];
+    grid_dependency_wait();
+    grid_dependents_go();
+    const int t = blockIdx.x, half = threadIdx.x >> 7, i0 = threadIdx.x & 127, hw = d / 2;      // (kc_gnorm's split of a row)
+    const size_t at = (size_t) t * d + (size_t) half * hw;
+    const float* const Dr = D + (size_t) t * k * d + (size_t) half * hw;
+    const float gate = 1.0f / (1.0f + expf(-sg[(size_t) t * sgld]));
+    float s = 0.0f;
+    for (int c0 = i0; c0 < hw; c0 += 8 * 128) {      // eight values a thread side by side
+        float a[8], xv[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int c = c0 + 128 * q;
+            if (c < hw) { a[q] = gate * sh[at + c]; xv[q] = x[at + c]; }
+        }
+#pragma unroll 4
+        for (int j = 0; j < k; ++j) {
+            const float wj = wt[t * k + j];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int c = c0 + 128 * q;
+                if (c < hw) a[q] += wj * Dr[(size_t) j * d + c];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int c = c0 + 128 * q;
+            if (c < hw) {
+                const float v = bf16_round(xv[q] + a[q]);
+                x[at + c] = v;
+                s = fmaf(v, v, s);
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    const float tot = ((part[4 * half] + part[4 * half + 1]) + part[4 * half + 2]) + part[4 * half + 3];
+    const float r = rsqrtf(tot / (float) hw + eps);
+    const uint16_t* wr = w + (size_t) half * hw;
+    for (int c = i0; c < hw; c += 128) y[at + c] = bf16_round(__uint_as_float((uint32_t) wr[c] << 16) * (x[at + c] * r));      // (x: this thread's own stores)
+}
+void launch_combine_residual_gnorm(cudaStream_t s, int d, int k, const float* D, const float* wt, const float* sh, const float* sg, int sgld, float* x,
+                                   float eps, const uint16_t* w, float* y, int T) {
+    launch(combine_residual_gnorm_kernel, (unsigned) T, 256, 0, s, d, k, D, wt, sh, sg, sgld, x, eps, w, y);
+    count_launch();
+}
+
 // The same without a shared expert over packed bf16 rows (d a multiple of 8: 16 bytes of each of the k rows a thread).
 __global__ void __launch_bounds__(256) combine_packed_kernel(int d8, int k, const uint4* __restrict__ D, const float* __restrict__ wt,
                                                              float4* __restrict__ out, int n) {

@@ -13,6 +13,8 @@
 // single-token call bit for bit, as the reference requires (tests/test_mova_kernels.c:173-183).
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "route.cuh"
 #include "seed_block.cuh"
@@ -1126,14 +1128,23 @@ __device__ __forceinline__ void dense_two_weights(const Words& wa, const Words& 
 }
 
 template <int PF, int NT>
-__global__ void __launch_bounds__(MV_THREADS, 2) mv_dense_kernel(MvParams a, KConst kc, RowShape sh) {
+__global__ void __launch_bounds__(MV_THREADS, 2) mv_dense_kernel(MvParams a, KConst kc, RowShape sh, DenseSet set) {
     extern __shared__ __align__(16) ulonglong2 dense_sx[];
     __shared__ StreamTab tab;
+    int block = blockIdx.x, blocks = gridDim.x;
+    if (set.n > 1) {
+        const int m = set_member(set, block);
+        block -= set.first[m];
+        blocks = set.first[m + 1] - set.first[m];
+        a.w0 = set.w[m];
+        a.R = a.ys = set.R[m];
+        a.y = set.y[m];
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lpr = 1 << sh.lpr_log2, rpw = 32 >> sh.lpr_log2, passes = 1 << (sh.lv - sh.lpr_log2);
     const int jc = lane & (lpr - 1), ro = lane >> sh.lpr_log2, ch = sh.ch;
-    const int steps = (a.R + rpw - 1) / rpw, stride = (int) gridDim.x * MV_WARPS;
-    int st = warp * (int) gridDim.x + (int) blockIdx.x, r = st * rpw + ro, base = 0, pass = 0;
+    const int steps = (a.R + rpw - 1) / rpw, stride = blocks * MV_WARPS;
+    int st = warp * blocks + block, r = st * rpw + ro, base = 0, pass = 0;
     Chunk k;
     if (st < steps && r < a.R && jc < ch) k = load_chunk<PF>(a.w0, (size_t) r * ch + jc);      // weights never change: requested before the wait
     load_stream_tab(tab, a.G, threadIdx.x, MV_THREADS);
@@ -1369,29 +1380,48 @@ static void launch_grp(cudaStream_t s, const MvParams& a, int lpr_log2) {
 }
 
 template <int PF, int NT>
-static void launch_dense_v(cudaStream_t s, const MvParams& a, size_t smem) {
+static void launch_dense_v(cudaStream_t s, const MvParams& a, size_t smem, DenseSet* set) {
     static bool attr_set[16];
     if (smem > 40 * 1024) allow_smem(mv_dense_kernel<PF, NT>, attr_set, (size_t) max_smem_optin() - 8192);
     const int bps = smem > 100 * 1024 ? 1 : 2;
-    const RowShape sh = row_shape(a.K / 64, a.R, sm_count() * bps * MV_WARPS);
-    const int steps = (a.R * (1 << sh.lpr_log2) + 31) / 32;
-    launch(mv_dense_kernel<PF, NT>, steps < sm_count() * bps ? steps : sm_count() * bps, MV_THREADS, smem, s, a, kconst(), sh);
+    long long rows = a.R;
+    for (int m = 1; set && m < set->n; ++m) rows += set->R[m];
+    const RowShape sh = row_shape(a.K / 64, rows, sm_count() * bps * MV_WARPS);
+    auto steps_of = [&](long long r) { return (int) ((r * (1 << sh.lpr_log2) + 31) / 32); };
+    int blocks = std::min(steps_of(rows), sm_count() * bps);
+    if (set) {      // each matrix gets its share of the blocks, at least one
+        int left = blocks > set->n ? blocks : set->n;
+        long long rest = rows;
+        for (int m = 0; m < DENSE_SET; ++m) {
+            int n = 0;
+            if (m < set->n) {
+                n = (int) ((2 * left * (long long) set->R[m] + rest) / (2 * rest));
+                n = std::max(1, std::min(n, left - (set->n - 1 - m)));
+                left -= n;
+                rest -= set->R[m];
+            }
+            set->first[m + 1] = set->first[m] + n;
+        }
+        blocks = set->first[DENSE_SET];
+    }
+    launch(mv_dense_kernel<PF, NT>, blocks, MV_THREADS, smem, s, a, kconst(), sh, set ? *set : DenseSet{1});
     count_launch();
 }
 // T rows on one slice; more rows than their inputs fit shared memory go in two launches (a row's bits do not depend on the rest).
 template <int PF>
-static void launch_dense(cudaStream_t s, MvParams a, int T) {
+static void launch_dense(cudaStream_t s, MvParams a, int T, DenseSet* set = NULL) {
     const size_t one = staged_bytes(a.K / 64), room = (size_t) max_smem_optin() - 8192;
     while (T > 0) {
         int n = T;
         while (n > 1 && n * one > room) n = (n + 1) / 2;
         switch (n) {
-#define NSL_CASE(N) case N: launch_dense_v<PF, N>(s, a, N * one); break;
+#define NSL_CASE(N) case N: launch_dense_v<PF, N>(s, a, N * one, set); break;
             NSL_CASE(1) NSL_CASE(2) NSL_CASE(3) NSL_CASE(4) NSL_CASE(5) NSL_CASE(6) NSL_CASE(7) NSL_CASE(8)
 #undef NSL_CASE
         }
         a.x += (size_t) n * a.xs;
         a.y += (size_t) n * a.ys;
+        for (int m = 0; set && m < set->n; ++m) set->y[m] += (size_t) n * set->R[m];
         T -= n;
     }
 }
@@ -1430,6 +1460,16 @@ static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse&
         if (a.P > GRP_MIN_PAIRS && !rf.logits && ch >= 4 && ch <= 32 && (ch & (ch - 1)) == 0) { launch_grp<MODE>(s, a, log2_floor(ch)); return; }
     }
     launch_pair<MODE, PF>(s, a, rf);
+}
+
+// A set of SEED4P4 matrices for up to MV_MAXT rows; false: a shape that needs the any-shape kernel.
+bool launch_seed_set(cudaStream_t s, DenseSet set, int K, const float* x, int T, const uint32_t* G) {
+    if (T < 1 || T > MV_MAXT || K < 64 || K % 64 || !aligned16(x) || staged_bytes(K / 64) > (size_t) max_smem_optin() - 10240) return false;
+    for (int m = 0; m < set.n; ++m)
+        if (set.R[m] < 1 || !slice_aligned(set.w[m])) return false;
+    MvParams a = {NULL, NULL, set.w[0], NULL, x, set.y[0], G, K, set.R[0], T, 1, K, set.R[0], 0, 0, NULL, NULL, 0};
+    launch_dense<4>(s, a, T, &set);
+    return true;
 }
 
 // The decode step in one launch; false (nothing launched) when a size is outside what the pair kernel serves.
