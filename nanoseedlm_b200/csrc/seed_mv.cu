@@ -316,62 +316,10 @@ __device__ __forceinline__ void pair_rows(const StreamTab& tab, const KConst& kc
     if (cnt) flush(st - cnt * STEPS * MV_WARPS, r - cnt * STEPS * S);
 }
 
-// The same for rows of any number of chunks: a row is cut into groups of lpr chunks, an ITEM is one group of the 32 / lpr rows of
-// a row step, and a block's warps take the items of its share one by one, so the work is even to within one chunk a warp
-// whatever the row's length.  A group's sum (the butterfly over its lanes) waits in shared memory; the row's is the groups'
-// sum in order.  PART_STEPS row steps at a time.
-constexpr int PART_FLOATS = 2048;
-__host__ __device__ __forceinline__ int part_steps(int groups, int lpr_log2, int mats) { return PART_FLOATS / (groups * (32 >> lpr_log2) * mats); }
-
-template <int MODE, int PF, typename Store>
-__device__ __forceinline__ void pair_items(const StreamTab& tab, const KConst& kc, const WSlice& wa, const WSlice& wb, const ulonglong2* sx, float* part,
-                                           RowShape sh, int R, int s_lo, int s_hi, Chunk ka, Chunk kb, Store store) {
-    constexpr int MATS = MODE == MODE_GU ? 2 : 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int lpr = 1 << sh.lpr_log2, rpw = 32 >> sh.lpr_log2, ch = sh.ch, groups = sh.groups;
-    const int jc = lane & (lpr - 1), ro = lane >> sh.lpr_log2;
-    const float sca = slice_scale(wa.eb + (8 - PF)), scb = slice_scale(wb.eb + (8 - PF));
-    const int span = part_steps(groups, sh.lpr_log2, MATS);
-    int done = s_lo, st = s_lo + warp / groups, g = warp % groups;      // this warp's item; its streams are in ka / kb
-    while (done < s_hi) {
-        const int upto = min(s_hi, done + span);
-        while (st < upto) {
-            int gn = g + MV_WARPS, sn = st;
-            while (gn >= groups) { gn -= groups; ++sn; }
-            const int r = st * rpw + ro, j = g * lpr + jc, rn = sn * rpw + ro, jn = gn * lpr + jc;
-            Chunk na, nb;
-            if (sn < s_hi && rn < R && jn < ch) {
-                na = load_chunk<PF>(wa, (size_t) rn * ch + jn);
-                if (MODE == MODE_GU) nb = load_chunk<PF>(wb, (size_t) rn * ch + jn);
-            }
-            u64 acc = 0ull, accu = 0ull;
-            if (r < R && j < ch) chunk_dots<MODE, PF>(tab, kc, ka, kb, sx + j * CX, acc, accu);
-            const float s = group_sum(pair_total(acc), lpr);
-            float su = 0.0f;
-            if (MODE == MODE_GU) su = group_sum(pair_total(accu), lpr);
-            if (jc == 0) {
-                float* at = part + (((st - done) * rpw + ro) * groups + g) * MATS;
-                at[0] = s;
-                if (MODE == MODE_GU) at[1] = su;
-            }
-            ka = na;
-            if (MODE == MODE_GU) kb = nb;
-            st = sn; g = gn;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < (upto - done) * rpw; i += MV_THREADS) {
-            const float* at = part + i * groups * MATS;
-            float s = at[0], su = MODE == MODE_GU ? at[1] : 0.0f;
-            for (int q = 1; q < groups; ++q) {
-                s += at[q * MATS];
-                if (MODE == MODE_GU) su += at[q * MATS + 1];
-            }
-            if (done * rpw + i < R) store(done * rpw + i, s * sca, su * scb);
-        }
-        done = upto;
-        if (done < s_hi) __syncthreads();      // the sums are read before the next span's are written
-    }
-}
+// Rows of any other number of chunks: a row is cut into groups of lpr chunks (item_shape), a group's sum is the butterfly over its
+// lanes, the row's the groups' sum in order.
+constexpr int PART_FLOATS = 4096, PART_FLOATS_MIN = 2048;      // groups' sums that wait in shared memory, if the inputs leave room for them (the longest rows: at least the ch floats of a step of 8 lanes a row)
+__host__ __device__ __forceinline__ int part_steps(int floats, int groups, int lpr_log2, int mats) { return floats / (groups * (32 >> lpr_log2) * mats); }
 
 // The router in a kernel's prologue: warp t picks token t's top-k experts; block 0 also stores ids and weights for the kernels that
 // follow.  Ends with a barrier.
@@ -533,54 +481,147 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KC
     }
 }
 
-// ---- the same for rows of any number of chunks (pair_items), two blocks of 8 warps per SM -----------------------------------
+// ---- the same for rows of any number of chunks ------------------------------------------------------------------------------
+// An ITEM is one group of the 32 / lpr rows of a row step (or, with spi = 2, of two steps of the one matrix, which then share the inputs'
+// loads), so the work is even to within one chunk a warp whatever the row's length; the warps fetch the items of a
+// window of row steps one by one.  The groups' sums wait in shared memory until the window is done: the end of a window is a
+// barrier, and a small call's share is one window.  (Two blocks of 8 warps an SM with the items dealt in advance: 47.9 us
+// for 5 rows, top 4, of a layer 1536 / 704 wide.)
 template <int MODE, int PF>
-__global__ void __launch_bounds__(MV_THREADS, 2) mv_items_kernel(MvParams a, KConst kc, RowShape sh, RouteFuse rf) {
-    extern __shared__ __align__(16) ulonglong2 pair_sx[];
+__global__ void __launch_bounds__(PAIR_THREADS, 1) mv_items_kernel(MvParams a, KConst kc, RowShape sh, int win, int part_floats, int spi, RouteFuse rf) {
+    extern __shared__ __align__(16) ulonglong2 pair_sx[];      // [win][ch * CX], then the sums
     __shared__ StreamTab tab;
-    __shared__ float part[PART_FLOATS];
     __shared__ int32_t r_ind[256];   // the fused router's picks
     __shared__ float r_wt[256];
-    load_stream_tab(tab, a.G, threadIdx.x, MV_THREADS);
+    __shared__ PairDesc desc[PAIR_WIN];
+    __shared__ int next_item;
+    constexpr int MATS = MODE == MODE_GU ? 2 : 1;
+    load_stream_tab(tab, a.G, threadIdx.x, PAIR_THREADS);
     grid_dependents_go();
     grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, ch = sh.ch, groups = sh.groups;
     const int lpr = 1 << sh.lpr_log2, rpw = 32 >> sh.lpr_log2;
-    const int ch = sh.ch;
+    const int jc = lane & (lpr - 1), ro = lane >> sh.lpr_log2;
     int P = a.count ? min(*a.count, a.P) : a.P;
     if (rf.logits) {
         route_prologue(rf, r_ind, r_wt);
         P = rf.T * rf.top_k;
     }
-    const int rs = (a.R + rpw - 1) / rpw;
+    float* const part = (float*) (pair_sx + (size_t) win * ch * CX);
+    const int rs = (a.R + rpw - 1) / rpw, span = part_steps(part_floats, groups, sh.lpr_log2, MATS);
     const long long total = (long long) P * rs;
     const long long begin = (long long) blockIdx.x * total / gridDim.x, end = (long long) (blockIdx.x + 1) * total / gridDim.x;
-    if (begin >= end) return;
-    const int p_first = (int) (begin / rs), p_last = (int) ((end - 1) / rs);
-    for (int pair = p_first; pair <= p_last; ++pair) {
-        const int s_lo = pair == p_first ? (int) (begin - (long long) pair * rs) : 0;
-        const int s_hi = pair == p_last ? (int) (end - (long long) pair * rs) : rs;
-        const int slice = rf.logits ? r_ind[pair] : (a.sel ? a.sel[pair] : 0);
-        const WSlice wa = a.ws ? a.ws[slice] : a.w0;
-        WSlice wb = wa;
-        if (MODE == MODE_GU) wb = a.wu[slice];
-        // this warp's first streams are requested before the inputs are staged: their DRAM latency runs under it
-        const int st = s_lo + warp / sh.groups, r = st * rpw + (lane >> sh.lpr_log2), jc = (lane & (lpr - 1)) + warp % sh.groups * lpr;
-        Chunk ka, kb;
-        if (st < s_hi && r < a.R && jc < ch) {
-            ka = load_chunk<PF>(wa, (size_t) r * ch + jc);
-            if (MODE == MODE_GU) kb = load_chunk<PF>(wb, (size_t) r * ch + jc);
+    const float inv_rs = 1.0f / (float) rs, inv_groups = 1.0f / (float) groups;
+    auto divide = [](int v, float inv, int d) {      // v / d for v < 2^23
+        int q = (int) ((float) v * inv);
+        if (q * d > v) --q;
+        return (q + 1) * d <= v ? q + 1 : q;
+    };
+    for (long long w0 = begin; w0 < end;) {
+        const int p0 = (int) (w0 / rs), lo = (int) (w0 - (long long) p0 * rs);      // the window's first pair, its first step there
+        const long long most = (long long) win * rs - lo;
+        const int n = (int) min(min(end - w0, (long long) span), most), np = (lo + n + rs - 1) / rs;
+        const int items = (n + spi - 1) / spi * groups;
+        if (w0 != begin) __syncthreads();      // the previous window is no longer read
+        if ((int) threadIdx.x < np) {
+            const int pair = p0 + threadIdx.x, slice = rf.logits ? r_ind[pair] : (a.sel ? a.sel[pair] : 0);
+            const WSlice wa = a.ws ? a.ws[slice] : a.w0;
+            PairDesc d = {wa.p[0], wa.p[1], wa.p[3], NULL, NULL, NULL, slice_scale(wa.eb + (8 - PF)), 0.0f, pair, 0};
+            if (MODE == MODE_GU) {
+                const WSlice wb = a.wu[slice];
+                d.sb = wb.p[0]; d.cb = wb.p[1]; d.db = wb.p[3];
+                d.scb = slice_scale(wb.eb + (8 - PF));
+            }
+            desc[threadIdx.x] = d;
         }
-        if (pair != p_first) __syncthreads();   // the previous pair's inputs are no longer read
-        const void* row = input_row(a, a.xrow ? a.xrow[pair] : pair / a.xdiv);
-        for (int i = threadIdx.x; i < ch * 4; i += MV_THREADS) {
+        if (threadIdx.x == 0) next_item = PAIR_WARPS;
+        for (int i = threadIdx.x; i < np * ch * 4; i += PAIR_THREADS) {
+            const int t = i / (ch * 4), e = i - t * (ch * 4), pair = p0 + t;
             float x[16];
-            stage_load(row, a.xbf16, i >> 2, i & 3, x);
-            stage_store<PF>(x, i >> 2, i & 3, pair_sx);
+            stage_load(input_row(a, a.xrow ? a.xrow[pair] : pair / a.xdiv), a.xbf16, e >> 2, e & 3, x);
+            stage_store<PF>(x, e >> 2, e & 3, pair_sx + (size_t) t * ch * CX);
         }
-        __syncthreads();   // inputs staged (and, for the block's first pair, the stream table loaded)
-        pair_items<MODE, PF>(tab, kc, wa, wb, pair_sx, part, sh, a.R, s_lo, s_hi, ka, kb,
-                             [&](int rr, float s, float su) { store_out<MODE>(a, pair, rr, s, su); });
+        __syncthreads();      // (and, the first time, the stream table is loaded)
+        auto locate = [&](int k, int& t, int& r) {      // the window's step k -> its pair, this lane's row
+            t = divide(lo + k, inv_rs, rs);
+            r = (lo + k - t * rs) * rpw + ro;
+        };
+        auto fetch_a = [&](const PairDesc& d, uint32_t at, Chunk& k) {
+            k.s = __ldg((const uint4*) d.sa + at);
+            k.c = __ldg((const uint4*) d.ca + at);
+            if (PF == 4) k.cd = __ldg((const uint32_t*) d.da + at);
+        };
+        struct At { int k, g, t, r; };      // an item: its (first) step, group, the step's pair, this lane's row
+        auto load = [&](int it, At& at_it, Chunk& ka, Chunk& kb) {
+            if (it >= items) return;
+            const int u = divide(it, inv_groups, groups), g = it - u * groups, j = g * lpr + jc;
+            int t, r;
+            locate(u * spi, t, r);
+            at_it = At{u * spi, g, t, r};
+            if (j >= ch) return;
+            if (r < a.R) {
+                const PairDesc& d = desc[t];
+                const uint32_t at = (uint32_t) (r * ch + j);
+                fetch_a(d, at, ka);
+                if (MODE == MODE_GU) {
+                    kb.s = __ldg((const uint4*) d.sb + at);
+                    kb.c = __ldg((const uint4*) d.cb + at);
+                    if (PF == 4) kb.cd = __ldg((const uint32_t*) d.db + at);
+                }
+            }
+            if (MODE != MODE_GU && spi == 2 && u * 2 + 1 < n) {
+                locate(u * 2 + 1, t, r);
+                if (r < a.R) fetch_a(desc[t], (uint32_t) (r * ch + j), kb);
+            }
+        };
+        int it = threadIdx.x >> 5;
+        Chunk ka, kb;
+        At cur = {0, 0, 0, 0};
+        load(it, cur, ka, kb);
+        while (it < items) {
+            int nx = 0;
+            if (lane == 0) nx = atomicAdd(&next_item, 1);
+            nx = __shfl_sync(0xFFFFFFFFu, nx, 0);
+            Chunk na, nb;
+            const At now = cur;
+            load(nx, cur, na, nb);
+            const int k = now.k, g = now.g, t = now.t, r = now.r, j = g * lpr + jc;
+            u64 acc[2] = {0ull, 0ull};
+            const ulonglong2* const cx = pair_sx + (size_t) (t * ch + j) * CX;
+            const bool two = MODE != MODE_GU && spi == 2 && k + 1 < n;
+            int t2 = t, r2 = r;
+            if (two) locate(k + 1, t2, r2);
+            if (j < ch) {
+                if (MODE == MODE_GU) {
+                    if (r < a.R) chunk_dots<MODE_GU, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);
+                } else if (two && t2 == t) {      // (r2 > r; a row that is not there: whatever the registers hold, never stored)
+                    if (r < a.R) chunk_dots<MODE_GU, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);
+                } else {
+                    if (r < a.R) chunk_dots<MODE_ROUND, PF>(tab, kc, ka, ka, cx, acc[0], acc[1]);
+                    if (two && r2 < a.R) chunk_dots<MODE_ROUND, PF>(tab, kc, kb, kb, pair_sx + (size_t) (t2 * ch + j) * CX, acc[1], acc[0]);
+                }
+            }
+            const float v[2] = {pair_total(acc[0]), pair_total(acc[1])};
+            const float mine = split_sum<2>(v, lpr, jc);      // value 0 ends in the row's lower lanes, value 1 in the upper ones
+            if (MODE == MODE_GU) {
+                if ((jc & (lpr / 2 - 1)) == 0) part[((k * rpw + ro) * groups + g) * 2 + (jc ? 1 : 0)] = mine;
+            } else if (jc == 0 || (two && jc == lpr / 2)) part[((k + (jc ? 1 : 0)) * rpw + ro) * groups + g] = mine;
+            it = nx;
+            ka = na;
+            kb = nb;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < n * rpw; i += PAIR_THREADS) {
+            const int k = i >> (5 - sh.lpr_log2), t = divide(lo + k, inv_rs, rs), r = (lo + k - t * rs) * rpw + (i & (rpw - 1));
+            const float* const at = part + (size_t) i * groups * MATS;
+            float s = at[0], su = MODE == MODE_GU ? at[1] : 0.0f;
+            for (int q = 1; q < groups; ++q) {
+                s += at[q * MATS];
+                if (MODE == MODE_GU) su += at[q * MATS + 1];
+            }
+            if (r < a.R) store_out<MODE>(a, desc[t].pair, r, s * desc[t].sca, su * desc[t].scb);
+        }
+        w0 += n;
     }
 }
 
@@ -1132,7 +1173,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_dense_kernel(MvParams a, KCo
     extern __shared__ __align__(16) ulonglong2 dense_sx[];
     __shared__ StreamTab tab;
     int block = blockIdx.x, blocks = gridDim.x;
-    if (set.n > 1) {
+    if (set.n > 1) {      // several matrices share the launch
         const int m = set_member(set, block);
         block -= set.first[m];
         blocks = set.first[m + 1] - set.first[m];
@@ -1343,7 +1384,7 @@ static RowShape item_shape(int ch) {
     for (int l = 3; l >= 1; --l) {
         const int groups = (ch + (1 << l) - 1) >> l;
         const double cost = (double) (groups << l) / ch + 0.05 * (3 - l);
-        if (cost < best_cost && part_steps(groups, l, 2) >= 1) { best.lpr_log2 = l; best.groups = groups; best_cost = cost; }
+        if (cost < best_cost && part_steps(PART_FLOATS_MIN, groups, l, 2) >= 1) { best.lpr_log2 = l; best.groups = groups; best_cost = cost; }
     }
     return best;
 }
@@ -1359,9 +1400,23 @@ static void launch_pair(cudaStream_t s, const MvParams& a, const RouteFuse& rf) 
         allow_smem(mv_pair_kernel<MODE, PF>, attr_set, (size_t) PAIR_WIN * 32 * CX * 16);
         launch(mv_pair_kernel<MODE, PF>, sms, PAIR_THREADS, win * staged_bytes(ch), s, a, kconst(), lpr_log2, win, rf);
     } else {
-        const size_t smem = staged_bytes(ch);
-        if (smem > 40 * 1024) allow_smem(mv_items_kernel<MODE, PF>, attr_set_items, (size_t) max_smem_optin() - 10240);
-        launch(mv_items_kernel<MODE, PF>, sms * 2, MV_THREADS, smem, s, a, kconst(), item_shape(ch), rf);
+        const RowShape sh = item_shape(ch);
+        const size_t room = (size_t) max_smem_optin() - 6144, one = staged_bytes(ch);      // 6144: the kernel's other shared memory (launch_mv has made sure that one row and the fewest sums fit)
+        const int rpw = 32 >> sh.lpr_log2;
+        const long long steps = ((long long) a.P * ((a.R + rpw - 1) / rpw) + sms - 1) / sms;      // of a block
+        int win = a.P / sms + 2;
+        if (win > PAIR_WIN) win = PAIR_WIN;
+        if (win > a.P) win = a.P;
+        while (win > 1 && win * one + PART_FLOATS * 4 > room) --win;
+        size_t part = (room - win * one) / 4;
+        if (part > PART_FLOATS) part = PART_FLOATS;
+        const size_t need = (size_t) (steps + 1) * sh.groups * rpw * (MODE == MODE_GU ? 2 : 1);
+        if (part > need) part = need;
+        // Two steps of the one matrix an item where a warp still gets eight items: they share the inputs' loads, but fewer items are
+        // dealt less evenly.
+        const int spi = MODE != MODE_GU && steps * sh.groups >= 16 * PAIR_WARPS ? 2 : 1;
+        allow_smem(mv_items_kernel<MODE, PF>, attr_set_items, room);
+        launch(mv_items_kernel<MODE, PF>, sms, PAIR_THREADS, win * one + part * 4, s, a, kconst(), sh, win, (int) part, spi, rf);
     }
     count_launch();
 }
@@ -1382,7 +1437,6 @@ static void launch_grp(cudaStream_t s, const MvParams& a, int lpr_log2) {
 template <int PF, int NT>
 static void launch_dense_v(cudaStream_t s, const MvParams& a, size_t smem, DenseSet* set) {
     static bool attr_set[16];
-    if (smem > 40 * 1024) allow_smem(mv_dense_kernel<PF, NT>, attr_set, (size_t) max_smem_optin() - 8192);
     const int bps = smem > 100 * 1024 ? 1 : 2;
     long long rows = a.R;
     for (int m = 1; set && m < set->n; ++m) rows += set->R[m];
@@ -1404,6 +1458,7 @@ static void launch_dense_v(cudaStream_t s, const MvParams& a, size_t smem, Dense
         }
         blocks = set->first[DENSE_SET];
     }
+    if (smem > 40 * 1024) allow_smem(mv_dense_kernel<PF, NT>, attr_set, (size_t) max_smem_optin() - 8192);
     launch(mv_dense_kernel<PF, NT>, blocks, MV_THREADS, smem, s, a, kconst(), sh, set ? *set : DenseSet{1});
     count_launch();
 }
