@@ -11,7 +11,8 @@
 #include "seed_mma.cuh"
 
 namespace nsl {
-void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* perm, uint16_t* y, int P, int xdiv, int d);
+void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* at, uint16_t* y, int T, int k, int d);
+void bucket(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles, int32_t* at);
 void launch_combine_packed(cudaStream_t s, int d, int k, const uint16_t* D, const float* wt, float* out, int T);
 }
 
@@ -123,7 +124,8 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
         nsl::PdlScope pdl(m->pdl);      // every kernel of the sequence waits on the device for its predecessor
         const int mt = P / MMT_BN + m->n_exp;
         nsl_route(s, m->n_exp, k, logits, m->n_exp, m->ind, m->wt, T);
-        kc_bucket(s, m->ind, P, m->n_exp, m->perm, m->tiles, m->ntiles);
+        int32_t* const at = (int32_t*) m->Gb;      // the pairs' places by expert, where the rows are packed in that order (Gb: the exact path's)
+        nsl::bucket(s, m->ind, P, m->n_exp, m->perm, m->tiles, m->ntiles, !nsl::seed_gemm_exact() && P / m->n_exp >= 96 ? at : NULL);
         if (!nsl::seed_gemm_exact() && d % 64 == 0 && ff % 64 == 0) {
             // gate, up and SwiGLU in one launch, results as packed bf16 (they are bf16 values); the down projections' rows stay packed too
             const int avg = P / m->n_exp;
@@ -135,7 +137,7 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
                 // the rows are packed in the order of the pairs by expert (4096 rows of config 1's layer: 549 -> 486 us; at 32
                 // rows an expert the copy costs what it saves)
                 uint16_t* const xs = D + (size_t) P * d;
-                nsl::launch_pack_sorted(s, x, m->perm, xs, P, k, d);
+                nsl::launch_pack_sorted(s, x, at, xs, T, k, d);
                 g.X = xs;
                 g.in_sorted = g.out_sorted = w.in_sorted = 1;
                 g.T_in = w.T_in = P;

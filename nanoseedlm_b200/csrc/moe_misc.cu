@@ -177,22 +177,30 @@ __global__ void pack_bf16_kernel(const float* __restrict__ x, uint16_t* __restri
     if (blockIdx.x == 0 && threadIdx.x < (n & 7)) y[n8 * 8 + threadIdx.x] = bf16_bits(x[n8 * 8 + threadIdx.x]);
 }
 
-// Row n of y = row perm[n] / xdiv of x as packed bf16 (d a multiple of 8; a thread: 8 values).
-__global__ void __launch_bounds__(256) pack_sorted_kernel(const float4* __restrict__ x, const int32_t* __restrict__ perm, uint4* __restrict__ y, int xdiv, int d8,
-                                                          int P) {
+// Packed bf16 rows in the order of the pairs by expert: row at[t * k + j] of y = row t of x for each of its k pairs (d a multiple of 8;
+// a thread: 8 values, read and converted once).  Bound by the writes: 32768 rows of 2048 from 4096 in 30 us; a row of y at a time, its
+// inputs read again for every pair, took 51.
+__global__ void __launch_bounds__(256) pack_sorted_kernel(const float4* __restrict__ x, const int32_t* __restrict__ at, uint4* __restrict__ y, int k, int d8,
+                                                          int T) {
+    __shared__ int pos[32];
     grid_dependency_wait();
     grid_dependents_go();
-    for (int row = blockIdx.x; row < P; row += gridDim.x) {
-        const float4* xp = x + (size_t) (__ldg(perm + row) / xdiv) * d8 * 2;
+    for (int t = blockIdx.x; t < T; t += gridDim.x) {
+        __syncthreads();      // the previous row's places are no longer read
+        if ((int) threadIdx.x < k) pos[threadIdx.x] = __ldg(at + (size_t) t * k + threadIdx.x);
+        __syncthreads();
+        const float4* xp = x + (size_t) t * d8 * 2;
         for (int c = threadIdx.x; c < d8; c += 256) {
             const float4 a = __ldg(xp + 2 * c), b = __ldg(xp + 2 * c + 1);
-            y[(size_t) row * d8 + c] = make_uint4(bf16x2_bits(a.x, a.y), bf16x2_bits(a.z, a.w), bf16x2_bits(b.x, b.y), bf16x2_bits(b.z, b.w));
+            const uint4 v = make_uint4(bf16x2_bits(a.x, a.y), bf16x2_bits(a.z, a.w), bf16x2_bits(b.x, b.y), bf16x2_bits(b.z, b.w));
+            for (int j = 0; j < k; ++j)
+                if ((unsigned) pos[j] < (unsigned) (T * k)) y[(size_t) pos[j] * d8 + c] = v;      // (a pair of no expert has no place)
         }
     }
 }
-void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* perm, uint16_t* y, int P, int xdiv, int d) {
+void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* at, uint16_t* y, int T, int k, int d) {
     const int cap = sm_count() * 8;
-    launch(pack_sorted_kernel, (unsigned) (P < cap ? P : cap), 256, 0, s, (const float4*) x, perm, (uint4*) y, xdiv, d / 8, P);
+    launch(pack_sorted_kernel, (unsigned) (T < cap ? T : cap), 256, 0, s, (const float4*) x, at, (uint4*) y, k, d / 8, T);
     count_launch();
 }
 
@@ -238,7 +246,7 @@ __global__ void __launch_bounds__(1024) bucket_count_kernel(const int32_t* __res
 // within the expert.
 __global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* __restrict__ inds, int count,
                                                             const int32_t* __restrict__ work, int32_t* __restrict__ perm,
-                                                            MmTile* __restrict__ tiles) {
+                                                            MmTile* __restrict__ tiles, int32_t* __restrict__ at_out) {
     __shared__ int wcount[32];
     const int e = blockIdx.x, n = gridDim.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     grid_dependency_wait();
@@ -279,7 +287,10 @@ __global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* __res
             int pos = at + __popc(m[0] & below) + __popc(m[1] & below) + __popc(m[2] & below) + __popc(m[3] & below);
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                if (f[q]) perm[pos++] = i + q;
+                if (f[q]) {
+                    if (at_out) at_out[i + q] = pos;      // the inverse of perm
+                    perm[pos++] = i + q;
+                }
             at += __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
         }
     }
@@ -288,6 +299,14 @@ __global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* __res
         MmTile tl = {e, begin + t * MMT_BN, total - t * MMT_BN < MMT_BN ? total - t * MMT_BN : MMT_BN, 0};
         tiles[t0 + t] = tl;
     }
+}
+
+// kc_bucket; at (optional, count ints): every pair's place in perm.
+void bucket(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles, int32_t* at) {
+    if (n < 1 || n > BUCKET_MAX_EXPERTS) { set_error("kc_bucket: %d experts, at most %d", n, BUCKET_MAX_EXPERTS); return; }
+    launch(bucket_count_kernel, 1, 1024, 0, s, inds, count, n, ntiles);
+    launch(bucket_place_kernel, (unsigned) n, 1024, 0, s, inds, count, (const int32_t*) ntiles, perm, tiles, at);
+    count_launch(2);
 }
 
 // ---- expert cache -----------------------------------------------------------------------------------------------------
@@ -547,12 +566,7 @@ void kc_pack_input_bf16(cudaStream_t s, const float* x, uint16_t* y, size_t n) {
     count_launch();
 }
 
-void kc_bucket(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles) {
-    if (n < 1 || n > BUCKET_MAX_EXPERTS) { set_error("kc_bucket: %d experts, at most %d", n, BUCKET_MAX_EXPERTS); return; }
-    launch(bucket_count_kernel, 1, 1024, 0, s, inds, count, n, ntiles);
-    launch(bucket_place_kernel, (unsigned) n, 1024, 0, s, inds, count, (const int32_t*) ntiles, perm, tiles);
-    count_launch(2);
-}
+void kc_bucket(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles) { nsl::bucket(s, inds, count, n, perm, tiles, ntiles, NULL); }
 
 void nsl_bucket_noalloc(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles_out) {
     if (n < 1 || n > BUCKET_MAX_EXPERTS) {
@@ -563,7 +577,7 @@ void nsl_bucket_noalloc(cudaStream_t s, const int32_t* inds, int count, int n, i
     if (!work) return;
     // every entry the placement reads is rewritten by the count kernel, so nothing has to be cleared between calls
     launch(bucket_count_kernel, 1, 1024, 0, s, inds, count, n, work);
-    launch(bucket_place_kernel, (unsigned) n, 1024, 0, s, inds, count, (const int32_t*) work, perm, tiles);
+    launch(bucket_place_kernel, (unsigned) n, 1024, 0, s, inds, count, (const int32_t*) work, perm, tiles, (int32_t*) NULL);
     launch(bucket_publish_kernel, 1, 32, 0, s, (const int32_t*) work, ntiles_out);
     count_launch(3);
 }

@@ -201,35 +201,54 @@ __device__ __forceinline__ float sigmoid(float g) {
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
 
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {      // each product rounded once
+    uint32_t d;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
 // The results of a unit, by the producer warps: warp w reads the tensor memory lanes of its quarter, 16 columns at a time, the
 // warpgroups taking turns.  col: the unit's first column.  bf16 results are turned round in 1 KB of shared memory a warp (box), so
 // that a lane stores 16 bytes of one row of outputs: with 2-byte stores straight from the registers the results of a 256-row unit
-// took 8400 clk, a quarter of its expansion.
-template <bool GU, int GROUPS>
+// took 8400 clk, a quarter of its expansion.  No MMA of the next unit runs meanwhile where a unit fills the accumulators, so the
+// instructions count: two columns at a time from the first rounding on (SwiGLU column by column: 6000 clk a unit), the places of
+// the next columns' rows requested ahead (AHEAD).
+template <bool GU, int GROUPS, bool AHEAD>
 __device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, uint16_t* box, int col, int start, int count, int r0) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lq = warp & 3;
     constexpr int ROWS = GU ? 16 : 32;      // rows of outputs' values a warp makes of its 32 lanes
     const int row0 = r0 + lq * ROWS;
+    auto place = [&](int c0) {      // lane j: column c0 + j's row of outputs
+        const int p = start + min(c0 + (lane & 15), count - 1);
+        return a.grouped && !a.out_sorted ? a.perm[p] : p;
+    };
+    int dst_next = AHEAD ? place((warp >> 2) * 16) : 0;
     for (int c0 = (warp >> 2) * 16; c0 < count; c0 += GROUPS * 16) {
         uint32_t v[16];
-        const int p = start + min(c0 + (lane & 15), count - 1), dst_lane = a.grouped && !a.out_sorted ? a.perm[p] : p;      // lane j: column c0 + j's place
+        const int dst_lane = AHEAD ? dst_next : place(c0);
         tmem_ld16(tmem + ((uint32_t) (lq * 32) << 16) + (uint32_t) (col + c0), v);
+        if (AHEAD) dst_next = place(c0 + GROUPS * 16);
         if (GU || a.out_bf16) {      // (R and ys are multiples of 8 here)
-            if (GU) {
-                uint16_t* const at = box + (lane & 1) * 8 * ROWS + (lane >> 1);      // even lanes finish columns 0..7, odd lanes 8..15
+            uint32_t two[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const float lo = __uint_as_float(v[j]), hi = __uint_as_float(v[j + 8]);
-                    const float from = __shfl_xor_sync(0xFFFFFFFFu, lane & 1 ? lo : hi, 1), mine = lane & 1 ? hi : lo;
-                    const float g = to_bf16(lane & 1 ? from : mine), up = to_bf16(lane & 1 ? mine : from);
-                    at[j * ROWS] = (uint16_t) bf16x2_bits(to_bf16(g * to_bf16(sigmoid(g))) * up, 0.0f);
+            for (int j = 0; j < 8; ++j) two[j] = bf16x2_bits(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+            if (GU) {
+                const bool odd = lane & 1;
+                uint16_t* const at = box + (odd ? 8 * ROWS : 0) + (lane >> 1);      // even lanes finish columns 0..7, odd lanes 8..15
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t mine = odd ? two[j + 4] : two[j], from = __shfl_xor_sync(0xFFFFFFFFu, odd ? two[j] : two[j + 4], 1);
+                    const uint32_t g = odd ? from : mine, up = odd ? mine : from;
+                    const uint32_t sg = bf16x2_bits(sigmoid(__uint_as_float(g << 16)), sigmoid(__uint_as_float(g & 0xFFFF0000u)));
+                    const uint32_t o = mul_bf16x2(mul_bf16x2(g, sg), up);
+                    at[2 * j * ROWS] = (uint16_t) o;
+                    at[(2 * j + 1) * ROWS] = (uint16_t) (o >> 16);
                 }
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const uint32_t two = bf16x2_bits(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-                    box[2 * j * ROWS + lane] = (uint16_t) two;
-                    box[(2 * j + 1) * ROWS + lane] = (uint16_t) (two >> 16);
+                    box[2 * j * ROWS + lane] = (uint16_t) two[j];
+                    box[(2 * j + 1) * ROWS + lane] = (uint16_t) (two[j] >> 16);
                 }
             }
             __syncwarp();
@@ -330,7 +349,7 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
             ok = __all_sync(0xFFFFFFFFu, ok);
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                unit_results<GU, GROUPS>(a, tmem, box + warp * 512, p_col, p_start, p_count, p_r0);
+                unit_results<GU, GROUPS, (TT > 1)>(a, tmem, box + warp * 512, p_col, p_start, p_count, p_r0);
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {
