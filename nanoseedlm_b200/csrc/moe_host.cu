@@ -13,6 +13,7 @@
 namespace nsl {
 void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* at, uint16_t* y, int T, int k, int d);
 void bucket(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles, int32_t* at);
+void bucket_pack(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles, const float* x, uint16_t* xp, size_t pack_n);
 void launch_combine_packed(cudaStream_t s, int d, int k, const uint16_t* D, const float* wt, float* out, int T);
 }
 
@@ -124,15 +125,17 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
         nsl::PdlScope pdl(m->pdl);      // every kernel of the sequence waits on the device for its predecessor
         const int mt = P / MMT_BN + m->n_exp;
         nsl_route(s, m->n_exp, k, logits, m->n_exp, m->ind, m->wt, T);
+        const int avg = P / m->n_exp;
+        const bool fast = !nsl::seed_gemm_exact() && d % 64 == 0 && ff % 64 == 0, sorted = fast && avg >= 96 && nsl::gemm_shares_tiles(mt);
         int32_t* const at = (int32_t*) m->Gb;      // the pairs' places by expert, where the rows are packed in that order (Gb: the exact path's)
-        nsl::bucket(s, m->ind, P, m->n_exp, m->perm, m->tiles, m->ntiles, !nsl::seed_gemm_exact() && P / m->n_exp >= 96 ? at : NULL);
-        if (!nsl::seed_gemm_exact() && d % 64 == 0 && ff % 64 == 0) {
+        if (sorted) nsl::bucket(s, m->ind, P, m->n_exp, m->perm, m->tiles, m->ntiles, at);
+        else nsl::bucket_pack(s, m->ind, P, m->n_exp, m->perm, m->tiles, m->ntiles, x, m->xp, (size_t) T * d);      // packed once: every row tile of every expert reads them
+        if (fast) {
             // gate, up and SwiGLU in one launch, results as packed bf16 (they are bf16 values); the down projections' rows stay packed too
-            const int avg = P / m->n_exp;
             uint16_t* const D = (uint16_t*) m->Dx;      // packed rows take half of the f32 buffer; the sorted inputs have the other half
             nsl::MmParams g = {m->wg, WSlice{}, m->xp, m->Ap, m->perm, m->tiles, m->ntiles, m->G, d, ff, 0, d, ff, k, 0, 1, 1, m->wu, 1, NULL, 0, 0, 0};
             nsl::MmParams w = {m->wd, WSlice{}, m->Ap, D, m->perm, m->tiles, m->ntiles, m->G, ff, d, 0, ff, d, 1, 0, 1, 1, NULL, 1, NULL, 0, 0, 0};
-            if (avg >= 96 && nsl::gemm_shares_tiles(mt)) {
+            if (sorted) {
                 // many rows an expert: one expansion for up to 384 of them, whose inputs are fetched as boxes of consecutive rows, so
                 // the rows are packed in the order of the pairs by expert (4096 rows of config 1's layer: 549 -> 486 us; at 32
                 // rows an expert the copy costs what it saves)
@@ -145,7 +148,6 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
                 nsl::launch_gemm_gu(s, g, mt);
                 nsl::launch_gemm(s, MF_SEED4P4, "nsl_moe_forward", w, mt);
             } else {
-                kc_pack_input_bf16(s, x, m->xp, (size_t) T * d);      // once: every row tile of every expert reads them
                 if (avg < 6) {      // few rows an expert: the kernel that keeps the weights in registers (128 experts, us, against the other: 209 / 227 at 1.5 rows, 263 / 265 at 4, 272 / 270 at 6, 282 / 269 at 7.5)
                     nsl::launch_seed_mma_grouped(s, g);
                     nsl::launch_seed_mma_grouped(s, w);
@@ -157,7 +159,6 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
             nsl::launch_combine_packed(s, d, k, D, m->wt, out, T);
             return 0;
         }
-        kc_pack_input_bf16(s, x, m->xp, (size_t) T * d);
         kc_mm_grouped_packed(s, MF_SEED4P4, m->wg, d, ff, m->xp, d, m->Gb, ff, k, m->perm, m->tiles, m->ntiles, mt, m->G);
         kc_mm_grouped_packed(s, MF_SEED4P4, m->wu, d, ff, m->xp, d, m->A, ff, k, m->perm, m->tiles, m->ntiles, mt, m->G);
         nsl_swiglu_packed(s, m->Gb, m->A, m->Ap, P * ff);

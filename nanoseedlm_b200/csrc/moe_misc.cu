@@ -161,20 +161,18 @@ __global__ void moe_combine_kernel(const float* __restrict__ D, const float* __r
     x[i] = bf16_round(x[i] + bf16_round(bf16_round(s) + shared[i]));
 }
 
+__device__ __forceinline__ void pack_bf16(const float* __restrict__ x, uint16_t* __restrict__ y, size_t n, unsigned block, unsigned blocks) {
+    const size_t n8 = n / 8;
+    for (size_t i = (size_t) block * blockDim.x + threadIdx.x; i < n8; i += (size_t) blocks * blockDim.x) {
+        const float4 a = ((const float4*) x)[2 * i], b = ((const float4*) x)[2 * i + 1];
+        ((uint4*) y)[i] = make_uint4(bf16x2_bits(a.x, a.y), bf16x2_bits(a.z, a.w), bf16x2_bits(b.x, b.y), bf16x2_bits(b.z, b.w));
+    }
+    if (block == 0 && threadIdx.x < (n & 7)) y[n8 * 8 + threadIdx.x] = bf16_bits(x[n8 * 8 + threadIdx.x]);
+}
 __global__ void pack_bf16_kernel(const float* __restrict__ x, uint16_t* __restrict__ y, size_t n) {
     grid_dependency_wait();
     grid_dependents_go();
-    const size_t n8 = n / 8;
-    for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t) gridDim.x * blockDim.x) {
-        const float4 a = ((const float4*) x)[2 * i], b = ((const float4*) x)[2 * i + 1];
-        uint4 o;
-        o.x = bf16_bits(a.x) | ((uint32_t) bf16_bits(a.y) << 16);
-        o.y = bf16_bits(a.z) | ((uint32_t) bf16_bits(a.w) << 16);
-        o.z = bf16_bits(b.x) | ((uint32_t) bf16_bits(b.y) << 16);
-        o.w = bf16_bits(b.z) | ((uint32_t) bf16_bits(b.w) << 16);
-        ((uint4*) y)[i] = o;
-    }
-    if (blockIdx.x == 0 && threadIdx.x < (n & 7)) y[n8 * 8 + threadIdx.x] = bf16_bits(x[n8 * 8 + threadIdx.x]);
+    pack_bf16(x, y, n, blockIdx.x, gridDim.x);
 }
 
 // Packed bf16 rows in the order of the pairs by expert: row at[t * k + j] of y = row t of x for each of its k pairs (d a multiple of 8;
@@ -208,14 +206,12 @@ void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* at, uint1
 // work (2n+3 ints): [0] tile count, [1..n+1] pair offset of each expert, [n+2..2n+2] tile offset of each expert.
 // One block: histogram by shared-memory atomics, then an exclusive scan of pairs and tiles over the experts (both in one 64-bit
 // word, by warp shuffles: two barriers).
-__global__ void __launch_bounds__(1024) bucket_count_kernel(const int32_t* __restrict__ inds, int count, int n,
-                                                            int32_t* __restrict__ work) {
+// The block's 1024 threads: pairs of expert tid (count_e), pairs (low half) and tiles (high half) of the experts before it, of all.
+__device__ __forceinline__ unsigned long long bucket_offsets(const int32_t* __restrict__ inds, int count, int n, int& count_e, unsigned long long& all) {
     __shared__ int cnt[BUCKET_MAX_EXPERTS];
     __shared__ unsigned long long wsum[32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     cnt[tid] = 0;
-    grid_dependency_wait();
-    grid_dependents_go();
     __syncthreads();
     auto add = [&](int e) { if (e >= 0 && e < n) atomicAdd(&cnt[e], 1); };
     const int n4 = aligned16_dev(inds) ? count / 4 : 0;
@@ -231,7 +227,12 @@ __global__ void __launch_bounds__(1024) bucket_count_kernel(const int32_t* __res
     const unsigned long long ws = wsum[lane];      // every warp scans the 32 warp sums itself
     unsigned long long wi = ws;
     for (int o = 1; o < 32; o <<= 1) { const unsigned long long v = __shfl_up_sync(FULL, wi, o); if (lane >= o) wi += v; }
-    const unsigned long long before = __shfl_sync(FULL, wi - ws, w) + inc - mine, all = __shfl_sync(FULL, wi, 31);
+    all = __shfl_sync(FULL, wi, 31);
+    count_e = c;
+    return __shfl_sync(FULL, wi - ws, w) + inc - mine;
+}
+__device__ __forceinline__ void bucket_work(int32_t* work, int n, unsigned long long before, unsigned long long all) {
+    const int tid = threadIdx.x;
     if (tid < n) {
         work[1 + tid] = (int) (unsigned) before;
         work[2 + n + tid] = (int) (before >> 32);
@@ -241,17 +242,22 @@ __global__ void __launch_bounds__(1024) bucket_count_kernel(const int32_t* __res
         work[2 + 2 * n] = work[0] = (int) (all >> 32);
     }
 }
+__global__ void __launch_bounds__(1024) bucket_count_kernel(const int32_t* __restrict__ inds, int count, int n,
+                                                            int32_t* __restrict__ work) {
+    grid_dependency_wait();
+    grid_dependents_go();
+    int c;
+    unsigned long long all;
+    const unsigned long long before = bucket_offsets(inds, count, n, c, all);
+    bucket_work(work, n, before, all);
+}
 // One block per expert.  Each warp owns a contiguous range of the pair list (a multiple of 128, four entries a lane): it counts its
 // matches, the block scans the 32 counts, then each warp writes its matches in order (ballot prefixes), so perm is ascending
 // within the expert.
-__global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* __restrict__ inds, int count,
-                                                            const int32_t* __restrict__ work, int32_t* __restrict__ perm,
-                                                            MmTile* __restrict__ tiles, int32_t* __restrict__ at_out) {
+__device__ __forceinline__ void bucket_place(const int32_t* __restrict__ inds, int count, int e, int begin, int total, int t0, int32_t* __restrict__ perm,
+                                             MmTile* __restrict__ tiles, int32_t* __restrict__ at_out) {
     __shared__ int wcount[32];
-    const int e = blockIdx.x, n = gridDim.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    grid_dependency_wait();
-    grid_dependents_go();
-    const int begin = work[1 + e], total = work[2 + e] - begin;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     if (total <= 0) return;
     const bool vec = aligned16_dev(inds);
     const int per = ((count + 31) / 32 + 127) & ~127;
@@ -294,13 +300,55 @@ __global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* __res
             at += __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
         }
     }
-    const int t0 = work[2 + n + e];
     for (int t = tid; t * MMT_BN < total; t += 1024) {
         MmTile tl = {e, begin + t * MMT_BN, total - t * MMT_BN < MMT_BN ? total - t * MMT_BN : MMT_BN, 0};
         tiles[t0 + t] = tl;
     }
 }
+__global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* __restrict__ inds, int count,
+                                                            const int32_t* __restrict__ work, int32_t* __restrict__ perm,
+                                                            MmTile* __restrict__ tiles, int32_t* __restrict__ at_out) {
+    const int e = blockIdx.x, n = gridDim.x;
+    grid_dependency_wait();
+    grid_dependents_go();
+    const int begin = work[1 + e];
+    bucket_place(inds, count, e, begin, work[2 + e] - begin, work[2 + n + e], perm, tiles, at_out);
+}
+// Short pair lists: both in one launch, every block counting the whole list itself (8 entries a thread at BUCKET_ONE_PAIRS); the blocks
+// beyond the experts' pack the layer's inputs (pack_n values of x), which nothing here needs.  Three launches in a row cost a prompt
+// of a few hundred rows three latencies, 3 us each.
+constexpr int BUCKET_ONE_PAIRS = 8192;
+__global__ void __launch_bounds__(1024) bucket_pack_kernel(const int32_t* __restrict__ inds, int count, int n, int32_t* __restrict__ work, int32_t* __restrict__ perm,
+                                                           MmTile* __restrict__ tiles, const float* __restrict__ x, uint16_t* __restrict__ xp, size_t pack_n) {
+    __shared__ int mine[3];
+    grid_dependency_wait();      // (its dependents go when it ends: the persistent GEMM's blocks would come in wherever an SM is free, and two with one unit more share one: 298 us for 512 rows instead of 274)
+    const int e = blockIdx.x;
+    if (e >= n) {
+        pack_bf16(x, xp, pack_n, (unsigned) (e - n), gridDim.x - (unsigned) n);
+        return;
+    }
+    int c;
+    unsigned long long all;
+    const unsigned long long before = bucket_offsets(inds, count, n, c, all);
+    if (e == 0) bucket_work(work, n, before, all);
+    if ((int) threadIdx.x == e) { mine[0] = (int) (unsigned) before; mine[1] = c; mine[2] = (int) (before >> 32); }
+    __syncthreads();
+    bucket_place(inds, count, e, mine[0], mine[1], mine[2], perm, tiles, NULL);
+}
 
+void bucket(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles, int32_t* at);
+// kc_bucket and kc_pack_input_bf16 (x -> xp, pack_n values) of a prompt.
+void bucket_pack(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles, const float* x, uint16_t* xp, size_t pack_n) {
+    if (n < 1 || n > BUCKET_MAX_EXPERTS || count > BUCKET_ONE_PAIRS) {
+        bucket(s, inds, count, n, perm, tiles, ntiles, NULL);
+        kc_pack_input_bf16(s, x, xp, pack_n);
+        return;
+    }
+    const size_t blocks = (pack_n / 8 + 1023) / 1024 + 1;
+    launch(bucket_pack_kernel, (unsigned) n + (unsigned) (blocks < (size_t) sm_count() * 4 ? blocks : (size_t) sm_count() * 4), 1024, 0, s, inds, count, n, ntiles, perm,
+           tiles, x, xp, pack_n);
+    count_launch();
+}
 // kc_bucket; at (optional, count ints): every pair's place in perm.
 void bucket(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles, int32_t* at) {
     if (n < 1 || n > BUCKET_MAX_EXPERTS) { set_error("kc_bucket: %d experts, at most %d", n, BUCKET_MAX_EXPERTS); return; }

@@ -16,7 +16,12 @@ F32B = 64 * 1.2e-7
                                              (256, 64, 5, 2, 233, 2.0),      # 93, some experts over 128, one with few
                                              (256, 64, 4, 2, 600, 0.0),      # 300: two and three tiles share an expansion
                                              (128, 64, 6, 3, 900, 3.0),      # up to 900 rows: several units an expert
-                                             (192, 320, 3, 1, 387, 0.0)])
+                                             (192, 320, 3, 1, 387, 0.0),
+                                             (320, 192, 100, 3, 190, 9.0),   # 5 rows an expert, some with over 32 and over 128; chunks that do not fill a step
+                                             (64, 64, 60, 2, 100, 0.0),      # one chunk a row
+                                             (576, 448, 30, 2, 80, 4.0),
+                                             (256, 64, 96, 8, 1024, 0.0),    # 8192 pairs: grouped in one launch
+                                             (256, 64, 96, 8, 1025, 0.0)])   # more: in two
 def test_layer_against_the_mat_vec_path(d, ff, E, k, T, skew):
     from nanoseedlm_b200 import moe
     layer = moe.DeviceLayer.from_host(moe.HostLayer(B, d, ff, E, seed=d + T))
