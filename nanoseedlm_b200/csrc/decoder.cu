@@ -12,6 +12,11 @@
 
 namespace nsl {
 bool launch_q4_mv(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add);      // q4_head.cu
+bool mv_groups(int K, int P, int slices);                                                                                         // seed_mv.cu
+void mv_gu_of(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K, int R, const float* x, int xs, float* out, int ys, const int32_t* sel, int P, int xdiv, int raw,
+              int n_exp, const uint32_t* G);
+void mv_sel_of(cudaStream_t s, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys, const int32_t* sel, int P, int xdiv, int raw, int n_exp,
+               const uint32_t* G);
 bool launch_bf16_set(cudaStream_t s, const DenseSet& set, int K, const float* x, int T);                                         // dense_bf16.cu
 bool launch_seed_set(cudaStream_t s, DenseSet set, int K, const float* x, int T, const uint32_t* G);                             // seed_mv.cu
 void launch_combine_residual_gnorm(cudaStream_t s, int d, int k, const float* D, const float* wt, const float* sh, const float* sg, int sgld, float* x,
@@ -210,12 +215,12 @@ int nsl_decoder_step(NslDecoder* m, cudaStream_t s, const int32_t* ids, const Ro
         dense(m, s, L.router, d, ld, m->h, m->logits, T, 0);
         if (!m->ep) {
             const int P = T * k;
-            if (T <= MV_MAXT) nsl_mv_gu_routed(s, L.eg, L.eu, d, ff, m->h, d, m->A, ff, c.n_exp, k, m->logits, ld, T, m->ind, m->wt, 0, m->G);
+            if (T <= MV_MAXT && !nsl::mv_groups(d, P, c.n_exp)) nsl_mv_gu_routed(s, L.eg, L.eu, d, ff, m->h, d, m->A, ff, c.n_exp, k, m->logits, ld, T, m->ind, m->wt, 0, m->G);
             else {
                 nsl_route(s, c.n_exp, k, m->logits, ld, m->ind, m->wt, T);
-                kc_mv_gu(s, MF_SEED4P4, L.eg, L.eu, d, ff, m->h, d, m->A, ff, m->ind, P, k, m->G);
+                nsl::mv_gu_of(s, L.eg, L.eu, d, ff, m->h, d, m->A, ff, m->ind, P, k, 0, c.n_exp, m->G);
             }
-            kc_mv_sel(s, MF_SEED4P4, L.ed, ff, d, m->A, ff, m->Dx, d, m->ind, P, 1, m->G);
+            nsl::mv_sel_of(s, L.ed, ff, d, m->A, ff, m->Dx, d, m->ind, P, 1, 0, c.n_exp, m->G);
             cudaStreamWaitEvent(s, m->ev_sh, 0);
             nsl::launch_combine_residual_gnorm(s, d, k, m->Dx, m->wt, m->sh, m->logits + c.n_exp, ld, m->x, c.eps, next_norm, m->h, T);
         } else {

@@ -14,6 +14,11 @@ namespace nsl {
 void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* at, uint16_t* y, int T, int k, int d);
 void bucket(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles, int32_t* at);
 void bucket_pack(cudaStream_t s, const int32_t* inds, int count, int n, int32_t* perm, MmTile* tiles, int32_t* ntiles, const float* x, uint16_t* xp, size_t pack_n);
+bool mv_groups(int K, int P, int slices);      // seed_mv.cu
+void mv_gu_of(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K, int R, const float* x, int xs, float* out, int ys, const int32_t* sel, int P, int xdiv, int raw,
+              int n_exp, const uint32_t* G);
+void mv_sel_of(cudaStream_t s, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys, const int32_t* sel, int P, int xdiv, int raw, int n_exp,
+               const uint32_t* G);
 void launch_combine_packed(cudaStream_t s, int d, int k, const uint16_t* D, const float* wt, float* out, int T);
 }
 
@@ -170,20 +175,18 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
     // as dependent launches (a kernel's blocks come in while the previous kernel drains and wait for its completion
     // before touching anything a neighbour writes)
     nsl::PdlScope pdl(m->pdl);
-    const bool fused = T <= MV_MAXT && d % 64 == 0 && d <= 32768 && nsl::aligned16(x);
+    const bool fits = T <= MV_MAXT && d % 64 == 0 && d <= 32768 && nsl::aligned16(x), fused = fits && !nsl::mv_groups(d, P, m->n_exp);
     // on request, one launch for the whole step where the fused kernel serves the sizes (measured slower than the three
     // dependent launches: 126.3 against 114.2 us at 8 rows, 70.1 / 65.5 at 4, 26.7 / 26.2 at 1)
-    if (fused && m->one_launch &&
+    if (fits && m->one_launch &&
         nsl_mv_step(s, m->wg, m->wu, m->wd, d, ff, x, d, m->n_exp, k, logits, m->n_exp, T, m->ind, m->wt, m->A, m->Dx, out, m->raw, m->step_sync, m->G))
         return 0;
     if (fused) nsl_mv_gu_routed(s, m->wg, m->wu, d, ff, x, d, m->A, ff, m->n_exp, k, logits, m->n_exp, T, m->ind, m->wt, m->raw, m->G);
     else {
         nsl_route(s, m->n_exp, k, logits, m->n_exp, m->ind, m->wt, T);
-        if (m->raw) nsl_mv_gu_raw(s, m->wg, m->wu, d, ff, x, d, m->A, ff, m->ind, P, k, m->G);
-        else kc_mv_gu(s, MF_SEED4P4, m->wg, m->wu, d, ff, x, d, m->A, ff, m->ind, P, k, m->G);
+        nsl::mv_gu_of(s, m->wg, m->wu, d, ff, x, d, m->A, ff, m->ind, P, k, m->raw, m->n_exp, m->G);
     }
-    if (m->raw) nsl_mv_raw(s, m->wd, ff, d, m->A, ff, m->Dx, d, m->ind, P, 1, m->G);
-    else kc_mv_sel(s, MF_SEED4P4, m->wd, ff, d, m->A, ff, m->Dx, d, m->ind, P, 1, m->G);
+    nsl::mv_sel_of(s, m->wd, ff, d, m->A, ff, m->Dx, d, m->ind, P, 1, m->raw, m->n_exp, m->G);
     kq4_moe_combine(s, d, k, m->Dx, m->wt, NULL, NULL, 0, out, T);
     return 0;
 }

@@ -37,6 +37,7 @@ struct MvParams {
     const int32_t* xrow;    // optional: pair p reads input row xrow[p] (instead of p / xdiv)
     const int32_t* count;   // optional: the pair count is read on the device (<= P)
     int xbf16;              // inputs are packed bf16 rows (row stride xs in bf16 elements)
+    int slices = 0;       // slices that sel chooses from (0: not known)
 };
 
 __device__ __forceinline__ float silu_bf(float g) {   // each op rounded to bf16 (engine/kernels_moe.cu:28-31)
@@ -1421,10 +1422,16 @@ static void launch_pair(cudaStream_t s, const MvParams& a, const RouteFuse& rf) 
     count_launch();
 }
 
-// Lists of more than GRP_MIN_PAIRS pairs go to the grouped kernel (one expansion per distinct slice, up to GRP_NT pairs a
-// unit): its plan and its costlier second pair pay once a good share of the pairs meet on a slice -- an expert-parallel
-// rank's list or all of a 64-row batch; a decode step's 8 .. 64 pairs over 128 experts run faster pair by pair.
+// Which pair lists go to the grouped kernel (one expansion per distinct slice, up to GRP_NT pairs a unit): its plan (and the router's
+// launch of its own) costs ~15 us a layer and its second pair half of a single one, so enough pairs have to meet on a slice.
+// P pairs of E slices meet P^2 / 2E times, and the line lies at 40 of them: config 1's layer with 64 pairs of 16 / 32 / 64 / 128
+// slices 90.4 / 93.8 / 100.0 / 105.5 us grouped, 98.9 / 99.2 / 99.3 / 99.6 pair by pair; two decoder layers with 96 pairs of 64 /
+// 128 / 512 397 / 408 / 429 and 416 / 416 / 422, with 160 of 512 605 and 589, with 200 719 and 714; 320 of 512 are faster
+// grouped.  Where the number of slices is not known: more than GRP_MIN_PAIRS pairs.
 constexpr int GRP_MIN_PAIRS = 64;
+static bool pairs_meet(int P, int slices) { return slices > 0 ? P >= 48 && (long long) P * P >= 80ll * slices : P > GRP_MIN_PAIRS; }
+static bool grp_serves(int K) { return K % 64 == 0 && K >= 256 && K <= 2048 && (K & (K - 1)) == 0; }
+bool mv_groups(int K, int P, int slices) { return grp_serves(K) && pairs_meet(P, slices); }
 
 template <int MODE>
 static void launch_grp(cudaStream_t s, const MvParams& a, int lpr_log2) {
@@ -1512,9 +1519,19 @@ static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse&
         if (dense) { launch_dense<PF>(s, a, T); return; }
     }
     if constexpr (PF == 4) {
-        if (a.P > GRP_MIN_PAIRS && !rf.logits && ch >= 4 && ch <= 32 && (ch & (ch - 1)) == 0) { launch_grp<MODE>(s, a, log2_floor(ch)); return; }
+        if (!rf.logits && mv_groups(a.K, a.P, a.slices)) { launch_grp<MODE>(s, a, log2_floor(ch)); return; }
     }
     launch_pair<MODE, PF>(s, a, rf);
+}
+
+// kc_mv_gu / nsl_mv_gu_raw and kc_mv_sel / nsl_mv_raw over a layer of n_exp SEED4P4 experts.
+void mv_gu_of(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K, int R, const float* x, int xs, float* out, int ys, const int32_t* sel, int P, int xdiv, int raw,
+              int n_exp, const uint32_t* G) {
+    launch_mv<MODE_GU, 4>(s, MvParams{wg, wu, WSlice{}, sel, x, out, G, K, R, P, xdiv, xs, ys, 0, raw, NULL, NULL, 0, n_exp}, 1);
+}
+void mv_sel_of(cudaStream_t s, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys, const int32_t* sel, int P, int xdiv, int raw, int n_exp,
+               const uint32_t* G) {
+    launch_mv<MODE_ROUND, 4>(s, MvParams{ws, NULL, WSlice{}, sel, x, y, G, K, R, P, xdiv, xs, ys, 0, raw, NULL, NULL, 0, n_exp}, 1);
 }
 
 // A set of SEED4P4 matrices for up to MV_MAXT rows; false: a shape that needs the any-shape kernel.

@@ -63,3 +63,19 @@ def test_router_in_front_at_any_number_of_chunks(K, R, T):
     rind, rwt = B.route(logits, k)
     assert np.array_equal(ind, rind) and np.allclose(wt, rwt, rtol=1e-6)
     assert np.array_equal(a, kernels.kt_mv_gu(w, u, ind.ravel(), k, x))
+
+
+@pytest.mark.parametrize("d,ff,E,k,T", [(256, 256, 28, 6, 8), (256, 256, 29, 6, 8), (256, 320, 8, 6, 8), (192, 512, 8, 6, 8), (2048, 64, 8, 8, 7)])
+def test_decode_rows_whose_pairs_meet(d, ff, E, k, T):
+    """A layer's decode rows either side of the line where pairs that meet on an expert share its expansion (48 pairs, 28 or 29 experts), and
+    with one of the two products outside the grouped kernel's widths: every row has the bits it has alone."""
+    from nanoseedlm_b200 import moe
+    m = moe.Moe(moe.DeviceLayer.from_host(moe.HostLayer(B, d, ff, E, seed=d + E)), k, T)
+    rng = np.random.default_rng(E)
+    x = B.bfr(rng.standard_normal((T, d)).astype(np.float32))
+    logits = rng.standard_normal((T, E)).astype(np.float32)
+    out, ind = m.forward_host(x, logits)
+    assert np.array_equal(ind, B.route(logits, k)[0])
+    for t in range(T):
+        assert np.array_equal(out[t], m.forward_host(x[t:t + 1], logits[t:t + 1])[0][0]), t
+    m.close()
