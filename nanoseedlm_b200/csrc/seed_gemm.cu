@@ -332,7 +332,11 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
     const int NB = a.K / 8, KT = (a.K + GM_BK - 1) / GM_BK, rows_u = GU ? GM_BM / 2 : GM_BM;
     const int row_tiles = (a.R + rows_u - 1) / rows_u;
     const int n_units = row_tiles * (a.grouped ? (TT > 1 ? n_heads : a.ntiles ? *a.ntiles : a.T) : (a.T + GM_BN * TT - 1) / (GM_BN * TT));
-    const int half_max = KT < GROUPS ? 0 : HALF;      // (a warpgroup without a step in a unit must not fall a unit behind the MMAs)
+    // Units of up to half_max rows alternate between the accumulators' halves.  Their MMAs do not wait for the previous unit's results to
+    // be read, so every warpgroup must still owe a step of unit u + 1 when it waits for unit u's MMAs (bar_done: two phases are told
+    // apart, a third would look like the first): results(u) follows its first step of u + 1, so it needs a second one.  With fewer
+    // steps every unit takes both halves, whose MMAs wait for the readers.
+    const int half_max = KT < 2 * GROUPS ? 0 : HALF;
     // Every role walks the same units and counts the same K steps (kr: its stage and the stage's phase) and units.
     int kr0 = 0, unit_run = 0;
     bool ok = true;

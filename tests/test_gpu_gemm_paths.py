@@ -51,3 +51,63 @@ def test_dense(p, R, K, T, packed):
     acc = x.astype(np.float64) @ W.T
     ref = B.bfr(acc.astype(np.float32)).astype(np.float64)
     assert (np.abs(y - ref) <= np.abs(ref) / 128 + F32B * (np.abs(x.astype(np.float64)) @ np.abs(W.T)) + 1e-30).all()
+
+
+def routed_layer(d, ff, counts, seed, scale=1.0):
+    """A layer of len(counts) experts, top 1, whose expert e gets counts[e] rows in a shuffled order -> (the handle's output, the rows'
+    experts, decoded bf16 weights per expert, inputs); everything on the device."""
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L, moe
+    E, T = len(counts), int(sum(counts))
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    layer = moe.DeviceLayer.random_on_device(d, ff, E, gen)
+    m = moe.Moe(layer, 1, T)
+    expert = torch.repeat_interleave(torch.arange(E, device="cuda"), torch.tensor(counts, device="cuda"))[torch.randperm(T, generator=gen, device="cuda")]
+    x = (torch.randn((T, d), generator=gen, device="cuda") * scale).to(torch.bfloat16).float()
+    logits = torch.zeros((T, E), device="cuda").scatter_(1, expert[:, None], 8.0)
+    out = torch.full((T, d), float("nan"), device="cuda")
+    m.forward_dev(x, logits, out)
+    again = torch.empty_like(out)
+    m.forward_dev(x, logits, again)
+    kernels._done()      # (raises when a GEMM block gave up on a wait)
+    assert torch.equal(out, again)
+    m.close()
+
+    def decoded(stack, R, K):      # all experts as one matrix: their streams follow one another
+        w = L.WSlice()
+        w.p[0], w.p[1], w.p[3], w.eb = stack.seeds.data_ptr(), stack.coefs.data_ptr(), stack.codes.data_ptr(), stack.eb[0]
+        o = torch.empty((E, R, K), dtype=torch.bfloat16, device="cuda")
+        L.load().nsl_decode_bf16(kernels._stream(), w, K, E * R, kernels._ptr(o), kernels._ptr(kernels.stream_table()))
+        return o
+    return out, expert, (decoded(layer.gate, ff, d), decoded(layer.up, ff, d), decoded(layer.down, d, ff)), x
+
+
+def layer_reference(weights, expert, x):
+    """The layer's rows with its rounding points, sums in double precision, and sum |w a| of every output."""
+    import torch
+    r = lambda t: t.float().to(torch.bfloat16).double()
+    ref, mag = torch.empty_like(x, dtype=torch.float64), torch.empty_like(x, dtype=torch.float64)
+    for e in range(weights[0].shape[0]):
+        rows = (expert == e).nonzero()[:, 0]
+        if not len(rows):
+            continue
+        wg, wu, wd = (w[e].double() for w in weights)
+        xe = x[rows].double()
+        g, u = r(xe @ wg.T), r(xe @ wu.T)
+        a = r(r(g * r(1.0 / (1.0 + torch.exp(-g)))) * u)
+        ref[rows], mag[rows] = r(a @ wd.T), a.abs() @ wd.abs().T
+    return ref, mag
+
+
+# Rows an expert: units of one to three tiles, at most and more than half of the accumulators (192 rows), full (384) and one beyond.
+UNITS = [97, 130, 192, 193, 110, 250, 100, 384, 96, 385, 120, 60, 140, 192, 150, 0]
+
+
+@pytest.mark.parametrize("d,ff,E", [(128, 256, 480), (256, 128, 480), (192, 320, 256), (448, 256, 256), (256, 448, 256), (320, 192, 256), (576, 512, 160)])
+def test_many_units_a_block_that_share_expansions(d, ff, E):
+    """Prompts whose experts' tiles share an expansion, several units a block, 2 .. 9 K steps a unit: a warpgroup has no, one or two
+    steps of a unit, and results are read under the next one.  Every element: an activation can round the other way, so an
+    output may differ by what it is to have all of its row's activations a bf16 unit off."""
+    out, expert, weights, x = routed_layer(d, ff, [UNITS[e % len(UNITS)] for e in range(E)], d + ff)
+    ref, mag = layer_reference(weights, expert, x)
+    assert ((out.double() - ref).abs() <= ref.abs() / 128 + mag / 128 + 1e-30).all()
