@@ -571,6 +571,7 @@ __global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax
     __shared__ int ci[ARG_CTAS];
     __shared__ float row_max;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, rank = blockIdx.x;      // (the grid's x is one cluster)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // this block has started: its shared memory may be written
     grid_dependents_go();
     grid_dependency_wait();
     const float* l = logits + (size_t) blockIdx.y * V;
@@ -603,6 +604,7 @@ __global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax
     block_best();
     if (lane == 0) { bv[w] = best; bi[w] = idx; }
     __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // the cluster's blocks have all started (a short row's end is soon reached)
     if (w == 0) {
         best = lane < ARG_T / 32 ? bv[lane] : -INFINITY;
         idx = lane < ARG_T / 32 ? bi[lane] : 0x7FFFFFFF;

@@ -62,3 +62,15 @@ def test_argmax_ties_to_the_lowest_id_and_probability(V, n):
     assert np.array_equal(out, ro) and out[0] == V // 2
     np.testing.assert_allclose(prob, rp, rtol=2e-5)
     assert np.array_equal(kernels.kt_argmax(logits), ro)
+
+
+@pytest.mark.parametrize("V,n", [(1, 1), (2, 700), (5, 300), (33, 2000), (4097, 61)])
+def test_argmax_of_many_short_rows(V, n):
+    """Rows with less than a value a block of the cluster: their blocks meet as soon as they have started."""
+    from nanoseedlm_b200 import kernels
+    logits = (np.random.default_rng(V + n).standard_normal((n, V)) * 3).astype(np.float32)
+    ro, rp = logits.argmax(axis=1), [1 / np.exp(r.astype(np.float64) - r.max()).sum() for r in logits]
+    for _ in range(3):
+        out, prob = kernels.kt_argmax(logits, prob=True)
+        assert np.array_equal(out, ro) and np.array_equal(kernels.kt_argmax(logits), ro)
+        np.testing.assert_allclose(prob, rp, rtol=2e-5)
