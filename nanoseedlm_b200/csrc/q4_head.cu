@@ -597,7 +597,10 @@ __global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax
             }
     }
     const int rest = head + 4 * n4, odd = tid < head ? tid : rest + (tid - head);      // the head's ids, then the tail's
-    if (rank == 0 && odd < V && (tid < head || odd >= rest)) arg_better(best, idx, l[odd], odd);
+    if (rank == 0 && odd < V && (tid < head || odd >= rest)) {
+        const float v = l[odd];
+        if (v > -INFINITY) arg_better(best, idx, v, odd);      // (a row without a larger value has no best id: 0)
+    }
     auto block_best = [&]() {
         for (int o = 16; o > 0; o >>= 1) arg_better(best, idx, __shfl_xor_sync(0xFFFFFFFFu, best, o), __shfl_xor_sync(0xFFFFFFFFu, idx, o));
     };

@@ -74,3 +74,16 @@ def test_argmax_of_many_short_rows(V, n):
         out, prob = kernels.kt_argmax(logits, prob=True)
         assert np.array_equal(out, ro) and np.array_equal(kernels.kt_argmax(logits), ro)
         np.testing.assert_allclose(prob, rp, rtol=2e-5)
+
+
+@pytest.mark.parametrize("V,row", [(33, 1000), (7, 2), (8, 1), (1023, 3)])
+def test_argmax_without_a_largest_value(V, row):
+    """A row of -inf (rows that start on and off a 16-byte boundary, with and without a tail) gives id 0; -inf beside a finite value never wins."""
+    from nanoseedlm_b200 import kernels
+    logits = np.random.default_rng(V).standard_normal((row + 2, V)).astype(np.float32)
+    logits[row] = -np.inf
+    logits[row + 1] = -np.inf
+    logits[row + 1, V - 1] = -3e38
+    out = kernels.kt_argmax(logits)
+    assert out[row] == 0 and out[row + 1] == V - 1
+    assert np.array_equal(out[:row], logits[:row].argmax(axis=1))
