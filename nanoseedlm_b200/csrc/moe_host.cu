@@ -153,13 +153,8 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
                 nsl::launch_gemm_gu(s, g, mt);
                 nsl::launch_gemm(s, MF_SEED4P4, "nsl_moe_forward", w, mt);
             } else {
-                if (avg < 6) {      // few rows an expert: the kernel that keeps the weights in registers (128 experts, us, against the other: 209 / 227 at 1.5 rows, 263 / 265 at 4, 272 / 270 at 6, 282 / 269 at 7.5)
-                    nsl::launch_seed_mma_grouped(s, g);
-                    nsl::launch_seed_mma_grouped(s, w);
-                } else {
-                    nsl::launch_gemm_gu(s, g, mt);
-                    nsl::launch_gemm(s, MF_SEED4P4, "nsl_moe_forward", w, mt);
-                }
+                nsl::launch_gemm_gu(s, g, mt);
+                nsl::launch_gemm(s, MF_SEED4P4, "nsl_moe_forward", w, mt);
             }
             nsl::launch_combine_packed(s, d, k, D, m->wt, out, T);
             return 0;

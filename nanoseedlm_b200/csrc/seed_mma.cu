@@ -1,5 +1,4 @@
-// Seed-decode products of a few rows (up to 32 a tile) on warp-level tensor instructions: the grouped products of a batch over
-// many experts, and dense products of a decode batch.
+// Dense seed products of a few rows (up to 32 a tile) on warp-level tensor instructions: the projections of a decode batch.
 //
 // Y[n][r] = sum_k W[r][k] X[n][k], weights expanded exactly and rounded to bf16, inputs bf16, f32 accumulation.
 //
@@ -13,12 +12,9 @@
 // lies in global memory but for an exclusive-or that spreads the lanes' 16-byte loads over the banks.  All of the tile's inputs
 // are resident where they fit (8 rows of 2048: 32 KB), so that a warp runs through its rows without a barrier; else two buffers
 // of whole super-steps take turns.
-// A tile that stages weights in shared memory for tcgen05.mma pays the stores, the address arithmetic, the proxy fence and the
-// waits of producers that run ahead on top (165-189 instructions a block): a layer of 512 experts, 64 rows, top 10 took 1022 us
-// that way.
-//
-// GU: the tile's 16 rows are 8 rows of the gate matrix and the same 8 of the up matrix, so a lane ends with both sums of the same
-// (row, token) and applies SwiGLU in registers.
+// The products of an expert layer do not come here: the pieces of a routed batch have any number of rows, each 32 of them would be
+// expanded again, and a row's bits would depend on how many others its expert got.  (A form for few rows an expert was 8 % faster for
+// 64 rows, top 10 of 512 experts, routed evenly, and 1.8 times slower where most rows went to a few experts: 231 / 127 us.)
 #include "common.cuh"
 #include "seed_block.cuh"
 #include "seed_mma.cuh"
@@ -64,11 +60,6 @@ __device__ __forceinline__ void pair_fragments(const StreamTab& tab, uint32_t sw
         f[i] = bf16x2_bits(a0, a1);
         f[4 + i] = bf16x2_bits(b0, b1);
     }
-}
-
-__device__ __forceinline__ float silu_round(float g) {   // each op rounded to bf16 (engine/kernels_moe.cu:28-31)
-    const float s = bf16_round(1.0f / (1.0f + expf(-g)));
-    return bf16_round(g * s);
 }
 
 // 16-byte unit u (k = 8 u .. 8 u + 7) of row n of a super-step's inputs: for one step j = u & 7 the eight lanes (two rows, four
@@ -204,15 +195,9 @@ __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, 
             const int dst = sh.drow[8 * i + 2 * t + e];
             const float va = acc[i][e], vb = acc[i][2 + e];
             if (dst < 0) continue;
-            if (a.out_bf16) {
-                uint16_t* y = (uint16_t*) a.Y + (size_t) dst * a.ys;
-                if (okA) y[rowA] = bf16_bits(va);
-                if (okB) y[rowB] = bf16_bits(vb);
-            } else {
-                float* y = (float*) a.Y + (size_t) dst * a.ys;
-                if (okA) y[rowA] = a.add ? bf16_round(y[rowA] + bf16_round(va)) : bf16_round(va);   // engine/kernels_moe.cu:214
-                if (okB) y[rowB] = a.add ? bf16_round(y[rowB] + bf16_round(vb)) : bf16_round(vb);
-            }
+            float* y = (float*) a.Y + (size_t) dst * a.ys;
+            if (okA) y[rowA] = a.add ? bf16_round(y[rowA] + bf16_round(va)) : bf16_round(va);   // engine/kernels_moe.cu:214
+            if (okB) y[rowB] = a.add ? bf16_round(y[rowB] + bf16_round(vb)) : bf16_round(vb);
         }
     }
 }
@@ -248,191 +233,6 @@ static void launch_smm_v(cudaStream_t s, const SmmParams& a, dim3 grid, size_t s
         done[dev & 15] = true;
     }
     launch(seed_mma_kernel<P>, grid, SMM_THREADS, smem, s, a, kconst());
-    count_launch();
-}
-
-// ---- grouped: few rows an expert ---------------------------------------------------------------------------------------------
-// An ITEM is 16 rows of weights of one tile, the whole of K, and belongs to one warp; nothing is shared between warps, so there is
-// no barrier.  One block of 16 warps an SM; block b's items come in runs of SMG_RUN: runs b, b + grid, ... of the tile-major
-// sequence, so that a tile of many rows is spread over many blocks, and its warps fetch them one by one from a counter (a warp
-// that the scheduler favours takes more).  The inputs are read through L1 straight into the B fragments: 16 bytes a lane, the
-// tile's few rows stay there while its items last.  What the next item needs (its slices' table entries, its pairs) is
-// copied into shared memory two steps before the end of the current one, and its first streams are requested in the last step.
-// With blocks of 8 warps a tile's 64 or 128 rows, their inputs staged in shared memory, a block's slowest warp and its
-// start-up (table entries, pairs, inputs, first streams, one after the other) took a fifth of the time.
-constexpr int SMG_WARPS = 16, SMG_THREADS = 32 * SMG_WARPS, SMG_RUN = 8;
-
-struct __align__(16) SmgItem {
-    int slice, start, count, r0;      // its tile, its first row of weights
-    WSlice wa, wb;
-    int perm[SMM_TILE];      // the first SMM_TILE pairs
-};
-struct SmgShared {
-    StreamTab tab;
-    SmgItem item[SMG_WARPS][2];
-    int next;
-};
-
-// One pass of an item: up to 8 NT rows of inputs.  ca / cb: the first step's streams; on return what last() has requested.
-template <int NT, bool GU, typename Step, typename Last>
-__device__ __forceinline__ void smg_pass(const MmParams& a, const KConst& kc, const StreamTab& tab, const SmgItem& d, int count,
-                                         MmaChunk& ca, MmaChunk& cb, Step step, Last last) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int ch = a.K / 64, nss = (ch + 3) / 4;
-    const float baseA = exact_base<4>(d.wa.eb), baseB = GU ? exact_base<4>(d.wb.eb) : baseA;
-    const uint16_t* x[NT];
-#pragma unroll
-    for (int i = 0; i < NT; ++i) x[i] = (const uint16_t*) a.X + (size_t) (d.perm[8 * i + g < count ? 8 * i + g : 0] / a.xdiv) * a.xs;      // (a row that is not there: any, its sums are dropped)
-    float acc[NT][4];
-#pragma unroll
-    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-    for (int it = 0; it < nss; ++it) {
-        const int c = min(it * 4 + t, ch - 1);
-        const uint32_t sA[4] = {ca.s.x, ca.s.y, ca.s.z, ca.s.w}, cA[4] = {ca.c.x, ca.c.y, ca.c.z, ca.c.w}, cdA = ca.cd;
-        const uint32_t sB[4] = {cb.s.x, cb.s.y, cb.s.z, cb.s.w}, cB[4] = {cb.c.x, cb.c.y, cb.c.z, cb.c.w}, cdB = cb.cd;
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            if (jj == 3) {      // the next streams, into the registers that these leave free: a quarter of a step ahead is enough
-                if (it + 1 < nss) step(it, ca, cb);
-                else last(ca, cb);
-            }
-            constexpr int AHEAD = NT <= 2 ? 2 : 1;      // steps whose inputs are requested before the expansion
-            uint4 xv[AHEAD][NT];
-#pragma unroll
-            for (int e = 0; e < AHEAD; ++e)
-#pragma unroll
-                for (int i = 0; i < NT; ++i) xv[e][i] = __ldg((const uint4*) (x[i] + c * 64) + 2 * jj + e);
-            uint32_t fa[8], fb[8];
-            pair_fragments<4>(tab, sA[jj], cA[jj], code_scale_pair(cdA, jj, kc), baseA, kc, fa);
-            pair_fragments<4>(tab, sB[jj], cB[jj], code_scale_pair(cdB, jj, kc), baseB, kc, fb);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                if (AHEAD == 1 && e == 1) {
-#pragma unroll
-                    for (int i = 0; i < NT; ++i) xv[0][i] = __ldg((const uint4*) (x[i] + c * 64) + 2 * jj + 1);
-                }
-#pragma unroll
-                for (int i = 0; i < NT; ++i) {
-                    const uint4 v = xv[AHEAD == 1 ? 0 : e][i];
-                    mma16816(acc[i], fa[4 * e], fb[4 * e], fa[4 * e + 1], fb[4 * e + 1], v.x, v.y);
-                    mma16816(acc[i], fa[4 * e + 2], fb[4 * e + 2], fa[4 * e + 3], fb[4 * e + 3], v.z, v.w);
-                }
-            }
-        }
-    }
-    // lane (g, t): rows 8 i + 2 t and + 1 of the inputs (elements 0, 1 of weight row A; 2, 3 of row B)
-    const int rowA = d.r0 + g, rowB = rowA + 8;
-#pragma unroll
-    for (int i = 0; i < NT; ++i) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int n = 8 * i + 2 * t + e;
-            const float va = acc[i][e], vb = acc[i][2 + e];
-            if (n >= count) continue;
-            uint16_t* y = (uint16_t*) a.Y + (size_t) d.perm[n] * a.ys;
-            if (GU) {
-                const float v = bf16_round(silu_round(bf16_round(va)) * bf16_round(vb));
-                if (rowA < a.R) y[rowA] = (uint16_t) (__float_as_uint(v) >> 16);
-            } else {
-                if (rowA < a.R) y[rowA] = bf16_bits(va);
-                if (rowB < a.R) y[rowB] = bf16_bits(vb);
-            }
-        }
-    }
-}
-
-template <bool GU>
-__global__ void __launch_bounds__(SMG_THREADS, 1) seed_mma_grouped_kernel(MmParams a, KConst kc) {
-    __shared__ SmgShared sh;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    constexpr int ROWS = GU ? 8 : 16;
-    load_stream_tab(sh.tab, a.G, tid, SMG_THREADS);
-    if (tid == 0) sh.next = 0;
-    grid_dependents_go();
-    grid_dependency_wait();
-    __syncthreads();
-    const int ch = a.K / 64, nss = (ch + 3) / 4;
-    const int groups = (a.R + ROWS - 1) / ROWS, rpt = (groups + SMG_RUN - 1) / SMG_RUN, runs = *a.ntiles * rpt;      // runs a tile, in all
-    auto fetch = [&](int buf) {      // the warp's next item, into one of its two places
-        for (;;) {
-            int i = 0;
-            if (lane == 0) i = atomicAdd(&sh.next, 1);
-            i = __shfl_sync(0xFFFFFFFFu, i, 0);
-            const int run = i / SMG_RUN * (int) gridDim.x + (int) blockIdx.x;
-            if (run >= runs) return false;
-            const int tile = run / rpt, grp = (run - tile * rpt) * SMG_RUN + i % SMG_RUN;
-            if (grp >= groups) continue;
-            if (lane == 0) {
-                const int4 tl = __ldg((const int4*) a.tiles + tile);
-                *(int4*) &sh.item[warp][buf] = make_int4(tl.x, tl.y, min(tl.z, MMT_BN), grp * ROWS);
-            }
-            __syncwarp();
-            return true;
-        }
-    };
-    auto describe = [&](int buf) {      // requests its table entries and pairs
-        SmgItem& d = sh.item[warp][buf];
-        const int words = (int) sizeof(WSlice) / 8, w = lane & 15;
-        if (w < words && (GU || lane < 16)) {
-            const WSlice* from = (lane < 16 ? a.ws : a.wu) + d.slice;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t) __cvta_generic_to_shared(lane < 16 ? &d.wa : &d.wb) + w * 8), "l"((const char*) from + w * 8) : "memory");
-        }
-        if (lane < d.count) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t) __cvta_generic_to_shared(d.perm + lane)), "l"(a.perm + d.start + lane) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    auto described = [&]() {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncwarp();
-    };
-    auto load = [&](const SmgItem& d, int it, MmaChunk& ca, MmaChunk& cb) {      // (rows that are not there: the last one, its sums are dropped)
-        const int c = it * 4 + t, cc = min(c, ch - 1), rowA = min(d.r0 + g, a.R - 1), rowB = GU ? rowA : min(d.r0 + g + 8, a.R - 1);
-        ca = load_mma_chunk<4>(d.wa, (uint32_t) (rowA * ch + cc));
-        cb = load_mma_chunk<4>(GU ? d.wb : d.wa, (uint32_t) (rowB * ch + cc));
-        if (it * 4 + 4 > ch && c >= ch) ca = cb = MmaChunk{};      // a chunk that is not there: zero coefficients, zero weights
-    };
-    int buf = 0;
-    if (!fetch(0)) return;
-    MmaChunk ca, cb;
-    describe(0);
-    described();
-    load(sh.item[warp][0], 0, ca, cb);
-    for (;;) {
-        const bool next = fetch(buf ^ 1);
-        SmgItem& d = sh.item[warp][buf];
-        for (int n0 = 0; n0 < d.count; n0 += SMM_TILE) {      // (a tile of more rows is expanded again: rare where this kernel is chosen)
-            const int count = min(d.count - n0, SMM_TILE);
-            if (n0) {
-                __syncwarp();
-                if (lane < count) d.perm[lane] = a.perm[d.start + n0 + lane];
-                __syncwarp();
-            }
-            const bool more = n0 + SMM_TILE < d.count, ahead = !more && next;
-            auto step = [&](int it, MmaChunk& na, MmaChunk& nb) {
-                if (it == nss - 2 && ahead) describe(buf ^ 1);
-                load(d, it + 1, na, nb);
-            };
-            auto last = [&](MmaChunk& na, MmaChunk& nb) {
-                if (more) load(d, 0, na, nb);
-                else if (next) {
-                    if (nss == 1) describe(buf ^ 1);
-                    described();
-                    load(sh.item[warp][buf ^ 1], 0, na, nb);
-                }
-            };
-            if (count <= 8) smg_pass<1, GU>(a, kc, sh.tab, d, count, ca, cb, step, last);
-            else if (count <= 16) smg_pass<2, GU>(a, kc, sh.tab, d, count, ca, cb, step, last);
-            else smg_pass<4, GU>(a, kc, sh.tab, d, count, ca, cb, step, last);
-        }
-        if (!next) break;
-        buf ^= 1;
-        __syncwarp();      // the place that the item after the next one goes to is no longer read
-    }
-}
-
-void launch_seed_mma_grouped(cudaStream_t s, const MmParams& m) {
-    if (m.R <= 0) return;
-    if (m.wu) launch(seed_mma_grouped_kernel<true>, sm_count(), SMG_THREADS, 0, s, m, kconst());
-    else launch(seed_mma_grouped_kernel<false>, sm_count(), SMG_THREADS, 0, s, m, kconst());
     count_launch();
 }
 

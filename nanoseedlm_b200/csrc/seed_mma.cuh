@@ -26,9 +26,8 @@ void launch_gemm_gu(cudaStream_t s, const MmParams& a, int tiles_y);
 void launch_gemm(cudaStream_t s, int fmt, const char* who, MmParams a, int tiles_y);
 bool gemm_shares_tiles(int max_tiles);
 
-// The same for a few rows (seed_mma.cu): dense, and grouped with few rows an expert (SEED4P4, packed inputs and results, K a multiple of 64).
+// The same for a dense call of a few rows (seed_mma.cu; K a multiple of 64).
 bool smm_serves(int K, const void* X, int xs, int packed);
 void launch_seed_mma(cudaStream_t s, int fmt, const MmParams& m);
-void launch_seed_mma_grouped(cudaStream_t s, const MmParams& m);
 
 }   // namespace nsl

@@ -111,3 +111,27 @@ def test_many_units_a_block_that_share_expansions(d, ff, E):
     out, expert, weights, x = routed_layer(d, ff, [UNITS[e % len(UNITS)] for e in range(E)], d + ff)
     ref, mag = layer_reference(weights, expert, x)
     assert ((out.double() - ref).abs() <= ref.abs() / 128 + mag / 128 + 1e-30).all()
+
+
+@pytest.mark.parametrize("d,ff,E,k", [(512, 256, 32, 4), (320, 192, 12, 3), (1000, 504, 16, 2)])
+def test_a_prompt_row_has_the_same_bits_in_every_batch(d, ff, E, k):
+    """1 .. 500 rows an expert, evenly and unevenly routed: the batch's size and routing choose units, loaders and shared expansions,
+    never the order of a row's sums."""
+    import torch
+    from nanoseedlm_b200 import kernels, moe
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    layer = moe.DeviceLayer.random_on_device(d, ff, E, gen)
+    T = 500 * E // k
+    m = moe.Moe(layer, k, T)
+    x = torch.randn((T, d), generator=gen, device="cuda").to(torch.bfloat16).float()
+    logits = torch.randn((T, E), generator=gen, device="cuda")
+    logits[T // 2:] -= 12.0 * torch.arange(E, device="cuda") / E
+    outs = {}
+    for n in (9, 16, 33, 64, 65, 100, 6 * E // k, 97 * E // k, T):
+        out = torch.empty((n, d), device="cuda")
+        m.forward_dev(x[:n].contiguous(), logits[:n].contiguous(), out)
+        outs[n] = out
+    kernels._done()
+    for n, out in outs.items():
+        assert torch.equal(out, outs[T][:n]), n
+    m.close()
