@@ -41,7 +41,8 @@ void nsl_moe_set_one_launch(NslMoe* m, int on);
 /* 0, or 1 when a bounded wait inside a one-launch step ran out since the last call (that step's output is not valid).
  * Reads device memory: call it after the layer's work has been waited for. */
 int nsl_moe_step_status(NslMoe* m);
-/* x [T][d], logits [T][n_exp] and out [T][d] in device memory; launches only. */
+/* x [T][d], logits [T][n_exp] and out [T][d] in device memory; launches only.  On the grouped prompt path x must be 16-byte aligned
+ * (else -1, nothing launched); out may be any float pointer. */
 int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* logits, int T, float* out);
 /* The same with host buffers: staged through pinned memory, copied both ways on the layer's stream, synchronised.
  * ind_out (optional): the T * top_k routed expert ids. */

@@ -127,6 +127,7 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
     if (T < 1 || T > m->max_tokens) { nsl::set_error("nsl_moe_forward: %d rows, at most %d", T, m->max_tokens); return -1; }
     const int k = m->top_k, P = T * k, d = m->d, ff = m->ff;
     if (T >= m->grouped_min_tokens) {
+        if (!nsl::aligned16(x)) { nsl::set_error("nsl_moe_forward: a prompt's rows must be 16-byte aligned"); return -1; }
         nsl::PdlScope pdl(m->pdl);      // every kernel of the sequence waits on the device for its predecessor
         const int mt = P / MMT_BN + m->n_exp;
         nsl_route(s, m->n_exp, k, logits, m->n_exp, m->ind, m->wt, T);

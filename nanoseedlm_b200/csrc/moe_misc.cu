@@ -112,9 +112,10 @@ void launch_combine_residual_gnorm(cudaStream_t s, int d, int k, const float* D,
     count_launch();
 }
 
-// The same without a shared expert over packed bf16 rows (d a multiple of 8: 16 bytes of each of the k rows a thread).
+// The same without a shared expert over packed bf16 rows (d a multiple of 8: 16 bytes of each of the k rows a thread).  vec: out is
+// 16-byte aligned (the caller's pointer may be any).
 __global__ void __launch_bounds__(256) combine_packed_kernel(int d8, int k, const uint4* __restrict__ D, const float* __restrict__ wt,
-                                                             float4* __restrict__ out, int n) {
+                                                             float* __restrict__ out, int n, int vec) {
     grid_dependency_wait();
     grid_dependents_go();
     const int i = blockIdx.x * 256 + threadIdx.x;
@@ -141,12 +142,18 @@ __global__ void __launch_bounds__(256) combine_packed_kernel(int d8, int k, cons
                 }
             }
     }
-    out[2 * (size_t) i] = make_float4(a[0], a[1], a[2], a[3]);
-    out[2 * (size_t) i + 1] = make_float4(a[4], a[5], a[6], a[7]);
+    float* const o = out + 8 * (size_t) i;
+    if (vec) {
+        ((float4*) o)[0] = make_float4(a[0], a[1], a[2], a[3]);
+        ((float4*) o)[1] = make_float4(a[4], a[5], a[6], a[7]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = a[e];
+    }
 }
 void launch_combine_packed(cudaStream_t s, int d, int k, const uint16_t* D, const float* wt, float* out, int T) {
     const int n = T * (d / 8);
-    launch(combine_packed_kernel, (unsigned) (n + 255) / 256, 256, 0, s, d / 8, k, (const uint4*) D, wt, (float4*) out, n);
+    launch(combine_packed_kernel, (unsigned) (n + 255) / 256, 256, 0, s, d / 8, k, (const uint4*) D, wt, out, n, (int) aligned16(out));
     count_launch();
 }
 

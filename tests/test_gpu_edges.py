@@ -49,3 +49,35 @@ def test_bucket_of_no_pairs_gives_no_tiles(oracle):
     from nanoseedlm_b200 import kernels
     perm, tiles, nt = kernels.kt_bucket(np.zeros(0, np.int32), 8)
     assert nt == 0 and tiles == [] and perm.size == 0
+
+
+@pytest.mark.parametrize("d,T", [(256, 20), (256, 700), (200, 20)])
+def test_a_layer_with_unaligned_rows(oracle, d, T):
+    """Output rows anywhere: the aligned call's bits.  Input rows of a prompt: refused, nothing written; of a decode step: served."""
+    import torch
+    from nanoseedlm_b200 import kernels, moe
+    E, k, ff = 6, 2, 128
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    m = moe.Moe(moe.DeviceLayer.random_on_device(d, ff, E, gen), k, T)
+    x, logits = torch.randn((T, d), generator=gen, device="cuda").to(torch.bfloat16).float(), torch.randn((T, E), generator=gen, device="cuda")
+    ref = torch.empty((T, d), device="cuda")
+    m.forward_dev(x, logits, ref)
+    for shift in (1, 2, 3):
+        out = torch.full((T * d + 8,), 7.0, device="cuda")
+        m.forward_dev(x, logits, out[shift:])
+        kernels._done()
+        assert torch.equal(out[shift:shift + T * d].view(T, d), ref)
+        assert (out[:shift] == 7.0).all() and (out[shift + T * d:] == 7.0).all()
+    xs = torch.empty(T * d + 1, device="cuda")
+    xs[1:] = x.view(-1)
+    out = torch.full((T, d), 7.0, device="cuda")
+    with pytest.raises(RuntimeError, match="aligned"):
+        m.forward_dev(xs[1:].view(T, d), logits, out)
+    torch.cuda.synchronize()
+    assert (out == 7.0).all()
+    for n in (1, 5):
+        m.forward_dev(xs[1:].view(T, d)[:n], logits[:n], out[:n])
+        m.forward_dev(x[:n], logits[:n], ref[:n])
+        kernels._done()
+        assert ((out[:n] - ref[:n]).norm(dim=1) <= 1e-2 * ref[:n].norm(dim=1)).all()
+    m.close()
