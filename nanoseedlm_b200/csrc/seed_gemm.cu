@@ -136,15 +136,33 @@ __device__ __forceinline__ float to_bf16(float x) { return __uint_as_float(bf16x
 // A thread's share of one K step: the 8 blocks (64 weights) of its row.
 struct ChunkIn { uint4 s, c; uint32_t cd; };
 
-template <bool P3, bool VEC>
-__device__ __forceinline__ ChunkIn load_row_chunk(const WSlice& w, int row, int chunk, int R, int NB) {
+// VEC, how the streams may be read.  2: rows of whole chunks; 16, 16 and 4 bytes where the slice's streams are aligned for that (wide,
+// stream_wide), else as 1.  1: rows of whole half chunks (K a multiple of 32), streams aligned to 8, 8 and 2 bytes.  0: anything.
+template <bool P3>
+__device__ __forceinline__ bool stream_wide(const WSlice& w) {
+    return (((unsigned long long) w.p[0] | (unsigned long long) w.p[1]) & 15ull) == 0 && (P3 || ((unsigned long long) w.p[3] & 3ull) == 0);
+}
+template <bool P3, int VEC>
+__device__ __forceinline__ ChunkIn load_row_chunk(const WSlice& w, bool wide, int row, int chunk, int R, int NB) {
     ChunkIn q = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u), 0u};      // zero coefficients: zero weights
     if (row >= R || chunk * 8 >= NB) return q;
-    if (VEC) {      // rows of whole chunks: one aligned load per stream
+    if (VEC == 2 && wide) {
         const uint32_t i = (uint32_t) row * (uint32_t) (NB / 8) + (uint32_t) chunk;
         q.s = __ldg((const uint4*) w.p[0] + i);
         q.c = __ldg((const uint4*) w.p[1] + i);
         if (!P3) q.cd = __ldg((const uint32_t*) w.p[3] + i);
+    } else if (VEC) {
+        const size_t i = ((size_t) row * NB + chunk * 8) / 4;      // the chunk's first half
+        const uint2 s0 = __ldg((const uint2*) w.p[0] + i), c0 = __ldg((const uint2*) w.p[1] + i);
+        uint2 s1 = make_uint2(0u, 0u), c1 = s1;
+        if (!P3) q.cd = __ldg((const uint16_t*) w.p[3] + i);
+        if (VEC == 2 || chunk * 8 + 4 < NB) {
+            s1 = __ldg((const uint2*) w.p[0] + i + 1);
+            c1 = __ldg((const uint2*) w.p[1] + i + 1);
+            if (!P3) q.cd |= (uint32_t) __ldg((const uint16_t*) w.p[3] + i + 1) << 16;
+        }
+        q.s = make_uint4(s0.x, s0.y, s1.x, s1.y);
+        q.c = make_uint4(c0.x, c0.y, c1.x, c1.y);
     } else {
         uint32_t sw[4] = {0u, 0u, 0u, 0u}, cw[4] = {0u, 0u, 0u, 0u};
         const size_t g = (size_t) row * NB + chunk * 8;
@@ -274,9 +292,9 @@ __device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, u
 }
 
 // WF: the weights' form.  0: SEED4P4 blocks; 1: stored BF16 values; 2: SEED4 (P = 3) blocks.  TERMS: bf16 terms a weight (1, or 3:
-// exact).  TT: tiles of 128 rows of inputs that share one expansion.  VEC: K a multiple of 64, streams in aligned 16-byte pieces.
+// exact).  TT: tiles of 128 rows of inputs that share one expansion.  VEC: how the streams are read (load_row_chunk).
 // GU: gate + up + SwiGLU; row i of the gate matrix on lane 2 i, of the up matrix on lane 2 i + 1.
-template <int TERMS, int WF, int TT, bool VEC, bool GU, int IN>
+template <int TERMS, int WF, int TT, int VEC, bool GU, int IN>
 __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT, IN>::CTAS) seed_gemm_kernel(MmParams a, KConst kc, const __grid_constant__ CUtensorMap tm) {
     using Cfg = GmCfg<TERMS, TT, IN>;
     constexpr bool F32 = IN == IN_F32;
@@ -369,14 +387,15 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
             const WSlice w = GU && (lane & 1) ? u.wb : u.wa;
             const int grow = GU ? u.r0 + (rl >> 1) : u.r0 + rl;
             const float base = BF16W ? 0.0f : exact_base<P3 ? 3 : 4>(w.eb);
+            const bool wide = VEC == 2 && stream_wide<P3>(w);
             int kt = (group - kr0 % GROUPS + GROUPS) % GROUPS;
             ChunkIn cur = {};
-            if (!BF16W && kt < KT) cur = load_row_chunk<P3, VEC>(w, grow, kt, a.R, NB);
+            if (!BF16W && kt < KT) cur = load_row_chunk<P3, VEC>(w, wide, grow, kt, a.R, NB);
             for (; kt < KT && ok; kt += GROUPS) {
                 const int kr = kr0 + kt, s = kr % GM_STAGES;
                 const uint32_t ta = tmem_w + ((uint32_t) (lq * 32) << 16) + (uint32_t) (s * Cfg::A_COLS);
                 ChunkIn nxt = {};
-                if (!BF16W && kt + GROUPS < KT) nxt = load_row_chunk<P3, VEC>(w, grow, kt + GROUPS, a.R, NB);
+                if (!BF16W && kt + GROUPS < KT) nxt = load_row_chunk<P3, VEC>(w, wide, grow, kt + GROUPS, a.R, NB);
                 const uint32_t sw[4] = {cur.s.x, cur.s.y, cur.s.z, cur.s.w}, cw[4] = {cur.c.x, cur.c.y, cur.c.z, cur.c.w};
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {      // 32 weights = 16 words
@@ -606,7 +625,7 @@ static bool encode_inputs(CUtensorMap* tm, const MmParams& a) {
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int TERMS, int WF, int TT, bool VEC, bool GU, int IN>
+template <int TERMS, int WF, int TT, int VEC, bool GU, int IN>
 static void launch_gemm_v(cudaStream_t s, const MmParams& a, int units) {
     using Cfg = GmCfg<TERMS, TT, IN>;
     const size_t smem = (size_t) GM_STAGES * Cfg::X_BYTES + Cfg::PW * 1024 + 1024;
@@ -637,32 +656,40 @@ static int dense_tiles(const MmParams& a, int row_tiles) {
     }
     return best;
 }
+// Whether a slice's seeds and coefficient words are aligned to n bytes and its codes to n / 4.
+template <int WF>
+static bool streams_aligned(const WSlice& w, unsigned n) {
+    return (((uintptr_t) w.p[0] | (uintptr_t) w.p[1]) & (n - 1)) == 0 && (WF == 2 || ((uintptr_t) w.p[3] & (n / 4 - 1)) == 0);
+}
 template <int WF>
 static void launch_gemm_seed(cudaStream_t s, const MmParams& a, int row_tiles, int tiles_y) {
     const int units = row_tiles * tiles_y;
+    // how the streams can be read; slices in a device table (8-byte aligned) are looked at by the kernel
+    const int vec = a.K % 32 || (!a.grouped && !streams_aligned<WF>(a.w0, 8)) ? 0 : a.K % 64 ? 1 : 2;
     if (g_exact) {
-        if (a.packed) launch_gemm_v<3, WF, 1, false, false, IN_LIST>(s, a, units);
-        else if (a.K % 64 == 0) launch_gemm_v<3, WF, 1, true, false, IN_F32>(s, a, units);
-        else launch_gemm_v<3, WF, 1, false, false, IN_F32>(s, a, units);
-    } else if (a.K % 64) {
-        if (a.packed) launch_gemm_v<1, WF, 1, false, false, IN_LIST>(s, a, units);
-        else launch_gemm_v<1, WF, 1, false, false, IN_F32>(s, a, units);
+        if (a.packed) { if (vec) launch_gemm_v<3, WF, 1, 1, false, IN_LIST>(s, a, units); else launch_gemm_v<3, WF, 1, 0, false, IN_LIST>(s, a, units); }
+        else if (vec) launch_gemm_v<3, WF, 1, 1, false, IN_F32>(s, a, units);
+        else launch_gemm_v<3, WF, 1, 0, false, IN_F32>(s, a, units);
+    } else if (vec < 2) {
+        if (a.packed) { if (vec) launch_gemm_v<1, WF, 1, 1, false, IN_LIST>(s, a, units); else launch_gemm_v<1, WF, 1, 0, false, IN_LIST>(s, a, units); }
+        else if (vec) launch_gemm_v<1, WF, 1, 1, false, IN_F32>(s, a, units);
+        else launch_gemm_v<1, WF, 1, 0, false, IN_F32>(s, a, units);
     } else if (a.grouped) {
-        if (!a.packed) launch_gemm_v<1, WF, 1, true, false, IN_F32>(s, a, units);
-        else if (a.in_sorted && a.offs) launch_gemm_v<1, WF, 3, true, false, IN_TMA>(s, a, units);
-        else launch_gemm_v<1, WF, 1, true, false, IN_LIST>(s, a, units);
+        if (!a.packed) launch_gemm_v<1, WF, 1, 2, false, IN_F32>(s, a, units);
+        else if (a.in_sorted && a.offs) launch_gemm_v<1, WF, 3, 2, false, IN_TMA>(s, a, units);
+        else launch_gemm_v<1, WF, 1, 2, false, IN_LIST>(s, a, units);
     } else {
         const int tt = dense_tiles(a, row_tiles), u = row_tiles * ((a.T + GM_BN * tt - 1) / (GM_BN * tt));
-        if (a.packed) { if (tt == 1) launch_gemm_v<1, WF, 1, true, false, IN_TMA>(s, a, u); else launch_gemm_v<1, WF, 3, true, false, IN_TMA>(s, a, u); }
-        else if (tt == 1) launch_gemm_v<1, WF, 1, true, false, IN_F32>(s, a, u);
-        else if (tt == 2) launch_gemm_v<1, WF, 2, true, false, IN_F32>(s, a, u);
-        else launch_gemm_v<1, WF, 3, true, false, IN_F32>(s, a, u);
+        if (a.packed) { if (tt == 1) launch_gemm_v<1, WF, 1, 2, false, IN_TMA>(s, a, u); else launch_gemm_v<1, WF, 3, 2, false, IN_TMA>(s, a, u); }
+        else if (tt == 1) launch_gemm_v<1, WF, 1, 2, false, IN_F32>(s, a, u);
+        else if (tt == 2) launch_gemm_v<1, WF, 2, 2, false, IN_F32>(s, a, u);
+        else launch_gemm_v<1, WF, 3, 2, false, IN_F32>(s, a, u);
     }
 }
 void launch_gemm_gu(cudaStream_t s, const MmParams& a, int tiles_y) {
     const int units = (a.R + GM_BM / 2 - 1) / (GM_BM / 2) * tiles_y;
-    if (a.offs) launch_gemm_v<1, 0, 3, true, true, IN_TMA>(s, a, units);
-    else launch_gemm_v<1, 0, 1, true, true, IN_LIST>(s, a, units);
+    if (a.offs) launch_gemm_v<1, 0, 3, 2, true, IN_TMA>(s, a, units);
+    else launch_gemm_v<1, 0, 1, 2, true, IN_LIST>(s, a, units);
 }
 bool gemm_shares_tiles(int max_tiles) { return max_tiles <= GM_MAX_HEADS; }
 
@@ -681,11 +708,12 @@ void launch_gemm(cudaStream_t s, int fmt, const char* who, MmParams a, int tiles
     }
     if (a.grouped && !a.ntiles) a.T = tiles_y;
     // a dense call of a few rows: the weights stay in registers (64 rows: 2 tiles there)
-    if (fmt != MF_BF16 && !g_exact && !a.grouped && a.T <= 64 && smm_serves(a.K, a.X, a.xs, a.packed)) { launch_seed_mma(s, fmt, a); return; }
+    if (fmt != MF_BF16 && !g_exact && !a.grouped && a.T <= 64 && (fmt == MF_SEED4 ? streams_aligned<2>(a.w0, 16) : streams_aligned<0>(a.w0, 16)) &&
+        smm_serves(a.K, a.X, a.xs, a.packed)) { launch_seed_mma(s, fmt, a); return; }
     const int row_tiles = (a.R + GM_BM - 1) / GM_BM;
     if (fmt == MF_BF16) {      // stored BF16 weights (p[0] = [R][K]): no expansion, one term
-        if (a.packed) launch_gemm_v<1, 1, 1, true, false, IN_LIST>(s, a, row_tiles * tiles_y);
-        else launch_gemm_v<1, 1, 1, true, false, IN_F32>(s, a, row_tiles * tiles_y);
+        if (a.packed) launch_gemm_v<1, 1, 1, 0, false, IN_LIST>(s, a, row_tiles * tiles_y);
+        else launch_gemm_v<1, 1, 1, 0, false, IN_F32>(s, a, row_tiles * tiles_y);
     } else if (fmt == MF_SEED4) launch_gemm_seed<2>(s, a, row_tiles, tiles_y);
     else launch_gemm_seed<0>(s, a, row_tiles, tiles_y);
 }

@@ -135,3 +135,70 @@ def test_a_prompt_row_has_the_same_bits_in_every_batch(d, ff, E, k):
     for n, out in outs.items():
         assert torch.equal(out, outs[T][:n]), n
     m.close()
+
+
+def shifted(t, by):
+    """The tensor's bytes `by` bytes into a fresh buffer -> (address, buffer)."""
+    import torch
+    raw = t.contiguous().view(torch.uint8).flatten()
+    buf = torch.empty(raw.numel() + 16, dtype=torch.uint8, device="cuda")
+    buf[by:by + raw.numel()] = raw
+    return buf.data_ptr() + by, buf
+
+
+@pytest.mark.parametrize("p", [4, 3])
+@pytest.mark.parametrize("R,K,T", [(130, 192, 20), (130, 192, 64), (70, 1088, 70), (140, 96, 300), (33, 160, 65), (40, 72, 40)])
+@pytest.mark.parametrize("by", [0, 2, 8])
+def test_dense_streams_of_any_alignment(p, R, K, T, by):
+    """K of whole chunks, of half chunks and of neither; streams on 16, on 8 and on 2 bytes (codes on 4, 2 and 1)."""
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L
+    m = B.Matrix(R, K, R + K, eb=-21) if p == 4 else B.Matrix3(R, K, R + K, eb=-21)
+    W = B.bfr(B.decode_rows_f32(m) if p == 4 else B.decode3_rows_f32(m)).astype(np.float64)
+    w0 = kernels.SeedWeight.from_matrices([m]) if p == 4 else kernels.SeedWeight3([m])
+    keep = [shifted(w0.seeds, by), shifted(w0.coefs if p == 4 else w0.nibs, by)] + ([shifted(w0.codes, {0: 0, 2: 1, 8: 2}[by])] if p == 4 else [])
+    w = w0.slice(0)
+    w.p[0], w.p[1] = keep[0][0], keep[1][0]
+    if p == 4:
+        w.p[3] = keep[2][0]
+    x = B.bfr(np.random.default_rng(K).standard_normal((T, K)).astype(np.float32))
+    xd = kernels.dev(x)
+    ref = x.astype(np.float64) @ W.T
+    bound = F32B * (np.abs(x.astype(np.float64)) @ np.abs(W.T)) + 1e-30
+    ref = B.bfr(ref.astype(np.float32)).astype(np.float64)
+    for packed in (False, True):
+        y = torch.full((T, R), float("nan"), device="cuda")
+        xin = xd.to(torch.bfloat16) if packed else xd
+        (L.load().kc_mm_packed if packed else L.load().kc_mm)(kernels._stream(), L.MF_SEED4P4 if p == 4 else L.MF_SEED4, w, K, R, kernels._ptr(xin), K,
+                                                              kernels._ptr(y), R, T, 0, kernels._ptr(kernels.stream_table()))
+        kernels._done()
+        assert (np.abs(y.cpu().numpy() - ref) <= np.abs(ref) / 128 + bound).all()
+
+
+@pytest.mark.parametrize("d,ff,T", [(256, 128, 100), (192, 320, 1200)])
+def test_a_layer_whose_streams_lie_on_8_bytes(d, ff, T):
+    """The slices of a device table are looked at by the kernels: the same bits from streams that are only 8-byte (codes 2-byte) aligned, in
+    every second expert."""
+    import ctypes as C
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L, moe
+    E, k = 6, 2
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    layer = moe.DeviceLayer.random_on_device(d, ff, E, gen)
+    x, logits = torch.randn((T, d), generator=gen, device="cuda").to(torch.bfloat16).float(), torch.randn((T, E), generator=gen, device="cuda")
+    m = moe.Moe(layer, k, T)
+    ref, out = torch.empty((T, d), device="cuda"), torch.empty((T, d), device="cuda")
+    m.forward_dev(x, logits, ref)
+    tables, keep = [], []
+    for st in (layer.gate, layer.up, layer.down):
+        arr = (L.WSlice * E)()
+        for e in range(E):
+            s = [shifted(t[e], by if e & 1 else 0) for t, by in ((st.seeds, 8), (st.coefs, 8), (st.codes, 2))]
+            keep.append(s)
+            arr[e].p[0], arr[e].p[1], arr[e].p[3], arr[e].eb = s[0][0], s[1][0], s[2][0], st.eb[e]
+        tables.append(torch.frombuffer(bytearray(bytes(arr)), dtype=torch.uint8).cuda())
+    m.lib.nsl_moe_set_layer(m.h, *(kernels._ptr(t) for t in tables))
+    m.forward_dev(x, logits, out)
+    kernels._done()
+    assert torch.equal(out, ref)
+    m.close()
