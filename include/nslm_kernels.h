@@ -39,7 +39,9 @@ enum { CACHE_PROTECT_PREV = 2 };  /* engine/kernels_cuda.h:51 */
 
 /* One slice's streams (engine/kernels_cuda.h:19-24).  SEED4P4: p[0] seeds u16 [R][K/8], p[1] coefficient words u16
  * [R][K/8], p[3] exponent codes, two per byte, block g = r*(K/8)+b in nibble g&1 of byte g>>1; eb the slice's
- * exponent bias.  Streams may live in device memory or in mapped pinned host memory. */
+ * exponent bias.  Streams may live in device memory or in mapped pinned host memory.  The slices of a device table have p[0]
+ * and p[1] 16-byte and p[3] 4-byte aligned (any rows * cols that is a multiple of 64 keeps a stack of slices so); 8 and 2 bytes do for
+ * the grouped GEMMs, any address for P = 3 gathers of rows that are not 64 * 2^j <= 2048 weights.  Dense calls take any address. */
 typedef struct {
     const void* p[4];
     int32_t eb;

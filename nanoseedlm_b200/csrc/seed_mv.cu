@@ -90,6 +90,17 @@ __device__ __forceinline__ Chunk load_chunk(const WSlice& w, size_t chunk_index)
     return k;
 }
 
+// Eight 16-bit values of a stream of any alignment.  (P = 3 gathers over rows that are not 2^j <= 32 chunks take slices from any address; the
+// other forms of a device table have always been read 16 bytes at a time.)
+__device__ __forceinline__ bool chunk_aligned(const void* s, const void* c) { return (((unsigned long long) s | (unsigned long long) c) & 15ull) == 0; }
+__device__ __noinline__ uint4 load_any_16(const void* p, uint32_t chunk) {
+    const uint16_t* q = (const uint16_t*) p + (size_t) chunk * 8;
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = (uint32_t) __ldg(q + 2 * i) | ((uint32_t) __ldg(q + 2 * i + 1) << 16);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 __device__ __forceinline__ float pair_total(u64 acc2) {
     float lo, hi;
     unpack2(acc2, lo, hi);
@@ -355,7 +366,7 @@ constexpr int PAIR_WARPS = 16, PAIR_THREADS = 32 * PAIR_WARPS, PAIR_WIN = 8;
 struct PairDesc {      // what an item needs of its pair
     const void *sa, *ca, *da, *sb, *cb, *db;
     float sca, scb;
-    int pair, pad;
+    int pair, any;      // any: bit 0 / 1: the first / second matrix's streams are not 16-byte aligned (mv_items_kernel, P = 3)
 };
 
 template <int MODE, int PF>
@@ -533,6 +544,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_items_kernel(MvParams a, K
                 d.sb = wb.p[0]; d.cb = wb.p[1]; d.db = wb.p[3];
                 d.scb = slice_scale(wb.eb + (8 - PF));
             }
+            if (PF == 3) d.any = (int) !chunk_aligned(d.sa, d.ca) | (MODE == MODE_GU && !chunk_aligned(d.sb, d.cb) ? 2 : 0);
             desc[threadIdx.x] = d;
         }
         if (threadIdx.x == 0) next_item = PAIR_WARPS;
@@ -547,11 +559,17 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_items_kernel(MvParams a, K
             t = divide(lo + k, inv_rs, rs);
             r = (lo + k - t * rs) * rpw + ro;
         };
-        auto fetch_a = [&](const PairDesc& d, uint32_t at, Chunk& k) {
-            k.s = __ldg((const uint4*) d.sa + at);
-            k.c = __ldg((const uint4*) d.ca + at);
-            if (PF == 4) k.cd = __ldg((const uint32_t*) d.da + at);
+        auto fetch = [&](const void* sp, const void* cp, const void* dp, bool any, uint32_t at, Chunk& k) {
+            if (PF == 3 && any) {
+                k.s = load_any_16(sp, at);
+                k.c = load_any_16(cp, at);
+                return;
+            }
+            k.s = __ldg((const uint4*) sp + at);
+            k.c = __ldg((const uint4*) cp + at);
+            if (PF == 4) k.cd = __ldg((const uint32_t*) dp + at);
         };
+        auto fetch_a = [&](const PairDesc& d, uint32_t at, Chunk& k) { fetch(d.sa, d.ca, d.da, d.any & 1, at, k); };
         struct At { int k, g, t, r; };      // an item: its (first) step, group, the step's pair, this lane's row
         auto load = [&](int it, At& at_it, Chunk& ka, Chunk& kb) {
             if (it >= items) return;
@@ -564,11 +582,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_items_kernel(MvParams a, K
                 const PairDesc& d = desc[t];
                 const uint32_t at = (uint32_t) (r * ch + j);
                 fetch_a(d, at, ka);
-                if (MODE == MODE_GU) {
-                    kb.s = __ldg((const uint4*) d.sb + at);
-                    kb.c = __ldg((const uint4*) d.cb + at);
-                    if (PF == 4) kb.cd = __ldg((const uint32_t*) d.db + at);
-                }
+                if (MODE == MODE_GU) fetch(d.sb, d.cb, d.db, d.any & 2, at, kb);
             }
             if (MODE != MODE_GU && spi == 2 && u * 2 + 1 < n) {
                 locate(u * 2 + 1, t, r);
@@ -1488,10 +1502,10 @@ static void launch_dense(cudaStream_t s, MvParams a, int T, DenseSet* set = NULL
     }
 }
 
-// The streams of a slice given by value (a dense call) can be checked on the host; slices in a device table are the
-// table builder's to check (nsl_wslice_table does).
-static bool slice_aligned(const WSlice& w) {
-    return aligned16(w.p[0]) && aligned16(w.p[1]) && ((uintptr_t) w.p[3] & 3u) == 0;
+// The streams of a slice given by value (a dense call) are checked on the host.  Slices in a device table are not: their streams must be
+// 16-byte aligned (codes 4) in every form but the one that load_any_16 serves.
+static bool slice_aligned(const WSlice& w, int pf) {
+    return aligned16(w.p[0]) && aligned16(w.p[1]) && (pf == 3 || ((uintptr_t) w.p[3] & 3u) == 0);
 }
 
 // PF = 4: SEED4P4; 3: SEED4.  The chunked kernels read whole chunks with 16-byte loads: rows of inputs and (checked where
@@ -1504,7 +1518,7 @@ static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse&
     if (T > MV_MAXT) { set_error("seed mat-vec: %d tokens, at most %d", T, MV_MAXT); return; }
     const bool dense = a.sel == NULL && rf.logits == NULL;
     const int ch = a.K / 64;
-    const bool chunked = a.K % 64 == 0 && aligned16(a.x) && a.xs % (a.xbf16 ? 8 : 4) == 0 && (a.ws != NULL || slice_aligned(a.w0)) &&
+    const bool chunked = a.K % 64 == 0 && aligned16(a.x) && a.xs % (a.xbf16 ? 8 : 4) == 0 && (a.ws != NULL || slice_aligned(a.w0, PF)) &&
                          staged_bytes(ch) <= (size_t) max_smem_optin() - 10240;
     if (!chunked) {
         if (a.xrow || a.count || a.xbf16 || rf.logits) {
@@ -1538,7 +1552,7 @@ void mv_sel_of(cudaStream_t s, const WSlice* ws, int K, int R, const float* x, i
 bool launch_seed_set(cudaStream_t s, DenseSet set, int K, const float* x, int T, const uint32_t* G) {
     if (T < 1 || T > MV_MAXT || K < 64 || K % 64 || !aligned16(x) || staged_bytes(K / 64) > (size_t) max_smem_optin() - 10240) return false;
     for (int m = 0; m < set.n; ++m)
-        if (set.R[m] < 1 || !slice_aligned(set.w[m])) return false;
+        if (set.R[m] < 1 || !slice_aligned(set.w[m], 4)) return false;
     MvParams a = {NULL, NULL, set.w[0], NULL, x, set.y[0], G, K, set.R[0], T, 1, K, set.R[0], 0, 0, NULL, NULL, 0};
     launch_dense<4>(s, a, T, &set);
     return true;

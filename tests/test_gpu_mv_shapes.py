@@ -79,3 +79,32 @@ def test_decode_rows_whose_pairs_meet(d, ff, E, k, T):
     for t in range(T):
         assert np.array_equal(out[t], m.forward_host(x[t:t + 1], logits[t:t + 1])[0][0]), t
     m.close()
+
+
+@pytest.mark.parametrize("K,R", [(64 * 3, 40), (64 * 11, 37), (64 * 24, 130), (64 * 45, 33)])
+@pytest.mark.parametrize("by", [2, 8])
+def test_p3_gathers_from_any_address(K, R, by):
+    """Slices of a device table whose streams start off the 16-byte grid, between ones that do not: the aligned streams' bits."""
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L
+    _, w = matrices(3, 3, R, K, K + R)
+    _, u = matrices(3, 3, R, K, 7 * K + R)
+    x = B.bfr(np.random.default_rng(K).standard_normal((7, K)).astype(np.float32))
+    sel = np.array([2, 0, 1, 1, 2, 0, 1], np.int32)
+    ref = kernels.kt_mv3_sel(w, sel, 1, x), kernels.kt_mv3_gu(w, u, sel, 1, x), kernels.kt_mv3(w, x[:5], 5, s=1)
+    for m, odd in ((w, (1,)), (u, (0, 1))):
+        arr = (L.WSlice * 3)()
+        for s in range(3):
+            arr[s] = m.slice(s)
+            for i, t in enumerate((m.seeds, m.nibs)):
+                if s in odd:
+                    buf = torch.empty(t[s].numel() + 8, dtype=t.dtype, device="cuda")
+                    buf[by // 2:by // 2 + t[s].numel()] = t[s]
+                    arr[s].p[i] = buf.data_ptr() + by
+                    m.__dict__.setdefault("keep", []).append(buf)
+        m.table = torch.frombuffer(bytearray(bytes(arr)), dtype=torch.uint8).cuda()
+        m.slice = lambda s, arr=arr: arr[s]
+    assert np.array_equal(kernels.kt_mv3_sel(w, sel, 1, x), ref[0])
+    assert np.array_equal(kernels.kt_mv3_gu(w, u, sel, 1, x), ref[1])
+    for t in range(5):
+        assert (np.abs(kernels.kt_mv3(w, x[:5], 5, s=1)[t] - ref[2][t]) <= np.abs(ref[2][t]) / 64 + 1e-4 * np.abs(ref[2]).max()).all()
