@@ -351,7 +351,7 @@ __device__ __forceinline__ void route_prologue(const RouteFuse& rf, int32_t* r_i
 }
 
 // ---- one expansion per pair, inputs in shared memory, one block of 16 warps per SM -----------------------------------------
-// Rows of 2 .. 32 chunks (a power of two).  The work is the pair-major sequence of items (RowItem); blocks take contiguous equal
+// Rows of 1, 2, 4 .. 32 chunks.  The work is the pair-major sequence of items (RowItem); blocks take contiguous equal
 // shares of it, and a block's warps fetch its items one by one from a counter in shared memory: the schedulers favour some warps,
 // and with items dealt in advance the favoured ones left the others alone for the last third of the launch (13.5 of 16 warps
 // active on average).  Inputs, stream addresses and scales of up to PAIR_WIN pairs are staged at a time.
@@ -482,6 +482,15 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KC
                 else chunk_dots<MODE_ROUND, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);      // (a pair's last, single step)
             }
             const float v[2] = {pair_total(acc[0]), pair_total(acc[1])};
+            if (lpr == 1) {      // rows of one chunk: every lane has its rows' sums (two lanes a row in mv_items_kernel, one idle: 1300 pairs of 640 rows 103 / 55 us)
+                const PairDesc& d = desc[t];
+                if (r < a.R) store_out<MODE>(a, d.pair, r, v[0] * d.sca, MODE == MODE_GU ? v[1] * d.scb : 0.0f);
+                if (MODE != MODE_GU && r + rpw < a.R) store_out<MODE>(a, d.pair, r + rpw, v[1] * d.sca, 0.0f);
+                it = nx;
+                ka = na;
+                kb = nb;
+                continue;
+            }
             const float mine = split_sum<2>(v, lpr, jc);
             if (slot == cnt) { keep = mine; kept = it; }
             if (++cnt == h) flush();
@@ -1407,7 +1416,7 @@ template <int MODE, int PF>
 static void launch_pair(cudaStream_t s, const MvParams& a, const RouteFuse& rf) {
     const int ch = a.K / 64, sms = sm_count();
     static bool attr_set[16], attr_set_items[16];
-    if (ch >= 2 && ch <= 32 && (ch & (ch - 1)) == 0) {
+    if (ch <= 32 && (ch & (ch - 1)) == 0) {
         const int lpr_log2 = log2_floor(ch);
         int win = a.P / sms + 2;      // a share's pairs, whole or in part
         if (win > PAIR_WIN) win = PAIR_WIN;

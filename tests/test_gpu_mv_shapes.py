@@ -108,3 +108,10 @@ def test_p3_gathers_from_any_address(K, R, by):
     assert np.array_equal(kernels.kt_mv3_gu(w, u, sel, 1, x), ref[1])
     for t in range(5):
         assert (np.abs(kernels.kt_mv3(w, x[:5], 5, s=1)[t] - ref[2][t]) <= np.abs(ref[2][t]) / 64 + 1e-4 * np.abs(ref[2]).max()).all()
+
+
+@pytest.mark.parametrize("p", [4, 3])
+@pytest.mark.parametrize("R", [1, 31, 33, 64, 65, 130])
+def test_rows_of_one_chunk(p, R):
+    """K = 64: a lane is a row and keeps both of an item's sums; rows either side of one and two row steps."""
+    test_any_number_of_chunks(p, 64, R)
