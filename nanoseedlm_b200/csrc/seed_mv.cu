@@ -263,7 +263,7 @@ __device__ __forceinline__ float split_sum(const float* v, int lpr, int jc) {
     return m;
 }
 
-// Rows of 2^j = 2 .. 32 chunks: a row step = the 32 / lpr rows a warp expands at once, a lane owning one chunk of its row; the
+// Rows of 2^j = 1 .. 32 chunks: a row step = the 32 / lpr rows a warp expands at once, a lane owning one chunk of its row; the
 // steps [s_lo, s_hi) of a pair go to the block's warps in turn.  A warp takes two rows of streams at a time against the same
 // inputs (an ITEM): a row of the gate and of the up matrix, or two of its steps of the one matrix.
 template <int MODE>
@@ -316,11 +316,16 @@ __device__ __forceinline__ void pair_rows(const StreamTab& tab, const KConst& kc
             else chunk_dots<MODE_ROUND, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);
         }
         const float v[2] = {pair_total(acc[0]), pair_total(acc[1])};
-        const float mine = split_sum<2>(v, lpr, jc);
-        if (slot == cnt) keep = mine;
-        if (++cnt == h) {
-            flush(st - (h - 1) * STEPS * MV_WARPS, r - (h - 1) * STEPS * S);
-            cnt = 0;
+        if (lpr == 1) {      // rows of one chunk: every lane has its rows' sums
+            if (r < R) store(r, v[0] * sca, MODE == MODE_GU ? v[1] * scb : 0.0f);
+            if (MODE != MODE_GU && st + MV_WARPS < s_hi && r + S < R) store(r + S, v[1] * sca, 0.0f);
+        } else {
+            const float mine = split_sum<2>(v, lpr, jc);
+            if (slot == cnt) keep = mine;
+            if (++cnt == h) {
+                flush(st - (h - 1) * STEPS * MV_WARPS, r - (h - 1) * STEPS * S);
+                cnt = 0;
+            }
         }
         ka = na;
         kb = nb;
@@ -1571,7 +1576,7 @@ bool launch_seed_set(cudaStream_t s, DenseSet set, int K, const float* x, int T,
 static bool launch_mv_step(cudaStream_t s, const StepParams& p) {
     const int cd = p.d / 64, cf = p.ff / 64;
     if (p.T < 1 || p.T > MV_MAXT || p.top_k < 1 || p.top_k > 32 || p.T * p.top_k > 256 || p.n_exp < p.top_k || p.n_exp > 32 * ROUTE_PER_LANE) return false;
-    if (p.d % 64 || p.ff % 64 || cd < 2 || cf < 2 || (cd & (cd - 1)) || (cf & (cf - 1)) || cd > 32 || cf > 32) return false;
+    if (p.d % 64 || p.ff % 64 || cd < 1 || cf < 1 || (cd & (cd - 1)) || (cf & (cf - 1)) || cd > 32 || cf > 32) return false;
     if (!aligned16(p.x) || p.xs % 4 || !aligned16(p.A) || !aligned16(p.D)) return false;
     launch(mv_step_kernel, sm_count() * 2, MV_THREADS, 0, s, p, kconst(), log2_floor(cd), log2_floor(cf));
     count_launch();

@@ -273,3 +273,28 @@ def test_one_launch_step_called_directly_its_status_word_and_refusals(oracle):
     assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
     assert call(dd=d + 8) == 0 and call(TT=9) == 0      # not 64 * 2^j; more rows than a decode step has
     m.close()
+
+
+@pytest.mark.parametrize("d,ff,E,k", [(64, 64, 12, 2), (64, 512, 12, 3), (512, 64, 12, 8)])
+def test_one_launch_step_with_rows_of_one_chunk(oracle, d, ff, E, k):
+    """The smallest widths nsl_mv_step serves: it launches (1) and gives the three launches' bits."""
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L, moe
+    lib, T = L.load(), 5
+    layer = moe.DeviceLayer.from_host(moe.HostLayer(oracle, d, ff, E, seed=d + ff))
+    m = moe.Moe(layer, k, 8)
+    x, logits = oracle.normal(7, T * d, bf16=True).reshape(T, d), oracle.normal(8, T * E).reshape(T, E)
+    want, wind = m.forward_host(x, logits)
+    dx, dl, P = torch.from_numpy(x).cuda(), torch.from_numpy(logits).cuda(), T * k
+    A, D, out = torch.zeros(P, ff, device="cuda"), torch.zeros(P, d, device="cuda"), torch.zeros(T, d, device="cuda")
+    ind, wt, sync = torch.zeros(P, dtype=torch.int32, device="cuda"), torch.zeros(P, device="cuda"), torch.zeros(2 + T + P, dtype=torch.int32, device="cuda")
+    G = kernels.stream_table()
+    for _ in range(3):
+        out.zero_()
+        assert lib.nsl_mv_step(None, layer.gate.table.data_ptr(), layer.up.table.data_ptr(), layer.down.table.data_ptr(), d, ff, dx.data_ptr(), d, E, k,
+                               dl.data_ptr(), E, T, ind.data_ptr(), wt.data_ptr(), A.data_ptr(), D.data_ptr(), out.data_ptr(), 0, sync.data_ptr(), G.data_ptr()) == 1
+        torch.cuda.synchronize()
+        assert not sync.any()
+        assert np.array_equal(ind.cpu().numpy().reshape(T, k), wind)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    m.close()
