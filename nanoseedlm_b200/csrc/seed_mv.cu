@@ -374,7 +374,8 @@ struct PairDesc {      // what an item needs of its pair
     int pair, any;      // any: bit 0 / 1: the first / second matrix's streams are not 16-byte aligned (mv_items_kernel, P = 3)
 };
 
-template <int MODE, int PF>
+// ONE: rows of one chunk (lpr_log2 = 0), a form of its own: the branch in the loop of the others cost config 1 at 8 rows 5 %.
+template <int MODE, int PF, bool ONE>
 __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KConst kc, int lpr_log2, int win, RouteFuse rf) {
     extern __shared__ __align__(16) ulonglong2 pair_sx[];      // [win][lpr * CX]
     __shared__ StreamTab tab;
@@ -487,7 +488,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KC
                 else chunk_dots<MODE_ROUND, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);      // (a pair's last, single step)
             }
             const float v[2] = {pair_total(acc[0]), pair_total(acc[1])};
-            if (lpr == 1) {      // rows of one chunk: every lane has its rows' sums (two lanes a row in mv_items_kernel, one idle: 1300 pairs of 640 rows 103 / 55 us)
+            if (ONE) {      // rows of one chunk: every lane has its rows' sums (two lanes a row in mv_items_kernel, one idle: 1300 pairs of 640 rows 103 / 55 us)
                 const PairDesc& d = desc[t];
                 if (r < a.R) store_out<MODE>(a, d.pair, r, v[0] * d.sca, MODE == MODE_GU ? v[1] * d.scb : 0.0f);
                 if (MODE != MODE_GU && r + rpw < a.R) store_out<MODE>(a, d.pair, r + rpw, v[1] * d.sca, 0.0f);
@@ -1426,8 +1427,11 @@ static void launch_pair(cudaStream_t s, const MvParams& a, const RouteFuse& rf) 
         int win = a.P / sms + 2;      // a share's pairs, whole or in part
         if (win > PAIR_WIN) win = PAIR_WIN;
         if (win > a.P) win = a.P;
-        allow_smem(mv_pair_kernel<MODE, PF>, attr_set, (size_t) PAIR_WIN * 32 * CX * 16);
-        launch(mv_pair_kernel<MODE, PF>, sms, PAIR_THREADS, win * staged_bytes(ch), s, a, kconst(), lpr_log2, win, rf);
+        if (ch == 1) launch(mv_pair_kernel<MODE, PF, true>, sms, PAIR_THREADS, win * staged_bytes(ch), s, a, kconst(), lpr_log2, win, rf);
+        else {
+            allow_smem(mv_pair_kernel<MODE, PF, false>, attr_set, (size_t) PAIR_WIN * 32 * CX * 16);
+            launch(mv_pair_kernel<MODE, PF, false>, sms, PAIR_THREADS, win * staged_bytes(ch), s, a, kconst(), lpr_log2, win, rf);
+        }
     } else {
         const RowShape sh = item_shape(ch);
         const size_t room = (size_t) max_smem_optin() - 6144, one = staged_bytes(ch);      // 6144: the kernel's other shared memory (launch_mv has made sure that one row and the fewest sums fit)
