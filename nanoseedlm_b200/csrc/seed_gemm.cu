@@ -211,12 +211,15 @@ __device__ __forceinline__ uint32_t input_at(uint32_t stage, int n, int uu) {
     return stage + (uint32_t) (n * 128 + ((uu ^ (n & 7)) << 4));
 }
 
-// 1 / (1 + e^-g): the hardware's reciprocal and one Newton step (within an ulp; rounded to bf16 by the caller).
+// 1 / (1 + e^-g): the hardware's reciprocal and one Newton-Raphson step r + r (1 - d r); where the result is subnormal (g under -87.3), which
+// the approximation flushes to zero, or e^-g is infinite, the division.  For every bf16 g the bf16 value is that of the division.
 __device__ __forceinline__ float sigmoid(float g) {
-    const float d = 1.0f + fminf(expf(-g), 1e38f);
+    const float d = 1.0f + expf(-g);
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    return fmaf(r, fmaf(-d, r, 1.0f), r);
+    r = fmaf(r, fmaf(-d, r, 1.0f), r);
+    if (d > 8e37f) r = 1.0f / d;
+    return r;
 }
 
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {      // each product rounded once

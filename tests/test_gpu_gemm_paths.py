@@ -202,3 +202,34 @@ def test_a_layer_whose_streams_lie_on_8_bytes(d, ff, T):
     kernels._done()
     assert torch.equal(out, ref)
     m.close()
+
+
+@pytest.mark.parametrize("T", [36, 216])      # the GEMM's two forms of the gate + up product
+def test_swiglu_over_the_range_of_gates(T):
+    """Rows whose gates all lie at one value, from where the sigmoid is a subnormal bf16 number (below -87.3; e^-g overflows f32 below -88.7)
+    to where it is 1.  A gate that rounds to the neighbouring bf16 value moves its own activation by up to e^0.5, one of 64: rows are
+    compared by their norms."""
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L, moe
+    d, ff = 1024, 64
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    layer = moe.DeviceLayer.random_on_device(d, ff, 1, gen)
+
+    def decoded(stack, R, K):
+        w = L.WSlice()
+        w.p[0], w.p[1], w.p[3], w.eb = stack.seeds.data_ptr(), stack.coefs.data_ptr(), stack.codes.data_ptr(), stack.eb[0]
+        o = torch.empty((1, R, K), dtype=torch.bfloat16, device="cuda")
+        L.load().nsl_decode_bf16(kernels._stream(), w, K, R, kernels._ptr(o), kernels._ptr(kernels.stream_table()))
+        return o
+    weights = decoded(layer.gate, ff, d), decoded(layer.up, ff, d), decoded(layer.down, d, ff)
+    gates = torch.tensor([-88.0, -87.75, -87.5, -87.25, -87.0, -80.0, -40.0, -8.0, -1.0, 1.0, 8.0, 100.0], device="cuda", dtype=torch.float64).repeat(T // 12)
+    x = (gates[:, None] * (torch.linalg.pinv(weights[0][0].double()) @ torch.ones(ff, device="cuda", dtype=torch.float64))).to(torch.bfloat16).float()
+    m = moe.Moe(layer, 1, T)
+    out = torch.empty((T, d), device="cuda")
+    m.forward_dev(x, torch.zeros((T, 1), device="cuda"), out)
+    kernels._done()
+    m.close()
+    ref, _ = layer_reference(weights, torch.zeros(T, dtype=torch.long, device="cuda"), x)
+    assert (ref.norm(dim=1) > 0).all()
+    err = (out.double() - ref).norm(dim=1) / ref.norm(dim=1)
+    assert (err < 0.25).all(), err[:12]
