@@ -31,6 +31,8 @@
 // TMEM and returns.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "seed_block.cuh"
 #include "seed_mma.cuh"
@@ -136,17 +138,17 @@ __device__ __forceinline__ float to_bf16(float x) { return __uint_as_float(bf16x
 // A thread's share of one K step: the 8 blocks (64 weights) of its row.
 struct ChunkIn { uint4 s, c; uint32_t cd; };
 
-// VEC, how the streams may be read.  2: rows of whole chunks; 16, 16 and 4 bytes where the slice's streams are aligned for that (wide,
-// stream_wide), else as 1.  1: rows of whole half chunks (K a multiple of 32), streams aligned to 8, 8 and 2 bytes.  0: anything.
+// VEC, how the streams may be read.  2: rows of whole chunks, streams aligned to 16, 16 and 4 bytes (stream_wide).  1: rows of whole half
+// chunks (K a multiple of 32), streams aligned to 8, 8 and 2 bytes.  0: anything.
 template <bool P3>
 __device__ __forceinline__ bool stream_wide(const WSlice& w) {
     return (((unsigned long long) w.p[0] | (unsigned long long) w.p[1]) & 15ull) == 0 && (P3 || ((unsigned long long) w.p[3] & 3ull) == 0);
 }
 template <bool P3, int VEC>
-__device__ __forceinline__ ChunkIn load_row_chunk(const WSlice& w, bool wide, int row, int chunk, int R, int NB) {
+__device__ __forceinline__ ChunkIn load_row_chunk(const WSlice& w, int row, int chunk, int R, int NB) {
     ChunkIn q = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u), 0u};      // zero coefficients: zero weights
     if (row >= R || chunk * 8 >= NB) return q;
-    if (VEC == 2 && wide) {
+    if (VEC == 2) {
         const uint32_t i = (uint32_t) row * (uint32_t) (NB / 8) + (uint32_t) chunk;
         q.s = __ldg((const uint4*) w.p[0] + i);
         q.c = __ldg((const uint4*) w.p[1] + i);
@@ -156,7 +158,7 @@ __device__ __forceinline__ ChunkIn load_row_chunk(const WSlice& w, bool wide, in
         const uint2 s0 = __ldg((const uint2*) w.p[0] + i), c0 = __ldg((const uint2*) w.p[1] + i);
         uint2 s1 = make_uint2(0u, 0u), c1 = s1;
         if (!P3) q.cd = __ldg((const uint16_t*) w.p[3] + i);
-        if (VEC == 2 || chunk * 8 + 4 < NB) {
+        if (chunk * 8 + 4 < NB) {
             s1 = __ldg((const uint2*) w.p[0] + i + 1);
             c1 = __ldg((const uint2*) w.p[1] + i + 1);
             if (!P3) q.cd |= (uint32_t) __ldg((const uint16_t*) w.p[3] + i + 1) << 16;
@@ -211,21 +213,45 @@ __device__ __forceinline__ uint32_t input_at(uint32_t stage, int n, int uu) {
     return stage + (uint32_t) (n * 128 + ((uu ^ (n & 7)) << 4));
 }
 
-// 1 / (1 + e^-g): the hardware's reciprocal and one Newton-Raphson step r + r (1 - d r); where the result is subnormal (g under -87.3), which
-// the approximation flushes to zero, or e^-g is infinite, the division.  For every bf16 g the bf16 value is that of the division.
-__device__ __forceinline__ float sigmoid(float g) {
+// 1 / (1 + e^-g).  The hardware's reciprocal and one Newton-Raphson step r + r (1 - d r): for every bf16 g above -87.3 the division's
+// value.  Below, the result is subnormal, which the approximation flushes to zero, or e^-g is infinite: largest collects the denominators,
+// so that the caller can go back and divide.
+template <bool DIVIDE>
+__device__ __forceinline__ float sigmoid(float g, float& largest) {
     const float d = 1.0f + expf(-g);
+    if (DIVIDE) return 1.0f / d;
+    largest = fmaxf(largest, d);
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    r = fmaf(r, fmaf(-d, r, 1.0f), r);
-    if (d > 8e37f) r = 1.0f / d;
-    return r;
+    return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
 
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {      // each product rounded once
     uint32_t d;
     asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
+}
+
+// SwiGLU of 16 columns of a warp: two = bf16 pairs of the gate's (even lanes) and the up matrix's (odd lanes) sums, two columns a word.
+// Even lanes finish columns 0..7, odd lanes 8..15, into the warp's box at `at`.  Returns the largest denominator.
+template <bool DIVIDE, int ROWS>
+__device__ __forceinline__ float swiglu_columns(const uint32_t* two, bool odd, uint16_t* at) {
+    float largest = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t mine = odd ? two[j + 4] : two[j], from = __shfl_xor_sync(0xFFFFFFFFu, odd ? two[j] : two[j + 4], 1);
+        const uint32_t g = odd ? from : mine, up = odd ? mine : from;
+        const uint32_t sg = bf16x2_bits(sigmoid<DIVIDE>(__uint_as_float(g << 16), largest), sigmoid<DIVIDE>(__uint_as_float(g & 0xFFFF0000u), largest));
+        const uint32_t o = mul_bf16x2(mul_bf16x2(g, sg), up);
+        at[2 * j * ROWS] = (uint16_t) o;
+        at[(2 * j + 1) * ROWS] = (uint16_t) (o >> 16);
+    }
+    return largest;
+}
+template <int ROWS>
+__device__ __noinline__ void swiglu_columns_divide(uint4 a, uint4 b, bool odd, uint16_t* at) {
+    const uint32_t two[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    swiglu_columns<true, ROWS>(two, odd, at);
 }
 
 // The results of a unit, by the producer warps: warp w reads the tensor memory lanes of its quarter, 16 columns at a time, the
@@ -256,15 +282,8 @@ __device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, u
             if (GU) {
                 const bool odd = lane & 1;
                 uint16_t* const at = box + (odd ? 8 * ROWS : 0) + (lane >> 1);      // even lanes finish columns 0..7, odd lanes 8..15
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t mine = odd ? two[j + 4] : two[j], from = __shfl_xor_sync(0xFFFFFFFFu, odd ? two[j] : two[j + 4], 1);
-                    const uint32_t g = odd ? from : mine, up = odd ? mine : from;
-                    const uint32_t sg = bf16x2_bits(sigmoid(__uint_as_float(g << 16)), sigmoid(__uint_as_float(g & 0xFFFF0000u)));
-                    const uint32_t o = mul_bf16x2(mul_bf16x2(g, sg), up);
-                    at[2 * j * ROWS] = (uint16_t) o;
-                    at[(2 * j + 1) * ROWS] = (uint16_t) (o >> 16);
-                }
+                if (__any_sync(0xFFFFFFFFu, swiglu_columns<false, ROWS>(two, odd, at) > 8e37f))      // (rare: out of line; a branch at every value cost a layer 1024 / 1024 wide 5 %)
+                    swiglu_columns_divide<ROWS>(make_uint4(two[0], two[1], two[2], two[3]), make_uint4(two[4], two[5], two[6], two[7]), odd, at);
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -295,7 +314,8 @@ __device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, u
 }
 
 // WF: the weights' form.  0: SEED4P4 blocks; 1: stored BF16 values; 2: SEED4 (P = 3) blocks.  TERMS: bf16 terms a weight (1, or 3:
-// exact).  TT: tiles of 128 rows of inputs that share one expansion.  VEC: how the streams are read (load_row_chunk).
+// exact).  TT: tiles of 128 rows of inputs that share one expansion.  VEC: how the streams are read (load_row_chunk; 2: slices that are not
+// aligned for it as 1).
 // GU: gate + up + SwiGLU; row i of the gate matrix on lane 2 i, of the up matrix on lane 2 i + 1.
 template <int TERMS, int WF, int TT, int VEC, bool GU, int IN>
 __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT, IN>::CTAS) seed_gemm_kernel(MmParams a, KConst kc, const __grid_constant__ CUtensorMap tm) {
@@ -390,68 +410,75 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
             const WSlice w = GU && (lane & 1) ? u.wb : u.wa;
             const int grow = GU ? u.r0 + (rl >> 1) : u.r0 + rl;
             const float base = BF16W ? 0.0f : exact_base<P3 ? 3 : 4>(w.eb);
-            const bool wide = VEC == 2 && stream_wide<P3>(w);
-            int kt = (group - kr0 % GROUPS + GROUPS) % GROUPS;
-            ChunkIn cur = {};
-            if (!BF16W && kt < KT) cur = load_row_chunk<P3, VEC>(w, wide, grow, kt, a.R, NB);
-            for (; kt < KT && ok; kt += GROUPS) {
-                const int kr = kr0 + kt, s = kr % GM_STAGES;
-                const uint32_t ta = tmem_w + ((uint32_t) (lq * 32) << 16) + (uint32_t) (s * Cfg::A_COLS);
-                ChunkIn nxt = {};
-                if (!BF16W && kt + GROUPS < KT) nxt = load_row_chunk<P3, VEC>(w, wide, grow, kt + GROUPS, a.R, NB);
-                const uint32_t sw[4] = {cur.s.x, cur.s.y, cur.s.z, cur.s.w}, cw[4] = {cur.c.x, cur.c.y, cur.c.z, cur.c.w};
+            auto steps = [&](auto how) {      // the unit's K steps of this warpgroup
+                constexpr int V = decltype(how)::value;
+                int kt = (group - kr0 % GROUPS + GROUPS) % GROUPS;
+                ChunkIn cur = {};
+                if (!BF16W && kt < KT) cur = load_row_chunk<P3, V>(w, grow, kt, a.R, NB);
+                for (; kt < KT && ok; kt += GROUPS) {
+                    const int kr = kr0 + kt, s = kr % GM_STAGES;
+                    const uint32_t ta = tmem_w + ((uint32_t) (lq * 32) << 16) + (uint32_t) (s * Cfg::A_COLS);
+                    ChunkIn nxt = {};
+                    if (!BF16W && kt + GROUPS < KT) nxt = load_row_chunk<P3, V>(w, grow, kt + GROUPS, a.R, NB);
+                    const uint32_t sw[4] = {cur.s.x, cur.s.y, cur.s.z, cur.s.w}, cw[4] = {cur.c.x, cur.c.y, cur.c.z, cur.c.w};
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {      // 32 weights = 16 words
-                    uint32_t v[TERMS][16];
-                    if (BF16W) {
+                    for (int q = 0; q < 2; ++q) {      // 32 weights = 16 words
+                        uint32_t v[TERMS][16];
+                        if (BF16W) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int k = kt * GM_BK + q * 32 + 8 * i;
-                            const uint4 t = grow < a.R && k < a.K ? __ldg((const uint4*) ((const uint16_t*) w.p[0] + (size_t) grow * a.K + k)) : make_uint4(0u, 0u, 0u, 0u);
-                            v[0][4 * i] = t.x; v[0][4 * i + 1] = t.y; v[0][4 * i + 2] = t.z; v[0][4 * i + 3] = t.w;
-                        }
-                    } else {
+                            for (int i = 0; i < 4; ++i) {
+                                const int k = kt * GM_BK + q * 32 + 8 * i;
+                                const uint4 t = grow < a.R && k < a.K ? __ldg((const uint4*) ((const uint16_t*) w.p[0] + (size_t) grow * a.K + k)) : make_uint4(0u, 0u, 0u, 0u);
+                                v[0][4 * i] = t.x; v[0][4 * i + 1] = t.y; v[0][4 * i + 2] = t.z; v[0][4 * i + 3] = t.w;
+                            }
+                        } else {
 #pragma unroll
-                        for (int b = 0; b < 2; ++b) {
-                            const int bp = 2 * q + b;
-                            u64 w2[8];
-                            const u64 e2 = P3 ? code_scale_pair3(cw[bp], kc) : code_scale_pair(cur.cd, bp, kc);
-                            pair_weights<P3 ? 3 : 4>(tab, sw[bp], cw[bp], e2, base, kc, w2);
-                            float wa[8], wb[8];
+                            for (int b = 0; b < 2; ++b) {
+                                const int bp = 2 * q + b;
+                                u64 w2[8];
+                                const u64 e2 = P3 ? code_scale_pair3(cw[bp], kc) : code_scale_pair(cur.cd, bp, kc);
+                                pair_weights<P3 ? 3 : 4>(tab, sw[bp], cw[bp], e2, base, kc, w2);
+                                float wa[8], wb[8];
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) unpack2(w2[i], wa[i], wb[i]);
+                                for (int i = 0; i < 8; ++i) unpack2(w2[i], wa[i], wb[i]);
 #pragma unroll
-                            for (int t = 0; t < TERMS; ++t) {      // term t = the bf16 value of what remains (exact subtraction)
+                                for (int t = 0; t < TERMS; ++t) {      // term t = the bf16 value of what remains (exact subtraction)
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    const uint32_t o = bf16x2_bits(wa[2 * i], wa[2 * i + 1]), p = bf16x2_bits(wb[2 * i], wb[2 * i + 1]);
-                                    v[t][8 * b + i] = o;
-                                    v[t][8 * b + 4 + i] = p;
-                                    if (t + 1 < TERMS) {
-                                        wa[2 * i] -= __uint_as_float(o << 16); wa[2 * i + 1] -= __uint_as_float(o & 0xFFFF0000u);
-                                        wb[2 * i] -= __uint_as_float(p << 16); wb[2 * i + 1] -= __uint_as_float(p & 0xFFFF0000u);
+                                    for (int i = 0; i < 4; ++i) {
+                                        const uint32_t o = bf16x2_bits(wa[2 * i], wa[2 * i + 1]), p = bf16x2_bits(wb[2 * i], wb[2 * i + 1]);
+                                        v[t][8 * b + i] = o;
+                                        v[t][8 * b + 4 + i] = p;
+                                        if (t + 1 < TERMS) {
+                                            wa[2 * i] -= __uint_as_float(o << 16); wa[2 * i + 1] -= __uint_as_float(o & 0xFFFF0000u);
+                                            wb[2 * i] -= __uint_as_float(p << 16); wb[2 * i + 1] -= __uint_as_float(p & 0xFFFF0000u);
+                                        }
                                     }
                                 }
                             }
                         }
-                    }
-                    if (q == 0) {      // the stage has to be free only now: half of the step is in registers
-                        if (kr >= GM_STAGES && !mbar_wait(bar_empty + 8 * s, ((kr / GM_STAGES) - 1) & 1, &abort_flag)) fail(1);
-                        ok = __all_sync(0xFFFFFFFFu, ok);
-                        if (!ok) break;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    }
+                        if (q == 0) {      // the stage has to be free only now: half of the step is in registers
+                            if (kr >= GM_STAGES && !mbar_wait(bar_empty + 8 * s, ((kr / GM_STAGES) - 1) & 1, &abort_flag)) fail(1);
+                            ok = __all_sync(0xFFFFFFFFu, ok);
+                            if (!ok) break;
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        }
 #pragma unroll
-                    for (int t = 0; t < TERMS; ++t) tmem_st16(ta + t * 32 + q * 16, v[t]);
+                        for (int t = 0; t < TERMS; ++t) tmem_st16(ta + t * 32 + q * 16, v[t]);
+                    }
+                    if (!ok) break;
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_full + 8 * s);
+                    cur = nxt;
+                    if (p_count) results();      // the previous unit's: its last MMAs ran under this step
                 }
-                if (!ok) break;
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_full + 8 * s);
-                cur = nxt;
-                if (p_count) results();      // the previous unit's: its last MMAs ran under this step
-            }
+            };
+            // A table's slices are looked at a unit at a time (512 / 4096 rows of config 1's layer 276.8 / 454.8 us, without the look 274.9 / 453.5; with
+            // predicated loads in one loop 276.8 / 461.3).
+            if (VEC != 2) steps(std::integral_constant<int, VEC>{});
+            else if (__all_sync(0xFFFFFFFFu, stream_wide<P3>(w))) steps(std::integral_constant<int, 2>{});
+            else steps(std::integral_constant<int, 1>{});
             if (ok && p_count) results();      // (a unit with fewer steps than warpgroups)
             kr0 += KT;
             ++unit_run;
