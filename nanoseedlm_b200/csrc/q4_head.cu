@@ -545,10 +545,14 @@ static void launch_q4_ring(cudaStream_t s, size_t total, int blocks, const WSlic
            (const uint16_t*) w.p[1], (const uint16_t*) w.p[2], K, R, x, xs, y, ys, T, add);
 }
 
-// Greedy arg-max of each row (ties: the lowest id) and, optionally, its softmax probability 1 / sum exp(l - max).  A row is shared by
-// a cluster of ARG_CTAS blocks, whose candidates meet in the first one's shared memory: one block a row left the chip idle
-// (15.6 us for 8 rows of 151936, a load's latency per 1024 values).
+// Greedy arg-max of each row (ties: the lowest id) and, optionally, its softmax probability 1 / sum exp(l - max).
+// A few long rows: each is shared by a cluster of ARG_CTAS blocks, whose candidates meet in the first one's shared memory (a block a
+// row leaves the chip idle).  Many rows fill it by themselves, and for short ones a cluster's barriers cost more than they share: a
+// block a row.  us, logits in L2, shared / a block a row: 151936 logits, 8 rows 3.9 / 6.7, 48 rows 6.2 / 6.7, 64 rows 7.3 / 6.8,
+// 256 rows 31 / 28; 32000: 8 rows 2.8 / 3.8, 32 rows 3.1 / 3.8, 48 rows 3.9 / 3.8; 16000: 8 rows 2.7 / 2.9; 8192: 8 rows 2.6 / 2.2;
+// 1000: 256 rows 9.7 / 2.6.
 constexpr int ARG_CTAS = 8, ARG_T = 512;
+static bool argmax_shared(int V, int n) { return V >= 24000 && n <= 32; }
 
 __device__ __forceinline__ void arg_better(float& v, int& i, float v2, int i2) {
     if (v2 > v || (v2 == v && i2 < i)) { v = v2; i = i2; }
@@ -651,6 +655,48 @@ __global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax
     }
 }
 
+// A block a row.
+__global__ void __launch_bounds__(1024) argmax_row_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, float* __restrict__ prob, int V) {
+    __shared__ float bv[32];
+    __shared__ int bi[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const float* l = logits + (size_t) blockIdx.x * V;
+    grid_dependents_go();
+    grid_dependency_wait();
+    float best = -INFINITY;
+    int idx = 0x7FFFFFFF;
+    for (int i = tid; i < V; i += 1024) {
+        const float v = l[i];
+        if (v > best) { best = v; idx = i; }      // ascending i: the first of equal values stays
+    }
+    auto warp_best = [&]() {
+        for (int o = 16; o > 0; o >>= 1) arg_better(best, idx, __shfl_xor_sync(0xFFFFFFFFu, best, o), __shfl_xor_sync(0xFFFFFFFFu, idx, o));
+    };
+    warp_best();
+    if (lane == 0) { bv[w] = best; bi[w] = idx; }
+    __syncthreads();
+    if (w == 0) {
+        best = bv[lane];
+        idx = bi[lane];
+        warp_best();
+        if (lane == 0) { out[blockIdx.x] = idx == 0x7FFFFFFF ? 0 : idx; bv[0] = best; }
+    }
+    if (!prob) return;
+    __syncthreads();
+    const float mx = bv[0];
+    float s = 0.0f;
+    for (int i = tid; i < V; i += 1024) s += expf(l[i] - mx);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    __syncthreads();      // every thread has read bv[0]
+    if (lane == 0) bv[w] = s;
+    __syncthreads();
+    if (tid == 0) {
+        float tot = 0.0f;
+        for (int i = 0; i < 32; ++i) tot += bv[i];
+        prob[blockIdx.x] = 1.0f / tot;
+    }
+}
+
 // kc_mv for fmt == MF_Q4, and the decoder's head for any number of tokens.  Returns false (with the error recorded) when the shape
 // is not served.
 bool launch_q4_mv(cudaStream_t s, const WSlice& w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add) {
@@ -712,10 +758,8 @@ extern "C" {
 
 void kc_argmax_p(cudaStream_t s, const float* logits, int32_t* out, float* prob, int V, int n) {
     if (V < 1 || n < 1) return;
-    for (int n0 = 0; n0 < n; n0 += 65535) {
-        const int m = n - n0 < 65535 ? n - n0 : 65535;
-        launch(argmax_kernel, dim3(ARG_CTAS, (unsigned) m), ARG_T, 0, s, logits + (size_t) n0 * V, out + n0, prob ? prob + n0 : (float*) NULL, V);
-    }
+    if (argmax_shared(V, n)) launch(argmax_kernel, dim3(ARG_CTAS, (unsigned) n), ARG_T, 0, s, logits, out, prob, V);
+    else launch(argmax_row_kernel, (unsigned) n, 1024, 0, s, logits, out, prob, V);
     count_launch();
 }
 

@@ -64,9 +64,10 @@ def test_argmax_ties_to_the_lowest_id_and_probability(V, n):
     assert np.array_equal(kernels.kt_argmax(logits), ro)
 
 
-@pytest.mark.parametrize("V,n", [(1, 1), (2, 700), (5, 300), (33, 2000), (4097, 61)])
+@pytest.mark.parametrize("V,n", [(1, 1), (2, 700), (5, 300), (33, 2000), (4097, 61), (23999, 32), (24000, 32), (24000, 33), (24003, 1)])
 def test_argmax_of_many_short_rows(V, n):
-    """Rows with less than a value a block of the cluster: their blocks meet as soon as they have started."""
+    """From one value a row to either side of the lines (24000 values, 32 rows) where a cluster of blocks shares a row, on and off a
+    16-byte boundary."""
     from nanoseedlm_b200 import kernels
     logits = (np.random.default_rng(V + n).standard_normal((n, V)) * 3).astype(np.float32)
     ro, rp = logits.argmax(axis=1), [1 / np.exp(r.astype(np.float64) - r.max()).sum() for r in logits]
@@ -76,7 +77,7 @@ def test_argmax_of_many_short_rows(V, n):
         np.testing.assert_allclose(prob, rp, rtol=2e-5)
 
 
-@pytest.mark.parametrize("V,row", [(33, 1000), (7, 2), (8, 1), (1023, 3)])
+@pytest.mark.parametrize("V,row", [(33, 1000), (7, 2), (8, 1), (1023, 3), (24001, 2), (24001, 30), (24002, 45)])
 def test_argmax_without_a_largest_value(V, row):
     """A row of -inf (rows that start on and off a 16-byte boundary, with and without a tail) gives id 0; -inf beside a finite value never wins."""
     from nanoseedlm_b200 import kernels
