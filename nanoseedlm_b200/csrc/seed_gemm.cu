@@ -655,8 +655,9 @@ static bool encode_inputs(CUtensorMap* tm, const MmParams& a) {
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// false (nothing launched): IN_TMA inputs that a tensor map cannot describe.
 template <int TERMS, int WF, int TT, int VEC, bool GU, int IN>
-static void launch_gemm_v(cudaStream_t s, const MmParams& a, int units) {
+static bool launch_gemm_v(cudaStream_t s, const MmParams& a, int units) {
     using Cfg = GmCfg<TERMS, TT, IN>;
     const size_t smem = (size_t) GM_STAGES * Cfg::X_BYTES + Cfg::PW * 1024 + 1024;
     static bool attr_set[16];
@@ -667,11 +668,13 @@ static void launch_gemm_v(cudaStream_t s, const MmParams& a, int units) {
         attr_set[dev & 15] = true;
     }
     CUtensorMap tm = {};
-    if (IN == IN_TMA && !encode_inputs(&tm, a)) { set_error("seed GEMM: no tensor map for packed inputs of row stride %d", a.xs); return; }
+    if (IN == IN_TMA && (a.xs < a.K || !encode_inputs(&tm, a))) return false;
     const int slots = sm_count() * Cfg::CTAS;
     launch(seed_gemm_kernel<TERMS, WF, TT, VEC, GU, IN>, (unsigned) (units < slots ? units : slots), Cfg::THREADS, smem, s, a, kconst(), tm);
     count_launch();
+    return true;
 }
+static void no_map(const MmParams& a) { set_error("seed GEMM: no tensor map for sorted inputs of row stride %d", a.xs); }
 // How many tiles of a dense call share an expansion: a unit takes the time of its expansion (twice that where two blocks share an
 // SM) or of its inputs' conversion (f32: nine tenths of it per tile), and the units go round the SMs.
 static int dense_tiles(const MmParams& a, int row_tiles) {
@@ -706,11 +709,14 @@ static void launch_gemm_seed(cudaStream_t s, const MmParams& a, int row_tiles, i
         else launch_gemm_v<1, WF, 1, 0, false, IN_F32>(s, a, units);
     } else if (a.grouped) {
         if (!a.packed) launch_gemm_v<1, WF, 1, 2, false, IN_F32>(s, a, units);
-        else if (a.in_sorted && a.offs) launch_gemm_v<1, WF, 3, 2, false, IN_TMA>(s, a, units);
+        else if (a.in_sorted && a.offs) { if (!launch_gemm_v<1, WF, 3, 2, false, IN_TMA>(s, a, units)) no_map(a); }
         else launch_gemm_v<1, WF, 1, 2, false, IN_LIST>(s, a, units);
     } else {
         const int tt = dense_tiles(a, row_tiles), u = row_tiles * ((a.T + GM_BN * tt - 1) / (GM_BN * tt));
-        if (a.packed) { if (tt == 1) launch_gemm_v<1, WF, 1, 2, false, IN_TMA>(s, a, u); else launch_gemm_v<1, WF, 3, 2, false, IN_TMA>(s, a, u); }
+        if (a.packed) {
+            if (!(tt == 1 ? launch_gemm_v<1, WF, 1, 2, false, IN_TMA>(s, a, u) : launch_gemm_v<1, WF, 3, 2, false, IN_TMA>(s, a, u)))
+                launch_gemm_v<1, WF, 1, 2, false, IN_LIST>(s, a, units);      // rows that overlap
+        }
         else if (tt == 1) launch_gemm_v<1, WF, 1, 2, false, IN_F32>(s, a, u);
         else if (tt == 2) launch_gemm_v<1, WF, 2, 2, false, IN_F32>(s, a, u);
         else launch_gemm_v<1, WF, 3, 2, false, IN_F32>(s, a, u);
@@ -718,7 +724,7 @@ static void launch_gemm_seed(cudaStream_t s, const MmParams& a, int row_tiles, i
 }
 void launch_gemm_gu(cudaStream_t s, const MmParams& a, int tiles_y) {
     const int units = (a.R + GM_BM / 2 - 1) / (GM_BM / 2) * tiles_y;
-    if (a.offs) launch_gemm_v<1, 0, 3, 2, true, IN_TMA>(s, a, units);
+    if (a.offs) { if (!launch_gemm_v<1, 0, 3, 2, true, IN_TMA>(s, a, units)) no_map(a); }
     else launch_gemm_v<1, 0, 1, 2, true, IN_LIST>(s, a, units);
 }
 bool gemm_shares_tiles(int max_tiles) { return max_tiles <= GM_MAX_HEADS; }

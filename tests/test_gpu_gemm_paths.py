@@ -233,3 +233,22 @@ def test_swiglu_over_the_range_of_gates(T):
     assert (ref.norm(dim=1) > 0).all()
     err = (out.double() - ref).norm(dim=1) / ref.norm(dim=1)
     assert (err < 0.25).all(), err[:12]
+
+
+@pytest.mark.parametrize("xs", [0, 64, 184, 192, 200])
+@pytest.mark.parametrize("T", [40, 70, 500])
+def test_packed_rows_at_any_distance(xs, T):
+    """Packed rows that repeat, overlap, follow one another or lie apart (a tensor map describes the last two)."""
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L
+    R, K = 150, 192
+    m = B.Matrix(R, K, 5, eb=-21)
+    w = kernels.SeedWeight.from_matrices([m])
+    W = B.bfr(B.decode_rows_f32(m)).astype(np.float64)
+    flat = B.bfr(np.random.default_rng(xs).standard_normal((T - 1) * xs + K).astype(np.float32))
+    x = np.stack([flat[t * xs:t * xs + K] for t in range(T)]).astype(np.float64)
+    xd, y = kernels.dev(flat).to(torch.bfloat16), torch.full((T, R), float("nan"), device="cuda")
+    L.load().kc_mm_packed(kernels._stream(), L.MF_SEED4P4, w.slice(0), K, R, kernels._ptr(xd), xs, kernels._ptr(y), R, T, 0, kernels._ptr(kernels.stream_table()))
+    kernels._done()
+    ref = B.bfr((x @ W.T).astype(np.float32)).astype(np.float64)
+    assert (np.abs(y.cpu().numpy() - ref) <= np.abs(ref) / 128 + F32B * (np.abs(x) @ np.abs(W.T)) + 1e-30).all()
