@@ -230,8 +230,9 @@ void nsl_mv_gu_raw(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K, in
 void nsl_decode_f32(cudaStream_t s, WSlice w, int K, int R, float* out, const uint32_t* G);
 void nsl_decode_bf16(cudaStream_t s, WSlice w, int K, int R, uint16_t* out, const uint32_t* G);
 /* 0, or the code of the first bounded device-side wait that ran out in a GEMM block since the last call (1 a producer
- * waiting for a free stage, 2 the epilogue waiting for the accumulator, 3 the MMA issuer waiting for a full stage); a
- * block that gives up frees its tensor memory and returns without storing.  Call after synchronising the stream. */
+ * waiting for a free stage, 2 results waiting for the accumulators, 3 the MMA issuer waiting for a full stage or for the
+ * results to have been read, 4 a loader waiting for a free stage); a block that gives up lets what it has in flight end, frees its tensor memory and
+ * returns without storing.  Call after synchronising the stream. */
 int nsl_mm_status(void);
 /* Fills a 65536-entry host array with the stream table the G arguments expect (lfsr_stream32 of every seed,
  * nslm/lfsr.h:53-59). */

@@ -27,8 +27,8 @@
 // Weight precision: default, seed weights rounded to bf16 (one term); kc_seed_gemm_f32(1), three bf16 terms whose sum is
 // the f32 weight exactly (three MMAs per step), as the reference's two modes (engine/kernels_moe.cu:405-412).
 //
-// Every wait on an mbarrier is bounded: after the limit the block records a status word, stops issuing work, frees its
-// TMEM and returns.
+// Every wait on an mbarrier is bounded: after the limit the block records a status word, stops issuing work, lets its copies and MMAs in
+// flight end, frees its TMEM and returns.
 #include <cuda.h>
 
 #include <type_traits>
@@ -630,6 +630,17 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (abort_flag) {      // a wait ran out: the block's copies and MMAs in flight have no barrier left to report to, so they get a millisecond before its memory goes
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        unsigned long long t0, t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+        for (int i = 0; i < 4096; ++i) {
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (t - t0 > 1000000ull) break;
+            __nanosleep(1000);
+        }
+        __syncthreads();
+    }
     if (warp == PW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::COLS) : "memory");
 }
 
@@ -792,8 +803,8 @@ void kc_mm_grouped_packed(cudaStream_t s, int fmt, const WSlice* ws, int K, int 
 }
 
 // 0, or the code of the first bounded wait that ran out in a GEMM block since the last call (1 producer waiting for a
-// free stage, 2 epilogue waiting for the accumulator, 3 MMA issuer waiting for a full stage).  Reads device memory: call
-// it after the stream has been synchronised.
+// free stage, 2 results waiting for the accumulators, 3 MMA issuer waiting for a full stage or for the results to have been read, 4 loader
+// waiting for a free stage).  Reads device memory: call it after the stream has been synchronised.
 int nsl_mm_status(void) {
     int v = 0, zero = 0;
     cudaMemcpyFromSymbol(&v, g_mm_status, sizeof v);
