@@ -60,7 +60,7 @@ struct KConst {
     uint32_t cor;       // 112 << 23: 2^(code - 15) from a code placed at bits 23..26
     unsigned long long coff_x2[4], two2;      // packed pairs: coff_x and 2 (operands from constant memory)
 };
-inline KConst kconst() {
+inline KConst make_kconst() {
     KConst k;
     for (int p = 0; p < 4; ++p) {
         k.cxor[p] = ((uint32_t) (215 - 5 * p) << 23) | (8u << (4 * p));
@@ -72,6 +72,10 @@ inline KConst kconst() {
     auto both = [](float v) { uint32_t u; memcpy(&u, &v, 4); return ((unsigned long long) u << 32) | u; };
     for (int p = 0; p < 4; ++p) k.coff_x2[p] = both(k.coff_x[p]);
     k.two2 = both(2.0f);
+    return k;
+}
+inline const KConst& kconst() {      // made once: sixteen ldexpf a launch otherwise
+    static const KConst k = make_kconst();
     return k;
 }
 #define NSL_XSCALE 18446744073709551616.0f   // 2^64: the mat-vec kernels' input scaling

@@ -65,6 +65,11 @@ struct GmCfg {
     static_assert(GM_STAGES >= GROUPS, "every warpgroup owns a stage");
 };
 
+// The inputs' tensor map, a parameter of the kernels that use one.
+struct NoMap {};
+template <int IN>
+using GmMap = typename std::conditional<IN == IN_TMA, CUtensorMap, NoMap>::type;
+
 __device__ int g_mm_status;   // 0, or the code of the first bounded wait that ran out
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t) __cvta_generic_to_shared(p); }
@@ -318,7 +323,7 @@ __device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, u
 // aligned for it as 1).
 // GU: gate + up + SwiGLU; row i of the gate matrix on lane 2 i, of the up matrix on lane 2 i + 1.
 template <int TERMS, int WF, int TT, int VEC, bool GU, int IN>
-__global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT, IN>::CTAS) seed_gemm_kernel(MmParams a, KConst kc, const __grid_constant__ CUtensorMap tm) {
+__global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT, IN>::CTAS) seed_gemm_kernel(MmParams a, KConst kc, const __grid_constant__ GmMap<IN> tm) {
     using Cfg = GmCfg<TERMS, TT, IN>;
     constexpr bool F32 = IN == IN_F32;
     constexpr bool BF16W = WF == 1, P3 = WF == 2;
@@ -678,8 +683,10 @@ static bool launch_gemm_v(cudaStream_t s, const MmParams& a, int units) {
         cudaFuncSetAttribute(seed_gemm_kernel<TERMS, WF, TT, VEC, GU, IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
         attr_set[dev & 15] = true;
     }
-    CUtensorMap tm = {};
-    if (IN == IN_TMA && (a.xs < a.K || !encode_inputs(&tm, a))) return false;
+    GmMap<IN> tm = {};
+    if constexpr (IN == IN_TMA) {
+        if (a.xs < a.K || !encode_inputs(&tm, a)) return false;
+    }
     const int slots = sm_count() * Cfg::CTAS;
     launch(seed_gemm_kernel<TERMS, WF, TT, VEC, GU, IN>, (unsigned) (units < slots ? units : slots), Cfg::THREADS, smem, s, a, kconst(), tm);
     count_launch();
