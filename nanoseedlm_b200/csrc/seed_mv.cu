@@ -1203,6 +1203,8 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_dense_kernel(MvParams a, KCo
     extern __shared__ __align__(16) ulonglong2 dense_sx[];
     __shared__ StreamTab tab;
     int block = blockIdx.x, blocks = gridDim.x;
+    a.x += (size_t) blockIdx.y * NT * a.xs;      // a small matrix: groups of NT rows of inputs side by side
+    a.y += (size_t) blockIdx.y * NT * a.ys;
     if (set.n > 1) {      // several matrices share the launch
         const int m = set_member(set, block);
         block -= set.first[m];
@@ -1474,14 +1476,14 @@ static void launch_grp(cudaStream_t s, const MvParams& a, int lpr_log2) {
 }
 
 template <int PF, int NT>
-static void launch_dense_v(cudaStream_t s, const MvParams& a, size_t smem, DenseSet* set) {
+static void launch_dense_v(cudaStream_t s, const MvParams& a, size_t smem, DenseSet* set, int groups = 1) {
     static bool attr_set[16];
     const int bps = smem > 100 * 1024 ? 1 : 2;
     long long rows = a.R;
     for (int m = 1; set && m < set->n; ++m) rows += set->R[m];
     const RowShape sh = row_shape(a.K / 64, rows, sm_count() * bps * MV_WARPS);
     auto steps_of = [&](long long r) { return (int) ((r * (1 << sh.lpr_log2) + 31) / 32); };
-    int blocks = std::min(steps_of(rows), sm_count() * bps);
+    int blocks = std::min(steps_of(rows), std::max(sm_count() * bps / groups, 1));
     if (set) {      // each matrix gets its share of the blocks, at least one
         int left = blocks > set->n ? blocks : set->n;
         long long rest = rows;
@@ -1498,13 +1500,29 @@ static void launch_dense_v(cudaStream_t s, const MvParams& a, size_t smem, Dense
         blocks = set->first[DENSE_SET];
     }
     if (smem > 40 * 1024) allow_smem(mv_dense_kernel<PF, NT>, attr_set, (size_t) max_smem_optin() - 8192);
-    launch(mv_dense_kernel<PF, NT>, blocks, MV_THREADS, smem, s, a, kconst(), sh, set ? *set : DenseSet{1});
+    launch(mv_dense_kernel<PF, NT>, dim3((unsigned) blocks, (unsigned) groups), MV_THREADS, smem, s, a, kconst(), sh, set ? *set : DenseSet{1});
     count_launch();
 }
 // T rows on one slice; more rows than their inputs fit shared memory go in two launches (a row's bits do not depend on the rest).
 template <int PF>
 static void launch_dense(cudaStream_t s, MvParams a, int T, DenseSet* set = NULL) {
     const size_t one = staged_bytes(a.K / 64), room = (size_t) max_smem_optin() - 8192;
+    // A matrix of fewer row steps than half the warps: its rows of inputs are shared out too (a P = 3 matrix of 512 x 2048, 8 rows: 12.3 us in one
+    // group, 9.1 in four, which is the call itself; 256 x 4096, 8 rows 13.0 and 9.2).
+    if (!set && T > 1) {
+        const int warps = sm_count() * 2 * MV_WARPS, ch = a.K / 64, per_step = ch < 32 ? 32 / ch : 1, steps = (a.R + per_step - 1) / per_step;
+        int g = T;
+        while (g > 1 && (T % g || (long long) steps * g > warps)) --g;
+        if (g > 1 && (size_t) (T / g) * one <= room) {
+            const int n = T / g;
+            switch (n) {
+                case 1: launch_dense_v<PF, 1>(s, a, n * one, NULL, g); return;
+                case 2: launch_dense_v<PF, 2>(s, a, n * one, NULL, g); return;
+                case 3: launch_dense_v<PF, 3>(s, a, n * one, NULL, g); return;
+                default: launch_dense_v<PF, 4>(s, a, n * one, NULL, g); return;
+            }
+        }
+    }
     while (T > 0) {
         int n = T;
         while (n > 1 && n * one > room) n = (n + 1) / 2;

@@ -115,3 +115,21 @@ def test_p3_gathers_from_any_address(K, R, by):
 def test_rows_of_one_chunk(p, R):
     """K = 64: a lane is a row and keeps both of an item's sums; rows either side of one and two row steps."""
     test_any_number_of_chunks(p, 64, R)
+
+
+@pytest.mark.parametrize("p", [4, 3])
+@pytest.mark.parametrize("K,R", [(512, 40), (2048, 296), (2048, 593), (4096, 1184), (64 * 45, 1185), (64 * 200, 30), (64 * 300, 30)])
+def test_dense_rows_of_small_matrices(p, K, R):
+    """Matrices whose row steps leave warps over: 2 .. 8 rows of inputs in one group, in several, or (long rows) in two launches; every
+    row has the bits it has alone, with the residual added too."""
+    from nanoseedlm_b200 import kernels
+    W, w = matrices(p, 1, R, K, K + R)
+    mv = kernels.kt_mv if p == 4 else kernels.kt_mv3
+    rng = np.random.default_rng(R)
+    x, y0 = (B.bfr(rng.standard_normal((8, n)).astype(np.float32)) for n in (K, R))
+    alone = [mv(w, x[t:t + 1], 1, add=1, y0=y0[t:t + 1])[0] for t in range(8)]
+    check(mv(w, x[:1], 1)[0], W[0], x[0].astype(np.float64))
+    for T in range(2, 9):
+        d = mv(w, x[:T], T, add=1, y0=y0[:T])
+        for t in range(T):
+            assert np.array_equal(d[t], alone[t]), (T, t)
