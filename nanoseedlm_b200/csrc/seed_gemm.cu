@@ -719,6 +719,7 @@ static void launch_gemm_seed(cudaStream_t s, const MmParams& a, int row_tiles, i
     const int vec = a.K % 32 || (!a.grouped && !streams_aligned<WF>(a.w0, 8)) ? 0 : a.K % 64 ? 1 : 2;
     if (g_exact) {
         if (a.packed) { if (vec) launch_gemm_v<3, WF, 1, 1, false, IN_LIST>(s, a, units); else launch_gemm_v<3, WF, 1, 0, false, IN_LIST>(s, a, units); }
+        else if (vec == 2) launch_gemm_v<3, WF, 1, 2, false, IN_F32>(s, a, units);
         else if (vec) launch_gemm_v<3, WF, 1, 1, false, IN_F32>(s, a, units);
         else launch_gemm_v<3, WF, 1, 0, false, IN_F32>(s, a, units);
     } else if (vec < 2) {
