@@ -44,16 +44,17 @@ constexpr int GM_MAX_HEADS = 2048;      // tiles of a launch whose experts' tile
 constexpr uint32_t GM_WAIT_LIMIT = 1u << 24;
 constexpr unsigned long long GM_WAIT_NS = 1000000000ull;
 // How the inputs reach shared memory.  IN_LIST: packed rows picked by a list (cp.async by the loader warps); IN_F32: f32 rows,
-// converted by the loaders, whose loads of a whole K step are held in registers meanwhile; IN_TMA: packed rows that follow one
+// converted by the loaders, whose loads of a whole K step are held in registers meanwhile (IN_F32_FEW: grouped, units of any number of
+// rows up to a tile); IN_TMA: packed rows that follow one
 // another (dense, or sorted by expert), by one thread.
-enum { IN_LIST = 0, IN_F32 = 1, IN_TMA = 2 };
+enum { IN_LIST = 0, IN_F32 = 1, IN_TMA = 2, IN_F32_FEW = 3 };
 // One block: PW producer warps, the MMA warp, LW loader warps.  Tensor memory: the accumulators (128 columns per tile of inputs),
 // then the stages' weights (32 columns per term: 64 k values as bf16 pairs).
 // LAUNCH_REGS: registers a thread at launch (what the launch bounds leave); PREGS, LREGS: of the producers' and of the other
 // warpgroups after the split, whose sum over the block is at most what the launch gave it.
 template <int TERMS, int TT, int IN>
 struct GmCfg {
-    static constexpr bool F32 = IN == IN_F32;
+    static constexpr bool F32 = IN == IN_F32 || IN == IN_F32_FEW;
     static constexpr int CTAS = TERMS == 1 && TT == 1 && !F32 ? 2 : 1, PW = TERMS == 3 || CTAS == 2 ? 8 : 16, LW = TERMS == 1 && F32 ? 7 : 3;
     static constexpr int WARPS = PW + 1 + LW, THREADS = WARPS * 32, GROUPS = PW / 4;
     static constexpr int ACC = GM_BN * TT, A_COLS = 32 * TERMS, COLS = ACC + GM_STAGES * A_COLS <= 256 ? 256 : 512;
@@ -325,14 +326,14 @@ __device__ __forceinline__ void unit_results(const MmParams& a, uint32_t tmem, u
 template <int TERMS, int WF, int TT, int VEC, bool GU, int IN>
 __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT, IN>::CTAS) seed_gemm_kernel(MmParams a, KConst kc, const __grid_constant__ GmMap<IN> tm) {
     using Cfg = GmCfg<TERMS, TT, IN>;
-    constexpr bool F32 = IN == IN_F32;
+    constexpr bool F32 = Cfg::F32, FEW = IN == IN_F32_FEW;
     constexpr bool BF16W = WF == 1, P3 = WF == 2;
     constexpr int PW = Cfg::PW, GROUPS = Cfg::GROUPS, HALF = Cfg::ACC / 2;
     extern __shared__ uint8_t smem_raw[];
     __shared__ StreamTab tab;
     __shared__ __align__(8) uint64_t bars[2 * GM_STAGES + 3];
     __shared__ uint32_t tmem_slot;
-    __shared__ int srow[GM_BN * TT];      // the unit's rows of inputs
+    __shared__ int srow[FEW ? Cfg::LW * 20 : GM_BN * TT];      // the unit's rows of inputs (FEW: 20 places a warp)
     __shared__ int abort_flag, n_heads;
     __shared__ uint16_t heads[TT > 1 ? GM_MAX_HEADS : 1];
 
@@ -564,10 +565,20 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
                 if (u.count <= 0) continue;
                 const int n16 = (u.count + 15) & ~15;
                 __syncwarp();
+                // FEW, units of few rows: groups of warps take the K steps in turn, so that two or three steps' rows are in flight instead of
+                // one (a memory latency a step).  us, 128 experts, 512 x 2048: 512 / 4096 pairs 122 / 154 -> 105 / 117; 7000 and 12000 (units
+                // of more than 60 rows) 162 / 174 -> 168 / 179.  The places of a warp's rows are its own: groups may be in different units.
+                int groups = 1, grp = 0, wi = lt >> 5, rpp = RPP, n_first = n_lo;
+                if (FEW) {
+                    if (n16 <= 40) { groups = 3; grp = min(wi >> 1, 2); wi -= 2 * grp; rpp = grp == 2 ? 12 : 8; }
+                    else if (n16 <= 60) { groups = 2; grp = wi >> 2; wi -= 4 * grp; rpp = grp ? 12 : 16; }
+                    n_first = 4 * wi + (lane >> 3);
+                }
+                const int mine = FEW ? (lt >> 5) * 20 : 0;
                 for (int i = lane;; i += 32) {      // this warp's own rows: 4 w .. 4 w + 3, then every RPP on
-                    const int n = ((lt >> 5) << 2) + (i & 3) + (i >> 2) * RPP;
+                    const int n = (wi << 2) + (i & 3) + (i >> 2) * (FEW ? rpp : RPP);
                     if (n >= n16) break;
-                    srow[n] = input_row_of(a, u, n);
+                    srow[FEW ? mine + i : n] = input_row_of(a, u, n);
                 }
                 __syncwarp();
                 constexpr int FLIGHT = 5;      // F32: 16-byte results in flight a thread (5 x 28 rows: a tile)
@@ -576,16 +587,17 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
                     const int k = kt * GM_BK + 8 * uu;
 #pragma unroll
                     for (int i = 0; i < FLIGHT; ++i) {
-                        const int n = n0 + i * RPP;
+                        const int n = n0 + i * (FEW ? rpp : RPP);
                         x[2 * i] = x[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                         if (n < n16 && k < a.K) {
-                            const float4* xp = (const float4*) ((const float*) a.X + ((size_t) srow[n] * a.xs + k));
+                            const float4* xp = (const float4*) ((const float*) a.X + ((size_t) srow[FEW ? mine + 4 * i + (lane >> 3) : n] * a.xs + k));
                             x[2 * i] = __ldg(xp);
                             x[2 * i + 1] = __ldg(xp + 1);
                         }
                     }
                 };
-                if (F32) request(0, n_lo);
+                if (F32 && grp < KT) request(grp, n_first);
+                int turn = 0;      // the group whose step this is
                 for (int kt = 0; kt < KT && ok; ++kt) {
                     const int kr = kr0 + kt, s = kr % GM_STAGES;
                     if (kr >= GM_STAGES && !mbar_wait(bar_empty + 8 * s, ((kr / GM_STAGES) - 1) & 1, &abort_flag)) fail(4);
@@ -605,6 +617,21 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
                             settle();
                         }
                         pending = s;
+                    } else if (FEW) {
+                        pending = s;
+                        if (turn == grp) {
+#pragma unroll
+                            for (int i = 0; i < FLIGHT; ++i) {
+                                const int n = n_first + i * rpp;
+                                if (n < n16)
+                                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(input_at(stage, n, uu)), "r"(bf16x2_bits(x[2 * i].x, x[2 * i].y)),
+                                                 "r"(bf16x2_bits(x[2 * i].z, x[2 * i].w)), "r"(bf16x2_bits(x[2 * i + 1].x, x[2 * i + 1].y)),
+                                                 "r"(bf16x2_bits(x[2 * i + 1].z, x[2 * i + 1].w)) : "memory");
+                            }
+                            if (kt + groups < KT) request(kt + groups, n_first);
+                        }
+                        settle();
+                        if (++turn == groups) turn = 0;
                     } else {
                         for (int n0 = n_lo;;) {
 #pragma unroll
@@ -727,7 +754,7 @@ static void launch_gemm_seed(cudaStream_t s, const MmParams& a, int row_tiles, i
         else if (vec) launch_gemm_v<1, WF, 1, 1, false, IN_F32>(s, a, units);
         else launch_gemm_v<1, WF, 1, 0, false, IN_F32>(s, a, units);
     } else if (a.grouped) {
-        if (!a.packed) launch_gemm_v<1, WF, 1, 2, false, IN_F32>(s, a, units);
+        if (!a.packed) launch_gemm_v<1, WF, 1, 2, false, IN_F32_FEW>(s, a, units);
         else if (a.in_sorted && a.offs) { if (!launch_gemm_v<1, WF, 3, 2, false, IN_TMA>(s, a, units)) no_map(a); }
         else launch_gemm_v<1, WF, 1, 2, false, IN_LIST>(s, a, units);
     } else {

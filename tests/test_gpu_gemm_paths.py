@@ -252,3 +252,48 @@ def test_packed_rows_at_any_distance(xs, T):
     kernels._done()
     ref = B.bfr((x @ W.T).astype(np.float32)).astype(np.float64)
     assert (np.abs(y.cpu().numpy() - ref) <= np.abs(ref) / 128 + F32B * (np.abs(x) @ np.abs(W.T)) + 1e-30).all()
+
+
+def decoded_stack(stack, E):
+    """A device stack's weights, exact and rounded to bf16 once: [E][R][K]."""
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L
+    w = L.WSlice()
+    w.p[0], w.p[1], w.p[3], w.eb = stack.seeds.data_ptr(), stack.coefs.data_ptr(), stack.codes.data_ptr(), stack.eb[0]
+    o = torch.empty((E, stack.R, stack.K), dtype=torch.bfloat16, device="cuda")
+    L.load().nsl_decode_bf16(kernels._stream(), w, stack.K, E * stack.R, kernels._ptr(o), kernels._ptr(kernels.stream_table()))
+    return o
+
+
+def within(y, x, W):
+    ref, mag = x.double() @ W.double().T, x.double().abs() @ W.double().abs().T
+    return ((y.double() - ref).abs() <= ref.abs() / 128 + F32B * mag + 1e-30).all()
+
+
+@pytest.mark.parametrize("K", [64, 128, 192, 256, 320, 448])
+@pytest.mark.parametrize("packed", [False, True])
+def test_grouped_tiles_of_every_size_many_units_a_block(K, packed):
+    """Tiles of 1 .. 128 rows, either side of where the loaders' warps share out the K steps (40, 60) and of half of the accumulators, in no
+    order, three to seven units a block; every element."""
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L, moe
+    counts = [1, 64, 128, 16, 17, 65, 40, 41, 48, 100, 49, 60, 61, 127, 32, 33, 8, 96, 80, 63, 112, 62, 24, 57, 56, 9]
+    E, R, P = len(counts), 5210, sum(counts)
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    st = moe.ExpertStack.random_on_device(E, R, K, gen)
+    W = decoded_stack(st, E)
+    sel = torch.repeat_interleave(torch.arange(E, device="cuda"), torch.tensor(counts, device="cuda"))
+    perm = torch.randperm(P, generator=gen, device="cuda").int()      # pair perm[i] belongs to the i-th place's expert
+    tiles = torch.zeros((E, 4), dtype=torch.int32)
+    tiles[:, 0], tiles[:, 2] = torch.arange(E), torch.tensor(counts)
+    tiles[1:, 1] = torch.tensor(counts).cumsum(0)[:-1]
+    x = torch.randn((P, K), generator=gen, device="cuda").to(torch.bfloat16)
+    xin, y, nt = (x if packed else x.float()), torch.full((P, R), float("nan"), device="cuda"), torch.tensor([E], dtype=torch.int32, device="cuda")
+    tiles = tiles.cuda()
+    f = L.load().kc_mm_grouped_packed if packed else L.load().kc_mm_grouped_dev
+    f(kernels._stream(), L.MF_SEED4P4, kernels._ptr(st.table), K, R, kernels._ptr(xin), K, kernels._ptr(y), R, 1, kernels._ptr(perm), kernels._ptr(tiles),
+      kernels._ptr(nt), E + 2, kernels._ptr(kernels.stream_table()))
+    kernels._done()
+    for e in range(E):
+        rows = perm[sel == e].long()
+        assert within(y[rows], x[rows].float(), W[e].float()), counts[e]
