@@ -297,3 +297,41 @@ def test_grouped_tiles_of_every_size_many_units_a_block(K, packed):
     for e in range(E):
         rows = perm[sel == e].long()
         assert within(y[rows], x[rows].float(), W[e].float()), counts[e]
+
+
+@pytest.mark.parametrize("R,K,T", [(75800, 64, 70), (75800, 192, 128), (75800, 256, 130), (115200, 320, 100), (40000, 448, 300), (40000, 128, 500)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_dense_calls_of_many_units_a_block(R, K, T, packed):
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L, moe
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    st = moe.ExpertStack.random_on_device(1, R, K, gen)
+    W = decoded_stack(st, 1)[0].float()
+    w = L.WSlice()
+    w.p[0], w.p[1], w.p[3], w.eb = st.seeds.data_ptr(), st.coefs.data_ptr(), st.codes.data_ptr(), st.eb[0]
+    x = torch.randn((T, K), generator=gen, device="cuda").to(torch.bfloat16)
+    xin, y = (x if packed else x.float()), torch.full((T, R), float("nan"), device="cuda")
+    (L.load().kc_mm_packed if packed else L.load().kc_mm)(kernels._stream(), L.MF_SEED4P4, w, K, R, kernels._ptr(xin), K, kernels._ptr(y), R, T, 0,
+                                                          kernels._ptr(kernels.stream_table()))
+    kernels._done()
+    assert within(y, x.float(), W)
+
+
+@pytest.mark.parametrize("p", [4, 3])
+@pytest.mark.parametrize("R,K", [(300, 256), (2048, 512), (130, 1088), (70, 96)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_a_dense_row_has_the_same_bits_up_to_64_rows_and_from_65_on(p, R, K, packed):
+    """Two kernels with their own orders of the sums; within each (and, where K is not a multiple of 64, over both ranges: one kernel) a row's
+    bits do not depend on the number of rows."""
+    from nanoseedlm_b200 import kernels
+    m = B.Matrix(R, K, R + K, eb=-21) if p == 4 else B.Matrix3(R, K, R + K, eb=-21)
+    w = kernels.SeedWeight.from_matrices([m]) if p == 4 else kernels.SeedWeight3([m])
+    x = B.bfr(np.random.default_rng(K).standard_normal((700, K)).astype(np.float32))
+    mm = lambda T: kernels.kt_mm(w, x[:T], T, packed=packed)
+    few, many = mm(64), mm(700)
+    for T in (1, 8, 9, 16, 17, 32, 33, 63):
+        assert np.array_equal(mm(T), few[:T]), T
+    for T in (65, 128, 129, 256, 257, 384, 385, 500):
+        assert np.array_equal(mm(T), many[:T]), T
+    if K % 64:
+        assert np.array_equal(few, many[:64])
