@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
     constexpr int ROW = Q4Ring<4>::ROW, STAGE = Q4Ring<4>::STAGE;
     constexpr int G = 4 * WARPS, KB = 128 * WARPS;      // groups and bytes of codes per row (K = 256 x WARPS)
     extern __shared__ __align__(16) uint32_t q4_smem[];
-    constexpr int TPI = 2 / NT;      // tiles of 16 rows an iteration: 256 outputs
+    constexpr int TPI = NT == 1 && WARPS == 16 ? 2 : 1;      // tiles of 16 rows an iteration
     float* part = (float*) q4_smem;                                              // [2 buffers][TPI][NT][WARPS][32][4]
     const int tok0 = blockIdx.y * 8 * NT;
     x += (size_t) tok0 * xs;
@@ -435,7 +435,8 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
 #pragma unroll
     for (int i = 0; i < NST - 1; ++i) issue();
 
-    // 256 outputs an iteration: one barrier and one reduction (a thread each) for all of them.
+    // A barrier and a reduction an iteration.  Two tiles in it pay where 16 warps meet (K = 4096, 151936 rows, 8 tokens: 86.8 -> 79.3 us); where two or
+    // four blocks share an SM and hide one another's barriers they do not (K = 2048: 44.3 with one tile, 45.7 with two).
     int stage = 0, pbuf = 0;
     for (int idx = 0; idx < my_tiles; idx += TPI, pbuf ^= 1) {
         float* pb = part + (size_t) pbuf * 2 * WARPS * 128;
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
                 *(float4*) (pb + (h * NT + tt) * WARPS * 128 + (warp * 32 + lane) * 4) = make_float4(out[tt][0], out[tt][1], out[tt][2], out[tt][3]);
         }
         __syncthreads();      // the block's partial sums of these tiles are in; the other buffer is free for the next ones
-        for (int e = threadIdx.x; e < 256; e += 32 * WARPS) {      // each output is the warps' sum in warp order
+        for (int e = threadIdx.x; e < 128 * TPI * NT; e += 32 * WARPS) {      // each output is the warps' sum in warp order
             const int h = e >> 7, o = e & 127, tile = idx + h / NT;      // (h: tile of rows, tile of tokens)
             if (tile >= my_tiles) break;
             const float* ps = pb + h * WARPS * 128 + o;
@@ -549,10 +550,10 @@ static void launch_q4_ring(cudaStream_t s, size_t total, int blocks, const WSlic
 // A few long rows: each is shared by a cluster of ARG_CTAS blocks, whose candidates meet in the first one's shared memory (a block a
 // row leaves the chip idle).  Many rows fill it by themselves, and for short ones a cluster's barriers cost more than they share: a
 // block a row.  us, logits in L2, shared / a block a row: 151936 logits, 8 rows 3.9 / 6.7, 48 rows 6.2 / 6.7, 64 rows 7.3 / 6.8,
-// 256 rows 31 / 28; 32000: 8 rows 2.8 / 3.8, 32 rows 3.1 / 3.8, 48 rows 3.9 / 3.8; 16000: 8 rows 2.7 / 2.9; 8192: 8 rows 2.6 / 2.2;
-// 1000: 256 rows 9.7 / 2.6.
+// 256 rows 31 / 28; 32000: 8 rows 2.8 / 3.8, 32 rows 3.1 / 3.8, 48 rows 3.9 / 3.8; 16000: 8 rows 2.7 / 2.9, 16 rows 3.0 / 2.9; 8192: 8 rows
+// 2.6 / 2.2; 1000: 256 rows 9.7 / 2.6.
 constexpr int ARG_CTAS = 8, ARG_T = 512;
-static bool argmax_shared(int V, int n) { return V >= 24000 && n <= 32; }
+static bool argmax_shared(int V, int n) { return n <= (V >= 24000 ? 32 : V >= 12000 ? 8 : 0); }
 
 __device__ __forceinline__ void arg_better(float& v, int& i, float v2, int i2) {
     if (v2 > v || (v2 == v && i2 < i)) { v = v2; i = i2; }

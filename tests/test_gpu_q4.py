@@ -64,9 +64,9 @@ def test_argmax_ties_to_the_lowest_id_and_probability(V, n):
     assert np.array_equal(kernels.kt_argmax(logits), ro)
 
 
-@pytest.mark.parametrize("V,n", [(1, 1), (2, 700), (5, 300), (33, 2000), (4097, 61), (23999, 32), (24000, 32), (24000, 33), (24003, 1)])
+@pytest.mark.parametrize("V,n", [(1, 1), (2, 700), (5, 300), (33, 2000), (4097, 61), (11999, 8), (12000, 8), (12003, 9), (23999, 32), (24000, 32), (24000, 33), (24003, 1)])
 def test_argmax_of_many_short_rows(V, n):
-    """From one value a row to either side of the lines (24000 values, 32 rows) where a cluster of blocks shares a row, on and off a
+    """From one value a row to either side of the lines (12000 and 24000 values, 8 and 32 rows) where a cluster of blocks shares a row, on and off a
     16-byte boundary."""
     from nanoseedlm_b200 import kernels
     logits = (np.random.default_rng(V + n).standard_normal((n, V)) * 3).astype(np.float32)
