@@ -375,15 +375,18 @@ struct PairDesc {      // what an item needs of its pair
 };
 
 // ONE: rows of one chunk (lpr_log2 = 0), a form of its own: the branch in the loop of the others cost config 1 at 8 rows 5 %.
-template <int MODE, int PF, bool ONE>
+// SINGLE: an item of the one matrix is one row step, not two: small calls, whose warps would not all have an item.  (Two steps one after the
+// other beside idle warps: 3 pairs of 1024 / 256 13.8 us a layer, 12.7 with one.)
+template <int MODE, int PF, bool ONE, bool SINGLE>
 __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KConst kc, int lpr_log2, int win, RouteFuse rf) {
+    constexpr bool TWO = MODE != MODE_GU && !SINGLE;
     extern __shared__ __align__(16) ulonglong2 pair_sx[];      // [win][lpr * CX]
     __shared__ StreamTab tab;
     __shared__ int32_t r_ind[256];   // the fused router's picks
     __shared__ float r_wt[256];
     __shared__ PairDesc desc[PAIR_WIN];
     __shared__ int next_item;
-    constexpr int STEPS = RowItem<MODE>::STEPS;
+    constexpr int STEPS = TWO ? 2 : 1;
     load_stream_tab(tab, a.G, threadIdx.x, PAIR_THREADS);
     grid_dependents_go();
     grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KC
                 kb.s = __ldg((const uint4*) d.sb + at);
                 kb.c = __ldg((const uint4*) d.cb + at);
                 if (PF == 4) kb.cd = __ldg((const uint32_t*) d.db + at);
-            } else if (r + rpw < a.R) {
+            } else if (TWO && r + rpw < a.R) {
                 kb.s = __ldg((const uint4*) d.sa + at + 32);      // the next row step: 32 chunks on
                 kb.c = __ldg((const uint4*) d.ca + at + 32);
                 if (PF == 4) kb.cd = __ldg((const uint32_t*) d.da + at + 32);
@@ -464,8 +467,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KC
                 const float su = __shfl_xor_sync(0xFFFFFFFFu, keep, h);
                 if (!upper && kept >= 0 && r < a.R) store_out<MODE>(a, d.pair, r, keep * d.sca, su * d.scb);
             } else {
-                r += upper ? rpw : 0;
-                if (kept >= 0 && r < a.R) store_out<MODE>(a, d.pair, r, keep * d.sca, 0.0f);
+                r += TWO && upper ? rpw : 0;
+                if (kept >= 0 && (TWO || !upper) && r < a.R) store_out<MODE>(a, d.pair, r, keep * d.sca, 0.0f);
             }
             kept = -1;
             cnt = 0;
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KC
             u64 acc[2] = {0ull, 0ull};
             if (r < a.R) {
                 const ulonglong2* cx = cx0 + t * (lpr * CX);
-                if (MODE == MODE_GU || (it - t * ips + 1) * STEPS <= rs) chunk_dots<MODE_GU, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);
+                if (MODE == MODE_GU || (TWO && (it - t * ips + 1) * STEPS <= rs)) chunk_dots<MODE_GU, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);
                 else chunk_dots<MODE_ROUND, PF>(tab, kc, ka, kb, cx, acc[0], acc[1]);      // (a pair's last, single step)
             }
             const float v[2] = {pair_total(acc[0]), pair_total(acc[1])};
@@ -1423,17 +1426,21 @@ static RowShape item_shape(int ch) {
 template <int MODE, int PF>
 static void launch_pair(cudaStream_t s, const MvParams& a, const RouteFuse& rf) {
     const int ch = a.K / 64, sms = sm_count();
-    static bool attr_set[16], attr_set_items[16];
+    static bool attr_set[16], attr_set_one[16], attr_set_single[16], attr_set_items[16];
     if (ch <= 32 && (ch & (ch - 1)) == 0) {
         const int lpr_log2 = log2_floor(ch);
         int win = a.P / sms + 2;      // a share's pairs, whole or in part
         if (win > PAIR_WIN) win = PAIR_WIN;
         if (win > a.P) win = a.P;
-        if (ch == 1) launch(mv_pair_kernel<MODE, PF, true>, sms, PAIR_THREADS, win * staged_bytes(ch), s, a, kconst(), lpr_log2, win, rf);
-        else {
-            allow_smem(mv_pair_kernel<MODE, PF, false>, attr_set, (size_t) PAIR_WIN * 32 * CX * 16);
-            launch(mv_pair_kernel<MODE, PF, false>, sms, PAIR_THREADS, win * staged_bytes(ch), s, a, kconst(), lpr_log2, win, rf);
-        }
+        const size_t smem = win * staged_bytes(ch);
+        auto go = [&](auto kernel, bool* done) {
+            allow_smem(kernel, done, (size_t) PAIR_WIN * 32 * CX * 16);
+            launch(kernel, sms, PAIR_THREADS, smem, s, a, kconst(), lpr_log2, win, rf);
+        };
+        const bool single = MODE != MODE_GU && (long long) a.P * ((a.R * ch + 31) / 32) <= (long long) PAIR_WARPS * sms;      // a warp each for all row steps
+        if (ch == 1) go(mv_pair_kernel<MODE, PF, true, false>, attr_set_one);
+        else if (single) go(mv_pair_kernel<MODE, PF, false, MODE != MODE_GU>, attr_set_single);
+        else go(mv_pair_kernel<MODE, PF, false, false>, attr_set);
     } else {
         const RowShape sh = item_shape(ch);
         const size_t room = (size_t) max_smem_optin() - 6144, one = staged_bytes(ch);      // 6144: the kernel's other shared memory (launch_mv has made sure that one row and the fewest sums fit)

@@ -133,3 +133,20 @@ def test_dense_rows_of_small_matrices(p, K, R):
         d = mv(w, x[:T], T, add=1, y0=y0[:T])
         for t in range(T):
             assert np.array_equal(d[t], alone[t]), (T, t)
+
+
+@pytest.mark.parametrize("p", [4, 3])
+@pytest.mark.parametrize("K,R", [(128, 592), (128, 577), (128, 15)])
+def test_gathers_either_side_of_one_row_step_an_item(p, K, R):
+    """64 and 65 pairs of 37 row steps are one item a warp of 148 multiprocessors, and one more pair: items of one row step and of two (the last
+    one single), with the same bits."""
+    from nanoseedlm_b200 import kernels
+    W, w = matrices(p, 3, R, K, K + R)
+    x = B.bfr(np.random.default_rng(R).standard_normal((66, K)).astype(np.float32))
+    sel = (np.arange(66) * 7 % 3).astype(np.int32)
+    mv_sel = kernels.kt_mv_sel if p == 4 else kernels.kt_mv3_sel
+    y = {P: mv_sel(w, sel[:P], 1, x[:P]) for P in (1, 2, 63, 64, 65, 66)}
+    for P, v in y.items():
+        assert np.array_equal(v, y[66][:P]), P
+    for i in (0, 1, 37, 63, 64, 65):
+        check(y[66][i], W[sel[i]], x[i].astype(np.float64))
