@@ -91,13 +91,7 @@ __device__ __forceinline__ uint16_t bf16_bits(float x) {
     return (uint16_t) (u >> 16);
 }
 
-// (a & MASK) | c and (a & MASK) ^ c as single LOP3s: MASK a literal, c a register.
-template <uint32_t MASK>
-__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "n"(MASK), "r"(c));
-    return d;
-}
+// (a & MASK) ^ c as a single LOP3: MASK a literal, c a register.
 template <uint32_t MASK>
 __device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t c) {
     uint32_t d;
@@ -105,7 +99,7 @@ __device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t c) {
     return d;
 }
 
-// The same on two words at once, the results packed as a 64-bit pair {lo, hi}: written as one unit so the assembler
+// The same, and (a & MASK) | c, on two words at once, the results packed as a 64-bit pair {lo, hi}: written as one unit so the assembler
 // places each result directly in its half of the pair (packing two separately produced values costs a move each).
 template <uint32_t MASK>
 __device__ __forceinline__ unsigned long long and_or_pair(uint32_t a0, uint32_t a1, uint32_t c) {
