@@ -88,7 +88,9 @@ void kc_mv_gu(cudaStream_t s, int fmt, const WSlice* wg, const WSlice* wu, int K
 /* ---- prompt GEMM (tcgen05 tensor-core path) ------------------------------------------------------------------------- */
 /* engine/kernels_cuda.h:96  1: seed weights exact in f32 (three bf16 terms); 0 (default): rounded to bf16. */
 void kc_seed_gemm_f32(int on);
-/* engine/kernels_cuda.h:97 */
+/* engine/kernels_cuda.h:97  A row's bits do not depend on T among calls of up to 64 rows, nor among calls of 65 and more; between the two they may
+ * (f32 sums in another order before the rounding to bf16: two kernels, for seed weights with K a multiple of 64 and bf16-rounded
+ * weights).  The grouped forms give a row the same bits in every call. */
 void kc_mm(cudaStream_t s, int fmt, WSlice w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add,
            const uint32_t* G);
 /* engine/kernels_cuda.h:99 */
@@ -205,7 +207,7 @@ void nsl_bucket_noalloc(cudaStream_t s, const int32_t* inds, int count, int n, i
 /* The whole decode step of an expert layer -- router, gate + up + SwiGLU, down projection, weighted combine (the four
  * launches of engine/qwen4_cuda.c:1033-1078) -- as ONE launch whose blocks pass from phase to phase and wait on counters
  * for what other blocks produce (every wait bounded).  Results are bit for bit those of nsl_mv_gu_routed + kc_mv_sel +
- * kq4_moe_combine.  Measured slower than those three as dependent launches (config 1, 8 rows: 126.3 against 114.2 us a
+ * kq4_moe_combine.  Measured slower than those three as dependent launches (config 1, 8 rows: 119 against 98.8 us a
  * step): the dependent launches already hide ramp and prologue, and a block here waits for its neighbours at each phase
  * change.  Returns 1 = launched; 0 = a size is outside what it serves (T <= MV_MAXT rows, d and ff = 64 * 2^j <=
  * 2048, aligned rows) and nothing was launched.  sync: 4 * (2 + T + T * top_k) bytes of device memory, zero before the
@@ -248,7 +250,7 @@ void nsl_decode3_f32(cudaStream_t s, WSlice w, int K, int R, float* out, const u
 void nsl_decode3_bf16(cudaStream_t s, WSlice w, int K, int R, uint16_t* out, const uint32_t* G);
 /* kc_mv_gu with the router folded into its prologue (one launch less on the decode path): T <= MV_MAXT rows of logits
  * [T][ld] -> ind / wt [T][top_k] as kq4_route gives them, and a [T * top_k][R] as kc_mv_gu gives it for sel = ind,
- * xdiv = top_k.  K = 64 * 2^j <= 2048; raw: unrounded f32 outputs.  n_exp <= 1024, top_k <= 32. */
+ * xdiv = top_k.  K a multiple of 64; raw: unrounded f32 outputs.  n_exp <= 1024, top_k <= 32. */
 void nsl_mv_gu_routed(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K, int R, const float* x, int xs, float* a, int ys,
                       int n_exp, int top_k, const float* logits, int ld, int T, int32_t* ind, float* wt, int raw,
                       const uint32_t* G);

@@ -3,7 +3,8 @@
  * It issues, for T rows, what the reference engine's moe() issues between the router logits and the combined output
  * (engine/qwen4_cuda.c:1023-1083): top-k routing, the routed experts' gate + up + SwiGLU and down projections over
  * the T * top_k (row, expert) pairs -- the mat-vec path for T <= MV_MAXT rows (:1071-1074), the grouped prompt path
- * for more (:1058-1065) -- and the weighted combine (:1078).  The reference has no stand-alone entry point for this
+ * for more (:1058-1065) -- and the weighted combine (:1078).  On either path a row's bits do not depend on the rows it shares the
+ * call with; between the two they may (exact weights / weights rounded to bf16).  The reference has no stand-alone entry point for this
  * slice (it is a static function of its engine object, engine/qwen4_eng.h:38-62); these calls give it one, with the
  * reference's conventions: int results are 0 or -1 with a message in nsl_last_error(), work buffers are allocated at
  * creation only, the device form only enqueues launches on the caller's stream. */
@@ -36,7 +37,7 @@ void nsl_moe_set_dependent_launch(NslMoe* m, int on);
  * (no device-to-host copy is enqueued).  0: the result goes to device memory and a copy brings it to the host. */
 void nsl_moe_set_direct_output(NslMoe* m, int on);
 /* 1: a decode step whose sizes nsl_mv_step serves is one launch; 0 (default): the three dependent launches, which
- * measured faster (config 1: 114.2 against 126.3 us at 8 rows, 26.2 against 26.7 us at 1 row). */
+ * measured faster (config 1: 98.8 against 119 us at 8 rows, 23.7 against 24.8 us at 1 row). */
 void nsl_moe_set_one_launch(NslMoe* m, int on);
 /* 0, or 1 when a bounded wait inside a one-launch step ran out since the last call (that step's output is not valid).
  * Reads device memory: call it after the layer's work has been waited for. */

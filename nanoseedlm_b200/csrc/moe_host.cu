@@ -1,8 +1,8 @@
 // Host side of one MoE expert layer above the kernel ABI: the sequence the reference engine's moe() issues
 // (engine/qwen4_cuda.c:1023-1083) -- router top-k, routed experts' gate+up+SwiGLU and down projections over the
 // (token, expert) pairs, weighted combine -- for a layer whose experts are resident in device memory.  Rows <= MV_MAXT
-// take the mat-vec path (kc_mv_gu + kc_mv_sel), more rows the grouped prompt path (kc_bucket + kc_mm_grouped_dev x 3 +
-// kc_swiglu), as the reference decides at engine/qwen4_cuda.c:1058-1075.  Work buffers are allocated once at creation;
+// take the mat-vec path (kc_mv_gu + kc_mv_sel), more rows the grouped prompt path (grouping and packing, gate + up + SwiGLU in
+// one GEMM, the down projection's, the combine), as the reference decides at engine/qwen4_cuda.c:1058-1075.  Work buffers are allocated once at creation;
 // a forward allocates nothing and, in its device form, only enqueues launches (graph-capturable).
 #include <cstdlib>
 #include <cstring>
@@ -173,7 +173,7 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
     nsl::PdlScope pdl(m->pdl);
     const bool fits = T <= MV_MAXT && d % 64 == 0 && d <= 32768 && nsl::aligned16(x), fused = fits && !nsl::mv_groups(d, P, m->n_exp);
     // on request, one launch for the whole step where the fused kernel serves the sizes (measured slower than the three
-    // dependent launches: 126.3 against 114.2 us at 8 rows, 70.1 / 65.5 at 4, 26.7 / 26.2 at 1)
+    // dependent launches: 119 against 98.8 us at 8 rows, 65 / 56.9 at 4, 24.8 / 23.7 at 1)
     if (fits && m->one_launch &&
         nsl_mv_step(s, m->wg, m->wu, m->wd, d, ff, x, d, m->n_exp, k, logits, m->n_exp, T, m->ind, m->wt, m->A, m->Dx, out, m->raw, m->step_sync, m->G))
         return 0;

@@ -674,12 +674,10 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_items_kernel(MvParams a, K
 // status 1, every other wait ends on seeing it, and the launch returns with its counters cleared (the last block to
 // finish clears them for the next launch; fin counts finished blocks and wraps to zero by itself).
 // Arithmetic and rounding points are those of the three kernels it replaces, operation for operation.
-// Measured (config 1, CUDA graph replay, us per step at 8 / 4 / 1 rows): 126.3 / 70.1 / 26.7 against 114.2 / 65.5 / 26.2
-// for the three dependent launches, so the host layer does not use it by default.  Under ncu the one launch lasts what
-// the three last back to back (130.5 against 129.2 us; the same 75.0 M instructions and 217 k active cycles an SM); what
-// the dependent launches hide between steps -- the next kernel's blocks resident with table, router and first streams
-// ready when the wait ends -- this form cannot, and its barrier stalls are 0.78 per issued instruction against 0.10:
-// at each phase change a block waits for the slowest of the ~6 blocks that share its pairs.
+// Measured (config 1, us per step at 8 / 4 / 1 rows): 119 / 65 / 24.8 against 98.8 / 56.9 / 23.7 for the three dependent launches, so the
+// host layer does not use it by default.  It keeps the blocks of 8 warps with row steps dealt in advance that the pair kernel had (the
+// same 75.0 M instructions then; 126 against 114 us), and at each phase change a block waits for the slowest of the ~6 blocks that share
+// its pairs (barrier stalls 0.78 per issued instruction against 0.10).
 struct StepSync {
     unsigned* ready;      // [T * top_k]
     unsigned* done;       // [T]
@@ -822,7 +820,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_step_kernel(StepParams p, KC
 
 
 // ---- pairs grouped by expert: one expansion per distinct slice ---------------------------------------------------------
-// Rows of 1, 2, 4, .. 32 chunks (K = 64 .. 2048).  Every block builds the same plan in its prologue: the pair list is
+// Rows of 4, 8, 16 or 32 chunks (K = 256 .. 2048: grp_serves).  Every block builds the same plan in its prologue: the pair list is
 // sorted by slice in shared memory, runs of pairs that use the same slice are cut into UNITS of at most GRP_NT pairs, and
 // a unit's rows are expanded once for all its pairs (the logic-pipe work is shared; each pair keeps its own sums, formed in
 // the same order as when it is alone, so a pair's result does not depend on its partners).  The work is the sequence of
