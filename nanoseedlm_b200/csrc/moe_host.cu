@@ -144,7 +144,9 @@ int nsl_moe_forward_dev(NslMoe* m, cudaStream_t s, const float* x, const float* 
             if (sorted) {
                 // many rows an expert: one expansion for up to 384 of them, whose inputs are fetched as boxes of consecutive rows, so
                 // the rows are packed in the order of the pairs by expert (4096 rows of config 1's layer: 549 -> 486 us; at 32
-                // rows an expert the copy costs what it saves)
+                // rows an expert the copy costs what it saves).  The line lies at 96 rows an expert on average: tile by tile / sorted, us, config 1's
+                // layer at 80 / 96 / 112 / 128 rows an expert 312 / 322 / 370 / 464 and 321 / 329 / 338 / 348; 32 experts of 1024 / 256
+                // 38.6 / 41.8 / 42.2 / 57.6 and 43.5 / 45.6 / 46.4 / 47.7; 60 of 1536 / 704 172 / 180 / 185 / 246 and 176 / 179 / 183 / 187
                 uint16_t* const xs = D + (size_t) P * d;
                 nsl::launch_pack_sorted(s, x, at, xs, T, k, d);
                 g.X = xs;

@@ -1466,7 +1466,9 @@ static void launch_pair(cudaStream_t s, const MvParams& a, const RouteFuse& rf) 
 // P pairs of E slices meet P^2 / 2E times, and the line lies at 40 of them: config 1's layer with 64 pairs of 16 / 32 / 64 / 128
 // slices 90.4 / 93.8 / 100.0 / 105.5 us grouped, 98.9 / 99.2 / 99.3 / 99.6 pair by pair; two decoder layers with 96 pairs of 64 /
 // 128 / 512 397 / 408 / 429 and 416 / 416 / 422, with 160 of 512 605 and 589, with 200 719 and 714; 320 of 512 are faster
-// grouped.  Where the number of slices is not known: more than GRP_MIN_PAIRS pairs.
+// grouped.  Fewer than 48 pairs stay pair by pair, where the two are within 5 % (config 1's widths, grouped / pair by pair, us: 28 and 32
+// pairs of 4 slices 51.4 / 49.9 and 53.2 / 56.0, 28 of 8 52.1 / 49.9, 40 of 8 63.9 / 66.6, 42 of 16 69.0 / 70.0; 48 of 8 and of 16 71.2 /
+// 76.4 and 73.2 / 76.4).  Where the number of slices is not known: more than GRP_MIN_PAIRS pairs.
 constexpr int GRP_MIN_PAIRS = 64;
 static bool pairs_meet(int P, int slices) { return slices > 0 ? P >= 48 && (long long) P * P >= 80ll * slices : P > GRP_MIN_PAIRS; }
 static bool grp_serves(int K) { return K % 64 == 0 && K >= 256 && K <= 2048 && (K & (K - 1)) == 0; }
