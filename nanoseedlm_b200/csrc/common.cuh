@@ -20,11 +20,20 @@ inline bool aligned16(const void* p) { return ((uintptr_t) p & 15u) == 0; }
 // which returns once the previous kernel has completed and its writes are visible.  Every kernel launched through
 // launch() calls grid_dependency_wait() before it reads or writes anything a neighbouring kernel touches; without the
 // scope the launch is an ordinary one and the wait returns at once.
-extern thread_local bool tl_pdl;
+enum { PDL_OWN = -1, PDL_OFF = 0, PDL_ON = 1 };      // the caller has not said (each entry point's own choice); ordinary launches; dependent ones
+extern thread_local int tl_pdl;
 struct PdlScope {
-    bool prev;
-    explicit PdlScope(bool on) : prev(tl_pdl) { tl_pdl = on; }
+    int prev;
+    explicit PdlScope(bool on) : prev(tl_pdl) { tl_pdl = on ? PDL_ON : PDL_OFF; }
     ~PdlScope() { tl_pdl = prev; }
+};
+// For entry points whose kernels follow another of this library's kernels as a rule and read nothing that it could have written before they wait: a
+// dependent launch unless the caller has asked for ordinary ones.  (After a kernel of the caller's own, which ends before its dependents start, and
+// after copies it is an ordinary launch.)
+struct FollowScope {
+    int prev;
+    FollowScope() : prev(tl_pdl) { if (prev == PDL_OWN) tl_pdl = PDL_ON; }
+    ~FollowScope() { tl_pdl = prev; }
 };
 
 template <typename... KArgs, typename... Args>
@@ -38,7 +47,7 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = tl_pdl ? 1 : 0;
+    cfg.numAttrs = tl_pdl == PDL_ON ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

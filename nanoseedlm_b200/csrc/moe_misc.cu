@@ -572,6 +572,7 @@ void nsl_route(cudaStream_t s, int n_exp, int top_k, const float* logits, int ld
         set_error("router: %d experts (at most %d), top %d (at most 32)", n_exp, 32 * ROUTE_PER_LANE, top_k);
         return;
     }
+    FollowScope follow;
     const dim3 grid((unsigned) (T + 3) / 4);
     if (n_exp <= 128) launch(route_kernel<4>, grid, 128, 0, s, n_exp, top_k, logits, ld, ind, wt, T);
     else if (n_exp <= 512) launch(route_kernel<16>, grid, 128, 0, s, n_exp, top_k, logits, ld, ind, wt, T);
@@ -589,6 +590,7 @@ void kq4_route(cudaStream_t s, const void* cfg, const float* logits, int32_t* in
 void kq4_moe_combine(cudaStream_t s, int d, int k, const float* D, const float* wt, const float* sh, const float* sg,
                      int sgld, float* out, int T) {
     if (T <= 0 || d <= 0) return;
+    FollowScope follow;
     launch(q4_combine_kernel, dim3((unsigned) (d + 255) / 256, (unsigned) T), 256, 0, s, d, k, D, wt, sh, sg, sgld, out);
     count_launch();
 }

@@ -759,6 +759,7 @@ extern "C" {
 
 void kc_argmax_p(cudaStream_t s, const float* logits, int32_t* out, float* prob, int V, int n) {
     if (V < 1 || n < 1) return;
+    FollowScope follow;      // the logits' product drains meanwhile
     if (argmax_shared(V, n)) launch(argmax_kernel, dim3(ARG_CTAS, (unsigned) n), ARG_T, 0, s, logits, out, prob, V);
     else launch(argmax_row_kernel, (unsigned) n, 1024, 0, s, logits, out, prob, V);
     count_launch();

@@ -1648,6 +1648,7 @@ void kc_mv(cudaStream_t s, int fmt, WSlice w, int K, int R, const float* x, int 
 void kc_mv_sel(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys,
                const int32_t* sel, int P, int xdiv, const uint32_t* G) {
     if (!seed_fmt(fmt, "kc_mv_sel")) return;
+    FollowScope follow;
     MvParams a = {ws, NULL, WSlice{}, sel, x, y, G, K, R, P, xdiv, xs, ys, 0, 0, NULL, NULL, 0};
     if (fmt == MF_SEED4) launch_mv<MODE_ROUND, 3>(s, a, 1);
     else launch_mv<MODE_ROUND, 4>(s, a, 1);
@@ -1656,6 +1657,7 @@ void kc_mv_sel(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const fl
 void kc_mv_gu(cudaStream_t s, int fmt, const WSlice* wg, const WSlice* wu, int K, int R, const float* x, int xs, float* out,
               int ys, const int32_t* sel, int P, int xdiv, const uint32_t* G) {
     if (!seed_fmt(fmt, "kc_mv_gu")) return;
+    FollowScope follow;
     MvParams a = {wg, wu, WSlice{}, sel, x, out, G, K, R, P, xdiv, xs, ys, 0, 0, NULL, NULL, 0};
     if (fmt == MF_SEED4) launch_mv<MODE_GU, 3>(s, a, 1);
     else launch_mv<MODE_GU, 4>(s, a, 1);
