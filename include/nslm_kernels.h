@@ -260,7 +260,9 @@ void nsl_mv_gu_routed(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K,
  * kc_rope_kv and nsl_residual_add.  While on, such a kernel may become resident before the previous kernel in its stream
  * has finished; it waits on the device for that kernel's completion before it reads or writes anything a neighbour
  * touches, so it is safe after any kernel; after a copy or another kind of node it is an ordinary launch.  Thread-local;
- * turn it off again (0) before launching anything else on the stream. */
+ * turn it off again (0) before launching anything else on the stream.  Off (the default), kq4_route*, nsl_route, kc_mv_sel,
+ * kc_mv_gu, kq4_moe_combine, kc_argmax*, the MF_Q4 form of kc_mv and kc_mm of seed weights are such launches all the same:
+ * before their wait they read nothing but the stream table G, which no kernel may write while calls that use it are queued. */
 void nsl_dependent_launch(int on);
 
 #ifdef __cplusplus

@@ -669,6 +669,7 @@ void kc_attn(cudaStream_t s, AttnArgs a, const float* q, KvView kv, const RowInf
         else if (group <= 8) launch_attn_split<1, ATT_SRC_BF16>(s, a, q, kv, ri, part, T);
         else launch_attn_split<2, ATT_SRC_BF16>(s, a, q, kv, ri, part, T);
     }
+    // (The first pass as a dependent launch too: its blocks wait beside the previous reduction's, 26.2 -> 28.5 us for 24 rows of 5000 keys.)
     PdlScope chain(true);      // the reduction's blocks come in while the first pass drains
     launch(attn_reduce_kernel, dim3((unsigned) a.n_head, (unsigned) T), ATT_HD, 0, s, a, (const float*) part, g, o, ri, T, n_blocks);
     count_launch(2);

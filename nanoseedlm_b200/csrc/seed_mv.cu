@@ -1631,6 +1631,7 @@ extern "C" {
 void kc_mv(cudaStream_t s, int fmt, WSlice w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add,
            const uint32_t* G) {
     if (fmt == MF_Q4) {      // the LM head's affine int4 (q4_head.cu)
+        FollowScope follow;
         if (T > MV_MAXT) set_error("kc_mv (Q4): %d tokens, at most %d", T, (int) MV_MAXT);
         else launch_q4_mv(s, w, K, R, x, xs, y, ys, T, add);
         return;

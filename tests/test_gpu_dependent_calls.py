@@ -1,0 +1,90 @@
+"""Calls that are dependent launches by themselves (router, gathers, combine, LM head and arg-max, prompt GEMM): queued one behind the other, with the
+buffers of the previous round still in flight and kernels of another library in between, they give the bits of calls that are waited for one by one."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def ptr(t):
+    return C.c_void_p(t.data_ptr() if t is not None else 0)
+
+
+@pytest.mark.parametrize("p", [4, 3])
+@pytest.mark.parametrize("T", [1, 8])
+def test_a_layer_by_its_own_calls(p, T):
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L
+    from oracle import binding as B
+    lib, G = L.load(), kernels.stream_table()
+    d, ff, E, k = 512, 256, 12, 4
+    if p == 4:
+        stack = lambda R, K, s: kernels.SeedWeight.from_matrices([B.Matrix(R, K, s + e, eb=-20) for e in range(E)])
+    else:
+        stack = lambda R, K, s: kernels.SeedWeight3([B.Matrix3(R, K, s + e, eb=-20) for e in range(E)])
+    gate, up, down = stack(ff, d, 1), stack(ff, d, 50), stack(d, ff, 99)
+    fmt = L.MF_SEED4P4 if p == 4 else L.MF_SEED4
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    xs = [torch.randn(T, d, generator=gen, device="cuda").to(torch.bfloat16).float() for _ in range(6)]
+    ls = [torch.randn(T, E, generator=gen, device="cuda") for _ in range(6)]
+    s = torch.cuda.Stream()
+    x, logits, out = torch.zeros(T, d, device="cuda"), torch.zeros(T, E, device="cuda"), torch.zeros(T, d, device="cuda")
+    ind, wt = torch.zeros(T, k, dtype=torch.int32, device="cuda"), torch.zeros(T, k, device="cuda")
+    A, D = torch.zeros(T * k, ff, device="cuda"), torch.zeros(T * k, d, device="cuda")
+
+    def run(wait):
+        res = []
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s):
+            st = C.c_void_p(s.cuda_stream)
+            done = (lambda: s.synchronize()) if wait else (lambda: None)
+            for rep in range(4):
+                for xi, li in zip(xs, ls):
+                    x.mul_(0.0).add_(xi)               # another library's kernels before and after
+                    logits.copy_(li)
+                    done(); lib.nsl_route(st, E, k, ptr(logits), E, ptr(ind), ptr(wt), T)
+                    done(); lib.kc_mv_gu(st, fmt, ptr(gate.table), ptr(up.table), d, ff, ptr(x), d, ptr(A), ff, ptr(ind), T * k, k, ptr(G))
+                    done(); lib.kc_mv_sel(st, fmt, ptr(down.table), ff, d, ptr(A), ff, ptr(D), d, ptr(ind), T * k, 1, ptr(G))
+                    done(); lib.kq4_moe_combine(st, d, k, ptr(D), ptr(wt), None, None, 0, ptr(out), T)
+                    done(); res.append(out.clone())
+        torch.cuda.synchronize()
+        L.check()
+        return torch.stack(res)
+
+    assert torch.equal(run(False), run(True))
+
+
+def test_prompt_product_head_and_tokens():
+    import torch
+    from nanoseedlm_b200 import kernels, lib as L, moe
+    lib, G = L.load(), kernels.stream_table()
+    K, V, T = 512, 9000, 8
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    st = moe.ExpertStack.random_on_device(1, K, K, gen)
+    w = L.WSlice()
+    w.p[0], w.p[1], w.p[3], w.eb = st.seeds.data_ptr(), st.coefs.data_ptr(), st.codes.data_ptr(), -22
+    codes = torch.randint(-2 ** 31, 2 ** 31 - 1, (V, K // 8), generator=gen, device="cuda", dtype=torch.int32)
+    sc = (torch.rand((V, K // 64), generator=gen, device="cuda") * 0.02 + 0.001).to(torch.bfloat16)
+    bi = (torch.rand((V, K // 64), generator=gen, device="cuda") * -0.2).to(torch.bfloat16)
+    q = L.WSlice()
+    q.p[0], q.p[1], q.p[2] = codes.data_ptr(), sc.data_ptr(), bi.data_ptr()
+    xs = [torch.randn(n, K, generator=gen, device="cuda").to(torch.bfloat16).float() for n in (100, 9, 300, 40)]
+    y, lg, tok = torch.zeros(300, K, device="cuda"), torch.zeros(T, V, device="cuda"), torch.zeros(T, dtype=torch.int32, device="cuda")
+
+    def run(wait):
+        res = []
+        torch.cuda.synchronize()
+        done = torch.cuda.synchronize if wait else (lambda: None)
+        for rep in range(5):
+            for x in xs:
+                done(); lib.kc_mm(None, L.MF_SEED4P4, w, K, K, ptr(x), K, ptr(y), K, x.shape[0], 0, ptr(G))
+                done(); lib.kc_mv(None, L.MF_Q4, q, K, V, ptr(y), K, ptr(lg), V, T, 0, None)
+                done(); lib.kc_argmax(None, ptr(lg), ptr(tok), V, T)
+                done(); res += [y[:x.shape[0]].clone().flatten(), lg.clone().flatten(), tok.float()]
+        torch.cuda.synchronize()
+        L.check()
+        return torch.cat(res)
+
+    assert torch.equal(run(False), run(True))
