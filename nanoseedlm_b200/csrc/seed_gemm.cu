@@ -15,6 +15,7 @@
 // issues tcgen05.mma (M 128, K 16, N = the tile's count rounded up to 16) and commits the stage back through an mbarrier.
 // Blocks are persistent: the stream table, the tensor memory and the barriers are set up once.
 //   TT = 1, packed inputs: 8 producer warps, two blocks an SM (256 of the 512 columns each).
+//   dense f32 inputs: 8 producer warps and 11 or 15 loaders, one block an SM (launch_dense_f32).
 //   otherwise: 16 producer warps, one block an SM.  TT = 3: up to three tiles of an expert share one expansion, which a prompt of
 //   thousands of rows needs (each tile expands its expert's weights again).
 // The accumulator is read back with tcgen05.ld by the producer warps (lane = weight row, column = row of inputs), rounded as the
@@ -46,21 +47,22 @@ constexpr unsigned long long GM_WAIT_NS = 1000000000ull;
 // How the inputs reach shared memory.  IN_LIST: packed rows picked by a list (cp.async by the loader warps); IN_F32: f32 rows,
 // converted by the loaders, whose loads of a whole K step are held in registers meanwhile (IN_F32_FEW: grouped, units of any number of
 // rows up to a tile); IN_TMA: packed rows that follow one
-// another (dense, or sorted by expert), by one thread.
-enum { IN_LIST = 0, IN_F32 = 1, IN_TMA = 2, IN_F32_FEW = 3 };
+// another (dense, or sorted by expert), by one thread.  IN_F32_DENSE: as IN_F32, with more loaders than producers.
+enum { IN_LIST = 0, IN_F32 = 1, IN_TMA = 2, IN_F32_FEW = 3, IN_F32_DENSE = 4 };
 // One block: PW producer warps, the MMA warp, LW loader warps.  Tensor memory: the accumulators (128 columns per tile of inputs),
 // then the stages' weights (32 columns per term: 64 k values as bf16 pairs).
 // LAUNCH_REGS: registers a thread at launch (what the launch bounds leave); PREGS, LREGS: of the producers' and of the other
 // warpgroups after the split, whose sum over the block is at most what the launch gave it.
 template <int TERMS, int TT, int IN>
 struct GmCfg {
-    static constexpr bool F32 = IN == IN_F32 || IN == IN_F32_FEW;
-    static constexpr int CTAS = TERMS == 1 && TT == 1 && !F32 ? 2 : 1, PW = TERMS == 3 || CTAS == 2 ? 8 : 16, LW = TERMS == 1 && F32 ? 7 : 3;
+    static constexpr bool DENSE = IN == IN_F32_DENSE, F32 = IN == IN_F32 || IN == IN_F32_FEW || DENSE;
+    static constexpr int CTAS = TERMS == 1 && TT == 1 && !F32 ? 2 : 1, PW = TERMS == 3 || CTAS == 2 || DENSE ? 8 : 16;
+    static constexpr int LW = DENSE ? (TT == 1 ? 11 : 15) : TERMS == 1 && F32 ? 7 : 3;
     static constexpr int WARPS = PW + 1 + LW, THREADS = WARPS * 32, GROUPS = PW / 4;
     static constexpr int ACC = GM_BN * TT, A_COLS = 32 * TERMS, COLS = ACC + GM_STAGES * A_COLS <= 256 ? 256 : 512;
     static constexpr int X_BYTES = TT * GM_BN * GM_BK * 2;      // a stage's inputs
     static constexpr bool SPLIT = TERMS == 1;
-    static constexpr int LAUNCH_REGS = CTAS == 1 && LW == 3 ? 96 : 80, LREGS = F32 ? 64 : 40, PREGS = F32 ? 88 : LAUNCH_REGS == 96 ? 104 : 96;
+    static constexpr int LAUNCH_REGS = CTAS == 1 && WARPS == 20 ? 96 : 80, LREGS = F32 ? 64 : 40, PREGS = DENSE ? 112 : F32 ? 88 : LAUNCH_REGS == 96 ? 104 : 96;
     static_assert(ACC + GM_STAGES * A_COLS <= COLS && CTAS * COLS <= 512, "tensor memory");
     static_assert(!SPLIT || PW * PREGS + (LW + 1) * LREGS <= WARPS * LAUNCH_REGS, "registers");
     static_assert(GM_STAGES >= GROUPS, "every warpgroup owns a stage");
@@ -576,7 +578,7 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
                     srow[FEW ? mine + i : n] = input_row_of(a, u, n);
                 }
                 __syncwarp();
-                constexpr int FLIGHT = 5;      // F32: 16-byte results in flight a thread (5 x 28 rows: a tile)
+                constexpr int FLIGHT = !Cfg::DENSE ? 5 : TT == 1 ? 3 : TT == 2 ? 5 : 4;      // F32: 16-byte results in flight a thread (5 x 28 rows, DENSE 3 x 44: a tile; 5 x 60: two)
                 float4 x[F32 ? 2 * FLIGHT : 1];
                 auto request = [&](int kt, int n0) {
                     const int k = kt * GM_BK + 8 * uu;
@@ -716,18 +718,30 @@ static bool launch_gemm_v(cudaStream_t s, const MmParams& a, int units) {
 }
 static void no_map(const MmParams& a) { set_error("seed GEMM: no tensor map for sorted inputs of row stride %d", a.xs); }
 // How many tiles of a dense call share an expansion: a unit takes the time of its expansion (twice that where two blocks share an
-// SM) or of its inputs' conversion (f32: nine tenths of it per tile), and the units go round the SMs.
+// SM) or of its inputs' conversion (f32; 31, 45 and 62 us a unit of one, two and three tiles at K = 2048), and the units go round the SMs.
 static int dense_tiles(const MmParams& a, int row_tiles) {
     int best = 1;
     double best_cost = 0.0;
     for (int tt = 1; tt <= 3; ++tt) {
         if (a.packed && tt == 2) continue;
         const int units = row_tiles * ((a.T + GM_BN * tt - 1) / (GM_BN * tt)), slots = sm_count() * (a.packed && tt == 1 ? 2 : 1);
-        const double unit = a.packed ? (tt == 1 && units > sm_count() ? 2.0 : 1.0) : tt == 1 ? 1.0 : 0.9 * tt;
+        const double unit = a.packed ? (tt == 1 && units > sm_count() ? 2.0 : 1.0) : 0.45 + 0.5 * tt;
         const double cost = (double) ((units + slots - 1) / slots) * unit;
         if (tt == 1 || cost < best_cost) { best = tt; best_cost = cost; }
     }
     return best;
+}
+// Dense f32 inputs.  Their loaders set the pace (load, convert, store and report a step, while the producers take most issue slots), and with
+// 16 producers and 7 loaders a step's rows also came in two or three passes, each a memory latency.  8 producers and 11 loaders take a tile
+// in one pass, 8 and 15 two tiles; both fit their registers, the 16 and 7 spill.  us, 16 + 7 / now: 2048 x 2048, 65 rows 34.8 / 34.4, 777 rows
+// 38.6 / 36.8, 2048 rows 58.8 / 50.7, 4096 rows 131.0 / 99.1; 8192 x 2048, 1024 rows 119 / 97; 8192 x 4096, 700 rows 154 / 131.  One tile and
+// several units a block: the results are read by the producers, which 16 do faster (151936 x 1024, 100 rows 158 / 166).
+template <int WF>
+static void launch_dense_f32(cudaStream_t s, const MmParams& a, int tt, int units) {
+    if (tt == 1 && units > sm_count()) launch_gemm_v<1, WF, 1, 2, false, IN_F32>(s, a, units);
+    else if (tt == 1) launch_gemm_v<1, WF, 1, 2, false, IN_F32_DENSE>(s, a, units);
+    else if (tt == 2) launch_gemm_v<1, WF, 2, 2, false, IN_F32_DENSE>(s, a, units);
+    else launch_gemm_v<1, WF, 3, 2, false, IN_F32_DENSE>(s, a, units);
 }
 // Whether a slice's seeds and coefficient words are aligned to n bytes and its codes to n / 4.
 template <int WF>
@@ -758,9 +772,7 @@ static void launch_gemm_seed(cudaStream_t s, const MmParams& a, int row_tiles, i
             if (!(tt == 1 ? launch_gemm_v<1, WF, 1, 2, false, IN_TMA>(s, a, u) : launch_gemm_v<1, WF, 3, 2, false, IN_TMA>(s, a, u)))
                 launch_gemm_v<1, WF, 1, 2, false, IN_LIST>(s, a, units);      // rows that overlap
         }
-        else if (tt == 1) launch_gemm_v<1, WF, 1, 2, false, IN_F32>(s, a, u);
-        else if (tt == 2) launch_gemm_v<1, WF, 2, 2, false, IN_F32>(s, a, u);
-        else launch_gemm_v<1, WF, 3, 2, false, IN_F32>(s, a, u);
+        else launch_dense_f32<WF>(s, a, tt, u);
     }
 }
 void launch_gemm_gu(cudaStream_t s, const MmParams& a, int tiles_y) {

@@ -335,3 +335,18 @@ def test_a_dense_row_has_the_same_bits_up_to_64_rows_and_from_65_on(p, R, K, pac
         assert np.array_equal(mm(T), many[:T]), T
     if K % 64:
         assert np.array_equal(few, many[:64])
+
+
+@pytest.mark.parametrize("p", [4, 3])
+@pytest.mark.parametrize("R,K,T", [(130, 64, 65), (130, 128, 129), (257, 192, 257), (300, 1024, 128), (-1, 128, 100), (0, 128, 100), (1, 128, 100),
+                                   (2048, 320, 1300), (2048, 64, 1409), (2050, 192, 2307), (1000, 128, 4100)])
+def test_dense_f32_rows_have_the_bits_of_the_packed_ones(p, R, K, T):
+    """Blocks of one unit with one, two or three tiles of rows, and (one tile) blocks of several: the same values meet in the same MMAs in
+    the same order as with packed inputs, whatever the loaders."""
+    import torch
+    from nanoseedlm_b200 import kernels
+    if R < 2: R += 128 * torch.cuda.get_device_properties(0).multi_processor_count      # just one unit an SM, and one more
+    m = B.Matrix(R, K, R + K, eb=-21) if p == 4 else B.Matrix3(R, K, R + K, eb=-21)
+    w = kernels.SeedWeight.from_matrices([m]) if p == 4 else kernels.SeedWeight3([m])
+    x = B.bfr(np.random.default_rng(T).standard_normal((T, K)).astype(np.float32))
+    assert np.array_equal(kernels.kt_mm(w, x, T, packed=False), kernels.kt_mm(w, x, T, packed=True))
