@@ -19,17 +19,17 @@ inline bool aligned16(const void* p) { return ((uintptr_t) p & 15u) == 0; }
 // kernel's blocks retire and run their prologue (the stream table, index arithmetic) until grid_dependency_wait(),
 // which returns once the previous kernel has completed and its writes are visible.  Every kernel launched through
 // launch() calls grid_dependency_wait() before it reads or writes anything a neighbouring kernel touches; without the
-// scope the launch is an ordinary one and the wait returns at once.
-enum { PDL_OWN = -1, PDL_OFF = 0, PDL_ON = 1 };      // the caller has not said (each entry point's own choice); ordinary launches; dependent ones
+// scope, and outside the entry points that open one themselves, the launch is an ordinary one and the wait returns at once.
+// The thread's state is one of: each entry point's own choice (until the caller says otherwise), ordinary launches, dependent ones.
+enum { PDL_OWN = -1, PDL_OFF = 0, PDL_ON = 1 };
 extern thread_local int tl_pdl;
 struct PdlScope {
     int prev;
     explicit PdlScope(bool on) : prev(tl_pdl) { tl_pdl = on ? PDL_ON : PDL_OFF; }
     ~PdlScope() { tl_pdl = prev; }
 };
-// For entry points whose kernels follow another of this library's kernels as a rule and read nothing that it could have written before they wait: a
-// dependent launch unless the caller has asked for ordinary ones.  (After a kernel of the caller's own, which ends before its dependents start, and
-// after copies it is an ordinary launch.)
+// For entry points whose kernels follow another of this library's kernels as a rule: a dependent launch unless the caller has asked for ordinary ones
+// (nsl_dependent_launch(0)).  After a copy, and after a kernel that does not let its dependents go early, nothing starts before the predecessor has ended.
 struct FollowScope {
     int prev;
     FollowScope() : prev(tl_pdl) { if (prev == PDL_OWN) tl_pdl = PDL_ON; }

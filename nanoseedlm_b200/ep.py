@@ -307,6 +307,7 @@ class CudaBackend:
             lib.nsl_ep_plan(s, base + lay["ind_off"], base + lay["wt_off"], ep.N, ep.t_loc, ep.k, lay["bytes"] // 4,
                             lay["rows"], ep.lo, ep.hi, *out)
         P = T * ep.k
+        before = lib.nsl_dependent_launch_state()
         lib.nsl_dependent_launch(1)   # the three kernels after the plan come in while their predecessor drains
         try:
             lib.nsl_mv_gu_rows(s, lyr.gate.table.data_ptr(), lyr.up.table.data_ptr(), lyr.d, lyr.ff, base, ep.d, 1,
@@ -319,7 +320,7 @@ class CudaBackend:
             else:
                 lib.nsl_ep_combine(s, self.D.data_ptr(), self.wsel.data_ptr(), self.tok_off.data_ptr(), T, ep.d, ep.partial.data_ptr())
         finally:
-            lib.nsl_dependent_launch(0)
+            lib.nsl_dependent_launch(before)
 
     def p2p_dispatch(self, ep):
         """The chunk route_and_pack left in send[0] -> every rank's window."""

@@ -116,6 +116,7 @@ PROTOTYPES = {
     "nsl_launch_count": (C.c_uint64, []),
     "nsl_sm_count": (_i, []),
     "nsl_dependent_launch": (None, [_i]),
+    "nsl_dependent_launch_state": (_i, []),
     "nsl_mv_gu_routed": (None, [_vp, _vp, _vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _vp, _i, _i, _vp, _vp, _i, _vp]),
     # include/nslm_moe.h
     "nsl_moe_create": (_vp, [_i, _i, _i, _i, _i, _vp, _vp, _vp, _vp]),

@@ -88,3 +88,71 @@ def test_prompt_product_head_and_tokens():
         return torch.cat(res)
 
     assert torch.equal(run(False), run(True))
+
+
+@pytest.fixture
+def switch():
+    """nsl_dependent_launch, set back afterwards."""
+    from nanoseedlm_b200 import lib as L
+    lib = L.load()
+    before = lib.nsl_dependent_launch_state()
+    yield lib.nsl_dependent_launch
+    lib.nsl_dependent_launch(before)
+
+
+def edges_of(calls):
+    """The calls captured into a graph of one stream: (programmatic edges, other edges)."""
+    import torch
+    rt = C.CDLL("libcudart.so.12")
+    s, graph = torch.cuda.Stream(), C.c_void_p()
+    torch.cuda.synchronize()
+    assert rt.cudaStreamBeginCapture(C.c_void_p(s.cuda_stream), 2) == 0
+    calls(C.c_void_p(s.cuda_stream))
+    assert rt.cudaStreamEndCapture(C.c_void_p(s.cuda_stream), C.byref(graph)) == 0
+    n = C.c_size_t(0)
+    assert rt.cudaGraphGetEdges_v2(graph, None, None, None, C.byref(n)) == 0
+    f, t, data = (C.c_void_p * n.value)(), (C.c_void_p * n.value)(), (C.c_uint8 * (8 * n.value))()      # an edge's data: from, to, type, 5 bytes reserved
+    assert rt.cudaGraphGetEdges_v2(graph, f, t, data, C.byref(n)) == 0
+    rt.cudaGraphDestroy(graph)
+    kinds = [data[8 * i + 2] for i in range(n.value)]
+    return sum(k == 1 for k in kinds), sum(k != 1 for k in kinds)
+
+
+class Layer:
+    """A SEED4P4 layer by its own calls on device buffers."""
+
+    def __init__(self, T, d=512, ff=256, E=12, k=4):
+        import torch
+        from nanoseedlm_b200 import kernels, lib as L, moe
+        gen = torch.Generator(device="cuda").manual_seed(7)
+        self.lib, self.G, self.d, self.ff, self.E, self.k, self.T = L.load(), kernels.stream_table(), d, ff, E, k, T
+        self.gate, self.up, self.down = (moe.ExpertStack.random_on_device(E, r, c, gen) for r, c in ((ff, d), (ff, d), (d, ff)))
+        self.x = torch.randn(T, d, generator=gen, device="cuda").to(torch.bfloat16).float()
+        self.logits = torch.randn(T, E, generator=gen, device="cuda")
+        self.ind, self.wt = torch.zeros(T, k, dtype=torch.int32, device="cuda"), torch.zeros(T, k, device="cuda")
+        self.A, self.D, self.out = torch.zeros(T * k, ff, device="cuda"), torch.zeros(T * k, d, device="cuda"), torch.zeros(T, d, device="cuda")
+
+    def calls(self, s, G=None):
+        from nanoseedlm_b200 import lib as L
+        G, f = ptr(self.G if G is None else G), L.MF_SEED4P4
+        self.lib.nsl_route(s, self.E, self.k, ptr(self.logits), self.E, ptr(self.ind), ptr(self.wt), self.T)
+        self.lib.kc_mv_gu(s, f, ptr(self.gate.table), ptr(self.up.table), self.d, self.ff, ptr(self.x), self.d, ptr(self.A), self.ff, ptr(self.ind), self.T * self.k,
+                          self.k, G)
+        self.lib.kc_mv_sel(s, f, ptr(self.down.table), self.ff, self.d, ptr(self.A), self.ff, ptr(self.D), self.d, ptr(self.ind), self.T * self.k, 1, G)
+        self.lib.kq4_moe_combine(s, self.d, self.k, ptr(self.D), ptr(self.wt), None, None, 0, ptr(self.out), self.T)
+
+
+def test_the_switch(switch):
+    """0: ordinary launches; positive: dependent ones; negative, and at the start: each entry point's own choice.  The bits are the same."""
+    import torch
+    layer, res = Layer(3), []
+    layer.calls(None)      # (functions are loaded before a capture)
+    assert edges_of(layer.calls) == (3, 0)
+    for on, edges in ((0, (0, 3)), (1, (3, 0)), (-1, (3, 0)), (0, (0, 3))):
+        switch(on)
+        assert layer.lib.nsl_dependent_launch_state() == on
+        assert edges_of(layer.calls) == edges
+        layer.out.zero_()
+        layer.calls(C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        res.append(layer.out.clone())
+    assert all(torch.equal(r, res[0]) for r in res) and bool(res[0].any())
