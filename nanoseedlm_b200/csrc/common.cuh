@@ -30,9 +30,12 @@ struct PdlScope {
 };
 // For entry points whose kernels follow another of this library's kernels as a rule: a dependent launch unless the caller has asked for ordinary ones
 // (nsl_dependent_launch(0)).  After a copy, and after a kernel that does not let its dependents go early, nothing starts before the predecessor has ended.
+// Such a kernel reads nothing at all before its wait, the stream table included (tab_and_wait): a caller that has asked for nothing may have made the
+// table in the kernel before, whose writes are visible after the wait and not sooner.
 struct FollowScope {
     int prev;
     FollowScope() : prev(tl_pdl) { if (prev == PDL_OWN) tl_pdl = PDL_ON; }
+    int own() const { return prev == PDL_OWN; }
     ~FollowScope() { tl_pdl = prev; }
 };
 

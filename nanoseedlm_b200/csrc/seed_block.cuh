@@ -25,6 +25,8 @@
 #include <stdint.h>
 #include <string.h>
 
+#include "common.cuh"
+
 namespace nsl {
 
 typedef unsigned long long u64;
@@ -35,12 +37,21 @@ struct StreamTab {
 };
 
 // G is linear over GF(2) (reference: tests/test_lfsr.c:87-93): G[s] = G[s & 0xFF] ^ G[s & 0xFF00], so 512 entries of
-// the caller's 65536-entry table are all a kernel needs.
-__device__ __forceinline__ void load_stream_tab(StreamTab& t, const uint32_t* __restrict__ G, int tid, int nthreads) {
+// the caller's 65536-entry table are all a kernel needs.  (Ordinary loads: the kernel before may have made the table.)
+__device__ __forceinline__ void load_stream_tab(StreamTab& t, const uint32_t* G, int tid, int nthreads) {
     for (int i = tid; i < 256; i += nthreads) {
-        t.lo[i] = __ldg(G + i);
-        t.hi[i] = __ldg(G + (i << 8));
+        const uint32_t lo = G[i], hi = G[i << 8];      // (both requested before either is stored)
+        t.lo[i] = lo;
+        t.hi[i] = hi;
     }
+}
+
+// The table, and the wait for the previous kernel in the stream.  late: the table only after the wait (common.cuh: FollowScope).
+__device__ __forceinline__ void tab_and_wait(StreamTab& t, const uint32_t* G, int late, int tid, int nthreads) {
+    if (late) grid_dependency_wait();
+    load_stream_tab(t, G, tid, nthreads);
+    grid_dependents_go();
+    grid_dependency_wait();
 }
 
 __device__ __forceinline__ uint32_t stream_bits(const StreamTab& t, uint32_t seed) {

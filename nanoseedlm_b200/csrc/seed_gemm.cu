@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
     uint16_t* const box = (uint16_t*) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023) + GM_STAGES * Cfg::X_BYTES / 2;      // 1 KB a producer warp
     const uint32_t smem_base = smem_u32((uint8_t*) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023));
     const uint32_t bar_full = smem_u32(&bars[0]), bar_empty = bar_full + 8 * GM_STAGES, bar_done = bar_empty + 8 * GM_STAGES, bar_read = bar_done + 8;
-    if (!BF16W) load_stream_tab(tab, a.G, tid, Cfg::THREADS);
+    if (!BF16W && !a.late) load_stream_tab(tab, a.G, tid, Cfg::THREADS);
     if (tid == 0) {
         abort_flag = 0;
         for (int s = 0; s < GM_STAGES; ++s) {
@@ -356,6 +356,7 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
     }
     grid_dependents_go();
     grid_dependency_wait();
+    if (!BF16W && a.late) load_stream_tab(tab, a.G, tid, Cfg::THREADS);
     if (TT > 1 && a.grouped && warp == 0) {      // the tiles that start a unit: every TT-th of a slice, in order
         const int nt = a.ntiles ? *a.ntiles : a.T;
         int n = 0;
@@ -822,7 +823,7 @@ void kc_mm(cudaStream_t s, int fmt, WSlice w, int K, int R, const float* x, int 
            const uint32_t* G) {
     if (fmt == MF_BF16 && launch_bf16_mm_skinny(s, w, K, R, x, xs, y, ys, T, add)) return;      // a decode batch (dense_bf16.cu)
     FollowScope follow;
-    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, K, R, T, xs, ys, 1, add, 0, 0, NULL, 0, NULL, 0, 0, 0};
+    MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, K, R, T, xs, ys, 1, add, 0, 0, NULL, 0, NULL, 0, 0, 0, follow.own()};
     launch_gemm(s, fmt, "kc_mm", a, (T + GM_BN - 1) / GM_BN);
 }
 void kc_mm_packed(cudaStream_t s, int fmt, WSlice w, int K, int R, const uint16_t* x, int xs, float* y, int ys, int T, int add,

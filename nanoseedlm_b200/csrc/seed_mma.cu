@@ -209,9 +209,7 @@ __global__ void __launch_bounds__(SMM_THREADS, 2) seed_mma_kernel(SmmParams sp, 
     __shared__ SmmShared sh;
     const MmParams& a = sp.m;
     const int tid = threadIdx.x;
-    load_stream_tab(sh.tab, a.G, tid, SMM_THREADS);
-    grid_dependents_go();
-    grid_dependency_wait();
+    tab_and_wait(sh.tab, a.G, a.late, tid, SMM_THREADS);
     const int start = (int) blockIdx.y * SMM_TILE, count = min(a.T - start, SMM_TILE), r0 = (int) blockIdx.x * sp.rw * 16;
     if (tid < SMM_TILE) {
         const int d = tid >= count ? -1 : start + tid;

@@ -18,6 +18,7 @@ struct MmParams {
     int out_bf16;
     const int32_t* offs;     // grouped: the slices' first pairs (kc_bucket's work), or NULL; given (with in_sorted): up to three tiles of a slice share an expansion
     int in_sorted, out_sorted, T_in;      // grouped, packed: row n of the inputs (of the outputs) belongs to pair perm[n]; T_in: rows of inputs
+    int late = 0;            // G may be read only after the wait for the previous kernel
 };
 
 bool seed_gemm_exact();      // kc_seed_gemm_f32's switch

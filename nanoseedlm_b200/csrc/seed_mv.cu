@@ -37,7 +37,7 @@ struct MvParams {
     const int32_t* xrow;    // optional: pair p reads input row xrow[p] (instead of p / xdiv)
     const int32_t* count;   // optional: the pair count is read on the device (<= P)
     int xbf16;              // inputs are packed bf16 rows (row stride xs in bf16 elements)
-    int slices = 0;       // slices that sel chooses from (0: not known)
+    int late = 0;         // G may be read only after the wait for the previous kernel
 };
 
 __device__ __forceinline__ float silu_bf(float g) {   // each op rounded to bf16 (engine/kernels_moe.cu:28-31)
@@ -387,9 +387,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_pair_kernel(MvParams a, KC
     __shared__ PairDesc desc[PAIR_WIN];
     __shared__ int next_item;
     constexpr int STEPS = TWO ? 2 : 1;
-    load_stream_tab(tab, a.G, threadIdx.x, PAIR_THREADS);
-    grid_dependents_go();
-    grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
+    tab_and_wait(tab, a.G, a.late, threadIdx.x, PAIR_THREADS);   // everything below may read what the previous kernel in the stream wrote
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2, h = lpr >> 1;
     const int jc = lane & (lpr - 1), ro = lane >> lpr_log2, slot = jc & (h - 1);
@@ -526,9 +524,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) mv_items_kernel(MvParams a, K
     __shared__ PairDesc desc[PAIR_WIN];
     __shared__ int next_item;
     constexpr int MATS = MODE == MODE_GU ? 2 : 1;
-    load_stream_tab(tab, a.G, threadIdx.x, PAIR_THREADS);
-    grid_dependents_go();
-    grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
+    tab_and_wait(tab, a.G, a.late, threadIdx.x, PAIR_THREADS);   // everything below may read what the previous kernel in the stream wrote
     const int lane = threadIdx.x & 31, ch = sh.ch, groups = sh.groups;
     const int lpr = 1 << sh.lpr_log2, rpw = 32 >> sh.lpr_log2;
     const int jc = lane & (lpr - 1), ro = lane >> sh.lpr_log2;
@@ -1048,9 +1044,7 @@ template <int MODE>
 __global__ void __launch_bounds__(GRP_THREADS, 1) mv_grp_kernel(MvParams a, KConst kc, int lpr_log2) {
     extern __shared__ __align__(16) unsigned char grp_smem[];
     GrpShared& sh = *reinterpret_cast<GrpShared*>(grp_smem);
-    load_stream_tab(sh.tab, a.G, threadIdx.x, GRP_THREADS);
-    grid_dependents_go();
-    grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
+    tab_and_wait(sh.tab, a.G, a.late, threadIdx.x, GRP_THREADS);   // everything below may read what the previous kernel in the stream wrote
     const int lpr = 1 << lpr_log2, rpw = 32 >> lpr_log2;
     int P = a.count ? min(*a.count, a.P) : a.P;
     if (P <= 0) return;
@@ -1289,9 +1283,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) mv_dense_kernel(MvParams a, KCo
 template <int MODE, int P>
 __global__ void __launch_bounds__(MV_THREADS) mv_generic_kernel(MvParams a, KConst kc, int T) {
     __shared__ StreamTab tab;
-    load_stream_tab(tab, a.G, threadIdx.x, MV_THREADS);
-    grid_dependents_go();
-    grid_dependency_wait();   // everything below may read what the previous kernel in the stream wrote
+    tab_and_wait(tab, a.G, a.late, threadIdx.x, MV_THREADS);   // everything below may read what the previous kernel in the stream wrote
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = a.K / 8, dense = a.sel == NULL;
@@ -1555,7 +1547,7 @@ static bool slice_aligned(const WSlice& w, int pf) {
 // the slice is on the host) the streams must be aligned for that, and one row of inputs must fit shared memory; anything else
 // goes to the any-shape kernel.
 template <int MODE, int PF>
-static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse& rf = RouteFuse{}) {
+static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse& rf = RouteFuse{}, int slices = 0) {      // slices that sel chooses from (0: not known)
     if (a.R <= 0 || a.P <= 0 || T <= 0) return;
     if (a.K <= 0 || a.K % 8) { set_error("seed mat-vec: K = %d is not a multiple of 8", a.K); return; }
     if (T > MV_MAXT) { set_error("seed mat-vec: %d tokens, at most %d", T, MV_MAXT); return; }
@@ -1576,7 +1568,7 @@ static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse&
         if (dense) { launch_dense<PF>(s, a, T); return; }
     }
     if constexpr (PF == 4) {
-        if (!rf.logits && mv_groups(a.K, a.P, a.slices)) { launch_grp<MODE>(s, a, log2_floor(ch)); return; }
+        if (!rf.logits && mv_groups(a.K, a.P, slices)) { launch_grp<MODE>(s, a, log2_floor(ch)); return; }
     }
     launch_pair<MODE, PF>(s, a, rf);
 }
@@ -1584,11 +1576,11 @@ static void launch_mv(cudaStream_t s, const MvParams& a, int T, const RouteFuse&
 // kc_mv_gu / nsl_mv_gu_raw and kc_mv_sel / nsl_mv_raw over a layer of n_exp SEED4P4 experts.
 void mv_gu_of(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K, int R, const float* x, int xs, float* out, int ys, const int32_t* sel, int P, int xdiv, int raw,
               int n_exp, const uint32_t* G) {
-    launch_mv<MODE_GU, 4>(s, MvParams{wg, wu, WSlice{}, sel, x, out, G, K, R, P, xdiv, xs, ys, 0, raw, NULL, NULL, 0, n_exp}, 1);
+    launch_mv<MODE_GU, 4>(s, MvParams{wg, wu, WSlice{}, sel, x, out, G, K, R, P, xdiv, xs, ys, 0, raw, NULL, NULL, 0}, 1, RouteFuse{}, n_exp);
 }
 void mv_sel_of(cudaStream_t s, const WSlice* ws, int K, int R, const float* x, int xs, float* y, int ys, const int32_t* sel, int P, int xdiv, int raw, int n_exp,
                const uint32_t* G) {
-    launch_mv<MODE_ROUND, 4>(s, MvParams{ws, NULL, WSlice{}, sel, x, y, G, K, R, P, xdiv, xs, ys, 0, raw, NULL, NULL, 0, n_exp}, 1);
+    launch_mv<MODE_ROUND, 4>(s, MvParams{ws, NULL, WSlice{}, sel, x, y, G, K, R, P, xdiv, xs, ys, 0, raw, NULL, NULL, 0}, 1, RouteFuse{}, n_exp);
 }
 
 // A set of SEED4P4 matrices for up to MV_MAXT rows; false: a shape that needs the any-shape kernel.
@@ -1650,7 +1642,7 @@ void kc_mv_sel(cudaStream_t s, int fmt, const WSlice* ws, int K, int R, const fl
                const int32_t* sel, int P, int xdiv, const uint32_t* G) {
     if (!seed_fmt(fmt, "kc_mv_sel")) return;
     FollowScope follow;
-    MvParams a = {ws, NULL, WSlice{}, sel, x, y, G, K, R, P, xdiv, xs, ys, 0, 0, NULL, NULL, 0};
+    MvParams a = {ws, NULL, WSlice{}, sel, x, y, G, K, R, P, xdiv, xs, ys, 0, 0, NULL, NULL, 0, follow.own()};
     if (fmt == MF_SEED4) launch_mv<MODE_ROUND, 3>(s, a, 1);
     else launch_mv<MODE_ROUND, 4>(s, a, 1);
 }
@@ -1659,7 +1651,7 @@ void kc_mv_gu(cudaStream_t s, int fmt, const WSlice* wg, const WSlice* wu, int K
               int ys, const int32_t* sel, int P, int xdiv, const uint32_t* G) {
     if (!seed_fmt(fmt, "kc_mv_gu")) return;
     FollowScope follow;
-    MvParams a = {wg, wu, WSlice{}, sel, x, out, G, K, R, P, xdiv, xs, ys, 0, 0, NULL, NULL, 0};
+    MvParams a = {wg, wu, WSlice{}, sel, x, out, G, K, R, P, xdiv, xs, ys, 0, 0, NULL, NULL, 0, follow.own()};
     if (fmt == MF_SEED4) launch_mv<MODE_GU, 3>(s, a, 1);
     else launch_mv<MODE_GU, 4>(s, a, 1);
 }

@@ -156,3 +156,47 @@ def test_the_switch(switch):
         layer.calls(C.c_void_p(torch.cuda.current_stream().cuda_stream))
         res.append(layer.out.clone())
     assert all(torch.equal(r, res[0]) for r in res) and bool(res[0].any())
+
+
+@pytest.mark.parametrize("kind,K,R,T", [("pair", 512, 256, 4), ("items", 1536, 256, 4), ("grp", 512, 256, 64), ("generic", 520, 256, 2), ("mma", 512, 256, 9),
+                                        ("gemm", 512, 256, 100), ("gemm", 520, 256, 100)])
+def test_a_table_made_by_the_kernel_before(kind, K, R, T):
+    """A call that is a dependent launch by its own choice may use a stream table that the kernel before it has made, one that lets its dependents
+    go early included (kc_pack_input_bf16: the table's halves as bf16 values)."""
+    import torch
+    from nanoseedlm_b200 import lib as L, moe, kernels
+    lib, E, k = L.load(), 6, 4
+    G = kernels.stream_table()
+    halves = (G.view(torch.int16).to(torch.int32) << 16).view(torch.float32)
+    made, want = torch.zeros_like(G), torch.zeros_like(G)
+    gen = torch.Generator(device="cuda").manual_seed(K + T)
+    st = moe.ExpertStack.random_on_device(E, R, K, gen)
+    x = torch.randn(T, K, generator=gen, device="cuda").to(torch.bfloat16).float()
+    sel = torch.randint(0, E, (T * k,), generator=gen, device="cuda", dtype=torch.int32)
+    busy = torch.randn(2048, 2048, device="cuda")
+    rows = T if kind in ("mma", "gemm") else T * k
+    w = L.WSlice()
+    w.p[0], w.p[1], w.p[3], w.eb = st.seeds.data_ptr(), st.coefs.data_ptr(), st.codes.data_ptr(), -22
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def calls(y, y2, table):
+        if kind in ("mma", "gemm"):
+            lib.kc_mm(s, L.MF_SEED4P4, w, K, R, ptr(x), K, ptr(y), R, T, 0, ptr(table))
+            return
+        lib.kc_mv_sel(s, L.MF_SEED4P4, ptr(st.table), K, R, ptr(x), K, ptr(y), R, ptr(sel), T * k, k, ptr(table))
+        lib.kc_mv_gu(s, L.MF_SEED4P4, ptr(st.table), ptr(st.table), K, R, ptr(x), K, ptr(y2), R, ptr(sel), T * k, k, ptr(table))
+
+    lib.kc_pack_input_bf16(s, ptr(halves), ptr(want), halves.numel())
+    torch.cuda.synchronize()
+    ref = [torch.zeros(rows, R, device="cuda") for _ in range(2)]
+    calls(*ref, want)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        got = [torch.zeros(rows, R, device="cuda") for _ in range(2)]
+        made.zero_()
+        for _ in range(4): busy @ busy      # the host gets ahead, so that the calls are queued when the table is made
+        lib.kc_pack_input_bf16(s, ptr(halves), ptr(made), halves.numel())
+        calls(*got, made)
+        torch.cuda.synchronize()
+        assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1]) and bool(ref[0].any())
+    L.check()
