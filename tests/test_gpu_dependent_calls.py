@@ -1,5 +1,5 @@
-"""Calls that are dependent launches by themselves (router, gathers, combine, LM head and arg-max, prompt GEMM): queued one behind the other, with the
-buffers of the previous round still in flight and kernels of another library in between, they give the bits of calls that are waited for one by one."""
+"""Calls that are dependent launches by themselves (router, gathers, combine, LM head and arg-max, prompt GEMM): queued one behind the other or captured in a
+graph, with the buffers of the previous round still in flight, they give the bits of calls that are waited for one by one; and the switch that decides."""
 import ctypes as C
 
 import numpy as np
@@ -12,14 +12,50 @@ def ptr(t):
     return C.c_void_p(t.data_ptr() if t is not None else 0)
 
 
+def three_ways(calls, results):
+    """calls(stream, done) issues a whole sequence, done() after each call; results() gives its outputs.  -> the outputs where each call is waited for;
+    where the sequence is queued before its first call starts (large products run in front of it meanwhile); and of a captured graph, replayed twice."""
+    import torch
+    got, s = [], torch.cuda.Stream()
+    st = C.c_void_p(s.cuda_stream)
+    a = torch.randn(8192, 8192, device="cuda").to(torch.bfloat16)
+    b = torch.empty_like(a)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        for r in results(): r.zero_()
+        calls(st, s.synchronize)
+        s.synchronize()
+        got.append([r.clone() for r in results()])
+        for r in results(): r.zero_()
+        for _ in range(12): torch.mm(a, a, out=b)
+        begin, end = torch.cuda.Event(), torch.cuda.Event()
+        begin.record(s)
+        calls(st, lambda: None)
+        assert not begin.query()      # nothing of the sequence has started yet
+        s.synchronize()
+        got.append([r.clone() for r in results()])
+    rt, graph, exe = C.CDLL("libcudart.so.12"), C.c_void_p(), C.c_void_p()
+    assert rt.cudaStreamBeginCapture(st, 2) == 0
+    calls(st, lambda: None)
+    assert rt.cudaStreamEndCapture(st, C.byref(graph)) == 0 and rt.cudaGraphInstantiate(C.byref(exe), graph, C.c_ulonglong(0)) == 0
+    with torch.cuda.stream(s):
+        for r in results(): r.zero_()
+        for _ in range(2): assert rt.cudaGraphLaunch(exe, st) == 0
+        s.synchronize()
+        got.append([r.clone() for r in results()])
+    rt.cudaGraphExecDestroy(exe)
+    rt.cudaGraphDestroy(graph)
+    return got
+
+
 @pytest.mark.parametrize("p", [4, 3])
-@pytest.mark.parametrize("T", [1, 8])
-def test_a_layer_by_its_own_calls(p, T):
+@pytest.mark.parametrize("T,d,ff,E,k", [(1, 512, 256, 12, 4), (8, 512, 256, 12, 4), (8, 1536, 704, 60, 4), (3, 520, 264, 12, 4), (32, 1024, 512, 16, 4)])
+def test_a_layer_by_its_own_calls(p, T, d, ff, E, k):
+    """Rounds of router, gate + up, down and combine over the same buffers, with nothing in between: a round overwrites what the round before has just read."""
     import torch
     from nanoseedlm_b200 import kernels, lib as L
     from oracle import binding as B
     lib, G = L.load(), kernels.stream_table()
-    d, ff, E, k = 512, 256, 12, 4
     if p == 4:
         stack = lambda R, K, s: kernels.SeedWeight.from_matrices([B.Matrix(R, K, s + e, eb=-20) for e in range(E)])
     else:
@@ -27,67 +63,54 @@ def test_a_layer_by_its_own_calls(p, T):
     gate, up, down = stack(ff, d, 1), stack(ff, d, 50), stack(d, ff, 99)
     fmt = L.MF_SEED4P4 if p == 4 else L.MF_SEED4
     gen = torch.Generator(device="cuda").manual_seed(3)
-    xs = [torch.randn(T, d, generator=gen, device="cuda").to(torch.bfloat16).float() for _ in range(6)]
-    ls = [torch.randn(T, E, generator=gen, device="cuda") for _ in range(6)]
-    s = torch.cuda.Stream()
-    x, logits, out = torch.zeros(T, d, device="cuda"), torch.zeros(T, E, device="cuda"), torch.zeros(T, d, device="cuda")
+    rounds = 12
+    x = torch.randn(rounds, T, d, generator=gen, device="cuda").to(torch.bfloat16).float()
+    logits, out = torch.randn(rounds, T, E, generator=gen, device="cuda"), torch.zeros(rounds, T, d, device="cuda")
     ind, wt = torch.zeros(T, k, dtype=torch.int32, device="cuda"), torch.zeros(T, k, device="cuda")
     A, D = torch.zeros(T * k, ff, device="cuda"), torch.zeros(T * k, d, device="cuda")
 
-    def run(wait):
-        res = []
-        torch.cuda.synchronize()
-        with torch.cuda.stream(s):
-            st = C.c_void_p(s.cuda_stream)
-            done = (lambda: s.synchronize()) if wait else (lambda: None)
-            for rep in range(4):
-                for xi, li in zip(xs, ls):
-                    x.mul_(0.0).add_(xi)               # another library's kernels before and after
-                    logits.copy_(li)
-                    done(); lib.nsl_route(st, E, k, ptr(logits), E, ptr(ind), ptr(wt), T)
-                    done(); lib.kc_mv_gu(st, fmt, ptr(gate.table), ptr(up.table), d, ff, ptr(x), d, ptr(A), ff, ptr(ind), T * k, k, ptr(G))
-                    done(); lib.kc_mv_sel(st, fmt, ptr(down.table), ff, d, ptr(A), ff, ptr(D), d, ptr(ind), T * k, 1, ptr(G))
-                    done(); lib.kq4_moe_combine(st, d, k, ptr(D), ptr(wt), None, None, 0, ptr(out), T)
-                    done(); res.append(out.clone())
-        torch.cuda.synchronize()
-        L.check()
-        return torch.stack(res)
+    def calls(st, done):
+        for i in range(rounds):
+            lib.nsl_route(st, E, k, ptr(logits[i]), E, ptr(ind), ptr(wt), T); done()
+            lib.kc_mv_gu(st, fmt, ptr(gate.table), ptr(up.table), d, ff, ptr(x[i]), d, ptr(A), ff, ptr(ind), T * k, k, ptr(G)); done()
+            lib.kc_mv_sel(st, fmt, ptr(down.table), ff, d, ptr(A), ff, ptr(D), d, ptr(ind), T * k, 1, ptr(G)); done()
+            lib.kq4_moe_combine(st, d, k, ptr(D), ptr(wt), None, None, 0, ptr(out[i]), T); done()
 
-    assert torch.equal(run(False), run(True))
+    waited, queued, graph = three_ways(calls, lambda: [out, ind, wt, A, D])
+    L.check()
+    assert bool(waited[0].any())
+    for a, b, c in zip(waited, queued, graph): assert torch.equal(a, b) and torch.equal(a, c)
 
 
-def test_prompt_product_head_and_tokens():
+# The head's forms: K split over the warps (two widths), streams through shared memory, streams from memory; the arg-max of a cluster a row and of a block a row.
+@pytest.mark.parametrize("K,V", [(2048, 24064), (4096, 13000), (1536, 30000), (1216, 24064), (512, 9000)])
+def test_prompt_product_head_and_tokens(K, V):
     import torch
     from nanoseedlm_b200 import kernels, lib as L, moe
-    lib, G = L.load(), kernels.stream_table()
-    K, V, T = 512, 9000, 8
+    lib, G, T = L.load(), kernels.stream_table(), 8
     gen = torch.Generator(device="cuda").manual_seed(5)
-    st = moe.ExpertStack.random_on_device(1, K, K, gen)
+    st4 = moe.ExpertStack.random_on_device(1, K, K, gen)
     w = L.WSlice()
-    w.p[0], w.p[1], w.p[3], w.eb = st.seeds.data_ptr(), st.coefs.data_ptr(), st.codes.data_ptr(), -22
+    w.p[0], w.p[1], w.p[3], w.eb = st4.seeds.data_ptr(), st4.coefs.data_ptr(), st4.codes.data_ptr(), -22
     codes = torch.randint(-2 ** 31, 2 ** 31 - 1, (V, K // 8), generator=gen, device="cuda", dtype=torch.int32)
     sc = (torch.rand((V, K // 64), generator=gen, device="cuda") * 0.02 + 0.001).to(torch.bfloat16)
     bi = (torch.rand((V, K // 64), generator=gen, device="cuda") * -0.2).to(torch.bfloat16)
     q = L.WSlice()
     q.p[0], q.p[1], q.p[2] = codes.data_ptr(), sc.data_ptr(), bi.data_ptr()
-    xs = [torch.randn(n, K, generator=gen, device="cuda").to(torch.bfloat16).float() for n in (100, 9, 300, 40)]
-    y, lg, tok = torch.zeros(300, K, device="cuda"), torch.zeros(T, V, device="cuda"), torch.zeros(T, dtype=torch.int32, device="cuda")
+    xs = [torch.randn(n, K, generator=gen, device="cuda").to(torch.bfloat16).float() for n in (100, 9, 300, 40, 65, 513)]
+    y, lg = torch.zeros(513, K, device="cuda"), torch.zeros(T, V, device="cuda")
+    tok, prob = torch.zeros(len(xs), T, dtype=torch.int32, device="cuda"), torch.zeros(len(xs), T, device="cuda")      # a probability depends on every logit
 
-    def run(wait):
-        res = []
-        torch.cuda.synchronize()
-        done = torch.cuda.synchronize if wait else (lambda: None)
-        for rep in range(5):
-            for x in xs:
-                done(); lib.kc_mm(None, L.MF_SEED4P4, w, K, K, ptr(x), K, ptr(y), K, x.shape[0], 0, ptr(G))
-                done(); lib.kc_mv(None, L.MF_Q4, q, K, V, ptr(y), K, ptr(lg), V, T, 0, None)
-                done(); lib.kc_argmax(None, ptr(lg), ptr(tok), V, T)
-                done(); res += [y[:x.shape[0]].clone().flatten(), lg.clone().flatten(), tok.float()]
-        torch.cuda.synchronize()
-        L.check()
-        return torch.cat(res)
+    def calls(st, done):
+        for i, x in enumerate(xs):
+            lib.kc_mm(st, L.MF_SEED4P4, w, K, K, ptr(x), K, ptr(y), K, x.shape[0], 0, ptr(G)); done()
+            lib.kc_mv(st, L.MF_Q4, q, K, V, ptr(y), K, ptr(lg), V, T, 0, None); done()
+            lib.kc_argmax_p(st, ptr(lg), ptr(tok[i]), ptr(prob[i]), V, T); done()
 
-    assert torch.equal(run(False), run(True))
+    waited, queued, graph = three_ways(calls, lambda: [tok, prob, y, lg])
+    L.check()
+    assert bool(waited[0].any()) and bool(torch.isfinite(waited[3]).all())
+    for a, b, c in zip(waited, queued, graph): assert torch.equal(a, b) and torch.equal(a, c)
 
 
 @pytest.fixture
@@ -200,3 +223,73 @@ def test_a_table_made_by_the_kernel_before(kind, K, R, T):
         torch.cuda.synchronize()
         assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1]) and bool(ref[0].any())
     L.check()
+
+
+def test_calls_behind_an_event(switch):
+    """The layer on a second stream that waits for the first one's event, joined again behind it: queued, and as a fork and join in a graph."""
+    import torch
+    layer = Layer(3)
+    src, x0 = layer.x.clone(), torch.zeros_like(layer.x)
+    big = torch.randn(4096, 4096, device="cuda")
+    layer.calls(None)
+    torch.cuda.synchronize()
+    want = layer.out.clone()
+    assert bool(want.any())
+    total = torch.zeros_like(want)
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def fork_and_join():
+        ev1, ev2 = torch.cuda.Event(), torch.cuda.Event()
+        with torch.cuda.stream(s1):
+            layer.x.zero_()
+            layer.x.copy_(src)
+            ev1.record(s1)
+            s2.wait_event(ev1)
+            layer.calls(C.c_void_p(s2.cuda_stream))
+            ev2.record(s2)
+            s1.wait_event(ev2)
+            total.add_(layer.out)
+
+    for on in (-1, 1, 0):
+        switch(on)
+        total.zero_()
+        layer.out.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s1):
+            for _ in range(4): torch.mm(big, big)
+        for _ in range(4): fork_and_join()
+        torch.cuda.synchronize()
+        assert torch.equal(total, want * 4), on
+        total.zero_()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s1):
+            for _ in range(2): fork_and_join()
+        for _ in range(2): g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(total, want * 4), on
+
+
+def test_the_switch_and_a_layer_handle_beside_it(switch):
+    """Calls with the switch turned between them, beside a layer whose own launches are ordinary: the bits stay."""
+    import torch
+    from nanoseedlm_b200 import moe
+    layer, gen = Layer(8), torch.Generator(device="cuda").manual_seed(1)
+    m = moe.Moe(moe.DeviceLayer.random_on_device(512, 256, 12, gen), 4, 8)
+    x, lg, out = torch.randn(8, 512, generator=gen, device="cuda"), torch.randn(8, 12, generator=gen, device="cuda"), torch.zeros(8, 512, device="cuda")
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    refs = []
+    for pdl in (1, 0):
+        m.lib.nsl_moe_set_dependent_launch(m.h, pdl)
+        for on in (0, -1, 1, -1):
+            switch(on)
+            layer.out.zero_()
+            out.zero_()
+            for _ in range(3):
+                layer.calls(s)
+                m.forward_dev(x, lg, out)
+                switch(on if _ else 0)
+            assert layer.lib.nsl_dependent_launch_state() == on
+            refs.append((layer.out.clone(), out.clone()))
+    m.close()
+    assert all(torch.equal(a, refs[0][0]) and torch.equal(b, refs[0][1]) for a, b in refs) and bool(refs[0][0].any()) and bool(refs[0][1].any())
