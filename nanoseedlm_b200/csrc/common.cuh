@@ -34,7 +34,7 @@ struct PdlScope {
 // table in the kernel before, whose writes are visible after the wait and not sooner.
 struct FollowScope {
     int prev;
-    FollowScope() : prev(tl_pdl) { if (prev == PDL_OWN) tl_pdl = PDL_ON; }
+    explicit FollowScope(bool follows = true) : prev(tl_pdl) { if (prev == PDL_OWN && follows) tl_pdl = PDL_ON; }
     int own() const { return prev == PDL_OWN; }
     ~FollowScope() { tl_pdl = prev; }
 };

@@ -822,7 +822,7 @@ void kc_seed_gemm_f32(int on) { g_exact = on; }
 void kc_mm(cudaStream_t s, int fmt, WSlice w, int K, int R, const float* x, int xs, float* y, int ys, int T, int add,
            const uint32_t* G) {
     if (fmt == MF_BF16 && launch_bf16_mm_skinny(s, w, K, R, x, xs, y, ys, T, add)) return;      // a decode batch (dense_bf16.cu)
-    FollowScope follow;
+    FollowScope follow(fmt != MF_BF16);      // (products of stored weights have not been measured as such)
     MmParams a = {NULL, w, x, y, NULL, NULL, NULL, G, K, R, T, xs, ys, 1, add, 0, 0, NULL, 0, NULL, 0, 0, 0, follow.own()};
     launch_gemm(s, fmt, "kc_mm", a, (T + GM_BN - 1) / GM_BN);
 }

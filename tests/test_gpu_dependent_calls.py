@@ -225,6 +225,37 @@ def test_a_table_made_by_the_kernel_before(kind, K, R, T):
     L.check()
 
 
+def bf16_product():
+    import torch
+    from nanoseedlm_b200 import lib as L
+    lib, K, R, T = L.load(), 256, 384, 100      # (format 0: stored BF16)
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    wb, x = torch.randn(R, K, generator=gen, device="cuda").to(torch.bfloat16), torch.randn(T, K, generator=gen, device="cuda").to(torch.bfloat16).float()
+    y, w = torch.zeros(T, R, device="cuda"), L.WSlice()
+    w.p[0] = wb.data_ptr()
+    return lambda s, rows: lib.kc_mm(s, 0, w, K, R, ptr(x), K, ptr(y), R, rows, 0, None), (wb, x, y)
+
+
+@pytest.mark.parametrize("rows", [100, 9])      # the tile GEMM, the decode batch's kernel
+def test_products_of_stored_bf16_weights_are_ordinary_launches(switch, rows):
+    import torch
+    call, (wb, x, y) = bf16_product()
+
+    def both(s):
+        call(s, rows)
+        call(s, rows)
+
+    both(None)
+    assert edges_of(both) == (0, 1)
+    switch(1)
+    assert edges_of(both) == (1, 0)
+    switch(0)
+    assert edges_of(both) == (0, 1)
+    torch.cuda.synchronize()
+    ref = x[:rows].double() @ wb.double().T      # f32 sums of 256 products (at most 256 x 2^-24 of their magnitudes' sum) and one rounding to bf16 (8 significant bits: 2^-8)
+    assert bool(((y[:rows].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1.01 * 2.0 ** -16 * (x[:rows].double().abs() @ wb.double().abs().T)).all())
+
+
 def test_calls_behind_an_event(switch):
     """The layer on a second stream that waits for the first one's event, joined again behind it: queued, and as a fork and join in a graph."""
     import torch
