@@ -99,7 +99,7 @@ __device__ __forceinline__ const KvSeg& kv_seg_of(const KvView& kv, int abs_pos,
 }
 __device__ __forceinline__ uint4 ld_stream(const void* p) {      // read once
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 // The four codes of a word times the row's scale, as two bf16 pairs: byte ^ 0x80 under the exponent of 2^23 is the float
@@ -247,7 +247,7 @@ __device__ __forceinline__ void attn_merge(unsigned char* att_smem, int STAGE, i
 // A lane holds keys r0 and r0 + 8 of heads 2 q4 and 2 q4 + 1 of each tile: the maxima and sums of a head run over the 8
 // lanes of equal q4.  Ends with the block in step (shared memory reusable).
 template <int NSLOT, int NT>
-__device__ __forceinline__ void attn_keys_bf16(const AttnArgs& a, const float* __restrict__ q, const KvView& kv, int t, int kvh, int kv0,
+__device__ __forceinline__ void attn_keys_bf16(const AttnArgs& a, const float* q, const KvView& kv, int t, int kvh, int kv0,
                                           int p0, int p1, unsigned char* att_smem, float* pp, size_t head_stride) {
     constexpr int STAGE = NSLOT * ATT_SLOT, STRIDE = ATT_MMA_WARPS * ATT_MT;
     const int lane = threadIdx.x & 31, ring_id = threadIdx.x >> 5, q4 = lane & 3, r0 = lane >> 2;
@@ -336,7 +336,7 @@ __device__ __forceinline__ void attn_keys_bf16(const AttnArgs& a, const float* _
 // The next step's K rows are requested when this step's are in fragments, V rows likewise.  (Staged through shared memory and
 // expanded there a step took 4500 clk of latency: 26.7 us for 24 rows of 2500..5000 keys, 2 KV heads, 22 % of the HBM peak.)
 template <int NT>
-__device__ __forceinline__ void attn_keys_q8(const AttnArgs& a, const float* __restrict__ q, const KvView& kv, int t, int kvh, int kv0, int p0, int p1,
+__device__ __forceinline__ void attn_keys_q8(const AttnArgs& a, const float* q, const KvView& kv, int t, int kvh, int kv0, int p0, int p1,
                                              unsigned char* att_smem, float* pp, size_t head_stride) {
     constexpr int STRIDE = ATT_MMA_WARPS * ATT_MT;
     const int lane = threadIdx.x & 31, q4 = lane & 3, r0 = lane >> 2, group = a.n_head / a.n_kv;
@@ -351,7 +351,7 @@ __device__ __forceinline__ void attn_keys_q8(const AttnArgs& a, const float* __r
             const unsigned char* src = (const unsigned char*) sg.k + at * ATT_HD + 16 * q4;
             kr[i][0] = ld_stream(src);
             kr[i][1] = ld_stream(src + 64);
-            ks[i] = __ldg(sg.ks + at);
+            ks[i] = sg.ks[at];
         }
     };
     auto load_v = [&](int p) {
@@ -361,7 +361,7 @@ __device__ __forceinline__ void attn_keys_q8(const AttnArgs& a, const float* __r
             const KvSeg& sg = kv_seg_of(kv, kv0 + min(p + 2 * q4 + (i & 1) + (i >> 1) * 8, p1 - 1), row);
             const size_t at = (size_t) row * a.n_kv + kvh;
             vr[i] = ld_stream((const unsigned char*) sg.v + at * ATT_HD + 16 * r0);
-            vs[i] = __ldg(sg.vs + at);
+            vs[i] = sg.vs[at];
         }
     };
     int p = p0 + (int) (threadIdx.x >> 5) * ATT_MT;
@@ -430,7 +430,7 @@ __device__ __forceinline__ void attn_keys_q8(const AttnArgs& a, const float* __r
 // SRC: the cache's form.
 enum { ATT_SRC_BF16 = 0, ATT_SRC_Q8 = 2 };
 template <int NSLOT, int NT, int SRC>
-__device__ __forceinline__ void attn_keys(const AttnArgs& a, const float* __restrict__ q, const KvView& kv, int t, int kvh, int kv0, int p0, int p1,
+__device__ __forceinline__ void attn_keys(const AttnArgs& a, const float* q, const KvView& kv, int t, int kvh, int kv0, int p0, int p1,
                                           unsigned char* att_smem, float* pp, size_t head_stride) {
     if (SRC == ATT_SRC_Q8) attn_keys_q8<NT>(a, q, kv, t, kvh, kv0, p0, p1, att_smem, pp, head_stride);
     else attn_keys_bf16<NSLOT, NT>(a, q, kv, t, kvh, kv0, p0, p1, att_smem, pp, head_stride);
@@ -438,8 +438,8 @@ __device__ __forceinline__ void attn_keys(const AttnArgs& a, const float* __rest
 
 // One block per (split, KV head, row): the split's keys as the reference cuts them.
 template <int NSLOT, int NT, int SRC>
-__global__ void __launch_bounds__(32 * ATT_MMA_WARPS) attn_split_mma_kernel(AttnArgs a, const float* __restrict__ q, KvView kv,
-                                                                            const RowInfo* __restrict__ ri, float* __restrict__ part) {
+__global__ void __launch_bounds__(32 * ATT_MMA_WARPS) attn_split_mma_kernel(AttnArgs a, const float* q, KvView kv,
+                                                                            const RowInfo* ri, float* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char att_smem[];      // the warps' rings, later their states
     const int split = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
     const int group = a.n_head / a.n_kv;
@@ -466,7 +466,7 @@ struct AttnPlan {
 
 // u(t) = units of row t; pre[t] = u(0) + ... + u(t - 1), pre[T] = their sum.  Called by all threads of a block of NW warps.
 template <int NW>
-__device__ __forceinline__ AttnPlan attn_plan(const RowInfo* __restrict__ ri, int T, int n_kv, int n_splits, int n_blocks, int* pre) {
+__device__ __forceinline__ AttnPlan attn_plan(const RowInfo* ri, int T, int n_kv, int n_splits, int n_blocks, int* pre) {
     __shared__ int wsum[NW], wmax[NW];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int each = (T + 32 * NW - 1) / (32 * NW);      // <= 8 rows a thread
@@ -512,7 +512,7 @@ __device__ __forceinline__ AttnPlan attn_plan(const RowInfo* __restrict__ ri, in
 
 template <int NSLOT, int NT, int SRC>
 __global__ void __launch_bounds__(32 * ATT_MMA_WARPS, 3)      // (8-bit cache, four blocks of 128 registers: 26.2 us where three take 25.7)
-attn_flat_mma_kernel(AttnArgs a, const float* __restrict__ q, KvView kv, const RowInfo* __restrict__ ri, float* __restrict__ part, int T) {
+attn_flat_mma_kernel(AttnArgs a, const float* q, KvView kv, const RowInfo* ri, float* __restrict__ part, int T) {
     extern __shared__ __align__(16) unsigned char att_smem[];
     __shared__ int pre[ATT_MAX_ROWS + 1];
     const int group = a.n_head / a.n_kv;
@@ -548,8 +548,8 @@ __device__ __forceinline__ float softplus_ln2(float g) {   // softplus with beta
 
 // Merges a head's partials and applies the gate.  n_blocks = 0: the split form's n_splits partials (unused ones carry
 // m = -inf); otherwise the balanced form's, as many as the pair's units touch blocks.
-__global__ void __launch_bounds__(ATT_HD) attn_reduce_kernel(AttnArgs a, const float* __restrict__ part, const float* __restrict__ g,
-                                                             float* __restrict__ o, const RowInfo* __restrict__ ri, int T, int n_blocks) {
+__global__ void __launch_bounds__(ATT_HD) attn_reduce_kernel(AttnArgs a, const float* part, const float* g,
+                                                             float* __restrict__ o, const RowInfo* ri, int T, int n_blocks) {
     __shared__ int pre[ATT_MAX_ROWS + 1];
     const int h = blockIdx.x, t = blockIdx.y, d = threadIdx.x;
     grid_dependents_go();

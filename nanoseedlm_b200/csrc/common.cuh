@@ -20,6 +20,9 @@ inline bool aligned16(const void* p) { return ((uintptr_t) p & 15u) == 0; }
 // which returns once the previous kernel has completed and its writes are visible.  Every kernel launched through
 // launch() calls grid_dependency_wait() before it reads or writes anything a neighbouring kernel touches; without the
 // scope, and outside the entry points that open one themselves, the launch is an ordinary one and the wait returns at once.
+// What a neighbour may have written (activations, logits, routing, partial sums, cache rows) is read with ordinary loads: ld.global.nc (__ldg, and what
+// the compiler makes of a kernel's const __restrict__ parameters) is for memory that nobody writes while the kernel runs, and a dependent kernel runs
+// beside the one that writes its inputs.  Weight streams and other constants take it.
 // The thread's state is one of: each entry point's own choice (until the caller says otherwise), ordinary launches, dependent ones.
 enum { PDL_OWN = -1, PDL_OFF = 0, PDL_ON = 1 };
 extern thread_local int tl_pdl;

@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(256) embed_bf16_kernel(const uint16_t* __restr
 
 // One block per row; threads 0..127 own the first half of the row, 128..255 the second, so each half's mean square is a
 // reduction over four warps and no element asks which group it is in.
-__global__ void __launch_bounds__(256) gnorm_kernel(int d, float eps, const float* __restrict__ x, const uint16_t* __restrict__ w,
+__global__ void __launch_bounds__(256) gnorm_kernel(int d, float eps, const float* x, const uint16_t* __restrict__ w,
                                                     float* __restrict__ y) {
     __shared__ float part[8];
     grid_dependents_go();
@@ -41,18 +41,38 @@ __global__ void __launch_bounds__(256) gnorm_kernel(int d, float eps, const floa
     const float r = rsqrtf(tot / (float) hw + eps);
     const uint16_t* wr = w + (size_t) half * hw;
     float* yr = y + (size_t) t * d + (size_t) half * hw;
-    for (int c = i0; c < hw; c += 128) yr[c] = bf16_round(bf16_to_f32(wr[c]) * (xr[c] * r));
+    for (int c0 = i0; c0 < hw; c0 += 8 * 128) {      // eight values requested before one is stored
+        float v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = c0 + 128 * q < hw ? xr[c0 + 128 * q] : 0.0f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int c = c0 + 128 * q;
+            if (c < hw) yr[c] = bf16_round(bf16_to_f32(wr[c]) * (v[q] * r));
+        }
+    }
 }
 
 // One warp per (row, head): lane l rotates the pairs (l, l + 64) and (l + 32, l + 96).  Heads below n_head are query heads
 // (rotated in place); heads below n_kv also carry that KV head's key and value into the cache.
-__global__ void __launch_bounds__(128) rope_kv_kernel(float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, KvView kv,
-                                                      const RowInfo* __restrict__ ri, const float* __restrict__ inv, int n_head, int n_kv, int heads) {
+__global__ void __launch_bounds__(128) rope_kv_kernel(float* __restrict__ q, const float* k, const float* v, KvView kv,
+                                                      const RowInfo* ri, const float* __restrict__ inv, int n_head, int n_kv, int heads) {
     grid_dependents_go();
     grid_dependency_wait();
     const int lane = threadIdx.x & 31, head = blockIdx.x * 4 + (threadIdx.x >> 5), t = blockIdx.y;
     if (head >= heads) return;
-    const int pos = ri[t].pos;
+    const int pos = ri[t].pos, kv0 = ri[t].kv0;
+    float ka[2], kb[2], va[2], vb[2];      // requested before the query is stored
+    if (head < n_kv) {
+        const float* kh = k + ((size_t) t * n_kv + head) * HD;
+        const float* vh = v + ((size_t) t * n_kv + head) * HD;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int p = lane + 32 * j;
+            ka[j] = kh[p]; kb[j] = kh[p + 64];
+            va[j] = vh[p]; vb[j] = vh[p + 64];
+        }
+    }
     float sn[2], cs[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) sincosf((float) pos * inv[lane + 32 * j], &sn[j], &cs[j]);
@@ -67,19 +87,15 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(float* __restrict__ q, con
         }
     }
     if (head >= n_kv) return;      // uniform over the warp
-    const float* kh = k + ((size_t) t * n_kv + head) * HD;
-    const float* vh = v + ((size_t) t * n_kv + head) * HD;
     float kr[4], vr[4];      // dims lane, lane + 64, lane + 32, lane + 96
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-        const int p = lane + 32 * j;
-        const float a = kh[p], b = kh[p + 64];
-        kr[2 * j] = a * cs[j] - b * sn[j];
-        kr[2 * j + 1] = b * cs[j] + a * sn[j];
-        vr[2 * j] = vh[p];
-        vr[2 * j + 1] = vh[p + 64];
+        kr[2 * j] = ka[j] * cs[j] - kb[j] * sn[j];
+        kr[2 * j + 1] = kb[j] * cs[j] + ka[j] * sn[j];
+        vr[2 * j] = va[j];
+        vr[2 * j + 1] = vb[j];
     }
-    int row = ri[t].kv0 + pos;      // the sequence slot's cache row: positions below nv in segment a, the rest in b
+    int row = kv0 + pos;      // the sequence slot's cache row: positions below nv in segment a, the rest in b
     const KvSeg sg = row < kv.nv ? kv.a : kv.b;
     if (row >= kv.nv) row -= kv.nv;
     const size_t off = ((size_t) row * n_kv + head) * HD;
@@ -117,7 +133,7 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(float* __restrict__ q, con
 }
 
 // x[i] = bf16(x[i] + y[i]): the residual stream holds bf16-valued numbers.
-__global__ void residual_add_kernel(float* __restrict__ x, const float* __restrict__ y, size_t n) {
+__global__ void residual_add_kernel(float* __restrict__ x, const float* y, size_t n) {
     grid_dependents_go();
     grid_dependency_wait();
     for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x) x[i] = bf16_round(x[i] + y[i]);

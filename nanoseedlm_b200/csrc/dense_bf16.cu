@@ -9,7 +9,7 @@
 namespace nsl {
 
 template <int NT>
-__global__ void __launch_bounds__(256) bf16_mv_kernel(const uint16_t* __restrict__ W, int K, int R, const float* __restrict__ x, int xs,
+__global__ void __launch_bounds__(256) bf16_mv_kernel(const uint16_t* __restrict__ W, int K, int R, const float* x, int xs,
                                                       float* __restrict__ y, int ys, int T, int add) {
     grid_dependents_go();
     grid_dependency_wait();
@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(256) bf16_mv_kernel(const uint16_t* __restrict
             for (int t = 0; t < NT; ++t) {
                 if (t >= T) break;
                 const float4* xp = (const float4*) (x + (size_t) t * xs + 8 * c);
-                const float4 a = __ldg(xp), b = __ldg(xp + 1);
+                const float4 a = xp[0], b = xp[1];
                 float s = acc[t];
                 s = fmaf(w[0], a.x, s); s = fmaf(w[1], a.y, s); s = fmaf(w[2], a.z, s); s = fmaf(w[3], a.w, s);
                 s = fmaf(w[4], b.x, s); s = fmaf(w[5], b.y, s); s = fmaf(w[6], b.z, s); s = fmaf(w[7], b.w, s);
@@ -83,7 +83,7 @@ __device__ __forceinline__ void mma_bf16_16816(float* c, uint32_t a0, uint32_t a
 
 // The matrices of a set are sixteen-row tiles side by side.  (Three launches for q, k, v of one decoder row cost three latencies, 3 us
 // each, for 1 us of memory traffic.)
-__global__ void __launch_bounds__(256) bf16_mm_skinny_kernel(DenseSet set, int K, const float* __restrict__ x, int xs, int ys, int T, int add) {
+__global__ void __launch_bounds__(256) bf16_mm_skinny_kernel(DenseSet set, int K, const float* x, int xs, int ys, int T, int add) {
     extern __shared__ __align__(16) unsigned char xsm[];      // 8 rows of K bf16 inputs
     __shared__ float part[8][16][9];
     grid_dependents_go();
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(256) bf16_mm_skinny_kernel(DenseSet set, int K
             for (int c = threadIdx.x; c < 8 * kc8; c += 256) {
                 const int n = c / kc8, kc = c - n * kc8;
                 const float4* xp = (const float4*) (x + (size_t) min(tok0 + n, T - 1) * xs + 8 * kc);
-                const float4 x0 = __ldg(xp), x1 = __ldg(xp + 1);
+                const float4 x0 = xp[0], x1 = xp[1];
                 *(uint4*) (xsm + (size_t) n * stride + 16 * kc) =
                     make_uint4(bf16x2_bits(x0.x, x0.y), bf16x2_bits(x0.z, x0.w), bf16x2_bits(x1.x, x1.y), bf16x2_bits(x1.z, x1.w));
             }

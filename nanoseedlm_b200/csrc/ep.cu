@@ -14,7 +14,7 @@ constexpr uint32_t FULL = 0xFFFFFFFFu;
 // in the middle: the lower rank of the two takes the first ceil(n/2) pairs, the upper rank the rest.  Either rank's
 // share differs from the other's by at most one pair whatever the routing.  Local slice index: e - lo for the own
 // range, (hi - lo) + e - lo2 for the partner's.
-__global__ void __launch_bounds__(1024) ep_plan_kernel(const int32_t* __restrict__ ind, const float* __restrict__ wt, int n_ranks,
+__global__ void __launch_bounds__(1024) ep_plan_kernel(const int32_t* ind, const float* wt, int n_ranks,
                                                        int t_loc, int k, int rank_stride, int row_stride, int lo, int hi,
                                                        int32_t* __restrict__ sel, int32_t* __restrict__ xrow,
                                                        float* __restrict__ wsel, int32_t* __restrict__ tok_off,
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(1024) ep_plan_kernel(const int32_t* __restrict
     }
 }
 
-__global__ void ep_combine_kernel(const float* __restrict__ D, const float* __restrict__ wsel, const int32_t* __restrict__ tok_off,
+__global__ void ep_combine_kernel(const float* D, const float* wsel, const int32_t* tok_off,
                                   int d, float* __restrict__ partial) {
     const int g = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     grid_dependents_go();

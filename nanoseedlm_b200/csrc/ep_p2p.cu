@@ -29,7 +29,7 @@ __device__ __forceinline__ char* recv_slot(const NslEpWindow& w, int rank) {   /
 }
 
 // Dispatch of a ready-made chunk: block r copies it into slot `me` of rank r's receive area.
-__global__ void __launch_bounds__(1024) ep_dispatch_kernel(NslEpWindow w, const uint4* __restrict__ chunk) {
+__global__ void __launch_bounds__(1024) ep_dispatch_kernel(NslEpWindow w, const uint4* chunk) {
     grid_dependents_go();
     grid_dependency_wait();
     const int r = blockIdx.x;
@@ -96,8 +96,8 @@ __global__ void __launch_bounds__(32) ep_wait_dispatch_kernel(NslEpWindow w) {
 
 // Combine: block g pre-sums token g's local experts and stores the row into slot `me` of the partial-row area of the
 // rank that owns the token, then signals one row to that rank.
-__global__ void __launch_bounds__(256) ep_combine_p2p_kernel(NslEpWindow w, const float* __restrict__ D, const float* __restrict__ wsel,
-                                                             const int32_t* __restrict__ tok_off, int d) {
+__global__ void __launch_bounds__(256) ep_combine_p2p_kernel(NslEpWindow w, const float* D, const float* wsel,
+                                                             const int32_t* tok_off, int d) {
     grid_dependents_go();
     grid_dependency_wait();
     const int g = blockIdx.x, owner = g / w.t_loc, t = g - owner * w.t_loc;

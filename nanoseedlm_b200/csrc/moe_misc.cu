@@ -15,7 +15,7 @@ __device__ __forceinline__ bool aligned16_dev(const void* p) { return ((unsigned
 // ---- router ------------------------------------------------------------------------------------------------------------
 // One warp per row (route_row in route.cuh).
 template <int PER>                   // experts per lane held in registers: E <= 32 * PER
-__global__ void __launch_bounds__(128) route_kernel(int E, int k, const float* __restrict__ logits, int ld,
+__global__ void __launch_bounds__(128) route_kernel(int E, int k, const float* logits, int ld,
                                                     int32_t* __restrict__ ind, float* __restrict__ wt, int T) {
     const int lane = threadIdx.x & 31, t = blockIdx.x * 4 + (threadIdx.x >> 5);
     grid_dependency_wait();
@@ -45,8 +45,8 @@ __global__ void swiglu_packed_kernel(const float* __restrict__ g, const float* _
 
 // out[t][i] = sigmoid(sg[t*sgld]) sh[t][i] + sum_j wt[t][j] D[t*k+j][i], plain f32, j ascending; sh == NULL: no shared
 // expert term.
-__global__ void q4_combine_kernel(int d, int k, const float* __restrict__ D, const float* __restrict__ wt,
-                                  const float* __restrict__ sh, const float* __restrict__ sg, int sgld, float* __restrict__ out) {
+__global__ void q4_combine_kernel(int d, int k, const float* D, const float* wt,
+                                  const float* sh, const float* sg, int sgld, float* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
     grid_dependents_go();
     grid_dependency_wait();
@@ -60,8 +60,8 @@ __global__ void q4_combine_kernel(int d, int k, const float* __restrict__ D, con
 // The end of a decoder layer and the start of the next: the combine above, x = bf16(x + its result) (nsl_residual_add) and y = the
 // grouped RMSNorm of x (kc_gnorm), a block a row, each value formed as those three kernels form it.  For a decode batch
 // each of them is a launch's latency and little else.
-__global__ void __launch_bounds__(256) combine_residual_gnorm_kernel(int d, int k, const float* __restrict__ D, const float* __restrict__ wt,
-                                                                     const float* __restrict__ sh, const float* __restrict__ sg, int sgld,
+__global__ void __launch_bounds__(256) combine_residual_gnorm_kernel(int d, int k, const float* D, const float* wt,
+                                                                     const float* sh, const float* sg, int sgld,
                                                                      float* __restrict__ x, float eps,
                                                                      const uint16_t* __restrict__ w, float* __restrict__ y) {
     __shared__ float part[8];
@@ -114,7 +114,7 @@ void launch_combine_residual_gnorm(cudaStream_t s, int d, int k, const float* D,
 
 // The same without a shared expert over packed bf16 rows (d a multiple of 8: 16 bytes of each of the k rows a thread).  vec: out is
 // 16-byte aligned (the caller's pointer may be any).
-__global__ void __launch_bounds__(256) combine_packed_kernel(int d8, int k, const uint4* __restrict__ D, const float* __restrict__ wt,
+__global__ void __launch_bounds__(256) combine_packed_kernel(int d8, int k, const uint4* D, const float* wt,
                                                              float* __restrict__ out, int n, int vec) {
     grid_dependency_wait();
     grid_dependents_go();
@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(256) combine_packed_kernel(int d8, int k, cons
 #pragma unroll
         for (int q = 0; q < 8; ++q)
             if (j0 + q < k) {
-                v[q] = __ldg(D + ((size_t) t * k + j0 + q) * d8 + c);
-                w[q] = __ldg(wt + t * k + j0 + q);
+                v[q] = D[((size_t) t * k + j0 + q) * d8 + c];
+                w[q] = wt[t * k + j0 + q];
             }
 #pragma unroll
         for (int q = 0; q < 8; ++q)
@@ -168,7 +168,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ D, const float* __r
     x[i] = bf16_round(x[i] + bf16_round(bf16_round(s) + shared[i]));
 }
 
-__device__ __forceinline__ void pack_bf16(const float* __restrict__ x, uint16_t* __restrict__ y, size_t n, unsigned block, unsigned blocks) {
+__device__ __forceinline__ void pack_bf16(const float* x, uint16_t* __restrict__ y, size_t n, unsigned block, unsigned blocks) {
     const size_t n8 = n / 8;
     for (size_t i = (size_t) block * blockDim.x + threadIdx.x; i < n8; i += (size_t) blocks * blockDim.x) {
         const float4 a = ((const float4*) x)[2 * i], b = ((const float4*) x)[2 * i + 1];
@@ -176,7 +176,7 @@ __device__ __forceinline__ void pack_bf16(const float* __restrict__ x, uint16_t*
     }
     if (block == 0 && threadIdx.x < (n & 7)) y[n8 * 8 + threadIdx.x] = bf16_bits(x[n8 * 8 + threadIdx.x]);
 }
-__global__ void pack_bf16_kernel(const float* __restrict__ x, uint16_t* __restrict__ y, size_t n) {
+__global__ void pack_bf16_kernel(const float* x, uint16_t* __restrict__ y, size_t n) {
     grid_dependency_wait();
     grid_dependents_go();
     pack_bf16(x, y, n, blockIdx.x, gridDim.x);
@@ -185,18 +185,18 @@ __global__ void pack_bf16_kernel(const float* __restrict__ x, uint16_t* __restri
 // Packed bf16 rows in the order of the pairs by expert: row at[t * k + j] of y = row t of x for each of its k pairs (d a multiple of 8;
 // a thread: 8 values, read and converted once).  Bound by the writes: 32768 rows of 2048 from 4096 in 26 us (168 MB); a row of y at a time, its
 // inputs read again for every pair, took 51.
-__global__ void __launch_bounds__(256) pack_sorted_kernel(const float4* __restrict__ x, const int32_t* __restrict__ at, uint4* __restrict__ y, int k, int d8,
+__global__ void __launch_bounds__(256) pack_sorted_kernel(const float4* x, const int32_t* at, uint4* __restrict__ y, int k, int d8,
                                                           int T) {
     __shared__ int pos[32];
     grid_dependency_wait();
     grid_dependents_go();
     for (int t = blockIdx.x; t < T; t += gridDim.x) {
         __syncthreads();      // the previous row's places are no longer read
-        if ((int) threadIdx.x < k) pos[threadIdx.x] = __ldg(at + (size_t) t * k + threadIdx.x);
+        if ((int) threadIdx.x < k) pos[threadIdx.x] = at[(size_t) t * k + threadIdx.x];
         __syncthreads();
         const float4* xp = x + (size_t) t * d8 * 2;
         for (int c = threadIdx.x; c < d8; c += 256) {
-            const float4 a = __ldg(xp + 2 * c), b = __ldg(xp + 2 * c + 1);
+            const float4 a = xp[2 * c], b = xp[2 * c + 1];
             const uint4 v = make_uint4(bf16x2_bits(a.x, a.y), bf16x2_bits(a.z, a.w), bf16x2_bits(b.x, b.y), bf16x2_bits(b.z, b.w));
             for (int j = 0; j < k; ++j)
                 if ((unsigned) pos[j] < (unsigned) (T * k)) y[(size_t) pos[j] * d8 + c] = v;      // (a pair of no expert has no place)
@@ -214,7 +214,7 @@ void launch_pack_sorted(cudaStream_t s, const float* x, const int32_t* at, uint1
 // One block: histogram by shared-memory atomics, then an exclusive scan of pairs and tiles over the experts (both in one 64-bit
 // word, by warp shuffles: two barriers).
 // The block's 1024 threads: pairs of expert tid (count_e), pairs (low half) and tiles (high half) of the experts before it, of all.
-__device__ __forceinline__ unsigned long long bucket_offsets(const int32_t* __restrict__ inds, int count, int n, int& count_e, unsigned long long& all) {
+__device__ __forceinline__ unsigned long long bucket_offsets(const int32_t* inds, int count, int n, int& count_e, unsigned long long& all) {
     __shared__ int cnt[BUCKET_MAX_EXPERTS];
     __shared__ unsigned long long wsum[32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -249,7 +249,7 @@ __device__ __forceinline__ void bucket_work(int32_t* work, int n, unsigned long 
         work[2 + 2 * n] = work[0] = (int) (all >> 32);
     }
 }
-__global__ void __launch_bounds__(1024) bucket_count_kernel(const int32_t* __restrict__ inds, int count, int n,
+__global__ void __launch_bounds__(1024) bucket_count_kernel(const int32_t* inds, int count, int n,
                                                             int32_t* __restrict__ work) {
     grid_dependency_wait();
     grid_dependents_go();
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(1024) bucket_count_kernel(const int32_t* __res
 // One block per expert.  Each warp owns a contiguous range of the pair list (a multiple of 128, four entries a lane): it counts its
 // matches, the block scans the 32 counts, then each warp writes its matches in order (ballot prefixes), so perm is ascending
 // within the expert.
-__device__ __forceinline__ void bucket_place(const int32_t* __restrict__ inds, int count, int e, int begin, int total, int t0, int32_t* __restrict__ perm,
+__device__ __forceinline__ void bucket_place(const int32_t* inds, int count, int e, int begin, int total, int t0, int32_t* __restrict__ perm,
                                              MmTile* __restrict__ tiles, int32_t* __restrict__ at_out) {
     __shared__ int wcount[32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -271,11 +271,11 @@ __device__ __forceinline__ void bucket_place(const int32_t* __restrict__ inds, i
     const int lo = w * per, hi = lo + per < count ? lo + per : count;
     auto four = [&](int i, bool* f) {      // the lane's entries i .. i + 3
         if (vec && i + 3 < hi) {
-            const int4 v = __ldg((const int4*) (inds + i));
+            const int4 v = *(const int4*) (inds + i);
             f[0] = v.x == e; f[1] = v.y == e; f[2] = v.z == e; f[3] = v.w == e;
         } else {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) f[q] = i + q < hi && __ldg(inds + i + q) == e;
+            for (int q = 0; q < 4; ++q) f[q] = i + q < hi && inds[i + q] == e;
         }
     };
     int mine = 0;
@@ -312,8 +312,8 @@ __device__ __forceinline__ void bucket_place(const int32_t* __restrict__ inds, i
         tiles[t0 + t] = tl;
     }
 }
-__global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* __restrict__ inds, int count,
-                                                            const int32_t* __restrict__ work, int32_t* __restrict__ perm,
+__global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* inds, int count,
+                                                            const int32_t* work, int32_t* __restrict__ perm,
                                                             MmTile* __restrict__ tiles, int32_t* __restrict__ at_out) {
     const int e = blockIdx.x, n = gridDim.x;
     grid_dependency_wait();
@@ -325,8 +325,8 @@ __global__ void __launch_bounds__(1024) bucket_place_kernel(const int32_t* __res
 // beyond the experts' pack the layer's inputs (pack_n values of x), which nothing here needs.  Three launches in a row cost a prompt
 // of a few hundred rows three latencies, 3 us each.
 constexpr int BUCKET_ONE_PAIRS = 8192;
-__global__ void __launch_bounds__(1024) bucket_pack_kernel(const int32_t* __restrict__ inds, int count, int n, int32_t* __restrict__ work, int32_t* __restrict__ perm,
-                                                           MmTile* __restrict__ tiles, const float* __restrict__ x, uint16_t* __restrict__ xp, size_t pack_n) {
+__global__ void __launch_bounds__(1024) bucket_pack_kernel(const int32_t* inds, int count, int n, int32_t* __restrict__ work, int32_t* __restrict__ perm,
+                                                           MmTile* __restrict__ tiles, const float* x, uint16_t* __restrict__ xp, size_t pack_n) {
     __shared__ int mine[3];
     grid_dependency_wait();      // (its dependents go when it ends: the persistent GEMM's blocks would come in wherever an SM is free, and two with one unit more share one: 298 us for 512 rows instead of 274)
     const int e = blockIdx.x;
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(512) cache_copy_kernel(CachePool p) {
 constexpr int BUCKET_SCRATCH_INTS = 2 * BUCKET_MAX_EXPERTS + 3;
 static __device__ __align__(256) int32_t g_bucket_scratch[BUCKET_SCRATCH_INTS];
 
-__global__ void bucket_publish_kernel(const int32_t* __restrict__ work, int32_t* __restrict__ ntiles_out) {
+__global__ void bucket_publish_kernel(const int32_t* work, int32_t* __restrict__ ntiles_out) {
     grid_dependency_wait();
     grid_dependents_go();
     if (threadIdx.x == 0 && blockIdx.x == 0) ntiles_out[0] = work[0];

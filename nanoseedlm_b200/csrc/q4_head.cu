@@ -55,7 +55,7 @@ __device__ __forceinline__ bool aligned16_dev(const void* p) { return ((unsigned
 
 // Shared memory: xb[g][q][n][8] u32 (the B fragments of group g's four MMAs for thread (n, q)), then xsum[g][8] f32.
 __global__ void __launch_bounds__(Q4_THREADS) q4_mv_kernel(const uint32_t* __restrict__ codes, const uint16_t* __restrict__ S,
-                                                          const uint16_t* __restrict__ B, int K, int R, const float* __restrict__ x,
+                                                          const uint16_t* __restrict__ B, int K, int R, const float* x,
                                                           int xs, float* __restrict__ y, int ys, int T, int add) {
     extern __shared__ __align__(16) uint32_t q4_smem[];
     const int G = K / Q4_GROUP;
@@ -75,12 +75,12 @@ __global__ void __launch_bounds__(Q4_THREADS) q4_mv_kernel(const uint32_t* __res
             if (vec) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float4 t = __ldg((const float4*) xp + j);
+                    const float4 t = ((const float4*) xp)[j];
                     v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
                 }
             } else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = __ldg(xp + j);
+                for (int j = 0; j < 16; ++j) v[j] = xp[j];
             }
         } else {
 #pragma unroll
@@ -181,7 +181,7 @@ template <int GPP> struct Q4Ring {
 template <int NST, int WARPS, int GPP>
 __global__ void __launch_bounds__(32 * WARPS, 1) q4_mv_ring_kernel(const uint32_t* __restrict__ codes, const uint16_t* __restrict__ S,
                                                                    const uint16_t* __restrict__ B, int K, int R,
-                                                                   const float* __restrict__ x, int xs, float* __restrict__ y, int ys,
+                                                                   const float* x, int xs, float* __restrict__ y, int ys,
                                                                    int T, int add) {
     constexpr int ROW = Q4Ring<GPP>::ROW, STAGE = Q4Ring<GPP>::STAGE, CODES = Q4Ring<GPP>::CODES;
     extern __shared__ __align__(16) uint32_t q4_smem[];
@@ -227,12 +227,12 @@ __global__ void __launch_bounds__(32 * WARPS, 1) q4_mv_ring_kernel(const uint32_
             if (vec) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float4 t = __ldg((const float4*) xp + j);
+                    const float4 t = ((const float4*) xp)[j];
                     v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
                 }
             } else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = __ldg(xp + j);
+                for (int j = 0; j < 16; ++j) v[j] = xp[j];
             }
         } else {
 #pragma unroll
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) q4_mv_ring_kernel(const uint32_
 template <int WARPS, int NST, int BPS, int NT>
 __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uint32_t* __restrict__ codes, const uint16_t* __restrict__ S,
                                                                      const uint16_t* __restrict__ B, int K, int R,
-                                                                     const float* __restrict__ x, int xs, float* __restrict__ y,
+                                                                     const float* x, int xs, float* __restrict__ y,
                                                                      int ys, int T, int add) {
     constexpr int ROW = Q4Ring<4>::ROW, STAGE = Q4Ring<4>::STAGE;
     constexpr int G = 4 * WARPS, KB = 128 * WARPS;      // groups and bytes of codes per row (K = 256 x WARPS)
@@ -393,12 +393,12 @@ __global__ void __launch_bounds__(32 * WARPS, BPS) q4_mv_ksplit_kernel(const uin
             if (vec) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float4 t = __ldg((const float4*) xp + j);
+                    const float4 t = ((const float4*) xp)[j];
                     v[4 * j] = t.x; v[4 * j + 1] = t.y; v[4 * j + 2] = t.z; v[4 * j + 3] = t.w;
                 }
             } else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = __ldg(xp + j);
+                for (int j = 0; j < 16; ++j) v[j] = xp[j];
             }
         } else {
 #pragma unroll
@@ -568,7 +568,7 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
     return a;
 }
 
-__global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax_kernel(const float* __restrict__ logits, int32_t* __restrict__ out,
+__global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax_kernel(const float* logits, int32_t* __restrict__ out,
                                                                                        float* __restrict__ prob, int V) {
     __shared__ float bv[ARG_T / 32];
     __shared__ int bi[ARG_T / 32];
@@ -590,7 +590,7 @@ __global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax
         float4 v[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            if (i + q * ARG_T < hi) v[q] = __ldg(l4 + i + q * ARG_T);
+            if (i + q * ARG_T < hi) v[q] = l4[i + q * ARG_T];
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             if (i + q * ARG_T < hi) {      // ascending ids: the first of equal values stays
@@ -635,7 +635,7 @@ __global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax
     const float mx = row_max;
     float s = 0.0f;
     for (int i = lo + tid; i < hi; i += ARG_T) {
-        const float4 v = __ldg(l4 + i);
+        const float4 v = l4[i];
         s += (expf(v.x - mx) + expf(v.y - mx)) + (expf(v.z - mx) + expf(v.w - mx));
     }
     if (rank == 0 && odd < V && (tid < head || odd >= rest)) s += expf(l[odd] - mx);
@@ -657,7 +657,7 @@ __global__ void __cluster_dims__(ARG_CTAS, 1, 1) __launch_bounds__(ARG_T) argmax
 }
 
 // A block a row.
-__global__ void __launch_bounds__(1024) argmax_row_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, float* __restrict__ prob, int V) {
+__global__ void __launch_bounds__(1024) argmax_row_kernel(const float* logits, int32_t* __restrict__ out, float* __restrict__ prob, int V) {
     __shared__ float bv[32];
     __shared__ int bi[32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;

@@ -28,7 +28,7 @@ __device__ __forceinline__ float route_unkey(uint32_t k) {
 // Lane l holds experts l, l + 32, ...  E <= 32 * PER, k <= 32, k <= E.  ind_row / wt_row: k entries in global or shared
 // memory; ind_row is written by lane 0, wt_row by lanes 0..k-1.
 template <int PER>
-__device__ __forceinline__ void route_row(int E, int k, const float* __restrict__ l, int lane, int32_t* ind_row, float* wt_row) {
+__device__ __forceinline__ void route_row(int E, int k, const float* l, int lane, int32_t* ind_row, float* wt_row) {
     uint32_t key[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) {

@@ -110,7 +110,7 @@ __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, 
                     uint4 o = make_uint4(0u, 0u, 0u, 0u);
                     if (ok) {
                         const float4* xp = (const float4*) ((const float*) a.X + ((size_t) (uint32_t) so * 4 + k));
-                        const float4 x0 = __ldg(xp), x1 = __ldg(xp + 1);
+                        const float4 x0 = xp[0], x1 = xp[1];
                         o = make_uint4(bf16x2_bits(x0.x, x0.y), bf16x2_bits(x0.z, x0.w), bf16x2_bits(x1.x, x1.y), bf16x2_bits(x1.z, x1.w));
                     }
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + i * 4096), "r"(o.x), "r"(o.y), "r"(o.z), "r"(o.w) : "memory");

@@ -137,13 +137,13 @@ __device__ __forceinline__ void offsets_from_sum(u64 s2, u64* xm2) {
 __device__ __forceinline__ float input_sum(const float* x) { return ((x[0] + x[4]) + (x[1] + x[5])) + ((x[2] + x[6]) + (x[3] + x[7])); }
 
 // 16 inputs (chunk j of the row, block pair bp): from memory, and into a staged row.
-template <bool CG = false>      // CG: memory that other blocks of this grid have written (the loads bypass the non-coherent path)
+template <bool CG = false>      // CG: memory that other blocks of this grid have written (the loads bypass the L1)
 __device__ __forceinline__ void stage_load(const void* row, int bf16, int j, int bp, float* x) {
     if (bf16) {
         const uint4* xp = (const uint4*) ((const uint16_t*) row + (size_t) j * 64 + bp * 16);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const uint4 t = __ldg(xp + i);
+            const uint4 t = xp[i];
             const uint32_t u[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -155,7 +155,7 @@ __device__ __forceinline__ void stage_load(const void* row, int bf16, int j, int
         const float4* xp = (const float4*) ((const float*) row + (size_t) j * 64 + bp * 16);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float4 t = CG ? __ldcg(xp + i) : __ldg(xp + i);
+            const float4 t = CG ? __ldcg(xp + i) : xp[i];
             x[4 * i] = t.x; x[4 * i + 1] = t.y; x[4 * i + 2] = t.z; x[4 * i + 3] = t.w;
         }
     }
@@ -1316,7 +1316,9 @@ __global__ void __launch_bounds__(MV_THREADS) mv_generic_kernel(MvParams a, KCon
                     const float* xp = a.x + (size_t) (dense ? t : pair / a.xdiv) * a.xs + (size_t) j * 8;
                     float xr[8], xo[4];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) xr[c] = __ldg(xp + c) * NSL_XSCALE;
+                    for (int c = 0; c < 8; ++c) asm volatile("ld.global.f32 %0, [%1];" : "=f"(xr[c]) : "l"(xp + c));      // (in C++: 4 % slower, spills)
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) xr[c] *= NSL_XSCALE;
                     block_offsets(xr, xo);
                     const float d = P == 4 ? states_dot(v, q, xr, xo) : states_dot3(v, q, xr, xo);
                     if (half) su[t] = fmaf(d, e2, su[t]);
