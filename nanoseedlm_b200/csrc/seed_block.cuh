@@ -46,11 +46,12 @@ __device__ __forceinline__ void load_stream_tab(StreamTab& t, const uint32_t* G,
     }
 }
 
-// The table, and the wait for the previous kernel in the stream.  late: the table only after the wait (common.cuh: FollowScope).
-__device__ __forceinline__ void tab_and_wait(StreamTab& t, const uint32_t* G, int late, int tid, int nthreads) {
+// The table, and the wait for the previous kernel in the stream.  late: the table only after the wait (common.cuh: FollowScope).  go: the next kernel's
+// blocks may come in from now on; without, only when this kernel ends.
+__device__ __forceinline__ void tab_and_wait(StreamTab& t, const uint32_t* G, int late, int tid, int nthreads, bool go = true) {
     if (late) grid_dependency_wait();
     load_stream_tab(t, G, tid, nthreads);
-    grid_dependents_go();
+    if (go) grid_dependents_go();
     grid_dependency_wait();
 }
 

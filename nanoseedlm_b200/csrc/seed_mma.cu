@@ -72,7 +72,8 @@ struct SmmShared {
 };
 
 // One pass: up to 8 NT rows of inputs for this block's rows of weights.
-template <int NT, int P>
+// DEP: may be a dependent launch, whose inputs the kernel beside it may still be writing (common.cuh).
+template <int NT, int P, bool DEP>
 __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, SmmShared& sh, unsigned char* xs, int r0) {
     const MmParams& a = sp.m;
     const int kw = sp.kw, rw = sp.rw;
@@ -110,7 +111,7 @@ __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, 
                     uint4 o = make_uint4(0u, 0u, 0u, 0u);
                     if (ok) {
                         const float4* xp = (const float4*) ((const float*) a.X + ((size_t) (uint32_t) so * 4 + k));
-                        const float4 x0 = xp[0], x1 = xp[1];
+                        const float4 x0 = DEP ? xp[0] : __ldg(xp), x1 = DEP ? xp[1] : __ldg(xp + 1);
                         o = make_uint4(bf16x2_bits(x0.x, x0.y), bf16x2_bits(x0.z, x0.w), bf16x2_bits(x1.x, x1.y), bf16x2_bits(x1.z, x1.w));
                     }
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + i * 4096), "r"(o.x), "r"(o.y), "r"(o.z), "r"(o.w) : "memory");
@@ -203,13 +204,14 @@ __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, 
 }
 
 // 128 registers: the pass of 32 rows spills some (P = 4 72 / 112 bytes of stores / loads, P = 3 8 / 12).
-template <int P>
+template <int P, bool DEP>
 __global__ void __launch_bounds__(SMM_THREADS, 2) seed_mma_kernel(SmmParams sp, KConst kc) {
     extern __shared__ __align__(128) unsigned char smm_smem[];
     __shared__ SmmShared sh;
     const MmParams& a = sp.m;
     const int tid = threadIdx.x;
-    tab_and_wait(sh.tab, a.G, a.late, tid, SMM_THREADS);
+    if (DEP) tab_and_wait(sh.tab, a.G, a.late, tid, SMM_THREADS, !a.late);
+    else load_stream_tab(sh.tab, a.G, tid, SMM_THREADS);
     const int start = (int) blockIdx.y * SMM_TILE, count = min(a.T - start, SMM_TILE), r0 = (int) blockIdx.x * sp.rw * 16;
     if (tid < SMM_TILE) {
         const int d = tid >= count ? -1 : start + tid;
@@ -217,21 +219,21 @@ __global__ void __launch_bounds__(SMM_THREADS, 2) seed_mma_kernel(SmmParams sp, 
         sh.drow[tid] = d;
     }
     __syncthreads();
-    if (count <= 8) smm_pass<1, P>(sp, kc, sh, smm_smem, r0);
-    else if (count <= 16) smm_pass<2, P>(sp, kc, sh, smm_smem, r0);
-    else smm_pass<4, P>(sp, kc, sh, smm_smem, r0);
+    if (count <= 8) smm_pass<1, P, DEP>(sp, kc, sh, smm_smem, r0);
+    else if (count <= 16) smm_pass<2, P, DEP>(sp, kc, sh, smm_smem, r0);
+    else smm_pass<4, P, DEP>(sp, kc, sh, smm_smem, r0);
 }
 
-template <int P>
+template <int P, bool DEP>
 static void launch_smm_v(cudaStream_t s, const SmmParams& a, dim3 grid, size_t smem) {
     static bool done[16];
     int dev = 0;
     cudaGetDevice(&dev);
     if (!done[dev & 15]) {
-        cudaFuncSetAttribute(seed_mma_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 8192);
+        cudaFuncSetAttribute(seed_mma_kernel<P, DEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin() - 8192);
         done[dev & 15] = true;
     }
-    launch(seed_mma_kernel<P>, grid, SMM_THREADS, smem, s, a, kconst());
+    launch(seed_mma_kernel<P, DEP>, grid, SMM_THREADS, smem, s, a, kconst());
     count_launch();
 }
 
@@ -259,8 +261,20 @@ void launch_seed_mma(cudaStream_t s, int fmt, const MmParams& m) {
     if (red > smem) smem = red;
     const int wrows = a.rw * 16;
     const dim3 grid((unsigned) ((m.R + wrows - 1) / wrows), (unsigned) ((m.T + SMM_TILE - 1) / SMM_TILE));
-    if (fmt == MF_SEED4) launch_smm_v<3>(s, a, grid, smem);
-    else launch_smm_v<4>(s, a, grid, smem);
+    // Blocks of two calls beside one another leave some SMs with two and others with none, and a grid of long and short tiles of rows is dealt unevenly
+    // wherever it comes in behind another kernel.  So where kc_mm chose a dependent launch itself, the next kernel's blocks come in when this one ends,
+    // and the choice falls only where the blocks are alike or each has an SM of its own.  us, calls one behind the other, ordinary / dependent with the
+    // next call's blocks let in at once / now: 17858 x 2880, 9 rows 45.1 / 71.0 / 41.9; 8192 x 4096, 48 rows 61.7 / 69.7 / 60.2; 22888 x 768, 35 rows
+    // 31.0 / 34.4 / 31.0; 1138 x 512, 11 rows 6.5 / 6.1 / 6.1.  (In a decoder's chain, whose kernels differ, letting them in at once is no slower.)
+    const bool even = grid.y == 1 || (long long) grid.x * grid.y <= sm_count();
+    if (even || !m.late) {
+        if (fmt == MF_SEED4) launch_smm_v<3, true>(s, a, grid, smem);
+        else launch_smm_v<4, true>(s, a, grid, smem);
+    } else {
+        PdlScope off(false);
+        if (fmt == MF_SEED4) launch_smm_v<3, false>(s, a, grid, smem);
+        else launch_smm_v<4, false>(s, a, grid, smem);
+    }
 }
 
 }   // namespace nsl
