@@ -15,8 +15,9 @@
 // issues tcgen05.mma (M 128, K 16, N = the tile's count rounded up to 16) and commits the stage back through an mbarrier.
 // Blocks are persistent: the stream table, the tensor memory and the barriers are set up once.
 //   TT = 1, packed inputs: 8 producer warps, two blocks an SM (256 of the 512 columns each).
-//   dense f32 inputs: 8 producer warps and 11 or 15 loaders, one block an SM (launch_dense_f32).
-//   otherwise: 16 producer warps, one block an SM.  TT = 3: up to three tiles of an expert share one expansion, which a prompt of
+//   dense f32 inputs, K a multiple of 64, streams 8-byte aligned, two or three tiles or at most a unit an SM: 8 producer warps and 11 or 15
+//   loaders, one block an SM (launch_dense_f32).
+//   otherwise: 16 producer warps, one block an SM (three terms: 8).  TT = 3: up to three tiles of an expert share one expansion, which a prompt of
 //   thousands of rows needs (each tile expands its expert's weights again).
 // The accumulator is read back with tcgen05.ld by the producer warps (lane = weight row, column = row of inputs), rounded as the
 // reference's store_y does and written so that a warp stores 32 consecutive rows of one row of outputs: after each warpgroup's
@@ -719,14 +720,18 @@ static bool launch_gemm_v(cudaStream_t s, const MmParams& a, int units) {
 }
 static void no_map(const MmParams& a) { set_error("seed GEMM: no tensor map for sorted inputs of row stride %d", a.xs); }
 // How many tiles of a dense call share an expansion: a unit takes the time of its expansion (twice that where two blocks share an
-// SM) or of its inputs' conversion (f32; 31, 45 and 62 us a unit of one, two and three tiles at K = 2048), and the units go round the SMs.
+// SM) or of its inputs' conversion, and the units go round the SMs.  f32, us a round of units at K = 2048: one tile 34-35 in either kernel form
+// (launch_dense_f32) where a block has several units, two tiles 45-48, three 62-72; a block's only unit of one tile 31.  Three rounds of one tile and two
+// of two are a tie that the steps of a unit decide, one tile / two: 20000 x 2048, 200 rows 103.1 / 88.0, x 1024 55.9 / 51.1, x 512 32.9 / 33.0; 1906 x 1088,
+// 3673 rows 59.5 / 57.9; 5019 x 640, 1156 rows 39.5 / 40.7; 4869 x 512, 1218 rows 34.2 / 36.1.  Two rounds of one tile against one of three: 7120 x 1216,
+// 617 rows 44.9 / 47.9, 3235 x 2176, 1365 rows 72.7 / 76.1, 6943 x 576, 553 rows 25.7 / 29.7, 1698 x 3840, 2588 rows 133 / 126.
 static int dense_tiles(const MmParams& a, int row_tiles) {
     int best = 1;
     double best_cost = 0.0;
     for (int tt = 1; tt <= 3; ++tt) {
         if (a.packed && tt == 2) continue;
         const int units = row_tiles * ((a.T + GM_BN * tt - 1) / (GM_BN * tt)), slots = sm_count() * (a.packed && tt == 1 ? 2 : 1);
-        const double unit = a.packed ? (tt == 1 && units > sm_count() ? 2.0 : 1.0) : 0.45 + 0.5 * tt;
+        const double unit = a.packed ? (tt == 1 && units > sm_count() ? 2.0 : 1.0) : tt == 1 && units > sm_count() && a.K >= 1024 ? 0.97 : 0.45 + 0.5 * tt;
         const double cost = (double) ((units + slots - 1) / slots) * unit;
         if (tt == 1 || cost < best_cost) { best = tt; best_cost = cost; }
     }
@@ -735,8 +740,10 @@ static int dense_tiles(const MmParams& a, int row_tiles) {
 // Dense f32 inputs.  Their loaders set the pace (load, convert, store and report a step, while the producers take most issue slots), and with
 // 16 producers and 7 loaders a step's rows also came in two or three passes, each a memory latency.  8 producers and 11 loaders take a tile
 // in one pass, 8 and 15 two tiles; both fit their registers, the 16 and 7 spill.  us, 16 + 7 / now: 2048 x 2048, 65 rows 34.8 / 34.4, 777 rows
-// 38.6 / 36.8, 2048 rows 58.8 / 50.7, 4096 rows 131.0 / 99.1; 8192 x 2048, 1024 rows 119 / 97; 8192 x 4096, 700 rows 154 / 131.  One tile and
-// several units a block: the results are read by the producers, which 16 do faster (151936 x 1024, 100 rows 158 / 166).
+// 38.6 / 36.8, 2048 rows 58.8 / 50.7, 4096 rows 131.0 / 99.1; 8192 x 2048, 1024 rows 119 / 97; 8192 x 4096, 700 rows 154 / 131 (the last five with two or
+// three tiles).  One tile and several units a block: the results are read by the producers, which 16 do faster where a unit has few steps (16 + 7 / 8 + 11:
+// 20000 x 512, 100 rows 22.6 / 24.6, 40000 x 512 32.2 / 35.4, 151936 x 512 92.8 / 101.9; K = 1024 37.9 / 39.4, 54.7 / 57.4, 157.6 / 166.7; K = 2048 69.1 / 68.9,
+// 101.5 / 101.8; 20000 x 4096 130.1 / 127.7).
 template <int WF>
 static void launch_dense_f32(cudaStream_t s, const MmParams& a, int tt, int units) {
     if (tt == 1 && units > sm_count()) launch_gemm_v<1, WF, 1, 2, false, IN_F32>(s, a, units);
