@@ -590,8 +590,8 @@ __global__ void __launch_bounds__(GmCfg<TERMS, TT, IN>::THREADS, GmCfg<TERMS, TT
                         x[2 * i] = x[2 * i + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                         if (n < n16 && k < a.K) {
                             const float4* xp = (const float4*) ((const float*) a.X + ((size_t) srow[FEW ? mine + 4 * i + (lane >> 3) : n] * a.xs + k));
-                            x[2 * i] = xp[0];
-                            x[2 * i + 1] = xp[1];
+                            x[2 * i] = ld_in_order(xp);      // (C++ loads: 1.5 to 3 % slower)
+                            x[2 * i + 1] = ld_in_order(xp + 1);
                         }
                     }
                 };

@@ -1318,7 +1318,7 @@ __global__ void __launch_bounds__(MV_THREADS) mv_generic_kernel(MvParams a, KCon
                     const float* xp = a.x + (size_t) (dense ? t : pair / a.xdiv) * a.xs + (size_t) j * 8;
                     float xr[8], xo[4];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) asm volatile("ld.global.f32 %0, [%1];" : "=f"(xr[c]) : "l"(xp + c));      // (in C++: 4 % slower, spills)
+                    for (int c = 0; c < 8; ++c) xr[c] = ld_in_order(xp + c);      // (C++ loads: 4 % slower, spills)
 #pragma unroll
                     for (int c = 0; c < 8; ++c) xr[c] *= NSL_XSCALE;
                     block_offsets(xr, xo);
