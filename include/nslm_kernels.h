@@ -263,8 +263,9 @@ void nsl_mv_gu_routed(cudaStream_t s, const WSlice* wg, const WSlice* wu, int K,
  * set it back before launching anything else on the stream.  on > 0: as above.  0: ordinary launches.  Negative (how every thread
  * starts): each entry point's own choice, which is a dependent launch for kq4_route*, nsl_route, kc_mv_sel, kc_mv_gu,
  * kq4_moe_combine, kc_argmax*, the MF_Q4 form of kc_mv and kc_mm of seed weights and an ordinary one for the others;
- * such a kernel reads nothing before its wait.  With on > 0 the seed kernels read the stream table G before it (and kc_mv its
- * weights): no kernel may then write G or weights while calls that use them are queued behind it.
+ * such a kernel reads nothing before its wait.  (kc_mm of up to 64 rows: dependent where its blocks are alike or each has an SM.)
+ * With on > 0 the seed kernels read the stream table G before the wait, and kc_mv and kc_mm's decode-batch kernel their weights: no
+ * kernel may then write those while calls that use them are queued behind it.
  * (The layer and the decoder handles have switches of their own; kc_attn's second pass always comes in behind its first.) */
 void nsl_dependent_launch(int on);
 int nsl_dependent_launch_state(void);   /* what the calling thread has set: -1, 0 or 1 */

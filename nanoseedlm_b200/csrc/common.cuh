@@ -33,6 +33,10 @@ struct PdlScope {
 };
 // For entry points whose kernels follow another of this library's kernels as a rule: a dependent launch unless the caller has asked for ordinary ones
 // (nsl_dependent_launch(0)).  After a copy, and after a kernel that does not let its dependents go early, nothing starts before the predecessor has ended.
+// Which ones: the calls of a layer, of a head with its tokens and of a prompt product, as an engine queues them (us, calls one behind the other, ordinary /
+// dependent: a P = 3 layer of 8 rows 89.9 / 82.3, head and arg-max 52.4 / 49.7, 777 x (2048 x 2048) 39.0 / 37.4; with new inputs copied in before each, the
+// copies included, 97.8 / 89.8, 56.5 / 53.2, 43.1 / 41.0).  kc_mm_packed, kc_mm_grouped*, nsl_mv_raw, nsl_mv_gu_raw,
+// nsl_mv_gu_routed and the stored-BF16 products start the same or similar kernels, have not been measured that way and stay ordinary.
 // Such a kernel reads nothing at all before its wait, the stream table included (tab_and_wait): a caller that has asked for nothing may have made the
 // table in the kernel before, whose writes are visible after the wait and not sooner.
 struct FollowScope {

@@ -806,7 +806,8 @@ void launch_gemm(cudaStream_t s, int fmt, const char* who, MmParams a, int tiles
     if (a.grouped && !a.ntiles) a.T = tiles_y;
     // A dense call of a few rows: the weights stay in registers.  The line lies where the second tile of 32 rows has used up what that saves
     // (us, this kernel / that one: 2048 x 2048, 9 rows 34.9 / 12.5, 32 rows 34.9 / 16.5, 64 rows 37.0 / 30.6; 512 x 2048, 64 rows 36.8 / 16.5;
-    // 8192 x 4096, 9 rows 62.5 / 36.3, 48 rows 64.5 / 63.5, 64 rows 65.7 / 73.2; a third tile adds half as much again).  A row's bits differ
+    // 8192 x 4096, 9 rows 62.5 / 36.3, 48 rows 64.5 / 63.5, 64 rows 65.7 / 73.2; a third tile adds half as much again; one call behind the other
+    // that kernel now takes 9.2, 14.3, 27.7; 14.1; 33.5, 60.5 and 70.5).  A row's bits differ
     // between the two (the order of its sums), not within either.
     if (fmt != MF_BF16 && !g_exact && !a.grouped && a.T <= 64 && (fmt == MF_SEED4 ? streams_aligned<2>(a.w0, 16) : streams_aligned<0>(a.w0, 16)) &&
         smm_serves(a.K, a.X, a.xs, a.packed)) { launch_seed_mma(s, fmt, a); return; }

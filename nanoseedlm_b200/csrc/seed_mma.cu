@@ -203,7 +203,7 @@ __device__ __forceinline__ void smm_pass(const SmmParams& sp, const KConst& kc, 
     }
 }
 
-// 128 registers: the pass of 32 rows spills some (P = 4 72 / 112 bytes of stores / loads, P = 3 8 / 12).
+// 128 registers: the pass of 32 rows spills some (P = 4 84 / 144 bytes of stores / loads, 72 / 112 without DEP; P = 3 8 / 12).
 template <int P, bool DEP>
 __global__ void __launch_bounds__(SMM_THREADS, 2) seed_mma_kernel(SmmParams sp, KConst kc) {
     extern __shared__ __align__(128) unsigned char smm_smem[];
