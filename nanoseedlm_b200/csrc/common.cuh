@@ -17,8 +17,8 @@ inline bool aligned16(const void* p) { return ((uintptr_t) p & 15u) == 0; }
 // Programmatic dependent launch.  While a PdlScope(true) is alive on the calling thread, launch() marks the kernel as
 // allowed to start before the previous kernel in its stream has finished: its blocks become resident as the previous
 // kernel's blocks retire and run their prologue (the stream table, index arithmetic) until grid_dependency_wait(),
-// which returns once the previous kernel has completed and its writes are visible.  Every kernel launched through
-// launch() calls grid_dependency_wait() before it reads or writes anything a neighbouring kernel touches; without the
+// which returns once the previous kernel has completed and its writes are visible.  Every kernel that launch() may start
+// so calls grid_dependency_wait() before it reads or writes anything a neighbouring kernel touches; without the
 // scope, and outside the entry points that open one themselves, the launch is an ordinary one and the wait returns at once.
 // What a neighbour may have written (activations, logits, routing, partial sums, cache rows) is read with ordinary loads: ld.global.nc (__ldg, and what
 // the compiler makes of a kernel's const __restrict__ parameters) is for memory that nobody writes while the kernel runs, and a dependent kernel runs

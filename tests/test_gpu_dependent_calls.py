@@ -26,13 +26,16 @@ def three_ways(calls, results):
         calls(st, s.synchronize)
         s.synchronize()
         got.append([r.clone() for r in results()])
-        for r in results(): r.zero_()
-        for _ in range(12): torch.mm(a, a, out=b)
-        begin, end = torch.cuda.Event(), torch.cuda.Event()
-        begin.record(s)
-        calls(st, lambda: None)
-        assert not begin.query()      # nothing of the sequence has started yet
-        s.synchronize()
+        for attempt in range(4):      # (again where the host was held up meanwhile)
+            for r in results(): r.zero_()
+            for _ in range(12): torch.mm(a, a, out=b)
+            begin = torch.cuda.Event()
+            begin.record(s)
+            calls(st, lambda: None)
+            queued = not begin.query()      # nothing of the sequence has started yet
+            s.synchronize()
+            if queued: break
+        assert queued
         got.append([r.clone() for r in results()])
     rt, graph, exe = C.CDLL("libcudart.so.12"), C.c_void_p(), C.c_void_p()
     assert rt.cudaStreamBeginCapture(st, 2) == 0
